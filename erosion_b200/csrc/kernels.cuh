@@ -33,56 +33,107 @@ __global__ void k_wall_nodes(int nout, double a, double b, double p, double* __r
   y[k] = b * r * s;
 }
 
-// One CTA per curve of length n.  First and second spectral derivatives by
-// circulant convolution with dk[m] = (1/2)(-1)^m cot(pi m/n), the matrix of
-// fourierDiff (:348-388, even n); then speed, normal (-y', x')/|z'|,
-// curvature (y'x'' - x'y'')/|z'|^3 (:447-453), negated on the wall (:195-199).
-__global__ void k_geom(const double* __restrict__ x, const double* __restrict__ y, int n,
-                       const double* __restrict__ dk, int out_off, int negate,
-                       double2* __restrict__ xy, double2* __restrict__ nrm, double* __restrict__ sp,
-                       double* __restrict__ cur, double* __restrict__ w, double2* __restrict__ dz,
-                       double2* __restrict__ d1tmp) {
-  const int c = blockIdx.x;
-  const double* xc = x + (size_t)c * n;
-  const double* yc = y + (size_t)c * n;
-  double2* D1 = d1tmp + (size_t)c * n;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double ax = 0.0, ay = 0.0;
-    for (int k = 0; k < n; ++k) {
-      int m = j - k;
-      if (m < 0) m += n;
-      double d = __ldg(dk + m);
-      ax = fma(d, __ldg(xc + k), ax);
-      ay = fma(d, __ldg(yc + k), ay);
-    }
-    D1[j] = make_double2(ax, ay);
+// First and second spectral derivatives of every curve by circulant
+// convolution with dk[m] = (1/2)(-1)^m cot(pi m/n), the matrix of fourierDiff
+// (:348-388, even n): k_geom_d1 writes z', k_geom takes z'' from it and then
+// the speed, normal (-y', x')/|z'| and curvature (y'x'' - x'y'')/|z'|^3
+// (:447-453), both negated on the wall (:195-199).  One launch covers the wall
+// (ceil(nout/32) CTAs) and the bodies (ceil(n/32) CTAs each).  A CTA owns 32
+// nodes, one per lane; its GEOM_W warps split the n sources and meet in shared
+// memory in a fixed order.  The convolution is 4 n_c^2 FMAs per curve and has
+// two loads from L1 per pair of FMAs, so it is bound by load latency until
+// enough warps share it.  Both launches together take 76 us at 400 bodies x 256
+// nodes and 4096 wall nodes and 16 us at 10 x 128 and 1024; with one CTA for
+// the whole wall they took 3352 us and 228 us.
+constexpr int GEOM_W = 16;
+
+struct GeomIn {
+  const double* __restrict__ wx;   // wall nodes
+  const double* __restrict__ wy;
+  const double* __restrict__ bx;   // body nodes, body-major
+  const double* __restrict__ by;
+  const double* __restrict__ dkw;  // derivative kernels of the wall and of a body
+  const double* __restrict__ dkb;
+  int nout, n;
+};
+
+struct GeomTask {
+  int start, len, j0;   // first node of the curve (global), its length, first node of this CTA in it
+};
+
+__device__ __forceinline__ GeomTask geom_task(const GeomIn& I) {
+  const int nwb = (I.nout + 31) / 32;
+  if ((int)blockIdx.x < nwb) return {0, I.nout, 32 * (int)blockIdx.x};
+  const int nbb = (I.n + 31) / 32, r = (int)blockIdx.x - nwb, b = r / nbb;
+  return {I.nout + b * I.n, I.n, 32 * (r - b * nbb)};
+}
+
+// sum_k dk[(j - k) mod len] f(k) for node j = T.j0 + lane; valid in warp 0.
+template <class F>
+__device__ __forceinline__ double2 geom_circulant(const double* __restrict__ dk, const GeomTask& T, F f,
+                                                  double2 (*red)[32]) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = min(T.j0 + lane, T.len - 1);
+  const int ka = (int)((long long)T.len * wid / GEOM_W), kb = (int)((long long)T.len * (wid + 1) / GEOM_W);
+  double ax = 0.0, ay = 0.0;
+#pragma unroll 8
+  for (int k = ka; k < kb; ++k) {
+    int m = j - k;
+    if (m < 0) m += T.len;
+    const double d = __ldg(dk + m);
+    const double2 v = f(k);
+    ax = fma(d, v.x, ax);
+    ay = fma(d, v.y, ay);
   }
+  red[wid][lane] = make_double2(ax, ay);
   __syncthreads();
-  const double h = EB_TWOPI / n;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double bx = 0.0, by = 0.0;
-    for (int k = 0; k < n; ++k) {
-      int m = j - k;
-      if (m < 0) m += n;
-      double d = __ldg(dk + m);
-      double2 q = D1[k];
-      bx = fma(d, q.x, bx);
-      by = fma(d, q.y, by);
+  double2 s = make_double2(0.0, 0.0);
+  if (wid == 0) {
+#pragma unroll
+    for (int w = 0; w < GEOM_W; ++w) {
+      s.x += red[w][lane].x;
+      s.y += red[w][lane].y;
     }
-    double2 q = D1[j];
-    double Dx = q.x, Dy = q.y, DDx = bx, DDy = by;
-    double s = sqrt(Dx * Dx + Dy * Dy);
-    double px = -Dy / s, py = Dx / s;
-    double cu = (Dy * DDx - Dx * DDy) / (s * s * s);
-    if (negate) { px = -px; py = -py; cu = -cu; }
-    int g = out_off + c * n + j;
-    xy[g] = make_double2(xc[j], yc[j]);
-    nrm[g] = make_double2(px, py);
-    sp[g] = s;
-    cur[g] = cu;
-    w[g] = s * h / EB_PI;
-    dz[g] = make_double2(Dx * h, Dy * h);
   }
+  return s;
+}
+
+__global__ void __launch_bounds__(32 * GEOM_W) k_geom_d1(GeomIn I, double2* __restrict__ d1) {
+  __shared__ double2 red[GEOM_W][32];
+  const GeomTask T = geom_task(I);
+  const bool wall = T.start < I.nout;
+  const double* __restrict__ x = wall ? I.wx : I.bx + (T.start - I.nout);
+  const double* __restrict__ y = wall ? I.wy : I.by + (T.start - I.nout);
+  const double2 s = geom_circulant(wall ? I.dkw : I.dkb, T,
+                                   [=](int k) { return make_double2(__ldg(x + k), __ldg(y + k)); }, red);
+  const int j = T.j0 + (int)threadIdx.x;
+  if (threadIdx.x < 32 && j < T.len) d1[T.start + j] = s;
+}
+
+__global__ void __launch_bounds__(32 * GEOM_W)
+k_geom(GeomIn I, const double2* __restrict__ d1, double2* __restrict__ xy, double2* __restrict__ nrm,
+       double* __restrict__ sp, double* __restrict__ cur, double* __restrict__ w, double2* __restrict__ dz) {
+  __shared__ double2 red[GEOM_W][32];
+  const GeomTask T = geom_task(I);
+  const bool wall = T.start < I.nout;
+  const double2* __restrict__ D1 = d1 + T.start;
+  const double2 dd = geom_circulant(wall ? I.dkw : I.dkb, T, [=](int k) { return __ldg(D1 + k); }, red);
+  const int j = T.j0 + (int)threadIdx.x;
+  if (threadIdx.x >= 32 || j >= T.len) return;
+  const double h = EB_TWOPI / T.len;
+  const double2 q = D1[j];
+  const double Dx = q.x, Dy = q.y;
+  const double s = sqrt(Dx * Dx + Dy * Dy);
+  double px = -Dy / s, py = Dx / s;
+  double cu = (Dy * dd.x - Dx * dd.y) / (s * s * s);
+  if (wall) { px = -px; py = -py; cu = -cu; }
+  const int g = T.start + j;
+  xy[g] = wall ? make_double2(I.wx[j], I.wy[j]) : make_double2(I.bx[g - I.nout], I.by[g - I.nout]);
+  nrm[g] = make_double2(px, py);
+  sp[g] = s;
+  cur[g] = cu;
+  w[g] = s * h / EB_PI;
+  dz[g] = make_double2(Dx * h, Dy * h);
 }
 
 // Centroid (plain node mean, :151-160) and mean speed (the body radius of

@@ -224,11 +224,13 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     EB_LAUNCH_CHECK();
     k_wall_nodes<<<nblk(nout, 256), 256, 0, st>>>(nout, p->wall_a, p->wall_b, p->wall_order, wx, wy);
     EB_LAUNCH_CHECK();
-    k_geom<<<1, 1024, 0, st>>>(wx, wy, nout, dker_w, 0, 1, xy, nrm, sp, cur, w, dz, d1tmp);
+    const GeomIn gin{wx, wy, d_xx, d_yy, dker_w, dker_b, nout, n};
+    const unsigned gblk = nblk(nout, 32) + (unsigned)M * nblk(n, 32);
+    k_geom_d1<<<gblk, 32 * GEOM_W, 0, st>>>(gin, d1tmp);
+    EB_LAUNCH_CHECK();
+    k_geom<<<gblk, 32 * GEOM_W, 0, st>>>(gin, d1tmp, xy, nrm, sp, cur, w, dz);
     EB_LAUNCH_CHECK();
     if (M > 0) {
-      k_geom<<<M, 256, 0, st>>>(d_xx, d_yy, n, dker_b, nout, 0, xy, nrm, sp, cur, w, dz, d1tmp + nout);
-      EB_LAUNCH_CHECK();
       k_body_stats<<<M, 256, 0, st>>>(n, nout, xy, sp, cen, rb);
       EB_LAUNCH_CHECK();
     }

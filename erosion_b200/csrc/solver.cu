@@ -531,13 +531,13 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   s.ws.ensure(N); s.sq64.ensure(N); s.sigdotn.ensure(1);
   k_wall_nodes<<<nblk(pr.nout, 256), 256, 0, st>>>(pr.nout, pr.P.wall_a, pr.P.wall_b, pr.P.wall_order, s.wx.p, s.wy.p);
   EB_LAUNCH_CHECK();
-  k_geom<<<1, 1024, 0, st>>>(s.wx.p, s.wy.p, pr.nout, s.dker_wall.p, 0, 1, s.xy.p, s.nrm.p, s.sp.p, s.cur.p, s.w.p,
-                             s.dz.p, s.d1tmp.p);
+  const GeomIn gin{s.wx.p, s.wy.p, d_xx, d_yy, s.dker_wall.p, s.dker_body.p, pr.nout, pr.n};
+  const unsigned gblk = nblk(pr.nout, 32) + (unsigned)pr.M * nblk(pr.n, 32);
+  k_geom_d1<<<gblk, 32 * GEOM_W, 0, st>>>(gin, s.d1tmp.p);
+  EB_LAUNCH_CHECK();
+  k_geom<<<gblk, 32 * GEOM_W, 0, st>>>(gin, s.d1tmp.p, s.xy.p, s.nrm.p, s.sp.p, s.cur.p, s.w.p, s.dz.p);
   EB_LAUNCH_CHECK();
   if (pr.M > 0) {
-    k_geom<<<pr.M, 256, 0, st>>>(d_xx, d_yy, pr.n, s.dker_body.p, pr.nout, 0, s.xy.p, s.nrm.p, s.sp.p, s.cur.p,
-                                 s.w.p, s.dz.p, s.d1tmp.p + pr.nout);
-    EB_LAUNCH_CHECK();
     k_body_stats<<<pr.M, 256, 0, st>>>(pr.n, pr.nout, s.xy.p, s.sp.p, s.cen.p, s.rb.p);
     EB_LAUNCH_CHECK();
   }
