@@ -12,9 +12,10 @@ constexpr int FAR_NT = 256;        // CTA shape (threads x targets per thread) t
 constexpr int FAR_TPT = 2;         //   splits of the shear-stress and target sums
 constexpr int FAR_TS = 256;        // sources per shared-memory tile
 constexpr int WALL_TS = 32;        // wall nodes per tile (keeps FP32 offsets small)
-constexpr int NEAR_NT = 128;       // threads per CTA of the barycentric kernels
-constexpr int NEAR_TK = 128;       // source nodes per shared-memory tile
-constexpr int BD_NT = 256;         // threads per CTA of the boundary-value kernel
+constexpr int NEAR_W = 8;          // warps per CTA of the barycentric kernels: they split the sources,
+constexpr int NEAR_T = 32;         //   every lane of each warp holding one of the CTA's 32 targets
+constexpr int NEAR_NT = 32 * NEAR_W;
+constexpr int NEAR_TK = 256;       // source nodes per shared-memory tile
 
 // ---------------------------------------------------------------------------
 // Geometry (stokesSolver.f:136-204, :417-457).
@@ -311,6 +312,16 @@ __device__ __forceinline__ double rcp_newton64(double r2) {
     y = fma(y, e, y);
   }
   return r2 > 0.0 ? y : 0.0;
+}
+
+// rcp_newton64<2> without the select: NaN for r2 = 0.
+__device__ __forceinline__ double rcp_raw64(double r2) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+  double e = fma(-r2, y, 1.0);
+  y = fma(y, e, y);
+  e = fma(-r2, y, 1.0);
+  return fma(y, e, y);
 }
 
 // One Newton-Raphson step from the FP32 estimate: relative error ~2^-46
@@ -1336,32 +1347,70 @@ __device__ __forceinline__ void node_fields(const GeoDev& G, const double* __res
   f[4] = cmul(make_double2(sx * nn.y, sy * nn.y), ninv);
 }
 
+// v[q] summed over the CTA's NEAR_W warps for every lane, in a fixed order; all
+// warps receive the sums.  red: NEAR_W / 2 x (at least NV) x 32.
+template <int NV, int NR>
+__device__ __forceinline__ void near_reduce(double (&v)[NV], double (*red)[NR][32]) {
+  static_assert(NV <= NR, "reduction buffer");
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int H = NEAR_W / 2;
+  if (wid >= H) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[wid - H][q][lane] = v[q];
+  }
+  __syncthreads();
+  if (wid < H) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[wid][q][lane] += v[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    double t = red[0][q][lane];
+#pragma unroll
+    for (int w = 1; w < H; ++w) t += red[w][q][lane];
+    v[q] = t;
+  }
+  __syncthreads();
+}
+
 // Boundary values of the five fields on one source curve
 // (compute_bdval_in :5103-5146, compute_bdval_ex :5382-5427):
 //   S_j = -sum_{k != j} (f_k - f_j) z'_k dt/(z_k - z_j) - dt f'_j
 //   interior: -i S_j/(2pi) - f_j        exterior: i S_j/(2pi)
-// with f' the spectral derivative.  One CTA per (curve, 256 nodes j).
-__global__ void __launch_bounds__(BD_NT)
+// with f' the spectral derivative, sum_k d_{j-k} f_k.  The derivative matrix
+// annihilates constants, so its sum takes the differences f_k - f_j too and
+// h d_{j-k} joins the real part of the Cauchy weight: one weight per pair for
+// both sums.  The first three fields are real and cost half a complex one:
+// 36 FP64 operations per pair.  One CTA per (curve, 32 nodes j), a node per
+// lane; the NEAR_W warps split the sources and meet in shared memory in a
+// fixed order.  Bound by the FP64 pipe for long curves and by the latency of a
+// warp's chain of sources for short ones, which the split shortens 8-fold.
+// 8.7 us for 3 bodies of 64 nodes near a wall of 256 (one thread per node and
+// two weights: 66.4 us), 155 us for all curves of 400 bodies of 256 nodes and a
+// wall of 4096 (1081 us).
+__global__ void __launch_bounds__(NEAR_NT)
 k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
         const int* __restrict__ src_curve, const long long* __restrict__ bd_off,
         const double* __restrict__ dker_wall, const double* __restrict__ dker_body,
         double2* __restrict__ bd) {
-  __shared__ double2 sz[BD_NT], sdz[BD_NT];
-  __shared__ double2 sf[5][BD_NT];
+  __shared__ double2 sz[NEAR_TK], sdz[NEAR_TK], s01[NEAR_TK], s3[NEAR_TK], s4[NEAR_TK];
+  __shared__ double s2[NEAR_TK];
+  __shared__ double red[NEAR_W / 2][10][32];
   const int s = work[blockIdx.x].x, j0 = work[blockIdx.x].y;
   const int c = src_curve[s];
   const int start = curve_start(G, c), len = curve_len(G, c);
   const double* __restrict__ dk = (c == 0) ? dker_wall : dker_body;
-  const int j = j0 + threadIdx.x;
-  const bool act = j < len;
-  const int jc = act ? j : len - 1;
-  const double2 zj = G.xy[start + jc];
+  const double h = EB_TWOPI / len;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = min(j0 + lane, len - 1);
+  const double2 zj = G.xy[start + j];
   double2 fj[5];
-  node_fields(G, den, start + jc, fj);
-  double2 S[5], D[5];
+  node_fields(G, den, start + j, fj);
+  double S[10];   // the five sums, real and imaginary part
 #pragma unroll
-  for (int q = 0; q < 5; ++q) { S[q] = make_double2(0, 0); D[q] = make_double2(0, 0); }
-  for (int k0 = 0; k0 < len; k0 += BD_NT) {
+  for (int q = 0; q < 10; ++q) S[q] = 0.0;
+  for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
     __syncthreads();
     const int kl = k0 + threadIdx.x;
     if (kl < len) {
@@ -1370,63 +1419,79 @@ k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
       sdz[threadIdx.x] = G.dz[g];
       double2 f[5];
       node_fields(G, den, g, f);
-#pragma unroll
-      for (int q = 0; q < 5; ++q) sf[q][threadIdx.x] = f[q];
+      s01[threadIdx.x] = make_double2(f[0].x, f[1].x);
+      s2[threadIdx.x] = f[2].x;
+      s3[threadIdx.x] = f[3];
+      s4[threadIdx.x] = f[4];
     }
     __syncthreads();
-    const int kt = min(BD_NT, len - k0);
-    for (int kk = 0; kk < kt; ++kk) {
-      const int k = k0 + kk;
-      int m = jc - k;
+    const int kt = min(NEAR_TK, len - k0);
+    const int ka = kt * wid / NEAR_W, kb = kt * (wid + 1) / NEAR_W;
+#pragma unroll 2
+    for (int kk = ka; kk < kb; ++kk) {
+      int m = j - (k0 + kk);
       if (m < 0) m += len;
-      const double dd = __ldg(dk + m);
-      double2 cc = make_double2(0.0, 0.0);
-      if (k != jc) cc = cmul(sdz[kk], cinv(csub(sz[kk], zj)));
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const double2 fk = sf[q][kk];
-        D[q].x = fma(dd, fk.x, D[q].x);
-        D[q].y = fma(dd, fk.y, D[q].y);
-        const double2 df = csub(fk, fj[q]);
-        S[q].x -= df.x * cc.x - df.y * cc.y;
-        S[q].y -= df.x * cc.y + df.y * cc.x;
-      }
+      const double dx = sz[kk].x - zj.x, dy = sz[kk].y - zj.y;
+      const double inv = m == 0 ? 0.0 : rcp_raw64(fma(dx, dx, dy * dy));   // no term for k = j
+      const double2 dz = sdz[kk];
+      const double cx = fma(h, __ldg(dk + m), inv * fma(dz.x, dx, dz.y * dy));
+      const double cy = inv * fma(dz.y, dx, -dz.x * dy);
+      const double2 f01 = s01[kk];
+      const double d0 = f01.x - fj[0].x, d1 = f01.y - fj[1].x, d2 = s2[kk] - fj[2].x;
+      const double2 d3 = csub(s3[kk], fj[3]), d4 = csub(s4[kk], fj[4]);
+      S[0] = fma(-d0, cx, S[0]); S[1] = fma(-d0, cy, S[1]);
+      S[2] = fma(-d1, cx, S[2]); S[3] = fma(-d1, cy, S[3]);
+      S[4] = fma(-d2, cx, S[4]); S[5] = fma(-d2, cy, S[5]);
+      S[6] = fma(-d3.x, cx, fma(d3.y, cy, S[6]));
+      S[7] = fma(-d3.x, cy, fma(-d3.y, cx, S[7]));
+      S[8] = fma(-d4.x, cx, fma(d4.y, cy, S[8]));
+      S[9] = fma(-d4.x, cy, fma(-d4.y, cx, S[9]));
     }
   }
-  if (!act) return;
-  const double h = EB_TWOPI / len;
-  const long long base = bd_off[s];
+  near_reduce(S, red);
+  if (wid >= 5 || j0 + lane >= len) return;   // warp q writes field q
+  const long long at = bd_off[s] + (long long)wid * len + j0 + lane;
+  double2 Sq = make_double2(0, 0), fq = make_double2(0, 0);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    double2 Sq = make_double2(S[q].x - h * D[q].x, S[q].y - h * D[q].y);
-    double2 r;
-    if (c == 0) r = make_double2(Sq.y / EB_TWOPI - fj[q].x, -Sq.x / EB_TWOPI - fj[q].y);
-    else r = make_double2(-Sq.y / EB_TWOPI, Sq.x / EB_TWOPI);
-    bd[base + (long long)q * len + j] = r;
-  }
+  for (int q = 0; q < 5; ++q)
+    if (q == wid) { Sq = make_double2(S[2 * q], S[2 * q + 1]); fq = fj[q]; }
+  if (c == 0) bd[at] = make_double2(Sq.y / EB_TWOPI - fq.x, -Sq.x / EB_TWOPI - fq.y);
+  else bd[at] = make_double2(-Sq.y / EB_TWOPI, Sq.x / EB_TWOPI);
 }
 
-// Source-curve tile of the barycentric kernels.
+// Source-curve tile of the barycentric kernels, and their reduction buffer.
 struct BaryTile {
   double2 z[NEAR_TK], dz[NEAR_TK], za[NEAR_TK], b[5][NEAR_TK];
+  double red[NEAR_W / 2][12][32];
 };
 
 __device__ __forceinline__ void bary_load_tile(BaryTile& T, const GeoDev& G, int start, int len, int k0,
                                                const double2* __restrict__ bdc, bool ext, double2 a) {
   __syncthreads();
-  for (int t = threadIdx.x; t < NEAR_TK; t += blockDim.x) {
-    int k = k0 + t;
-    if (k < len) {
-      int g = start + k;
-      double2 z = G.xy[g];
-      T.z[t] = z;
-      T.dz[t] = G.dz[g];
-      T.za[t] = ext ? cinv(csub(z, a)) : make_double2(0, 0);
+  const int t = threadIdx.x, k = k0 + t;
+  if (t < NEAR_TK && k < len) {
+    const int g = start + k;
+    const double2 z = G.xy[g];
+    T.z[t] = z;
+    T.dz[t] = G.dz[g];
+    T.za[t] = ext ? cinv(csub(z, a)) : make_double2(0, 0);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) T.b[q][t] = bdc[(long long)q * len + k];
-    }
+    for (int q = 0; q < 5; ++q) T.b[q][t] = bdc[(long long)q * len + k];
   }
   __syncthreads();
+}
+
+// 1/d of a target-source difference, NaN for d = 0 (a target on a node of
+// another curve).
+__device__ __forceinline__ double2 bary_inv(double2 d) {
+  const double r = rcp_raw64(fma(d.x, d.x, d.y * d.y));
+  return make_double2(d.x * r, -d.y * r);
+}
+
+// (ax, ay) += b * c
+__device__ __forceinline__ void cfma2(double& ax, double& ay, double2 b, double2 c) {
+  ax = fma(b.x, c.x, fma(-b.y, c.y, ax));
+  ay = fma(b.x, c.y, fma(b.y, c.x, ay));
 }
 
 // Result of one barycentric Stokes evaluation.
@@ -1459,100 +1524,128 @@ __device__ double2 bary_coincident(const GeoDev& G, int start, int len, const do
 }
 
 // Evaluates the Stokes DLP (and for NDER = 2 its gradient) of source curve c
-// at the target zt.  All threads of the CTA call it for the same curve; the
-// curve is streamed through shared memory three times (value, first and
-// second derivative passes, :5190-5228 / :5468-5525).
+// at the target zt of every lane.  All threads of the CTA call it for the same
+// curve; warp w holds the same 32 targets as the others and takes its share of
+// the sources, and the sums meet in near_reduce, so that every thread returns
+// the result of its lane.  The curve is read in passes over its shared-memory
+// tiles (value, first and second derivative, :5190-5228 / :5468-5525); a curve
+// of at most NEAR_TK nodes is staged once for all of them.  Bound by the FP64
+// pipe with many targets and by a warp's chain of sources with few: against one
+// thread per target and a correctly rounded division, the near pairs of 3
+// bodies x 64 nodes take 11.8 us (69.6), of 400 x 256 28.7 us (78.1), and the
+// gradients of the latter's shear stress 454 us (2200).
 template <int NDER>
 __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* __restrict__ bdc, double2 zt,
                             bool act) {
   const int start = curve_start(G, c), len = curve_len(G, c);
-  const bool ext = c != 0;
+  const bool ext = c != 0, whole = len <= NEAR_TK;
+  const int wid = threadIdx.x >> 5;
   double2 a = make_double2(0, 0);
   if (ext) a = G.cen[c - 1];
   // Pass 1: values.
-  double2 den = make_double2(0, 0), num[5];
+  double v1[12];   // the denominator, then the five numerators
 #pragma unroll
-  for (int q = 0; q < 5; ++q) num[q] = make_double2(0, 0);
+  for (int q = 0; q < 12; ++q) v1[q] = 0.0;
   for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
     bary_load_tile(T, G, start, len, k0, bdc, ext, a);
     const int kt = min(NEAR_TK, len - k0);
-    for (int kk = 0; kk < kt; ++kk) {
-      const double2 c1 = cmul(T.dz[kk], cinv(csub(T.z[kk], zt)));
-      den = cadd(den, c1);
+    const int kb = kt * (wid + 1) / NEAR_W;
+#pragma unroll 2
+    for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
+      const double2 c1 = cmul(T.dz[kk], bary_inv(csub(T.z[kk], zt)));
+      v1[0] += c1.x;
+      v1[1] += c1.y;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) cfma(num[q], T.b[q][kk], c1);
+      for (int q = 0; q < 5; ++q) cfma2(v1[2 + 2 * q], v1[3 + 2 * q], T.b[q][kk], c1);
     }
   }
+  near_reduce(v1, T.red);
+  const double2 den = make_double2(v1[0], v1[1]);
   double2 u[5];
   {
     const double2 dd = ext ? make_double2(den.x, den.y - EB_TWOPI) : den;
     const double2 di = cinv(dd);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) u[q] = cmul(num[q], di);
+    for (int q = 0; q < 5; ++q) u[q] = cmul(make_double2(v1[2 + 2 * q], v1[3 + 2 * q]), di);
   }
-  // Pass 2: first derivative.
-  double2 den2 = make_double2(0, 0), num2[5];
+  // Pass 2: first derivative (of all five fields when the gradient is asked for).
+  constexpr int ND = NDER == 2 ? 5 : 3;
+  double v2[2 + 2 * ND];
 #pragma unroll
-  for (int q = 0; q < 5; ++q) num2[q] = make_double2(0, 0);
+  for (int q = 0; q < 2 + 2 * ND; ++q) v2[q] = 0.0;
   bool coinc = false;
   for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
-    bary_load_tile(T, G, start, len, k0, bdc, ext, a);
+    if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
     const int kt = min(NEAR_TK, len - k0);
-    for (int kk = 0; kk < kt; ++kk) {
+    const int kb = kt * (wid + 1) / NEAR_W;
+#pragma unroll 2
+    for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
       const double2 d = csub(T.z[kk], zt);
-      const double2 inv = cinv(d);
+      const double2 inv = bary_inv(d);
       const double2 c1 = cmul(T.dz[kk], inv);
       if (ext) {
-        den2 = cadd(den2, cmul(c1, T.za[kk]));
+        cfma2(v2[0], v2[1], c1, T.za[kk]);
         if (cabs2(d) <= 1e-20) { coinc = true; continue; }
       }
       const double2 c2 = cmul(c1, inv);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) cfma(num2[q], csub(T.b[q][kk], u[q]), c2);
+      for (int q = 0; q < ND; ++q) cfma2(v2[2 + 2 * q], v2[3 + 2 * q], csub(T.b[q][kk], u[q]), c2);
     }
   }
-  if (ext && coinc && act) {
+  if (ext) {
+    // a warp adds the branch of the coincident nodes in its own share
+    if (coinc && act) {
 #pragma unroll 1
-    for (int q = 0; q < 5; ++q) {
-      double2 tmp1 = make_double2(0, 0), tmp2 = make_double2(0, 0);
-      for (int k = 0; k < len; ++k) {
-        const double2 d = csub(G.xy[start + k], zt);
-        if (cabs2(d) <= 1e-20) num2[q] = cadd(num2[q], bary_coincident(G, start, len, bdc, q, k, zt, a, tmp1, tmp2));
+      for (int q = 0; q < ND; ++q) {
+        double2 tmp1 = make_double2(0, 0), tmp2 = make_double2(0, 0), add = make_double2(0, 0);
+        for (int k = 0; k < len; ++k) {
+          const double2 d = csub(G.xy[start + k], zt);
+          const int kk = k % NEAR_TK, kt = min(NEAR_TK, len - (k - kk));
+          if (kk >= kt * wid / NEAR_W && kk < kt * (wid + 1) / NEAR_W && cabs2(d) <= 1e-20)
+            add = cadd(add, bary_coincident(G, start, len, bdc, q, k, zt, a, tmp1, tmp2));
+        }
+#pragma unroll
+        for (int p = 0; p < ND; ++p)
+          if (p == q) { v2[2 + 2 * p] += add.x; v2[3 + 2 * p] += add.y; }
       }
     }
   }
+  near_reduce(v2, T.red);
   double2 du[5];
   double2 fac;
-  if (ext) fac = cinv(cmul(csub(zt, a), den2));
+  if (ext) fac = cinv(cmul(csub(zt, a), make_double2(v2[0], v2[1])));
   else fac = cinv(den);
 #pragma unroll
-  for (int q = 0; q < 5; ++q) du[q] = cmul(num2[q], fac);
+  for (int q = 0; q < ND; ++q) du[q] = cmul(make_double2(v2[2 + 2 * q], v2[3 + 2 * q]), fac);
   DLPVal r;
   r.ux = du[0].x - zt.x * du[1].x - zt.y * du[2].x + u[3].x;
   r.uy = -du[0].y + zt.x * du[1].y + zt.y * du[2].y + u[4].x;
   r.u1x = r.u1y = r.u2x = r.u2y = 0.0;
-  if (NDER == 2) {
+  if constexpr (NDER == 2) {
     // Pass 3: second derivative.
-    double2 num3[5];
+    double v3[10];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) num3[q] = make_double2(0, 0);
+    for (int q = 0; q < 10; ++q) v3[q] = 0.0;
     for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
-      bary_load_tile(T, G, start, len, k0, bdc, ext, a);
+      if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
       const int kt = min(NEAR_TK, len - k0);
-      for (int kk = 0; kk < kt; ++kk) {
+      const int kb = kt * (wid + 1) / NEAR_W;
+#pragma unroll 2
+      for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
         const double2 d = csub(T.z[kk], zt);
-        const double2 inv = cinv(d);
+        const double2 inv = bary_inv(d);
         const double2 c3 = cmul(cmul(cmul(T.dz[kk], inv), inv), inv);
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
-          double2 t = csub(csub(T.b[q][kk], u[q]), cmul(du[q], d));
-          cfma(num3[q], t, c3);
+          const double2 t = csub(csub(T.b[q][kk], u[q]), cmul(du[q], d));
+          cfma2(v3[2 * q], v3[2 * q + 1], t, c3);
         }
       }
     }
+    near_reduce(v3, T.red);
     double2 dd[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) dd[q] = cscale(cmul(num3[q], fac), 2.0);
+    for (int q = 0; q < 5; ++q) dd[q] = cscale(cmul(make_double2(v3[2 * q], v3[2 * q + 1]), fac), 2.0);
     r.u1x = dd[0].x - du[1].x - zt.x * dd[1].x - zt.y * dd[2].x + du[3].x;
     r.u1y = -dd[0].y + zt.x * dd[1].y - du[2].x + zt.y * dd[2].y - du[3].y;
     r.u2x = -dd[0].y + du[1].y + zt.x * dd[1].y + zt.y * dd[2].y + du[4].x;
@@ -1561,8 +1654,8 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
   return r;
 }
 
-// Near-pair list evaluation: CTA = (source s, pairs [p0, p1)), one thread per
-// (target, source curve) pair.  Output: (ux, uy) per pair.
+// Near-pair list evaluation: CTA = (source s, pairs [p0, p1) of at most NEAR_T),
+// one lane per (target, source curve) pair.  Output: (ux, uy) per pair.
 __global__ void __launch_bounds__(NEAR_NT)
 k_bary_list(GeoDev G, const int4* __restrict__ work, const int* __restrict__ src_curve,
             const long long* __restrict__ bd_off, const double2* __restrict__ bd,
@@ -1571,11 +1664,11 @@ k_bary_list(GeoDev G, const int4* __restrict__ work, const int* __restrict__ src
   const int4 wk = work[blockIdx.x];
   const int s = wk.x, p0 = wk.y, p1 = wk.z;
   const int c = src_curve[s];
-  const int p = p0 + threadIdx.x;
+  const int p = p0 + (threadIdx.x & 31);
   const bool act = p < p1;
   const double2 zt = txy[pair_tgt[act ? p : p1 - 1]];
   DLPVal r = bary_eval<1>(T, G, c, bd + bd_off[s], zt, act);
-  if (act) out[p] = make_double2(r.ux, r.uy);
+  if (act && threadIdx.x < 32) out[p] = make_double2(r.ux, r.uy);
 }
 
 // ---------------------------------------------------------------------------

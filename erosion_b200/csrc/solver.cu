@@ -154,9 +154,9 @@ static void build_near(State& s, const std::vector<double2>& hxy, const std::vec
     int len = c == 0 ? nout : n;
     hbdoff.push_back(bdtot);
     bdtot += 5LL * len;
-    for (int j0 = 0; j0 < len; j0 += BD_NT) hbdw.push_back(make_int2(sidx, j0));
-    for (long long p0 = cnt[c]; p0 < cnt[c + 1]; p0 += NEAR_NT)
-      hbw.push_back(make_int4(sidx, (int)p0, (int)std::min<long long>(p0 + NEAR_NT, cnt[c + 1]), 0));
+    for (int j0 = 0; j0 < len; j0 += NEAR_T) hbdw.push_back(make_int2(sidx, j0));
+    for (long long p0 = cnt[c]; p0 < cnt[c + 1]; p0 += NEAR_T)
+      hbw.push_back(make_int4(sidx, (int)p0, (int)std::min<long long>(p0 + NEAR_T, cnt[c + 1]), 0));
   }
   nr.h_src_ptr.push_back((int)P);
   for (long long q = 0; q < P; ++q) nr.h_pair_tgt[q] = pt[order[q]];
@@ -874,7 +874,7 @@ void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
   k_self64<<<s.n_self_tasks, 256, 0, st>>>(G, s.ws.p, s.self_tasks.p, s.selfsum.p, SELF_CHUNK_BODY);
   EB_LAUNCH_CHECK();
   if (nr.npairs > 0) {
-    k_bdval<<<nr.n_bd_work, BD_NT, 0, st>>>(G, d_den, nr.bd_work.p, nr.src_curve.p, nr.bd_off.p, s.dker_wall.p,
+    k_bdval<<<nr.n_bd_work, NEAR_NT, 0, st>>>(G, d_den, nr.bd_work.p, nr.src_curve.p, nr.bd_off.p, s.dker_wall.p,
                                             s.dker_body.p, s.bd.p);
     EB_LAUNCH_CHECK();
     k_bary_list<<<nr.n_bary_work, NEAR_NT, 0, st>>>(G, nr.bary_work.p, nr.src_curve.p, nr.bd_off.p, s.bd.p,

@@ -23,7 +23,7 @@ k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict_
   __shared__ BaryTile T;
   const int4 tk = tasks[blockIdx.x];
   const int split = blockIdx.y;
-  const int t = tk.x + threadIdx.x;
+  const int t = tk.x + (threadIdx.x & 31);
   const bool act = t < tk.y;
   const double2 zt = txy[act ? t : tk.y - 1];
   double a[6] = {0, 0, 0, 0, 0, 0};
@@ -32,7 +32,7 @@ k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict_
     DLPVal r = bary_eval<NDER>(T, G, c, bd_all + bd_all_off(G, c), zt, act);
     a[0] += r.ux; a[1] += r.uy; a[2] += r.u1x; a[3] += r.u1y; a[4] += r.u2x; a[5] += r.u2y;
   }
-  if (act) {
+  if (act && threadIdx.x < 32) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) out[((size_t)split * 6 + q) * ntar + t] = a[q];
   }
@@ -261,31 +261,26 @@ k_stress_near_mask(GeoDev G, const double* __restrict__ wall_d2h, const double2*
 }
 
 // Barycentric Stokes DLP gradient of the near source curves only: CTA = task
-// (up to NEAR_NT nodes of one body); the CTA visits, in curve order, every
-// curve that is near for at least one of its nodes, and a node keeps the
-// value only for the curves near to it.  out[q * nb + i], q as k_bary_sum
-// (one split).
+// (up to NEAR_T nodes of one body, one per lane of every warp); the CTA visits,
+// in curve order, every curve that is near for at least one of its nodes, and a
+// node keeps the value only for the curves near to it.  With 32 nodes a CTA
+// visits fewer curves that only some of its nodes need than with 128, and the
+// warps share each curve's nodes (bary_eval).  out[q * nb + i], q as
+// k_bary_sum (one split).
 __global__ void __launch_bounds__(NEAR_NT)
 k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict__ tasks,
                 const unsigned* __restrict__ mask, int mw, double* __restrict__ out) {
   __shared__ BaryTile T;
-  __shared__ unsigned tmask;
   const int nb = G.n * G.M;
   const int4 tk = tasks[blockIdx.x];
-  const int t = tk.x + threadIdx.x;
+  const int t = tk.x + (threadIdx.x & 31);
   const bool act = t < tk.y;
   const int tc = act ? t : tk.y - 1;
   const double2 zt = G.xy[G.nout + tc];
   double a[6] = {0, 0, 0, 0, 0, 0};
   for (int w = 0; w < mw; ++w) {
     const unsigned my = act ? mask[(size_t)tc * mw + w] : 0u;
-    __syncthreads();
-    if (threadIdx.x == 0) tmask = 0u;
-    __syncthreads();
-    const unsigned wor = __reduce_or_sync(0xffffffffu, my);
-    if ((threadIdx.x & 31) == 0 && wor) atomicOr(&tmask, wor);
-    __syncthreads();
-    unsigned bits = tmask;   // block-uniform
+    unsigned bits = __reduce_or_sync(0xffffffffu, my);   // the same in every warp
     while (bits) {
       const int q = __ffs(bits) - 1;
       bits &= bits - 1u;
@@ -296,7 +291,7 @@ k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const int4* __rest
       }
     }
   }
-  if (act) {
+  if (act && threadIdx.x < 32) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) out[(size_t)q * nb + t] = a[q];
   }
@@ -607,7 +602,7 @@ static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all) {
     curves[c] = c;
     off[c] = c == 0 ? 0 : 5LL * pr.nout + 5LL * (c - 1) * pr.n;
     int len = c == 0 ? pr.nout : pr.n;
-    for (int j0 = 0; j0 < len; j0 += BD_NT) work.push_back(make_int2(c, j0));
+    for (int j0 = 0; j0 < len; j0 += NEAR_T) work.push_back(make_int2(c, j0));
   }
   static DBuf<int> d_curves;
   static DBuf<long long> d_off;
@@ -616,7 +611,7 @@ static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all) {
   h2d(d_off.ensure(off.size()), off.data(), off.size(), s.st);
   h2d(d_work.ensure(work.size()), work.data(), work.size(), s.st);
   bd_all.ensure(5LL * pr.nout + 5LL * pr.n * pr.M);
-  k_bdval<<<(unsigned)work.size(), BD_NT, 0, s.st>>>(G, d_den, d_work.p, d_curves.p, d_off.p, s.dker_wall.p,
+  k_bdval<<<(unsigned)work.size(), NEAR_NT, 0, s.st>>>(G, d_den, d_work.p, d_curves.p, d_off.p, s.dker_wall.p,
                                                       s.dker_body.p, bd_all.p);
   EB_LAUNCH_CHECK();
   EB_CK(cudaStreamSynchronize(s.st));   // host vectors go out of scope
@@ -748,8 +743,8 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     bdval_all(s, d_den, bd_all);
     std::vector<int4> tasks;
     for (int b = 0; b < pr.M; ++b)
-      for (int k0 = 0; k0 < pr.n; k0 += NEAR_NT)
-        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_NT), 1 + b, 0));
+      for (int k0 = 0; k0 < pr.n; k0 += NEAR_T)
+        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_T), 1 + b, 0));
     std::vector<int> sc;
     const int nsplit = source_splits((int)tasks.size(), pr.M + 1, sc);
     h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
@@ -776,8 +771,8 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     bdval_all(s, d_den, bd_all);
     std::vector<int4> tasks;
     for (int b = 0; b < pr.M; ++b)
-      for (int k0 = 0; k0 < pr.n; k0 += NEAR_NT)
-        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_NT), 1 + b, 0));
+      for (int k0 = 0; k0 < pr.n; k0 += NEAR_T)
+        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_T), 1 + b, 0));
     h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
     k_bary_sum_near<<<(unsigned)tasks.size(), NEAR_NT, 0, s.st>>>(G, bd_all.p, d_tasks.p, smask.p, mw,
                                                                    pnear.ensure(6LL * nb));
@@ -833,8 +828,8 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
   if (ibary) {
     bdval_all(s, d_den, bd_all);
     std::vector<int4> tasks;
-    for (long long t0 = 0; t0 < ntar; t0 += NEAR_NT)
-      tasks.push_back(make_int4((int)t0, (int)std::min<long long>(ntar, t0 + NEAR_NT), -1, 0));
+    for (long long t0 = 0; t0 < ntar; t0 += NEAR_T)
+      tasks.push_back(make_int4((int)t0, (int)std::min<long long>(ntar, t0 + NEAR_T), -1, 0));
     std::vector<int> sc;
     ns2 = source_splits((int)tasks.size(), pr.M + 1, sc);
     h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
