@@ -1,0 +1,590 @@
+// The far field by clusters.  A cluster is a far-field tile (an arc of 32 wall
+// nodes, or up to 256 nodes of one body).  For every target cluster the source
+// clusters fall into two lists: the separated ones act through their multipole
+// expansion, shifted to a local expansion about the target cluster's centre
+// and evaluated at its nodes; the others are summed pair by pair.
+//
+// In complex notation (z a target, s_j a source, n_j its normal and v_j its
+// weighted strength as complex numbers) the double-layer sum is
+//   u = sum_j (r.n)(r.v) r / |r|^4 = 1/4 [ phi - z conj(phi') + conj(chi) ],
+//   phi(z) = sum A_j/(z - s_j),  A = n v,
+//   chi(z) = sum B_j/(z - s_j) - A_j conj(s_j)/(z - s_j)^2,  B = 2 Re(n conj(v)),
+// z and s_j measured from one common origin.  A and B follow from the pair
+// tensor (n_x v_x, n_x v_y + n_y v_x, n_y v_y) that the direct sums read.  A
+// body's stokeslet l and rotlet xi sit at the centre of its cluster (when the
+// body is a single cluster) and add
+//   phi: -2 q L log,  chi: -2 q conj(L) log + 2 q conj(L) + 4 i xi / (z - c),
+// L = l_x + i l_y, q = 1/(4 pi); of the logarithm only log|.| is kept in the
+// constants, where the imaginary parts of phi and conj(chi) cancel.
+//
+// About a source cluster's centre c with radius R the expansions are
+//   phi = sum_k a_k (R/y)^k / y,  chi = sum_k x_k (R/y)^k / y,  y = z - c,
+//   a_k = sum A t^k,  x_k = sum B t^k - k sum A conj(t) t^(k-1),  t = (s - c)/R,
+// and taking chi to a target centre c + D adds conj(D)/R k a_(k-1) to x_k.  The
+// local coefficients about that centre, w = (z - c - D)/R', are
+//   alpha_l = (-R'/D)^l sum_k C(k + l, l) a_k (R/D)^k / D,
+// a product of one real matrix of binomials with the scaled multipoles of all
+// pairs: FP64 tensor-core work (mma m8n8k4).
+//
+// Accuracy.  Clusters are separated when R <= theta (|D| - R') and R' <= theta
+// (|D| - R), theta = 1/3: cutting both series after CL_P = 32 terms leaves
+// 3^-32 = 5e-16 of the cluster's field, FP64 rounding.  Measured against a
+// direct sum in FP64, the operator on 400 bodies x 256 nodes is as far from
+// the 64-bit value as the direct kernels are (their geometry's rounding).
+//
+// Cost.  Per pair of clusters 4 x 32 x 32 multiply-adds and ~40% around them,
+// against 256 x 256 x ~18 operations for the pairs of two bodies.
+#pragma once
+#include "kernels.cuh"
+
+namespace {
+
+constexpr int CL_P = 32;                 // terms of an expansion
+constexpr double CL_THETA = 1.0 / 3.0;   // separation
+constexpr int CL_MP = 3 * CL_P;          // multipole record of a cluster: a_k, x_k, k a_(k-1)
+constexpr int CL_MAX_TILES = 4096;       // above this the lists (tiles^2 entries) are not built
+
+struct BinomTable {
+  double c[CL_P][CL_P];   // c[l][k] = C(k + l, l)
+  constexpr BinomTable() : c{} {
+    for (int l = 0; l < CL_P; ++l)
+      for (int k = 0; k < CL_P; ++k) c[l][k] = (l == 0 || k == 0) ? 1.0 : c[l - 1][k] + c[l][k - 1];
+  }
+};
+__device__ const BinomTable kBinom{};
+
+// Centre and radius of every cluster: the node mean (of a body that is one
+// cluster the body's own centre, where its stokeslet and rotlet sit) and the
+// largest distance of a node from it.  One warp per cluster.
+__global__ void __launch_bounds__(128)
+k_cl_geom(GeoDev G, int ntile, const int4* __restrict__ tiles, double2* __restrict__ cen, double* __restrict__ rad) {
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= ntile) return;
+  const int4 T = tiles[t];
+  double sx = 0.0, sy = 0.0;
+  for (int k = lane; k < T.y; k += 32) {
+    const double2 p = G.xy[T.x + k];
+    sx += p.x;
+    sy += p.y;
+  }
+  double2 c = make_double2(warp_sum(sx) / T.y, warp_sum(sy) / T.y);
+  if (T.z > 0 && T.y == G.n) c = G.cen[T.z - 1];
+  double r2 = 0.0;
+  for (int k = lane; k < T.y; k += 32) {
+    const double2 p = G.xy[T.x + k];
+    r2 = fmax(r2, cabs2(csub(p, c)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+  if (lane == 0) {
+    cen[t] = c;
+    rad[t] = fmax(sqrt(r2), 1e-30);
+  }
+}
+
+// The lists of target cluster blockIdx.x + tile0.  mask: bit c of node i's row
+// (node index less mask0) marks the source curves that another rule evaluates
+// at that node; a cluster pair with any marked node stays in the near list.
+// expand = 0 puts every cluster there.  A body's own clusters are in neither
+// list (k_self64); the wall's are, its own pairs included.  pairs[0], pairs[1]
+// += node pairs of the near lists with wall and with body sources, unmasked.
+__global__ void __launch_bounds__(256)
+k_cl_lists(GeoDev G, int ntile, int nwt, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
+           const double* __restrict__ rad, const unsigned* __restrict__ mask, int mw, int mask0, int expand,
+           int* __restrict__ near, int* __restrict__ far, double* __restrict__ lnd, int4* __restrict__ cnt,
+           unsigned long long* __restrict__ pairs) {
+  extern __shared__ int marked[];   // marked nodes of this cluster per source curve
+  __shared__ int wn[8], wf[8];
+  const int t = blockIdx.x + tile0;
+  const int4 T = tiles[t];
+  const double2 ct = cen[t];
+  const double rt = rad[t];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (mask) {
+    for (int c = threadIdx.x; c < 32 * mw; c += blockDim.x) marked[c] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < T.y * mw; e += blockDim.x) {
+      const int w = e % mw;
+      unsigned m = mask[(size_t)(T.x - mask0) * mw + e];
+      while (m) {
+        atomicAdd(&marked[32 * w + __ffs(m) - 1], 1);
+        m &= m - 1;
+      }
+    }
+    __syncthreads();
+  }
+  int n0 = 0, f0 = 0;   // entries so far
+  int4 c4 = make_int4(0, 0, 0, 0);
+  unsigned long long pw = 0, pb = 0;
+  for (int s0 = 0; s0 < ntile; s0 += 256) {
+    const int s = s0 + threadIdx.x;
+    bool isn = false, isf = false;
+    double ld = 0.0;
+    if (s < ntile) {
+      const int4 S = tiles[s];
+      if (S.z == 0 || S.z != T.z) {
+        const int mk = mask ? marked[S.z] : 0;
+        const double2 d = csub(ct, cen[s]);
+        const double D = sqrt(cabs2(d)), rs = rad[s];
+        isf = expand && mk == 0 && rs <= CL_THETA * (D - rt) && rt <= CL_THETA * (D - rs);
+        isn = !isf;
+        if (isf) ld = log(D);
+        if (isn) {
+          const unsigned long long p = (unsigned long long)(T.y - mk) * S.y - (s == t ? T.y : 0);
+          if (S.z == 0) pw += p;
+          else pb += p;
+        }
+      }
+    }
+    const unsigned bn = __ballot_sync(0xffffffffu, isn), bf = __ballot_sync(0xffffffffu, isf);
+    if (lane == 0) { wn[wid] = __popc(bn); wf[wid] = __popc(bf); }
+    __syncthreads();
+    int on = n0, of = f0, tn = 0, tf = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < wid) { on += wn[w]; of += wf[w]; }
+      tn += wn[w];
+      tf += wf[w];
+    }
+    const unsigned below = (1u << lane) - 1u;
+    const int in = on + __popc(bn & below), jf = of + __popc(bf & below);
+    if (isn) near[(size_t)t * ntile + in] = s;
+    if (isf) { far[(size_t)t * ntile + jf] = s; lnd[(size_t)t * ntile + jf] = ld; }
+    if (s == nwt) { c4.x = in; c4.z = jf; }   // entries before the first body cluster
+    n0 += tn;
+    f0 += tf;
+    __syncthreads();
+  }
+  // exactly one thread saw s == nwt; without body clusters nobody did
+  if (ntile == nwt) {
+    c4.x = n0;
+    c4.z = f0;
+  }
+  if (threadIdx.x == nwt % 256) cnt[t] = make_int4(c4.x, n0, c4.z, f0);
+  for (int o = 16; o > 0; o >>= 1) {
+    pw += __shfl_xor_sync(0xffffffffu, pw, o);
+    pb += __shfl_xor_sync(0xffffffffu, pb, o);
+  }
+  if (lane == 0 && pw) atomicAdd(pairs, pw);
+  if (lane == 0 && pb) atomicAdd(pairs + 1, pb);
+}
+
+// Multipoles of cluster blockIdx.x + tile0: mp[t][0..31] = a_k, [32..63] = x_k,
+// [64..95] = k a_(k-1) (entry 0: 2 q R L of the stokeslet), lam[t] = -2 q L.
+// den: the density the stokeslets and rotlets are read from (nullptr: none).
+// Warp w sums the powers 4w..4w+3 over all nodes, a node per lane: 11 complex
+// products a node instead of a chain of 32, then the lanes meet in a fixed
+// tree.  Bound by latency (a few hundred FP64 operations per thread).
+__global__ void __launch_bounds__(256)
+k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
+          const double* __restrict__ rad, const double4* __restrict__ sq, const double* __restrict__ den,
+          double2* __restrict__ mp, double2* __restrict__ lam) {
+  __shared__ double2 sA[FAR_TS], sT[FAR_TS];
+  __shared__ double sB[FAR_TS];
+  __shared__ double2 ka[CL_P], ke[CL_P], kb[CL_P];
+  const int t = blockIdx.x + tile0;
+  const int4 T = tiles[t];
+  const double2 c = cen[t];
+  const double R = rad[t], iR = 1.0 / R;
+  for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
+    const double4 S = sq[T.x + j];
+    sA[j] = make_double2(S.x - S.z, S.y);
+    sB[j] = 2.0 * (S.x + S.z);
+    sT[j] = cscale(csub(G.xy[T.x + j], c), iR);
+  }
+  __syncthreads();
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a[4][6];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int v = 0; v < 6; ++v) a[q][v] = 0.0;
+  for (int j = lane; j < T.y; j += 32) {
+    const double2 A = sA[j], tj = sT[j];
+    const double B = sB[j];
+    double2 p = make_double2(1.0, 0.0);   // t^(4 wid)
+    double2 tp = cmul(tj, tj);
+    tp = cmul(tp, tp);
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      if ((wid >> b) & 1) p = cmul(p, tp);
+      tp = cmul(tp, tp);
+    }
+    const double2 At = cmul(A, make_double2(tj.x, -tj.y));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      cfma2(a[q][0], a[q][1], A, p);
+      cfma2(a[q][2], a[q][3], At, p);
+      a[q][4] = fma(B, p.x, a[q][4]);
+      a[q][5] = fma(B, p.y, a[q][5]);
+      p = cmul(p, tj);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int v = 0; v < 6; ++v) a[q][v] = warp_sum(a[q][v]);
+  if (lane == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      ka[4 * wid + q] = make_double2(a[q][0], a[q][1]);
+      ke[4 * wid + q] = make_double2(a[q][2], a[q][3]);
+      kb[4 * wid + q] = make_double2(a[q][4], a[q][5]);
+    }
+  }
+  __syncthreads();
+  const int k = threadIdx.x;
+  if (k >= CL_P) return;
+  double2 x = kb[k], d = make_double2(0, 0);
+  if (k > 0) {
+    x = make_double2(fma(-(double)k, ke[k - 1].x, x.x), fma(-(double)k, ke[k - 1].y, x.y));
+    d = cscale(ka[k - 1], k);
+  } else {
+    double2 L = make_double2(0, 0);
+    double xi = 0.0;
+    if (den && T.z > 0 && T.y == G.n) {
+      L = make_double2(den[ic_of(G, T.z - 1, 0)], den[ic_of(G, T.z - 1, 1)]);
+      xi = den[ic_of(G, T.z - 1, 2)];
+    }
+    const double q2 = 1.0 / EB_TWOPI;   // 2 q
+    x.y += 4.0 * xi;
+    d = cscale(L, q2 * R);
+    lam[t] = cscale(L, -q2);
+  }
+  double2* o = mp + (size_t)t * CL_MP;
+  o[k] = ka[k];
+  o[CL_P + k] = x;
+  o[2 * CL_P + k] = d;
+}
+
+// One FP64 tensor-core product: c (8 x 8) += a (8 x 4) b (4 x 8); a: row
+// lane/4, column lane%4; b: row lane%4, column lane/4; c: row lane/4, columns
+// 2 (lane%4) and the next.
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// The local expansion of the far list of cluster t: loc[0][l] = alpha_l,
+// loc[1][l] = those of chi, valid for all threads on return.  wall_only: only
+// the wall's clusters as sources.  Every warp takes two sources at a time;
+// their phi and chi, real and imaginary, are the 8 columns of the product with
+// the 32 x 32 binomials that a warp holds in registers (a lane 32 of them).
+// Each lane forms its own operand: its component of the scaled multipole of
+// the order k it holds, the power of R/D by recurrence from k to k + 4.  The
+// products stay in registers until they are scaled by (-R'/D)^l and added to
+// the lane's sums, which the warps combine at the end in a fixed order.
+struct ClShared {
+  double2 red[8][CL_P][2];
+  double2 loc[2][CL_P];
+};
+
+__device__ __forceinline__ void cl_shift(const ClView& L, int t, bool wall_only, const double2* __restrict__ mp,
+                                         const double2* __restrict__ lam, ClShared& sh) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int4 c4 = L.cnt[t];
+  const int nf = wall_only ? c4.z : c4.w;
+  const double2 ct = L.cen[t];
+  const double rt = L.rad[t];
+  const int* __restrict__ far = L.far + (size_t)t * L.T;
+  const double* __restrict__ lnd = L.lnd + (size_t)t * L.T;
+  const int kq = lane & 3, bsrc = lane >> 4, bfn = (lane >> 3) & 1, bri = (lane >> 2) & 1;
+  const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
+  double P[4][8];
+#pragma unroll
+  for (int lt = 0; lt < 4; ++lt)
+#pragma unroll
+    for (int kt = 0; kt < 8; ++kt) P[lt][kt] = kBinom.c[8 * lt + row][4 * kt + kq];
+  double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
+  for (int i = 2 * wid; i < nf; i += 16) {
+    const bool vb = i + bsrc < nf;
+    const int s = far[min(i + bsrc, nf - 1)];
+    const double2 D = csub(ct, L.cen[s]);
+    const double R = L.rad[s];
+    const double id2 = rcp_raw64(cabs2(D));
+    const double2 rho = make_double2(D.x * id2, -D.y * id2);   // 1/D
+    const double2 q1 = cscale(rho, R), q2 = cmul(q1, q1), q4 = cmul(q2, q2);
+    double2 g = vb ? rho : make_double2(0, 0);                 // (R/D)^k / D, k = kq
+    if (kq & 1) g = cmul(g, q1);
+    if (kq & 2) g = cmul(g, q2);
+    const double2 kap = bfn ? cscale(make_double2(D.x, -D.y), 1.0 / R) : make_double2(0, 0);
+    const double2* __restrict__ m = mp + (size_t)s * CL_MP;
+    const double2* __restrict__ mb = m + bfn * CL_P;
+    double c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int kt = 0; kt < 8; ++kt) {
+      const int k = 4 * kt + kq;
+      double2 y = mb[k];
+      const double2 d = m[2 * CL_P + k];
+      cfma2(y.x, y.y, kap, d);
+      const double b = bri ? fma(y.x, g.y, y.y * g.x) : fma(y.x, g.x, -y.y * g.y);
+#pragma unroll
+      for (int lt = 0; lt < 4; ++lt) mma_f64(c0[lt], c1[lt], P[lt][kt], b);
+      g = cmul(g, q4);
+    }
+    // scale by (-R'/D)^l of the lane's own source
+    const int from = csrc << 4;
+    const double2 r1 = make_double2(__shfl_sync(0xffffffffu, rho.x, from), __shfl_sync(0xffffffffu, rho.y, from));
+    const int sc = __shfl_sync(0xffffffffu, s, from);
+    const bool vc = i + csrc < nf;
+    const double2 p1 = cscale(r1, -rt), p2 = cmul(p1, p1), p4 = cmul(p2, p2), p8 = cmul(p4, p4);
+    double2 pw = vc ? make_double2(1.0, 0.0) : make_double2(0, 0);
+    if (row & 1) pw = cmul(pw, p1);
+    if (row & 2) pw = cmul(pw, p2);
+    if (row & 4) pw = cmul(pw, p4);
+    double2 lm = lam[sc];
+    if (cfn) lm.y = -lm.y;
+    const double l0 = lnd[min(i + csrc, nf - 1)] - cfn;
+#pragma unroll
+    for (int lt = 0; lt < 4; ++lt) {
+      const int l = 8 * lt + row;
+      const double f = l == 0 ? l0 : -1.0 / l;
+      cfma2(ax[lt], ay[lt], make_double2(fma(lm.x, f, c0[lt]), fma(lm.y, f, c1[lt])), pw);
+      pw = cmul(pw, p8);
+    }
+  }
+#pragma unroll
+  for (int lt = 0; lt < 4; ++lt) {
+    ax[lt] += __shfl_xor_sync(0xffffffffu, ax[lt], 2);
+    ay[lt] += __shfl_xor_sync(0xffffffffu, ay[lt], 2);
+    if (csrc == 0) sh.red[wid][8 * lt + row][cfn] = make_double2(ax[lt], ay[lt]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * CL_P) {
+    const int l = threadIdx.x >> 1, f = threadIdx.x & 1;
+    double2 v = sh.red[0][l][f];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) v = cadd(v, sh.red[w][l][f]);
+    sh.loc[f][l] = v;
+  }
+  __syncthreads();
+}
+
+// The separated sources' velocity at the nodes of cluster blockIdx.x + tile0.
+__global__ void __launch_bounds__(256)
+k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, int wall_only,
+           const double2* __restrict__ mp, const double2* __restrict__ lam, double2* __restrict__ out) {
+  __shared__ ClShared sh;
+  const int t = blockIdx.x + tile0;
+  const int4 T = tiles[t];
+  cl_shift(L, t, wall_only != 0, mp, lam, sh);
+  const double2 c = L.cen[t];
+  const double iR = 1.0 / L.rad[t];
+  for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
+    const double2 w = cscale(csub(G.xy[T.x + j], c), iR);
+    double2 f = sh.loc[0][CL_P - 1], df = make_double2(0, 0), x = sh.loc[1][CL_P - 1];
+#pragma unroll 4
+    for (int l = CL_P - 2; l >= 0; --l) {
+      df = cadd(cmul(df, w), f);
+      f = cadd(cmul(f, w), sh.loc[0][l]);
+      x = cadd(cmul(x, w), sh.loc[1][l]);
+    }
+    const double2 e = cmul(w, make_double2(df.x, -df.y));
+    out[T.x + j] = make_double2(0.25 * (f.x - e.x + x.x), 0.25 * (f.y - e.y - x.y));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The near lists, pair by pair.  CTA = item (target cluster, first node in
+// it): up to 32 targets (FP64) or 64 (FP32, two per lane).  The CTA stages up to
+// 256 sources of consecutive list entries at a time and its 8 warps split
+// them, so that a cluster with few targets still fills 8 warps; the warps' sums
+// meet in a fixed order.  blockIdx.y takes a contiguous part of every list into
+// a slot of its own (out[part * N + i]): few items alone leave SMs idle and a
+// CTA with a long chain of stages.  Bound by the FP64 (FP32) pipe as k_far64
+// (k_far32), whose arithmetic and near masks they share, at thousands of items,
+// by the latency of the stages at tens.
+constexpr int CL_MAXE = 64;   // list entries whose tiles are read at a time
+
+template <int RCP, bool MASK>
+__global__ void __launch_bounds__(256)
+k_cl_near64(GeoDev G, ClView L, const int2* __restrict__ items, const int4* __restrict__ tiles, int wall_only,
+            const double4* __restrict__ sq, const unsigned* __restrict__ mask, int mw, double2* __restrict__ out) {
+  __shared__ double4 sg[FAR_TS];
+  __shared__ double sw[FAR_TS];
+  __shared__ double red[NEAR_W / 2][2][32];
+  __shared__ int4 ent[CL_MAXE];
+  const int2 it = items[blockIdx.x];
+  const int4 T = tiles[it.x];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool act = it.y + lane < T.y;
+  const int i = T.x + (act ? it.y + lane : T.y - 1);
+  const double2 p = G.xy[i];
+  const int4 c4 = L.cnt[it.x];
+  const int nt = wall_only ? c4.x : c4.y;
+  const int ne = (int)((long long)nt * (blockIdx.y + 1) / gridDim.y);
+  const int* __restrict__ near = L.near + (size_t)it.x * L.T;
+  double a[2] = {0.0, 0.0};
+  int eb = 0, nb = 0;   // the entries held in ent: [eb, eb + nb)
+  for (int e0 = (int)((long long)nt * blockIdx.y / gridDim.y); e0 < ne;) {
+    __syncthreads();
+    if (e0 >= eb + nb || (eb + nb < ne && e0 - eb > CL_MAXE / 2)) {   // refill
+      eb = e0;
+      nb = min(CL_MAXE, ne - e0);
+      if ((int)threadIdx.x < nb) ent[threadIdx.x] = tiles[near[e0 + threadIdx.x]];
+      __syncthreads();
+    }
+    // stage the entries from e0 that fit (the same walk in every thread)
+    int m = 0, len = 0;
+    while (e0 + m < eb + nb) {
+      const int4 S = ent[e0 + m - eb];
+      if (len + S.y > FAR_TS) break;
+      if ((int)threadIdx.x >= len && (int)threadIdx.x < len + S.y) {
+        const int g = S.x + (int)threadIdx.x - len;
+        const double2 q = G.xy[g];
+        const double4 s4 = sq[g];
+        sg[threadIdx.x] = make_double4(q.x, q.y, s4.x, s4.y);
+        sw[threadIdx.x] = s4.z;
+      }
+      len += S.y;
+      ++m;
+    }
+    __syncthreads();
+    const int ka = len * wid / NEAR_W, kb = len * (wid + 1) / NEAR_W;
+    int at = 0;   // first staged source of entry e
+    for (int e = e0 - eb; e < e0 - eb + m; ++e) {
+      const int lo = max(ka, at), hi = min(kb, at + ent[e].y);
+      at += ent[e].y;
+      if (lo >= hi) continue;
+      bool use = true;
+      if (MASK) {
+        const int c = ent[e].z;
+        use = !((__ldg(mask + (size_t)i * mw + (c >> 5)) >> (c & 31)) & 1u);
+        if (!__any_sync(0xffffffffu, use)) continue;
+      }
+      double tx = 0.0, ty = 0.0;
+#pragma unroll 4
+      for (int j = lo; j < hi; ++j) {
+        const double4 s = sg[j];   // x, y, S_xx, 2 S_xy
+        const double syy = sw[j];
+        const double rx = p.x - s.x, ry = p.y - s.y;
+        const double ry2 = ry * ry;
+        const double rho2 = fma(rx, rx, ry2);
+        const double tt = fma(s.w, ry, s.z * rx);
+        const double qq = fma(tt, rx, syy * ry2);
+        const double inv = rcp_variant<RCP>(rho2);   // 0 for a wall node on itself
+        const double c = qq * inv * inv;
+        tx = fma(c, rx, tx);
+        ty = fma(c, ry, ty);
+      }
+      if (use) { a[0] += tx; a[1] += ty; }
+    }
+    e0 += m;
+  }
+  __syncthreads();
+  near_reduce(a, red);
+  if (act && wid == 0) out[(size_t)blockIdx.y * G.N + i] = make_double2(a[0], a[1]);
+}
+
+// FP32 pair terms as k_far32's (chunks of F32_CHUNK sources summed in FP32 and
+// added to FP64 accumulators); body sources [cnt.x, cnt.y) of the near list, or
+// the wall's [0, cnt.x) with wall_only.
+template <bool MASK>
+__global__ void __launch_bounds__(256)
+k_cl_near32(GeoDev G, ClView L, const int2* __restrict__ items, const int4* __restrict__ tiles, int wall_only,
+            const float4* __restrict__ src, const float2* __restrict__ tgt, const double2* __restrict__ anchor,
+            const double2* __restrict__ tile_c, const float4* __restrict__ sq32, const unsigned* __restrict__ mask,
+            int mw, double2* __restrict__ out) {
+  __shared__ float4 s_pos[F32_TS], s_q1[F32_TS];
+  __shared__ float2 s_q2[F32_TS];
+  __shared__ double red[NEAR_W / 2][4][32];
+  __shared__ int4 ent[CL_MAXE];
+  __shared__ double2 ecen[CL_MAXE];
+  const int2 it = items[blockIdx.x];
+  const int4 T = tiles[it.x];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k0 = it.y + lane, k1 = k0 + 32;
+  const int i0 = T.x + min(k0, T.y - 1), i1 = T.x + min(k1, T.y - 1);
+  const double2 an = anchor[i0];   // one cluster: one anchor
+  const float2 o0 = tgt[i0], o1 = tgt[i1];
+  const int4 c4 = L.cnt[it.x];
+  const int n0 = wall_only ? 0 : c4.x, nt = (wall_only ? c4.x : c4.y) - n0;
+  const int ne = n0 + (int)((long long)nt * (blockIdx.y + 1) / gridDim.y);
+  const int* __restrict__ near = L.near + (size_t)it.x * L.T;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+  int eb = 0, nb = 0;   // the entries held in ent: [eb, eb + nb)
+  for (int e0 = n0 + (int)((long long)nt * blockIdx.y / gridDim.y); e0 < ne;) {
+    __syncthreads();
+    if (e0 >= eb + nb || (eb + nb < ne && e0 - eb > CL_MAXE / 2)) {   // refill
+      eb = e0;
+      nb = min(CL_MAXE, ne - e0);
+      if ((int)threadIdx.x < nb) {
+        const int ti = near[e0 + threadIdx.x];
+        ent[threadIdx.x] = tiles[ti];
+        ecen[threadIdx.x] = tile_c[ti];
+      }
+      __syncthreads();
+    }
+    int m = 0, len = 0;   // entries and sources staged, every entry padded to whole chunks
+    while (e0 + m < eb + nb) {
+      const int4 S = ent[e0 + m - eb];
+      const int pl = (S.y + F32_CHUNK - 1) / F32_CHUNK * F32_CHUNK;
+      if (len + pl > F32_TS) break;
+      const int k = (int)threadIdx.x - len;
+      if (k >= 0 && k < pl) {
+        if (k < S.y) {
+          const float4 x = src[S.x + k], q = sq32[S.x + k];
+          s_pos[threadIdx.x] = make_float4(-x.x, -x.x, -x.y, -x.y);
+          s_q1[threadIdx.x] = make_float4(q.x, q.x, q.y, q.y);
+          s_q2[threadIdx.x] = make_float2(q.z, q.z);
+        } else {   // zero strength, far from every target: exactly zero terms
+          s_pos[threadIdx.x] = make_float4(-1e4f, -1e4f, -1e4f, -1e4f);
+          s_q1[threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+          s_q2[threadIdx.x] = make_float2(0.f, 0.f);
+        }
+      }
+      len += pl;
+      ++m;
+    }
+    __syncthreads();
+    const int nch = len / F32_CHUNK;
+    const int ca = nch * wid / NEAR_W, cb = nch * (wid + 1) / NEAR_W;
+    int at = 0;   // first chunk of entry e
+    for (int e = e0 - eb; e < e0 - eb + m; ++e) {
+      const int nc = (ent[e].y + F32_CHUNK - 1) / F32_CHUNK;
+      const int lo = max(ca, at), hi = min(cb, at + nc);
+      at += nc;
+      if (lo >= hi) continue;
+      bool u0 = true, u1 = true;
+      if (MASK) {
+        const int c = ent[e].z;
+        u0 = !((__ldg(mask + (size_t)i0 * mw + (c >> 5)) >> (c & 31)) & 1u);
+        u1 = !((__ldg(mask + (size_t)i1 * mw + (c >> 5)) >> (c & 31)) & 1u);
+        if (!__any_sync(0xffffffffu, u0 || u1)) continue;
+      }
+      const double2 cs = ecen[e];
+      const float dx = (float)(an.x - cs.x), dy = (float)(an.y - cs.y);
+      const float2 PX = make_float2(dx + o0.x, dx + o1.x), PY = make_float2(dy + o0.y, dy + o1.y);
+      for (int c = lo; c < hi; ++c) {
+        float2 TX = make_float2(0.f, 0.f), TY = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int j = c * F32_CHUNK; j < (c + 1) * F32_CHUNK; ++j) {
+          const float4 A = s_pos[j], B = s_q1[j];
+          const float2 qyy = s_q2[j];
+          const float2 rx = __fadd2_rn(PX, make_float2(A.x, A.y));
+          const float2 ry = __fadd2_rn(PY, make_float2(A.z, A.w));
+          const float2 ry2 = __fmul2_rn(ry, ry);
+          const float2 rho2 = __ffma2_rn(rx, rx, ry2);
+          const float2 inv = make_float2(rcp_approx(rho2.x), rcp_approx(rho2.y));
+          const float2 t = __ffma2_rn(make_float2(B.z, B.w), ry, __fmul2_rn(make_float2(B.x, B.y), rx));
+          const float2 q = __ffma2_rn(t, rx, __fmul2_rn(qyy, ry2));
+          const float2 cc = __fmul2_rn(__fmul2_rn(q, inv), inv);
+          TX = __ffma2_rn(cc, rx, TX);
+          TY = __ffma2_rn(cc, ry, TY);
+        }
+        if (u0) { a[0] += (double)TX.x; a[1] += (double)TY.x; }
+        if (u1) { a[2] += (double)TX.y; a[3] += (double)TY.y; }
+      }
+    }
+    e0 += m;
+  }
+  __syncthreads();
+  near_reduce(a, red);
+  if (wid == 0) {
+    double2* o = out + (size_t)blockIdx.y * G.N;
+    if (k0 < T.y) o[i0] = make_double2(a[0], a[1]);
+    if (k1 < T.y) o[i1] = make_double2(a[2], a[3]);
+  }
+}
+
+}  // namespace

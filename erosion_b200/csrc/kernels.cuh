@@ -17,6 +17,55 @@ constexpr int NEAR_T = 32;         //   every lane of each warp holding one of t
 constexpr int NEAR_NT = 32 * NEAR_W;
 constexpr int NEAR_TK = 256;       // source nodes per shared-memory tile
 
+// v[q] summed over the CTA's NEAR_W warps for every lane, in a fixed order; all
+// warps receive the sums.  red: NEAR_W / 2 x (at least NV) x 32.
+template <int NV, int NR>
+__device__ __forceinline__ void near_reduce(double (&v)[NV], double (*red)[NR][32]) {
+  static_assert(NV <= NR, "reduction buffer");
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int H = NEAR_W / 2;
+  if (wid >= H) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[wid - H][q][lane] = v[q];
+  }
+  __syncthreads();
+  if (wid < H) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[wid][q][lane] += v[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    double t = red[0][q][lane];
+#pragma unroll
+    for (int w = 1; w < H; ++w) t += red[w][q][lane];
+    v[q] = t;
+  }
+  __syncthreads();
+}
+
+// Lists of the target clusters.  near/far: row t holds the source clusters in
+// ascending order (the wall's first), T entries apart; cnt[t] = (wall entries
+// of near, entries of near, wall entries of far, entries of far); lnd: log |D|
+// of the far entries.
+struct ClView {
+  int T = 0;
+  const double2* __restrict__ cen = nullptr;
+  const double* __restrict__ rad = nullptr;
+  const int* __restrict__ near = nullptr;
+  const int* __restrict__ far = nullptr;
+  const int4* __restrict__ cnt = nullptr;
+  const double* __restrict__ lnd = nullptr;
+};
+
+// Cluster of a node (the tiling of build_tiles).
+__device__ __forceinline__ int tile_of(const GeoDev& G, int g) {
+  const int nwt = (G.nout + WALL_TS - 1) / WALL_TS;
+  if (g < G.nout) return g / WALL_TS;
+  const int r = g - G.nout, b = r / G.n, k = r - b * G.n;
+  return nwt + b * ((G.n + FAR_TS - 1) / FAR_TS) + k / FAR_TS;
+}
+
 // ---------------------------------------------------------------------------
 // Geometry (stokesSolver.f:136-204, :417-457).
 
@@ -263,10 +312,11 @@ __global__ void __launch_bounds__(256) k_prep(GeoDev G, const double* __restrict
 
 // ---------------------------------------------------------------------------
 // Far field, FP64: u_i = sum_{j != i} (r.n_j)(r.w_j sigma_j)/rho^4 r,
-// r = x_i - x_j, over every pair of distinct curves except the (target,
-// source curve) pairs that the near-field bookkeeping replaces (bit c of
-// mask[i]); pairs within a curve are summed by k_self64 with the full density,
-// the far field uses the density less its rigid part (see k_prep).  This is the
+// r = x_i - x_j, over every pair of distinct curves and of distinct wall nodes
+// except the (target, source curve) pairs that the near-field bookkeeping
+// replaces (bit c of mask[i]); pairs within a body are summed by k_self64 with
+// the full density, the far field uses the density less its rigid part (see
+// k_prep; the wall has none).  This is the
 // sum the reference's FMM approximates (stokesSolver.f:636-680; direct form
 // :1563-1584).  Sources are staged tile by tile in shared memory; a tile never
 // crosses a curve, so the mask test is one bit per tile and target.  blockIdx.y
@@ -405,7 +455,7 @@ __device__ __forceinline__ void far64_cta(const GeoDev& G, const double4* __rest
     }
 #pragma unroll
     for (int q = 0; q < TPT; ++q) {
-      bool use = T.z != cv[q];
+      bool use = T.z != cv[q] || T.z == 0;
       if (MASK) use = use && !((__ldg(mask + (size_t)it[q] * mw + (T.z >> 5)) >> (T.z & 31)) & 1u);
       if (use) { ax[q] += tx[q]; ay[q] += ty[q]; }
     }
@@ -714,54 +764,50 @@ __global__ void k_geom32(int ntile, const int4* __restrict__ tiles, const double
   }
 }
 
-// FP64 pairs within each curve (i != j), with the full density: the
-// self-interaction part of the far-field sum.  Task = (first target, count
-// <= 256, curve, source chunk); the wall's sources are split into chunks of
-// SELF_CHUNK and a body's into chunks of body_chunk, whose partial sums land in
-// separate slots (out[slot*N + i]) added in a fixed order by k_combine.
-constexpr int SELF_CHUNK = 512;
-constexpr int SELF_CHUNK_BODY = 64;
-__global__ void __launch_bounds__(256)
-k_self64(GeoDev G, const double2* __restrict__ ws, const int4* __restrict__ tasks, double2* __restrict__ out,
-         int body_chunk) {
-  __shared__ double4 sg[256];
-  __shared__ double2 sw[256];
-  const int4 tk = tasks[blockIdx.x];   // target start, count, curve, chunk
-  const int c = tk.z, chunk = tk.w;
-  const int start = curve_start(G, c), len = curve_len(G, c);
-  const int csz = c == 0 ? SELF_CHUNK : body_chunk;
-  const int kb = chunk * csz, ke = min(len, kb + csz);
-  const int i = tk.x + threadIdx.x;
-  const bool act = threadIdx.x < tk.y;
-  const int ic = act ? i : tk.x;
-  const double2 p = G.xy[ic];
-  double ax = 0.0, ay = 0.0;
-  for (int k0 = kb; k0 < ke; k0 += 256) {
+// FP64 pairs within each body (i != j), with the full density: the
+// self-interaction part of the far-field sum (the wall's is part of the far
+// field).  CTA = 32 nodes of a body, one per lane; its 8 warps split the body's
+// sources and meet in a fixed order.  n^2 pairs of ~18 FP64 operations per
+// body: bound by the FP64 pipe at 400 bodies of 256 nodes, by a warp's chain of
+// n/8 sources for few bodies.
+__global__ void __launch_bounds__(NEAR_NT)
+k_self64(GeoDev G, const double2* __restrict__ ws, double2* __restrict__ out) {
+  __shared__ double4 sg[FAR_TS];
+  __shared__ double sw[FAR_TS];
+  __shared__ double red[NEAR_W / 2][2][32];
+  const int per = (G.n + 31) / 32, b = blockIdx.x / per;
+  const int start = G.nout + b * G.n, k = 32 * (blockIdx.x - b * per) + (threadIdx.x & 31);
+  const int wid = threadIdx.x >> 5;
+  const double2 p = G.xy[start + min(k, G.n - 1)];
+  double a[2] = {0.0, 0.0};
+  for (int k0 = 0; k0 < G.n; k0 += FAR_TS) {
     __syncthreads();
     const int kl = k0 + threadIdx.x;
-    if (kl < ke) {
-      int g = start + kl;
-      double2 q = G.xy[g], nn = G.nrm[g];
-      sg[threadIdx.x] = make_double4(q.x, q.y, nn.x, nn.y);
-      sw[threadIdx.x] = ws[g];
+    if (kl < G.n) {
+      const double2 q = G.xy[start + kl];
+      const double4 S = pair_tensor64(G.nrm[start + kl], ws[start + kl]);
+      sg[threadIdx.x] = make_double4(q.x, q.y, S.x, S.y);
+      sw[threadIdx.x] = S.z;
     }
     __syncthreads();
-    const int kt = min(256, ke - k0);
+    const int kt = min(FAR_TS, G.n - k0);
+    const int hi = kt * (wid + 1) / NEAR_W;
 #pragma unroll 4
-    for (int j = 0; j < kt; ++j) {
+    for (int j = kt * wid / NEAR_W; j < hi; ++j) {
       const double4 s = sg[j];
-      const double2 a = sw[j];
-      double rx = p.x - s.x, ry = p.y - s.y;
-      double rho2 = fma(rx, rx, ry * ry);
-      double rdn = fma(rx, s.z, ry * s.w);
-      double rds = fma(rx, a.x, ry * a.y);
-      double inv = rcp_or_zero(rho2);
-      double cc = rdn * rds * inv * inv;
-      ax = fma(cc, rx, ax);
-      ay = fma(cc, ry, ay);
+      const double rx = p.x - s.x, ry = p.y - s.y;
+      const double ry2 = ry * ry;
+      const double t = fma(s.w, ry, s.z * rx);
+      const double q = fma(t, rx, sw[j] * ry2);
+      const double inv = rcp_newton64<2>(fma(rx, rx, ry2));   // 0 for i = j
+      const double c = q * inv * inv;
+      a[0] = fma(c, rx, a[0]);
+      a[1] = fma(c, ry, a[1]);
     }
   }
-  if (act) out[(size_t)chunk * G.N + i] = make_double2(ax, ay);
+  __syncthreads();
+  near_reduce(a, red);
+  if (threadIdx.x < 32 && k < G.n) out[start + k] = make_double2(a[0], a[1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1315,16 +1361,19 @@ __global__ void __launch_bounds__(256) k_cg_prolong(GeoDev G, const double* __re
   if (threadIdx.x < 3) z[ic_of(G, b, threadIdx.x)] += cs[3 * b + threadIdx.x];
 }
 
-// z_wall = -2 v_wall, and the FP32 source tensors of w * z_wall on the wall
-// (pair_tensor32) for the coupling sum.
-__global__ void k_pc_wall(GeoDev G, const double* __restrict__ v, double* __restrict__ z, float4* __restrict__ sq32) {
+// z_wall = -2 v_wall, and the source tensors of w * z_wall on the wall
+// (pair_tensor32/64) for the coupling sum.
+__global__ void k_pc_wall(GeoDev G, const double* __restrict__ v, double* __restrict__ z, float4* __restrict__ sq32,
+                          double4* __restrict__ sq64) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G.nout) return;
   const double zx = -2.0 * v[g], zy = -2.0 * v[G.nout + g];
   z[g] = zx;
   z[G.nout + g] = zy;
   const double w = G.w[g];
-  sq32[g] = pair_tensor32(G.nrm[g], make_double2(w * zx, w * zy));
+  const double2 nn = G.nrm[g], q = make_double2(w * zx, w * zy);
+  sq32[g] = pair_tensor32(nn, q);
+  sq64[g] = pair_tensor64(nn, q);
 }
 
 // ---------------------------------------------------------------------------
@@ -1345,33 +1394,6 @@ __device__ __forceinline__ void node_fields(const GeoDev& G, const double* __res
   double2 ninv = cinv(nn);
   f[3] = cmul(make_double2(sx * nn.x, sy * nn.x), ninv);
   f[4] = cmul(make_double2(sx * nn.y, sy * nn.y), ninv);
-}
-
-// v[q] summed over the CTA's NEAR_W warps for every lane, in a fixed order; all
-// warps receive the sums.  red: NEAR_W / 2 x (at least NV) x 32.
-template <int NV, int NR>
-__device__ __forceinline__ void near_reduce(double (&v)[NV], double (*red)[NR][32]) {
-  static_assert(NV <= NR, "reduction buffer");
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int H = NEAR_W / 2;
-  if (wid >= H) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) red[wid - H][q][lane] = v[q];
-  }
-  __syncthreads();
-  if (wid < H) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) red[wid][q][lane] += v[q];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double t = red[0][q][lane];
-#pragma unroll
-    for (int w = 1; w < H; ++w) t += red[w][q][lane];
-    v[q] = t;
-  }
-  __syncthreads();
 }
 
 // Boundary values of the five fields on one source curve
@@ -1679,13 +1701,16 @@ k_bary_list(GeoDev G, const int4* __restrict__ work, const int* __restrict__ src
 // COMBINE_G consecutive threads share one node: they split the partial-sum
 // slots, the near pairs and the bodies of the stokeslet/rotlet sum, and their
 // sums meet by warp shuffles (launch nblk(N * COMBINE_G, 256) CTAs of 256).
+// L.T = 0: every body's stokeslet and rotlet is summed here (a logarithm and a
+// division each, 206 us at 400 bodies x 256 nodes), otherwise those of the
+// cluster's near list and the node's own body.
 constexpr int SR_CHUNK = 256;
 constexpr int COMBINE_G = 4;
 __global__ void __launch_bounds__(256)
 k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ partial, int nsplit,
           const int* __restrict__ tptr, const int* __restrict__ tpairs, const double2* __restrict__ pair_out,
-          const double* __restrict__ sigdotn, const double2* __restrict__ selfp, int nself, int nself_body,
-          double* __restrict__ vel) {
+          const double* __restrict__ sigdotn, const double2* __restrict__ selfp, ClView L,
+          const int4* __restrict__ tiles, double* __restrict__ vel) {
   __shared__ double4 sc[SR_CHUNK];   // cx, cy, stokeslet x, stokeslet y
   __shared__ double sr[SR_CHUNK];    // rotlet
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1698,12 +1723,9 @@ k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ 
     double2 v = partial[(size_t)q * G.N + gc];
     ux += v.x; uy += v.y;
   }
-  if (selfp) {
-    const int ns = gc < G.nout ? nself : nself_body;
-    for (int q = sub; q < ns; q += COMBINE_G) {
-      double2 v = selfp[(size_t)q * G.N + gc];
-      ux += v.x; uy += v.y;
-    }
+  if (gc >= G.nout && sub == 0) {
+    double2 v = selfp[gc];
+    ux += v.x; uy += v.y;
   }
   if (tptr) {
     for (int e = tptr[gc] + sub; e < tptr[gc + 1]; e += COMBINE_G) {
@@ -1711,28 +1733,37 @@ k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ 
       ux += v.x; uy += v.y;
     }
   }
-  for (int b0 = 0; b0 < G.M; b0 += SR_CHUNK) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < SR_CHUNK; t += blockDim.x) {
-      int b = b0 + t;
-      if (b < G.M) {
-        double2 cc = G.cen[b];
-        sc[t] = make_double4(cc.x, cc.y, den[ic_of(G, b, 0)], den[ic_of(G, b, 1)]);
-        sr[t] = den[ic_of(G, b, 2)];
-      }
+  auto singular = [&](double2 c, double2 l, double rot) {
+    const double rx = p.x - c.x, ry = p.y - c.y;
+    const double rho2 = rx * rx + ry * ry;
+    const double rd = rx * l.x + ry * l.y;
+    const double lg = log(rho2);
+    const double ir = 1.0 / rho2;
+    ux += 0.5 / EB_TWOPI * (-0.5 * lg * l.x + rd * ir * rx) + rot * ry * ir;
+    uy += 0.5 / EB_TWOPI * (-0.5 * lg * l.y + rd * ir * ry) - rot * rx * ir;
+  };
+  if (L.T > 0) {   // the bodies of the node's near list and its own; the others came with the expansions
+    const int t = tile_of(G, gc), own = tiles[t].z;
+    const int4 c4 = L.cnt[t];
+    for (int e = c4.x - 1 + sub; e < c4.y; e += COMBINE_G) {
+      const int c = e < c4.x ? own : tiles[L.near[(size_t)t * L.T + e]].z;
+      if (c > 0)
+        singular(G.cen[c - 1], make_double2(den[ic_of(G, c - 1, 0)], den[ic_of(G, c - 1, 1)]), den[ic_of(G, c - 1, 2)]);
     }
-    __syncthreads();
-    const int bt = min(SR_CHUNK, G.M - b0);
-    for (int t = sub; t < bt; t += COMBINE_G) {
-      const double4 q = sc[t];
-      const double rot = sr[t];
-      const double rx = p.x - q.x, ry = p.y - q.y;
-      const double rho2 = rx * rx + ry * ry;
-      const double rd = rx * q.z + ry * q.w;
-      const double lg = log(rho2);
-      const double ir = 1.0 / rho2;
-      ux += 0.5 / EB_TWOPI * (-0.5 * lg * q.z + rd * ir * rx) + rot * ry * ir;
-      uy += 0.5 / EB_TWOPI * (-0.5 * lg * q.w + rd * ir * ry) - rot * rx * ir;
+  } else {
+    for (int b0 = 0; b0 < G.M; b0 += SR_CHUNK) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < SR_CHUNK; t += blockDim.x) {
+        int b = b0 + t;
+        if (b < G.M) {
+          double2 cc = G.cen[b];
+          sc[t] = make_double4(cc.x, cc.y, den[ic_of(G, b, 0)], den[ic_of(G, b, 1)]);
+          sr[t] = den[ic_of(G, b, 2)];
+        }
+      }
+      __syncthreads();
+      const int bt = min(SR_CHUNK, G.M - b0);
+      for (int t = sub; t < bt; t += COMBINE_G) singular(make_double2(sc[t].x, sc[t].y), make_double2(sc[t].z, sc[t].w), sr[t]);
     }
   }
 #pragma unroll

@@ -41,11 +41,11 @@ constexpr size_t NA_SCRATCH_BYTES = size_t(24) << 20;
 constexpr int NA_MAX_DEVICES = 64;
 
 // Per-layout tables the host-side operator builds on the CPU: tiles of the
-// far-field sum, their split-K ranges, the self-curve tasks (same order and
-// contents as build_tiles in solver.cu) and the two circulant derivative
+// far-field sum, their split-K ranges (same order and contents as build_tiles
+// in solver.cu) and the two circulant derivative
 // kernels d[m] = (1/2)(-1)^m cot(pi m/n) (fourierDiff, stokesSolver.f:348-388).
-__global__ void k_na_layout(int nout, int n, int M, int nsplit, int nslots, int4* __restrict__ tiles,
-                            int* __restrict__ split_ptr, int4* __restrict__ tasks, double* __restrict__ dker_w,
+__global__ void k_na_layout(int nout, int n, int M, int nsplit, int4* __restrict__ tiles,
+                            int* __restrict__ split_ptr, double* __restrict__ dker_w,
                             double* __restrict__ dker_b) {
   const int nwt = (nout + WALL_TS - 1) / WALL_TS;
   const int tpb = M > 0 ? (n + FAR_TS - 1) / FAR_TS : 0;
@@ -60,18 +60,6 @@ __global__ void k_na_layout(int nout, int n, int M, int nsplit, int nslots, int4
     }
   }
   for (int q = threadIdx.x; q <= nsplit; q += blockDim.x) split_ptr[q] = (int)((long long)q * ntile / nsplit);
-  const int wpt = (nout + 255) / 256;
-  const int nwtask = nslots * wpt;
-  const int bpt = M > 0 ? (n + 255) / 256 : 0;
-  for (int t = threadIdx.x; t < nwtask + M * bpt; t += blockDim.x) {
-    if (t < nwtask) {
-      const int ch = t / wpt, o = (t % wpt) * 256;
-      tasks[t] = make_int4(o, min(256, nout - o), 0, ch);
-    } else {
-      const int r = t - nwtask, b = r / bpt, o = (r % bpt) * 256;
-      tasks[t] = make_int4(nout + b * n + o, min(256, n - o), 1 + b, 0);
-    }
-  }
   for (int m = threadIdx.x; m < nout + n; m += blockDim.x) {
     const int len = m < nout ? nout : n, k = m < nout ? m : m - nout;
     double d = 0.0;
@@ -182,8 +170,6 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     const long long ntot = 2LL * N + 3LL * M;
     const int nwt = (nout + WALL_TS - 1) / WALL_TS;
     const int ntile = nwt + (M > 0 ? M * ((n + FAR_TS - 1) / FAR_TS) : 0);
-    const int nslots = (nout + SELF_CHUNK - 1) / SELF_CHUNK;
-    const int ntask = nslots * ((nout + 255) / 256) + (M > 0 ? M * ((n + 255) / 256) : 0);
 
     Carve cv{nd.base};
     double* wx = cv.take<double>(nout);
@@ -204,8 +190,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     float4* sq32 = cv.take<float4>(N);
     double* sigdotn = cv.take<double>(1);
     int4* tiles = cv.take<int4>(ntile);
-    int4* tasks = cv.take<int4>(ntask);
-    double2* selfsum = cv.take<double2>((size_t)nslots * N);
+    double2* selfsum = cv.take<double2>(N);
     // split-K of the far field as the host-side operator chooses it, capped by
     // the room left in the array
     const int TB = (int)nblk(N, FAR_NT * FAR_TPT);
@@ -220,7 +205,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     G.n = n; G.M = M; G.nout = nout; G.N = N; G.ntot = ntot;
     G.xy = xy; G.nrm = nrm; G.sp = sp; G.cur = cur; G.w = w; G.dz = dz; G.cen = cen; G.rb = rb;
 
-    k_na_layout<<<1, 256, 0, st>>>(nout, n, M, nsplit, nslots, tiles, split_ptr, tasks, dker_w, dker_b);
+    k_na_layout<<<1, 256, 0, st>>>(nout, n, M, nsplit, tiles, split_ptr, dker_w, dker_b);
     EB_LAUNCH_CHECK();
     k_wall_nodes<<<nblk(nout, 256), 256, 0, st>>>(nout, p->wall_a, p->wall_b, p->wall_order, wx, wy);
     EB_LAUNCH_CHECK();
@@ -239,10 +224,12 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     k_far64<false, FAR_NT, FAR_TPT, 0><<<dim3((unsigned)TB, (unsigned)nsplit), FAR_NT, 0, st>>>(
         G, sq64, tiles, split_ptr, nullptr, 0, partial);
     EB_LAUNCH_CHECK();
-    k_self64<<<ntask, 256, 0, st>>>(G, ws, tasks, selfsum, n);   // one chunk per body
-    EB_LAUNCH_CHECK();
-    k_combine<<<nblk((long long)N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, partial, nsplit, nullptr, nullptr, nullptr, sigdotn, selfsum,
-                                            nslots, 1, d_vel);
+    if (M > 0) {
+      k_self64<<<M * nblk(n, 32), NEAR_NT, 0, st>>>(G, ws, selfsum);
+      EB_LAUNCH_CHECK();
+    }
+    k_combine<<<nblk((long long)N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, partial, nsplit, nullptr, nullptr, nullptr,
+                                                                  sigdotn, selfsum, ClView{}, nullptr, d_vel);
     EB_LAUNCH_CHECK();
     set_status(EROSION_OK, "");
     return EROSION_OK;

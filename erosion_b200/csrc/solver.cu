@@ -1,7 +1,7 @@
 // Host orchestration of the boundary operator and the GMRES solve, and the
 // C ABI entry points that replace the reference's libstokes.so.
 #include "state.h"
-#include "kernels.cuh"
+#include "cluster.cuh"
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -239,24 +239,23 @@ static void build_tiles(State& s) {
   s.nsplit = far_split_count(pr.N, s.ntile, FAR_NT * FAR_TPT);
   upload_splits(s, s.split_ptr, s.nsplit, 0, s.ntile);
   s.partial.ensure((size_t)s.nsplit * pr.N);
-  // self-curve tasks: (first target, count <= 256, curve, source chunk)
-  std::vector<int4> st;
-  s.n_self_slots = 1;
-  s.n_self_wall = s.n_self_body = 1;
-  for (int c = 0; c <= pr.M; ++c) {
-    int start = c == 0 ? 0 : pr.nout + (c - 1) * pr.n, len = c == 0 ? pr.nout : pr.n;
-    const int csz = c == 0 ? SELF_CHUNK : SELF_CHUNK_BODY;
-    int nch = (len + csz - 1) / csz;
-    if (c == 0) s.n_self_wall = nch;
-    else s.n_self_body = nch;
-    s.n_self_slots = std::max(s.n_self_slots, nch);
-    for (int ch = 0; ch < nch; ++ch)
-      for (int o = 0; o < len; o += 256) st.push_back(make_int4(start + o, std::min(256, len - o), c, ch));
+  // target items of the cluster kernels: (tile, first node in it)
+  std::vector<int2> i32, i64;
+  for (int t = 0; t < s.ntile; ++t) {
+    for (int o = 0; o < tl[t].y; o += 32) i32.push_back(make_int2(t, o));
+    for (int o = 0; o < tl[t].y; o += 64) i64.push_back(make_int2(t, o));
+    if (t == s.nwall_tiles - 1) {
+      s.n_items32_wall = (int)i32.size();
+      s.n_items64_wall = (int)i64.size();
+    }
   }
-  s.n_self_tasks = (int)st.size();
-  h2d(s.self_tasks.ensure(st.size()), st.data(), st.size(), s.st);
-  // pairs of distinct curves, less the near-masked ones (counted per launch)
-  long long same = (long long)pr.nout * (pr.nout - 1) + (long long)pr.M * pr.n * (pr.n - 1);
+  s.n_items32 = (int)i32.size();
+  s.n_items64 = (int)i64.size();
+  h2d(s.items32.ensure(i32.size()), i32.data(), i32.size(), s.st);
+  h2d(s.items64.ensure(i64.size()), i64.data(), i64.size(), s.st);
+  // pairs of distinct curves and of distinct wall nodes, less the near-masked
+  // ones (counted per launch)
+  long long same = (long long)pr.M * pr.n * (pr.n - 1);
   long long masked = 0, masked_wall = 0;
   for (int q = 0; q < s.near.nsrc; ++q) {
     int c = s.near.h_src_curve[q];
@@ -265,7 +264,7 @@ static void build_tiles(State& s) {
     if (c == 0) masked_wall += m;
   }
   s.far64_pairs = (long long)pr.N * (pr.N - 1) - same - masked;
-  s.farw_pairs = (long long)pr.nout * (pr.N - pr.nout) - masked_wall;
+  s.farw_pairs = (long long)pr.nout * (pr.N - 1) - masked_wall;
   s.far32_pairs = s.far64_pairs - s.farw_pairs;
   EB_CK(cudaStreamSynchronize(s.st));
 }
@@ -496,6 +495,133 @@ static void plan_far(State& s) {
   if (tune) { s.tune_N = pr.N; s.tune_ntile = s.ntile; s.tune_masked = masked; }
 }
 
+// ---------------------------------------------------------------------------
+// The far field by clusters.
+
+// Nodes from which the separated clusters act through expansions; below, every
+// cluster pair is summed directly.  Near lists, expansions and assembly with
+// and without them, FP64 (mixed): 2304 nodes 24.0 and 23.0 us (28.2 and 21.7),
+// 3072 nodes 29.9 and 34.8 us (32.7 and 28.8), 3584 nodes 29.0 and 47.2 us
+// (32.1 and 33.0), 8704 nodes 44.7 and 160.7 us (43.7 and 109.8); the
+// expansions are two launches more.
+constexpr int kExpandNodes = 3200;
+
+static ClView cl_view(const State& s, const ClLists& L) {
+  ClView v;
+  v.T = s.ntile;
+  v.cen = s.cl_cen.p;
+  v.rad = s.cl_rad.p;
+  v.near = L.near.p;
+  v.far = L.far.p;
+  v.cnt = L.cnt.p;
+  v.lnd = L.lnd.p;
+  return v;
+}
+
+// Lists of the target clusters from tile0 on (mask as k_cl_lists takes it).
+void build_lists(State& s, ClLists& L, int tile0, const unsigned* mask, int mw, int mask0, bool expand) {
+  const size_t T = s.ntile;
+  unsigned long long* pairs = L.pairs.ensure(2);
+  EB_CK(cudaMemsetAsync(pairs, 0, 2 * sizeof(unsigned long long), s.st));
+  const size_t smem = mask ? 32 * (size_t)mw * sizeof(int) : 0;
+  k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(s.geo(), s.ntile, s.nwall_tiles, tile0, s.tiles.p, s.cl_cen.p,
+                                                        s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),
+                                                        L.far.ensure(T * T), L.lnd.ensure(T * T), L.cnt.ensure(T),
+                                                        pairs);
+  EB_LAUNCH_CHECK();
+}
+
+// Parts of the near lists: about two CTAs per SM from items CTAs, at most 8.
+// 10 bodies x 128 nodes and 1024 wall nodes (72 items): 31.5 us in one part,
+// 18.3 us in 5.
+static int near_parts(int items) { return std::max(1, std::min(8, (2 * g_num_sms + items - 1) / items)); }
+
+// Decides how the current problem's far field is summed and builds the lists.
+// The direct sum over split tile ranges (launch_far) stays for a forced launch
+// shape and for more tiles than the lists are built for.
+static void plan_clusters(State& s) {
+  const Problem& pr = s.pr;
+  s.cl_active = s.ntile <= CL_MAX_TILES && s.force_shape[0] < 0 && s.force_shape[1] < 0 && s.force_shape[2] < 0;
+  s.cl_expand = s.cl_sing = false;
+  if (!s.cl_active) return;
+  k_cl_geom<<<nblk(s.ntile, 4), 128, 0, s.st>>>(s.geo(), s.ntile, s.tiles.p, s.cl_cen.ensure(s.ntile),
+                                               s.cl_rad.ensure(s.ntile));
+  EB_LAUNCH_CHECK();
+  s.cl_expand = pr.N >= kExpandNodes;
+  s.cl_sing = s.cl_expand && pr.n <= FAR_TS;   // a body in several clusters has no centre among theirs
+  const bool masked = s.near.npairs > 0;
+  build_lists(s, s.cl, 0, masked ? s.near.mask.p : nullptr, s.near.mw, 0, s.cl_expand);
+  s.cl_parts64 = near_parts(s.n_items32);
+  s.cl_parts32 = near_parts(s.n_items64);
+  s.partial.ensure((size_t)(s.cl_parts64 + s.cl_parts32 + 1) * pr.N);
+  if (s.cl_expand) {
+    s.cl_mp.ensure((size_t)s.ntile * CL_MP);
+    s.cl_lam.ensure(s.ntile);
+  }
+  unsigned long long pairs[2] = {0, 0};
+  d2h(pairs, s.cl.pairs.p, 2, s.st);
+  EB_CK(cudaStreamSynchronize(s.st));
+  s.farw_pairs = (long long)pairs[0];
+  s.far32_pairs = (long long)pairs[1];
+  s.far64_pairs = s.farw_pairs + s.far32_pairs;
+}
+
+// FP64 near-list sums (wall_only: of the wall's clusters) into cl_parts64 slots.
+static void launch_near64(State& s, bool wall_only, double2* out) {
+  const Near& nr = s.near;
+  const ClView L = cl_view(s, s.cl);
+  const dim3 g((unsigned)s.n_items32, (unsigned)s.cl_parts64);
+  if (nr.npairs > 0)
+    k_cl_near64<3, true><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
+                                                        nr.mask.p, nr.mw, out);
+  else
+    k_cl_near64<3, false><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
+                                                         nullptr, 0, out);
+  EB_LAUNCH_CHECK();
+}
+
+// FP32 near-list sums of the body clusters into cl_parts32 slots.
+static void launch_near32(State& s, double2* out) {
+  const Near& nr = s.near;
+  const ClView L = cl_view(s, s.cl);
+  const dim3 g((unsigned)s.n_items64, (unsigned)s.cl_parts32);
+  if (nr.npairs > 0)
+    k_cl_near32<true><<<g, 256, 0, s.st>>>(s.geo(), L, s.items64.p, s.tiles.p, 0, s.src32.p, s.tgt32.p,
+                                                     s.anchor.p, s.tile_c.p, s.sq32.p, nr.mask.p, nr.mw, out);
+  else
+    k_cl_near32<false><<<g, 256, 0, s.st>>>(s.geo(), L, s.items64.p, s.tiles.p, 0, s.src32.p, s.tgt32.p,
+                                                      s.anchor.p, s.tile_c.p, s.sq32.p, nullptr, 0, out);
+  EB_LAUNCH_CHECK();
+}
+
+// Expansions of every cluster and their sum over the far lists into out[N].
+static void launch_expansions(State& s, const double* d_den, double2* out) {
+  const GeoDev G = s.geo();
+  k_cl_form<<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p, s.cl_sing ? d_den : nullptr,
+                                       s.cl_mp.p, s.cl_lam.p);
+  EB_LAUNCH_CHECK();
+  k_cl_shift<<<s.ntile, 256, 0, s.st>>>(G, cl_view(s, s.cl), 0, s.tiles.p, 0, s.cl_mp.p, s.cl_lam.p, out);
+  EB_LAUNCH_CHECK();
+}
+
+// The wall's field at the body nodes for the preconditioner (strengths
+// pc_sq32, pc_sq64) into out[0..N) and, with expansions, out[N..2N).
+static void launch_wall_coupling(State& s, double2* out) {
+  const GeoDev G = s.geo();
+  const ClView L = cl_view(s, s.cl);
+  const int nit = s.n_items64 - s.n_items64_wall;
+  k_cl_near32<false><<<nit, 256, 0, s.st>>>(G, L, s.items64.p + s.n_items64_wall, s.tiles.p, 1, s.src32.p, s.tgt32.p,
+                                            s.anchor.p, s.tile_c.p, s.pc_sq32.p, nullptr, 0, out);
+  EB_LAUNCH_CHECK();
+  if (!s.cl_expand) return;
+  k_cl_form<<<s.nwall_tiles, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.pc_sq64.p, nullptr, s.cl_mp.p,
+                                             s.cl_lam.p);
+  EB_LAUNCH_CHECK();
+  k_cl_shift<<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, 1, s.cl_mp.p, s.cl_lam.p,
+                                                        out + s.pr.N);
+  EB_LAUNCH_CHECK();
+}
+
 void setup_problem(State& s, const Problem& in, const double* d_xx, const double* d_yy) {
   const auto t_start = std::chrono::steady_clock::now();
   Problem pr = in;
@@ -564,13 +690,14 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   s.sq32.ensure(N);
   s.tgt32.ensure(N);
   s.anchor.ensure(N);
-  s.selfsum.ensure((size_t)s.n_self_slots * N);
+  s.selfsum.ensure(N);
   s.tile_c.ensure(s.ntile);
   k_geom32<<<s.ntile, 256, 0, st>>>(s.ntile, s.tiles.p, s.xy.p, s.nrm.p, s.tile_c.p, s.src32.p, s.tgt32.p,
                                      s.anchor.p);
   EB_LAUNCH_CHECK();
   harvest_far_timing(s);
   plan_far(s);
+  plan_clusters(s);
   setup_preconditioner(s);
   s.geo_valid = true;
   s.setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
@@ -747,12 +874,16 @@ void setup_preconditioner(State& s) {
   // the wall-to-body coupling runs the FP32 far-field kernel over the wall
   // tiles: its tile splits (whole waves, as the far field's own) and its
   // partial sums, one N-long slot per split
-  {
+  s.pc_sq32.ensure(pr.nout);
+  s.pc_sq64.ensure(pr.nout);
+  if (s.cl_active) {
+    s.pc_wsplit = s.cl_expand ? 2 : 1;
+    s.pc_tw.ensure((size_t)s.pc_wsplit * pr.N);
+  } else {
     const int sh = s.far_shape[1];
     s.pc_wsplit = far_split_count(pr.N, s.nwall_tiles, shape_targets(1, sh), far_resident(1, sh, false));
     upload_splits(s, s.pc_split_ptr, s.pc_wsplit, 0, s.nwall_tiles);
     s.pc_tw.ensure((size_t)s.pc_wsplit * pr.N);
-    s.pc_sq32.ensure(pr.nout);
   }
   // keep the previous inverses (a lagged preconditioner) when allowed
   if (pr.P.precond_refresh > 1 && s.pc_valid && s.pc_M == pr.M && s.pc_n == n && s.pc_nout == pr.nout &&
@@ -828,10 +959,11 @@ void apply_preconditioner(State& s, const double* v, double* z) {
 static void apply_block_gs(State& s, const double* v, double* z) {
   const Problem& pr = s.pr;
   const GeoDev G = s.geo();
-  const int n = pr.n, m = 2 * n + 3, nb = n * pr.M;
-  k_pc_wall<<<nblk(pr.nout, 256), 256, 0, s.st>>>(G, v, z, s.pc_sq32.p);
+  const int n = pr.n, m = 2 * n + 3;
+  k_pc_wall<<<nblk(pr.nout, 256), 256, 0, s.st>>>(G, v, z, s.pc_sq32.p, s.pc_sq64.p);
   EB_LAUNCH_CHECK();
-  launch_far32_unmasked(s, s.pc_sq32.p, s.pc_split_ptr.p, s.pc_wsplit, s.pc_tw.p);
+  if (s.cl_active) launch_wall_coupling(s, s.pc_tw.p);
+  else launch_far32_unmasked(s, s.pc_sq32.p, s.pc_split_ptr.p, s.pc_wsplit, s.pc_tw.p);
   dim3 g(pr.M, (unsigned)std::max(1, (m + 63) / 64));
   k_pc_apply_bodies<<<g, 256, m * sizeof(float), s.st>>>(G, s.pcB.p, v, s.pc_tw.p + pr.nout, pr.N, s.pc_wsplit, z);
   EB_LAUNCH_CHECK();
@@ -863,6 +995,7 @@ void operator_prep(State& s, const double* d_den, double* d_vel) {
 }
 
 int far_slots(const State& s, int prec) {
+  if (s.cl_active) return (prec == 1 ? s.cl_parts32 : 0) + s.cl_parts64 + (s.cl_expand ? 1 : 0);
   return prec == 1 ? s.nsplit32 + s.nsplitw : (prec == 2 ? s.nsplit64f : s.nsplit64t);
 }
 
@@ -871,8 +1004,10 @@ void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
   const GeoDev G = s.geo();
   const Near& nr = s.near;
   cudaStream_t st = s.st;
-  k_self64<<<s.n_self_tasks, 256, 0, st>>>(G, s.ws.p, s.self_tasks.p, s.selfsum.p, SELF_CHUNK_BODY);
-  EB_LAUNCH_CHECK();
+  if (pr.M > 0) {
+    k_self64<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, st>>>(G, s.ws.p, s.selfsum.p);
+    EB_LAUNCH_CHECK();
+  }
   if (nr.npairs > 0) {
     k_bdval<<<nr.n_bd_work, NEAR_NT, 0, st>>>(G, d_den, nr.bd_work.p, nr.src_curve.p, nr.bd_off.p, s.dker_wall.p,
                                             s.dker_body.p, s.bd.p);
@@ -883,16 +1018,33 @@ void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
   }
   k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tptr.p : nullptr,
                                              nr.npairs ? nr.tpairs.p : nullptr, s.pair_out.p, s.sigdotn.p,
-                                             s.selfsum.p, s.n_self_wall, s.n_self_body, d_vel);
+                                             s.selfsum.p, s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel);
   EB_LAUNCH_CHECK();
 }
 
-void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
-  harvest_far_timing(s);
+// The far field of a prepared density into the partial slots, its launches
+// bracketed by the timing events (ef: body sources or all, ew: the wall's
+// sources of the mixed operator).
+static void far_field(State& s, const double* d_den, int kind) {
   const Problem& pr = s.pr;
   cudaStream_t st = s.st;
-  operator_prep(s, d_den, d_vel);
-  const int kind = prec == 1 ? 1 : (prec == 2 ? 2 : 0);
+  const size_t N = pr.N;
+  if (s.cl_active) {
+    EB_CK(cudaEventRecord(s.ef0, st));
+    if (kind != 1) launch_near64(s, false, s.partial.p);
+    else launch_near32(s, s.partial.p);
+    EB_CK(cudaEventRecord(s.ef1, st));
+    if (kind == 1) {   // the wall's sources stay FP64
+      EB_CK(cudaEventRecord(s.ew0, st));
+      launch_near64(s, true, s.partial.p + s.cl_parts32 * N);
+      EB_CK(cudaEventRecord(s.ew1, st));
+      s.farw_pending = true;
+    }
+    if (s.cl_expand) launch_expansions(s, d_den, s.partial.p + (far_slots(s, kind) - 1) * N);
+    s.far_kind = kind;
+    s.far_pending = true;
+    return;
+  }
   const int n1 = kind == 1 ? s.nsplit32 : (kind == 2 ? s.nsplit64f : s.nsplit64t);
   if (n1 > 0) {
     EB_CK(cudaEventRecord(s.ef0, st));
@@ -909,8 +1061,19 @@ void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
     launch_far(s, wk, s.far_shape[wk], s.split_ptrw.p, s.nsplitw, s.partial.p + (size_t)n1 * pr.N);
     EB_CK(cudaEventRecord(s.ew1, st));
     s.farw_pending = true;
+  }
+}
+
+void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
+  harvest_far_timing(s);
+  const Problem& pr = s.pr;
+  cudaStream_t st = s.st;
+  operator_prep(s, d_den, d_vel);
+  const int kind = prec == 1 ? 1 : (prec == 2 ? 2 : 0);
+  far_field(s, d_den, kind);
+  if (kind == 1) {
     s.stats.matvecs_fp32++;
-    if (s.nsplit32 > 0) s.stats.far32_launches++;
+    if (pr.M > 0) s.stats.far32_launches++;
     s.stats.farw_launches++;
   } else if (kind == 2) {
     s.stats.far64f_launches++;
@@ -1241,7 +1404,9 @@ void release_state_buffers(State& s) {
   s.cg_ready = false;
   s.pc_valid = false;
   s.src32.release(); s.sq32.release(); s.tgt32.release(); s.tile_c.release(); s.anchor.release();
-  s.self_tasks.release(); s.selfsum.release(); s.split_ptr32.release(); s.split_ptr64t.release(); s.split_ptrw.release();
+  s.selfsum.release(); s.cl.release(); s.cl_cen.release(); s.cl_rad.release(); s.cl_mp.release(); s.cl_lam.release();
+  s.items32.release(); s.items64.release(); s.pc_sq64.release();
+  s.split_ptr32.release(); s.split_ptr64t.release(); s.split_ptrw.release();
   s.split_tune.release(); s.split_ptr64f.release(); s.tune_N = -1;
   for (int k = 0; k < kFarKinds; ++k) s.tuned_shape[k] = -1;
   s.dker_body_n = s.dker_wall_n = -1;

@@ -102,6 +102,17 @@ struct Near {
   DBuf<unsigned> mask;
 };
 
+// Near and far lists of the clusters (ClView in kernels.cuh).
+struct ClLists {
+  DBuf<int> near, far;
+  DBuf<int4> cnt;
+  DBuf<double> lnd;
+  DBuf<unsigned long long> pairs;
+  void release() {
+    near.release(); far.release(); cnt.release(); lnd.release(); pairs.release();
+  }
+};
+
 struct State {
   std::mutex mu;
   bool init = false;
@@ -141,10 +152,19 @@ struct State {
   DBuf<float4> sq32;        // FP32 far-field source tensors (pair_tensor32)
   DBuf<float2> tgt32;
   DBuf<double2> tile_c, anchor;
-  DBuf<int4> self_tasks;
-  int n_self_tasks = 0, n_self_slots = 1, n_self_wall = 1, n_self_body = 1;
   int pc_wsplit = 1;        // wall-tile splits of the preconditioner's coupling sum
-  DBuf<double2> selfsum;
+  DBuf<double2> selfsum;    // k_self64: pairs within each body
+  // far field by clusters (cluster.cuh)
+  bool cl_active = false;   // the operator sums by clusters, not by split tile ranges
+  bool cl_expand = false;   // separated clusters act through expansions
+  bool cl_sing = false;     // ... and carry the stokeslets and rotlets
+  ClLists cl;
+  DBuf<double2> cl_cen, cl_mp, cl_lam;
+  DBuf<double> cl_rad;
+  DBuf<int2> items32, items64;   // (tile, first node) of 32 and of 64 targets, wall first
+  int n_items32 = 0, n_items64 = 0, n_items32_wall = 0, n_items64_wall = 0;
+  int cl_parts64 = 1, cl_parts32 = 1;   // parts of the near lists (k_cl_near64, k_cl_near32)
+  DBuf<double4> pc_sq64;    // wall pair tensors of the preconditioner's coupling sum
   long long far32_pairs = 0;
   // block Gauss-Seidel preconditioner
   bool pc_active = false;

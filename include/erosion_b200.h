@@ -42,7 +42,9 @@ enum {
  * right-hand side, then solves the double-layer boundary integral equation by
  * unrestarted GMRES to relative residual 1e-8.  density is the initial guess
  * on entry and the solution on exit; nits receives the GMRES iterations.
- * ifmm is accepted for ABI compatibility: the far field is an exact direct sum.
+ * ifmm is accepted for ABI compatibility: the far field is summed directly
+ * between close clusters of nodes and through expansions cut at FP64 rounding
+ * (5e-16 of a cluster's field) between separated ones.
  * ibary = 1 applies the barycentric near-singular corrections with the
  * selection rules of matvec_DLP_fmmbary (ifmm = 1) or to every pair of
  * distinct curves as matvec_DLP_bary does (ifmm = 0); ibary = 0 is the
@@ -115,7 +117,10 @@ typedef struct {
                            (reciprocal to ~1e-12 instead of FP64 rounding) while the
                            residual is above relax_tol and to the wall's sources
                            after, 0 the accurate one; true residuals always use
-                           the accurate one                                       */
+                           the accurate one.  Only the direct sums of a forced
+                           launch shape (erosion_set_far_shape) and of the ensemble
+                           distinguish the two; the sums by clusters are always
+                           accurate                                               */
   int32_t precond_refresh; /* block preconditioner: 0 or 1 rebuilds the body blocks
                            at every set-up; k > 1 keeps the previous inverses for up
                            to k - 1 further set-ups of the same size (consecutive
@@ -164,7 +169,9 @@ typedef struct {
   int64_t near_pairs;       /* (target node, source curve) barycentric pairs       */
   double ms_far32;          /* device time inside the FP32 far-field kernel        */
   int64_t far32_launches;   /* FP32 far-field kernel launches                      */
-  int64_t far32_pairs;      /* source-target pairs per FP32 far-field launch       */
+  int64_t far32_pairs;      /* source-target pairs per FP32 far-field launch (here and
+                               below: the pairs summed one by one, not those of
+                               separated clusters that act through expansions)     */
   double true_residual_checks; /* FP64 true-residual evaluations (mixed mode)      */
   double sweep_residual[8]; /* true residual after each refinement sweep          */
   int64_t sweep_iterations[8]; /* GMRES iterations of each sweep                   */
@@ -438,10 +445,13 @@ double erosion_peak_tflops(int32_t precision);
  * (threads per CTA x targets per thread x variant); by default an autotuner
  * times every candidate on the geometry at hand the first time a problem of
  * that size is set up (problems above 2e8 node pairs) and keeps the fastest.
+ * The shapes are those of the direct sum over every pair, which runs when one
+ * is forced, in ensembles and for more than 4096 clusters (wall arcs of 32
+ * nodes and bodies of up to 256); otherwise the far field is summed by clusters.
  * erosion_set_far_shape(kind, shape) forces candidate 'shape' (kind 0 = the
  * accurate FP64 kernel, 1 = the FP32 kernel, 2 = the fast FP64 kernel of the
  * mixed solve's early iterations) from the next set-up on; shape = -1
- * returns to the autotuner.  Returns EROSION_BAD_INPUT for an unknown kind
+ * returns to the sum by clusters and the autotuner.  Returns EROSION_BAD_INPUT for an unknown kind
  * or shape. */
 int erosion_set_far_shape(int32_t kind, int32_t shape);
 
