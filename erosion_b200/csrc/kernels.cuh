@@ -1406,7 +1406,8 @@ __device__ __forceinline__ void node_fields(const GeoDev& G, const double* __res
 // both sums.  The first three fields are real and cost half a complex one:
 // 36 FP64 operations per pair.  One CTA per (curve, 32 nodes j), a node per
 // lane; the NEAR_W warps split the sources and meet in shared memory in a
-// fixed order.  Bound by the FP64 pipe for long curves and by the latency of a
+// fixed order; work = nullptr takes every curve.  Bound by the FP64 pipe for
+// long curves and by the latency of a
 // warp's chain of sources for short ones, which the split shortens 8-fold.
 // 8.7 us for 3 bodies of 64 nodes near a wall of 256 (one thread per node and
 // two weights: 66.4 us), 155 us for all curves of 400 bodies of 256 nodes and a
@@ -1419,8 +1420,19 @@ k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
   __shared__ double2 sz[NEAR_TK], sdz[NEAR_TK], s01[NEAR_TK], s3[NEAR_TK], s4[NEAR_TK];
   __shared__ double s2[NEAR_TK];
   __shared__ double red[NEAR_W / 2][10][32];
-  const int s = work[blockIdx.x].x, j0 = work[blockIdx.x].y;
-  const int c = src_curve[s];
+  int c, j0;
+  long long off;
+  if (work) {
+    const int s = work[blockIdx.x].x;
+    j0 = work[blockIdx.x].y;
+    c = src_curve[s];
+    off = bd_off[s];
+  } else {   // every curve, the wall first, its fields at 5 times its first node
+    const int nwb = (G.nout + NEAR_T - 1) / NEAR_T, per = (G.n + NEAR_T - 1) / NEAR_T, r = (int)blockIdx.x - nwb;
+    c = r < 0 ? 0 : 1 + r / per;
+    j0 = NEAR_T * (r < 0 ? (int)blockIdx.x : r % per);
+    off = 5LL * curve_start(G, c);
+  }
   const int start = curve_start(G, c), len = curve_len(G, c);
   const double* __restrict__ dk = (c == 0) ? dker_wall : dker_body;
   const double h = EB_TWOPI / len;
@@ -1472,7 +1484,7 @@ k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
   }
   near_reduce(S, red);
   if (wid >= 5 || j0 + lane >= len) return;   // warp q writes field q
-  const long long at = bd_off[s] + (long long)wid * len + j0 + lane;
+  const long long at = off + (long long)wid * len + j0 + lane;
   double2 Sq = make_double2(0, 0), fq = make_double2(0, 0);
 #pragma unroll
   for (int q = 0; q < 5; ++q)

@@ -506,51 +506,24 @@ static void plan_far(State& s) {
 // expansions are two launches more.
 constexpr int kExpandNodes = 3200;
 
-static ClView cl_view(const State& s, const ClLists& L) {
-  ClView v;
-  v.T = s.ntile;
-  v.cen = s.cl_cen.p;
-  v.rad = s.cl_rad.p;
-  v.near = L.near.p;
-  v.far = L.far.p;
-  v.cnt = L.cnt.p;
-  v.lnd = L.lnd.p;
-  return v;
-}
-
-// Lists of the target clusters from tile0 on (mask as k_cl_lists takes it).
-void build_lists(State& s, ClLists& L, int tile0, const unsigned* mask, int mw, int mask0, bool expand) {
-  const size_t T = s.ntile;
-  unsigned long long* pairs = L.pairs.ensure(2);
-  EB_CK(cudaMemsetAsync(pairs, 0, 2 * sizeof(unsigned long long), s.st));
-  const size_t smem = mask ? 32 * (size_t)mw * sizeof(int) : 0;
-  k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(s.geo(), s.ntile, s.nwall_tiles, tile0, s.tiles.p, s.cl_cen.p,
-                                                        s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),
-                                                        L.far.ensure(T * T), L.lnd.ensure(T * T), L.cnt.ensure(T),
-                                                        pairs);
-  EB_LAUNCH_CHECK();
-}
-
 // Parts of the near lists: about two CTAs per SM from items CTAs, at most 8.
 // 10 bodies x 128 nodes and 1024 wall nodes (72 items): 31.5 us in one part,
 // 18.3 us in 5.
-static int near_parts(int items) { return std::max(1, std::min(8, (2 * g_num_sms + items - 1) / items)); }
+int near_parts(int items) { return std::max(1, std::min(8, (2 * g_num_sms + items - 1) / items)); }
 
 // Decides how the current problem's far field is summed and builds the lists.
 // The direct sum over split tile ranges (launch_far) stays for a forced launch
 // shape and for more tiles than the lists are built for.
 static void plan_clusters(State& s) {
   const Problem& pr = s.pr;
-  s.cl_active = s.ntile <= CL_MAX_TILES && s.force_shape[0] < 0 && s.force_shape[1] < 0 && s.force_shape[2] < 0;
-  s.cl_expand = s.cl_sing = false;
-  if (!s.cl_active) return;
+  s.cl_ready = s.ntile <= CL_MAX_TILES;
+  s.cl_active = s.cl_ready && s.force_shape[0] < 0 && s.force_shape[1] < 0 && s.force_shape[2] < 0;
+  s.cl_expand = s.cl_ready && pr.N >= kExpandNodes;
+  s.cl_sing = s.cl_expand && pr.n <= FAR_TS;   // a body in several clusters has no centre among theirs
+  if (!s.cl_ready) return;
   k_cl_geom<<<nblk(s.ntile, 4), 128, 0, s.st>>>(s.geo(), s.ntile, s.tiles.p, s.cl_cen.ensure(s.ntile),
                                                s.cl_rad.ensure(s.ntile));
   EB_LAUNCH_CHECK();
-  s.cl_expand = pr.N >= kExpandNodes;
-  s.cl_sing = s.cl_expand && pr.n <= FAR_TS;   // a body in several clusters has no centre among theirs
-  const bool masked = s.near.npairs > 0;
-  build_lists(s, s.cl, 0, masked ? s.near.mask.p : nullptr, s.near.mw, 0, s.cl_expand);
   s.cl_parts64 = near_parts(s.n_items32);
   s.cl_parts32 = near_parts(s.n_items64);
   s.partial.ensure((size_t)(s.cl_parts64 + s.cl_parts32 + 1) * pr.N);
@@ -558,6 +531,9 @@ static void plan_clusters(State& s) {
     s.cl_mp.ensure((size_t)s.ntile * CL_MP);
     s.cl_lam.ensure(s.ntile);
   }
+  if (!s.cl_active) return;
+  const bool masked = s.near.npairs > 0;
+  build_lists(s, s.cl, 0, masked ? s.near.mask.p : nullptr, s.near.mw, 0, s.cl_expand);
   unsigned long long pairs[2] = {0, 0};
   d2h(pairs, s.cl.pairs.p, 2, s.st);
   EB_CK(cudaStreamSynchronize(s.st));
@@ -572,11 +548,11 @@ static void launch_near64(State& s, bool wall_only, double2* out) {
   const ClView L = cl_view(s, s.cl);
   const dim3 g((unsigned)s.n_items32, (unsigned)s.cl_parts64);
   if (nr.npairs > 0)
-    k_cl_near64<3, true><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
-                                                        nr.mask.p, nr.mw, out);
+    k_cl_near64<false, true><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
+                                                 nr.mask.p, nr.mw, 0, out);
   else
-    k_cl_near64<3, false><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
-                                                         nullptr, 0, out);
+    k_cl_near64<false, false><<<g, 256, 0, s.st>>>(s.geo(), L, s.items32.p, s.tiles.p, wall_only, s.sq64.p,
+                                                  nullptr, 0, 0, out);
   EB_LAUNCH_CHECK();
 }
 
@@ -1018,7 +994,7 @@ void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
   }
   k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tptr.p : nullptr,
                                              nr.npairs ? nr.tpairs.p : nullptr, s.pair_out.p, s.sigdotn.p,
-                                             s.selfsum.p, s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel);
+                                             s.selfsum.p, s.cl_active && s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel);
   EB_LAUNCH_CHECK();
 }
 
@@ -1404,7 +1380,7 @@ void release_state_buffers(State& s) {
   s.cg_ready = false;
   s.pc_valid = false;
   s.src32.release(); s.sq32.release(); s.tgt32.release(); s.tile_c.release(); s.anchor.release();
-  s.selfsum.release(); s.cl.release(); s.cl_cen.release(); s.cl_rad.release(); s.cl_mp.release(); s.cl_lam.release();
+  s.selfsum.release(); s.cl.release(); s.cl_stress.release(); s.cl_cen.release(); s.cl_rad.release(); s.cl_mp.release(); s.cl_lam.release();
   s.items32.release(); s.items64.release(); s.pc_sq64.release();
   s.split_ptr32.release(); s.split_ptr64t.release(); s.split_ptrw.release();
   s.split_tune.release(); s.split_ptr64f.release(); s.tune_N = -1;

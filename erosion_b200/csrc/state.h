@@ -155,10 +155,11 @@ struct State {
   int pc_wsplit = 1;        // wall-tile splits of the preconditioner's coupling sum
   DBuf<double2> selfsum;    // k_self64: pairs within each body
   // far field by clusters (cluster.cuh)
+  bool cl_ready = false;    // clusters exist for this problem
   bool cl_active = false;   // the operator sums by clusters, not by split tile ranges
   bool cl_expand = false;   // separated clusters act through expansions
   bool cl_sing = false;     // ... and carry the stokeslets and rotlets
-  ClLists cl;
+  ClLists cl, cl_stress;    // lists of the operator's near mask and of the shear stress's
   DBuf<double2> cl_cen, cl_mp, cl_lam;
   DBuf<double> cl_rad;
   DBuf<int2> items32, items64;   // (tile, first node) of 32 and of 64 targets, wall first
@@ -217,6 +218,8 @@ struct State {
 
 State& state();
 int eb_num_sms();
+// Parts of the near lists for a launch of that many items.
+int near_parts(int items);
 // Raises a kernel's dynamic shared-memory cap to the device's opt-in maximum
 // (less the kernel's static shared memory).  Every caller sets the same value, so set-ups running concurrently on host
 // threads (the ensemble) that need different sizes never lower the cap under

@@ -2,7 +2,7 @@
 // and velocity/pressure/vorticity at target points (computeQoiTargets,
 // :3099-3323).
 #include "state.h"
-#include "kernels.cuh"
+#include "cluster.cuh"
 #include <cmath>
 
 namespace eb {
@@ -40,70 +40,71 @@ k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict_
 
 // Self-interaction of each body for the deformation tensor: the odd-even
 // trapezoid rule on the subtracted density (:2744-2833) plus the jump term
-// from the spectral tangential derivative of sigma (:2933-2958).  One CTA per
-// body; out[3][n*M] = E11, E12, E22.
-__global__ void __launch_bounds__(256)
+// from the spectral tangential derivative of sigma (:2933-2958).  CTA = 32
+// nodes of a body, one per lane; its 8 warps split the body's sources in pairs
+// of neighbours (one enters the rule, both the derivative) and meet in a fixed
+// order.  out[3][n*M] = E11, E12, E22.  A chain of n/16 pairs a thread: 7.6 us
+// at 37 bodies x 200 nodes and 66 us at 400 x 256 (a thread per node with all
+// sources and a correctly rounded division: 27.8 and 79.2 us).
+__global__ void __launch_bounds__(NEAR_NT)
 k_stress_self(GeoDev G, const double* __restrict__ den, const double* __restrict__ dk, double* __restrict__ out) {
-  extern __shared__ double sm[];
-  const int n = G.n, b = blockIdx.x, nb = G.n * G.M;
-  double* sx = sm;
-  double* sy = sm + n;
-  double* xs = sm + 2 * n;
-  double* ys = sm + 3 * n;
-  double* pxs = sm + 4 * n;
-  double* pys = sm + 5 * n;
-  double* ws = sm + 6 * n;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    int g = G.nout + b * n + k;
-    sx[k] = den[ix_of(G, g)];
-    sy[k] = den[iy_of(G, g)];
-    double2 p = G.xy[g], nn = G.nrm[g];
-    xs[k] = p.x; ys[k] = p.y; pxs[k] = nn.x; pys[k] = nn.y;
-    ws[k] = G.w[g];
+  __shared__ double2 ss[FAR_TS], xs[FAR_TS], ps[FAR_TS];
+  __shared__ double ws[FAR_TS];
+  __shared__ double red[NEAR_W / 2][5][32];
+  const int n = G.n, per = (n + 31) / 32, b = blockIdx.x / per, nb = n * G.M;
+  const int start = G.nout + b * n, wid = threadIdx.x >> 5;
+  const int kk = 32 * (blockIdx.x - b * per) + (threadIdx.x & 31), k = min(kk, n - 1), g = start + k;
+  const double2 x = G.xy[g];
+  const double sxk = den[ix_of(G, g)], syk = den[iy_of(G, g)];
+  const int odd = k & 1;
+  double e[5] = {0, 0, 0, 0, 0};   // E11, E12, E22, d sigma/d theta
+  for (int k0 = 0; k0 < n; k0 += FAR_TS) {
+    __syncthreads();
+    const int j = k0 + threadIdx.x;
+    if (j < n) {
+      const int gj = start + j;
+      ss[threadIdx.x] = make_double2(den[ix_of(G, gj)], den[iy_of(G, gj)]);
+      xs[threadIdx.x] = G.xy[gj];
+      ps[threadIdx.x] = G.nrm[gj];
+      ws[threadIdx.x] = G.w[gj];
+    }
+    __syncthreads();
+    const int kt = min(FAR_TS, n - k0) / 2;   // pairs of neighbours (n is even)
+    const int hi = kt * (wid + 1) / NEAR_W;
+    for (int q = kt * wid / NEAR_W; q < hi; ++q) {
+      const double2 s0 = ss[2 * q], s1 = ss[2 * q + 1];
+      int m = k - (k0 + 2 * q);
+      if (m < 0) m += n;
+      const int m1 = m > 0 ? m - 1 : n - 1;
+      const double d0 = __ldg(dk + m), d1 = __ldg(dk + m1);
+      e[3] = fma(d0, s0.x, fma(d1, s1.x, e[3]));
+      e[4] = fma(d0, s0.y, fma(d1, s1.y, e[4]));
+      const int o = 2 * q + 1 - odd;   // the neighbour of the other parity
+      const double2 p = ps[o], sj = odd ? s0 : s1;
+      const double rx = x.x - xs[o].x, ry = x.y - xs[o].y;
+      const double ir2 = rcp_raw64(fma(rx, rx, ry * ry));
+      const double ir4 = ir2 * ir2 * ws[o];
+      const double rdotn = fma(rx, p.x, ry * p.y), routn = fma(rx, p.y, ry * p.x);
+      const double dsx = sj.x - sxk, dsy = sj.y - syk;
+      const double rdots = fma(rx, dsx, ry * dsy), routs = fma(rx, dsy, ry * dsx);
+      const double A = 2.0 * rdotn * rdots * ir4, C = 4.0 * A * ir2;
+      e[0] += A + 2.0 * ir4 * rx * fma(rdots, p.x, rdotn * dsx) - C * rx * rx;
+      e[1] += ir4 * fma(rdots, routn, rdotn * routs) - C * rx * ry;
+      e[2] += A + 2.0 * ir4 * ry * fma(rdots, p.y, rdotn * dsy) - C * ry * ry;
+    }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    double e11 = 0, e12 = 0, e22 = 0;
-    const double xk = xs[k], yk = ys[k], sxk = sx[k], syk = sy[k];
-    for (int j = (k & 1) ? 0 : 1; j < n; j += 2) {
-      double rx = xk - xs[j], ry = yk - ys[j];
-      double rho2 = rx * rx + ry * ry;
-      double ir2 = 1.0 / rho2;
-      double ir4 = ir2 * ir2, ir6 = ir4 * ir2;
-      double px = pxs[j], py = pys[j];
-      double rdotn = rx * px + ry * py;
-      double routn = rx * py + ry * px;
-      double ssx = sx[j] - sxk, ssy = sy[j] - syk;
-      double rdots = rx * ssx + ry * ssy;
-      double routs = rx * ssy + ry * ssx;
-      double wg = ws[j];
-      e11 += 2.0 * 0.5 * (2.0 * rdotn * rdots * ir4 + 2.0 * rdots * ir4 * rx * px + 2.0 * rdotn * ir4 * rx * ssx -
-                          8.0 * rdotn * rdots * ir6 * rx * rx) * wg;
-      e12 += 2.0 * 0.5 * (rdots * routn * ir4 + rdotn * routs * ir4 - 8.0 * rdotn * rdots * rx * ry * ir6) * wg;
-      e22 += 2.0 * 0.5 * (2.0 * rdotn * rdots * ir4 + 2.0 * rdots * ir4 * ry * py + 2.0 * rdotn * ir4 * ry * ssy -
-                          8.0 * rdotn * rdots * ir6 * ry * ry) * wg;
-    }
-    // jump: t = (-py, px) at the target, d(sigma)/ds . t
-    double dx = 0, dy = 0;
-    for (int j = 0; j < n; ++j) {
-      int m = k - j;
-      if (m < 0) m += n;
-      double d = __ldg(dk + m);
-      dx = fma(d, sx[j], dx);
-      dy = fma(d, sy[j], dy);
-    }
-    const int g = G.nout + b * n + k;
-    const double spk = G.sp[g];
-    const double tx = -pys[k], ty = pxs[k];
-    const double dd = (dx / spk) * tx + (dy / spk) * ty;
-    e11 += 0.5 * dd * (tx * tx - ty * ty);
-    e12 += 0.5 * dd * 2.0 * tx * ty;
-    e22 += 0.5 * dd * (-tx * tx + ty * ty);
-    const int i = b * n + k;
-    out[i] = e11;
-    out[nb + i] = e12;
-    out[2 * nb + i] = e22;
-  }
+  near_reduce(e, red);
+  if (threadIdx.x >= 32 || kk >= n) return;
+  // jump: t = (-py, px) at the target, d(sigma)/ds . t
+  const double spk = G.sp[g];
+  const double2 nn = G.nrm[g];
+  const double tx = -nn.y, ty = nn.x;
+  const double dd = (e[3] / spk) * tx + (e[4] / spk) * ty;
+  const int i = b * n + k;
+  out[i] = e[0] + 0.5 * dd * (tx * tx - ty * ty);
+  out[nb + i] = e[1] + 0.5 * dd * 2.0 * tx * ty;
+  out[2 * nb + i] = e[2] + 0.5 * dd * (-tx * tx + ty * ty);
 }
 
 // Trapezoid deformation tensor of every other curve (deformation_on_boundary_trap,
@@ -260,22 +261,91 @@ k_stress_near_mask(GeoDev G, const double* __restrict__ wall_d2h, const double2*
   }
 }
 
-// Barycentric Stokes DLP gradient of the near source curves only: CTA = task
-// (up to NEAR_T nodes of one body, one per lane of every warp); the CTA visits,
+// The mask of k_stress_near_mask with the clusters at hand: CTA = item (32 nodes
+// of a body cluster, one per lane).  A curve or wall cluster is tested node by
+// node only when its disc, widened by STRESS_NEAR_H of its spacings, reaches
+// the disc of the item's cluster; the warps share the words of the mask and the
+// wall's clusters.  7.1 us at 37 bodies x 200 nodes and 55 us at 400 x 256
+// (every node against every body and wall node: 35 and 334 us).
+__global__ void __launch_bounds__(256)
+k_stress_near_items(GeoDev G, const int2* __restrict__ items, const int4* __restrict__ tiles, int nwt,
+                    const double2* __restrict__ cen, const double* __restrict__ rad, const double2* __restrict__ ext,
+                    int mw, unsigned* __restrict__ mask) {
+  __shared__ unsigned wall[8][32];
+  const int2 it = items[blockIdx.x];
+  const int4 T = tiles[it.x];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = min(it.y + lane, T.y - 1), i = T.x + k - G.nout, own = T.z;
+  const double2 p = G.xy[T.x + k], ct = cen[it.x];
+  const double rt = rad[it.x];
+  const double hs = EB_TWOPI / G.nout;
+  unsigned nearw = 0u;
+  for (int t = wid; t < nwt; t += 8) {
+    const int4 W = tiles[t];
+    const double hl = lane < W.y ? G.sp[W.x + lane] * hs : 0.0;
+    const double2 xl = G.xy[W.x + min(lane, W.y - 1)];
+    double hm = hl;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) hm = fmax(hm, __shfl_xor_sync(0xffffffffu, hm, o));
+    const double reach = rt + rad[t] + STRESS_NEAR_H * hm;
+    if (cabs2(csub(ct, cen[t])) > reach * reach * 1.0001) continue;
+    const double ih2 = 1.0 / (hl * hl);
+    for (int j = 0; j < W.y; ++j) {
+      const double wx = __shfl_sync(0xffffffffu, xl.x, j), wy = __shfl_sync(0xffffffffu, xl.y, j);
+      const double w2 = __shfl_sync(0xffffffffu, ih2, j);
+      const double dx = p.x - wx, dy = p.y - wy;
+      if ((dx * dx + dy * dy) * w2 <= STRESS_NEAR_H * STRESS_NEAR_H) nearw = 1u;
+    }
+  }
+  wall[wid][lane] = nearw;
+  __syncthreads();
+  for (int w = wid; w < mw; w += 8) {
+    const int c = 32 * w + lane;
+    bool cand = false;
+    double2 cc = make_double2(0, 0);
+    double R = 0.0;
+    if (c >= 1 && c <= G.M && c != own) {
+      cc = G.cen[c - 1];
+      const double2 e = ext[c - 1];
+      R = e.x + STRESS_NEAR_H * e.y;
+      const double reach = rt + R;
+      cand = cabs2(csub(ct, cc)) <= reach * reach * 1.0001;
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, cand), bits = 0u;
+    while (todo) {
+      const int q = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const double cx = __shfl_sync(0xffffffffu, cc.x, q), cy = __shfl_sync(0xffffffffu, cc.y, q);
+      const double Rq = __shfl_sync(0xffffffffu, R, q);
+      const double dx = p.x - cx, dy = p.y - cy;
+      if (dx * dx + dy * dy <= Rq * Rq) bits |= 1u << q;
+    }
+    if (w == 0) {
+      unsigned any = 0u;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) any |= wall[v][lane];
+      bits |= any;
+    }
+    if (it.y + lane < T.y) mask[(size_t)i * mw + w] = bits;
+  }
+}
+
+// Barycentric Stokes DLP gradient of the near source curves only: CTA =
+// NEAR_T nodes of one body, one per lane of every warp; the CTA visits,
 // in curve order, every curve that is near for at least one of its nodes, and a
 // node keeps the value only for the curves near to it.  With 32 nodes a CTA
 // visits fewer curves that only some of its nodes need than with 128, and the
 // warps share each curve's nodes (bary_eval).  out[q * nb + i], q as
 // k_bary_sum (one split).
 __global__ void __launch_bounds__(NEAR_NT)
-k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict__ tasks,
-                const unsigned* __restrict__ mask, int mw, double* __restrict__ out) {
+k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const unsigned* __restrict__ mask, int mw,
+                double* __restrict__ out) {
   __shared__ BaryTile T;
   const int nb = G.n * G.M;
-  const int4 tk = tasks[blockIdx.x];
-  const int t = tk.x + (threadIdx.x & 31);
-  const bool act = t < tk.y;
-  const int tc = act ? t : tk.y - 1;
+  const int per = (G.n + NEAR_T - 1) / NEAR_T, b = blockIdx.x / per;
+  const int k = NEAR_T * (blockIdx.x - b * per) + (threadIdx.x & 31);
+  const bool act = k < G.n;
+  const int t = b * G.n + k, tc = act ? t : b * G.n + G.n - 1;
   const double2 zt = G.xy[G.nout + tc];
   double a[6] = {0, 0, 0, 0, 0, 0};
   for (int w = 0; w < mw; ++w) {
@@ -483,6 +553,70 @@ k_stress_final(GeoDev G, const double* __restrict__ den, const double* __restric
   }
 }
 
+// The same assembly when the strain of the other curves comes by clusters:
+// near: barycentric strain (layout of k_bary_sum_near); part: nslot slots of
+// (E11, E12) per node, E22 = -E11; the stokeslets and rotlets of the bodies in
+// the node's near list and its own are summed here, the others came with the
+// expansions (sing = 0: all bodies are summed here).  COMBINE_G threads share a
+// node.
+__global__ void __launch_bounds__(256)
+k_stress_assemble(GeoDev G, const double* __restrict__ den, ClView L, const int4* __restrict__ tiles, int sing,
+                  const double* __restrict__ near, const double2* __restrict__ part, int nslot,
+                  const double* __restrict__ eself, double* __restrict__ tau, double* __restrict__ Eout) {
+  const int nb = G.n * G.M;
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(tid / COMBINE_G), sub = (int)(tid % COMBINE_G);
+  const bool act = i < nb;
+  const int ic = act ? i : nb - 1, g = G.nout + ic;
+  const double2 p = G.xy[g];
+  double e11 = 0, e12 = 0, e22 = 0;
+  for (int s = sub; s < nslot; s += COMBINE_G) {
+    const double2 v = part[(size_t)s * G.N + g];
+    e11 += v.x;
+    e12 += v.y;
+    e22 -= v.x;
+  }
+  auto singular = [&](int b) {
+    const double2 c = G.cen[b];
+    const double lx = den[ic_of(G, b, 0)], ly = den[ic_of(G, b, 1)], rot = den[ic_of(G, b, 2)];
+    const double rx = p.x - c.x, ry = p.y - c.y;
+    const double rd = rx * lx + ry * ly;
+    const double ir2 = 1.0 / (rx * rx + ry * ry), ir4 = ir2 * ir2;
+    e11 += 0.5 / EB_TWOPI * (rd * ir2 - 2 * rx * rx * rd * ir4) - 2.0 * rot * rx * ry * ir4;
+    e12 += rot * (rx * rx - ry * ry) * ir4 - 1.0 / EB_TWOPI * (rd * ir4 * rx * ry);
+    e22 += 0.5 / EB_TWOPI * (rd * ir2 - 2 * ry * ry * rd * ir4) + 2.0 * rot * rx * ry * ir4;
+  };
+  if (sing) {
+    const int t = tile_of(G, g), own = tiles[t].z;
+    const int4 c4 = L.cnt[t];
+    for (int e = c4.x - 1 + sub; e < c4.y; e += COMBINE_G)
+      singular((e < c4.x ? own : tiles[L.near[(size_t)t * L.T + e]].z) - 1);
+  } else {
+    for (int b = sub; b < G.M; b += COMBINE_G) singular(b);
+  }
+  if (sub == 0) {
+    e11 += near[2 * (size_t)nb + ic] + eself[ic];
+    e12 += 0.5 * (near[3 * (size_t)nb + ic] + near[4 * (size_t)nb + ic]) + eself[nb + ic];
+    e22 += near[5 * (size_t)nb + ic] + eself[2 * nb + ic];
+  }
+#pragma unroll
+  for (int o = 1; o < COMBINE_G; o <<= 1) {
+    e11 += __shfl_xor_sync(0xffffffffu, e11, o);
+    e12 += __shfl_xor_sync(0xffffffffu, e12, o);
+    e22 += __shfl_xor_sync(0xffffffffu, e22, o);
+  }
+  if (!act || sub != 0) return;
+  const double2 nn = G.nrm[g];
+  const double tx = -2.0 * e11 * nn.x - 2.0 * e12 * nn.y;
+  const double ty = -2.0 * e12 * nn.x - 2.0 * e22 * nn.y;
+  tau[i] = tx * nn.y - ty * nn.x;
+  if (Eout) {
+    Eout[i] = e11;
+    Eout[nb + i] = e12;
+    Eout[2 * nb + i] = e22;
+  }
+}
+
 // Trapezoid pressure (always) and velocity/vorticity (ibary = 0) at targets
 // from every node (:3170-3197, :3225-3255).  out[(split*4 + q)*ntar + t],
 // q = u, v, p, w.
@@ -594,27 +728,10 @@ k_qoi_final(GeoDev G, const double* __restrict__ den, int ntar, const double2* _
 // Boundary values of all curves (wall first, then every body).
 static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all) {
   const Problem& pr = s.pr;
-  const GeoDev G = s.geo();
-  std::vector<int> curves(pr.M + 1);
-  std::vector<long long> off(pr.M + 1);
-  std::vector<int2> work;
-  for (int c = 0; c <= pr.M; ++c) {
-    curves[c] = c;
-    off[c] = c == 0 ? 0 : 5LL * pr.nout + 5LL * (c - 1) * pr.n;
-    int len = c == 0 ? pr.nout : pr.n;
-    for (int j0 = 0; j0 < len; j0 += NEAR_T) work.push_back(make_int2(c, j0));
-  }
-  static DBuf<int> d_curves;
-  static DBuf<long long> d_off;
-  static DBuf<int2> d_work;
-  h2d(d_curves.ensure(curves.size()), curves.data(), curves.size(), s.st);
-  h2d(d_off.ensure(off.size()), off.data(), off.size(), s.st);
-  h2d(d_work.ensure(work.size()), work.data(), work.size(), s.st);
   bd_all.ensure(5LL * pr.nout + 5LL * pr.n * pr.M);
-  k_bdval<<<(unsigned)work.size(), NEAR_NT, 0, s.st>>>(G, d_den, d_work.p, d_curves.p, d_off.p, s.dker_wall.p,
-                                                      s.dker_body.p, bd_all.p);
+  k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, s.st>>>(
+      s.geo(), d_den, nullptr, nullptr, nullptr, s.dker_wall.p, s.dker_body.p, bd_all.p);
   EB_LAUNCH_CHECK();
-  EB_CK(cudaStreamSynchronize(s.st));   // host vectors go out of scope
 }
 
 int eb_num_sms();
@@ -734,9 +851,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
   static DBuf<int4> d_tasks;
   static DBuf<int> d_sc;
   eself.ensure(3LL * nb);
-  size_t smem = 7 * (size_t)pr.n * sizeof(double);
-  if (smem > 48 * 1024) allow_max_dynamic_smem((const void*)k_stress_self);
-  k_stress_self<<<pr.M, 256, smem, s.st>>>(G, d_den, s.dker_body.p, eself.p);
+  k_stress_self<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, s.st>>>(G, d_den, s.dker_body.p, eself.p);
   EB_LAUNCH_CHECK();
   const int bary = pr.P.ibary == 1;
   if (bary && pr.P.stress_all_bary) {   // every pair barycentric, as the reference evaluates it
@@ -762,20 +877,50 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     static DBuf<unsigned> smask;
     static DBuf<double> pnear;
     const int mw = (pr.M + 1 + 31) / 32;
-    k_stress_wall_dist<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.ensure(nb));
-    EB_LAUNCH_CHECK();
     k_body_extent<<<pr.M, 256, 0, s.st>>>(G, ext.ensure(pr.M));
     EB_LAUNCH_CHECK();
-    k_stress_near_mask<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.p, ext.p, mw, smask.ensure((size_t)nb * mw));
-    EB_LAUNCH_CHECK();
+    smask.ensure((size_t)nb * mw);
+    pnear.ensure(6LL * nb);
     bdval_all(s, d_den, bd_all);
-    std::vector<int4> tasks;
-    for (int b = 0; b < pr.M; ++b)
-      for (int k0 = 0; k0 < pr.n; k0 += NEAR_T)
-        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_T), 1 + b, 0));
-    h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
-    k_bary_sum_near<<<(unsigned)tasks.size(), NEAR_NT, 0, s.st>>>(G, bd_all.p, d_tasks.p, smask.p, mw,
-                                                                   pnear.ensure(6LL * nb));
+    const unsigned near_ctas = pr.M * nblk(pr.n, NEAR_T);
+    if (s.cl_ready) {
+      const int2* items = s.items32.p + s.n_items32_wall;
+      const int nit = s.n_items32 - s.n_items32_wall;
+      k_stress_near_items<<<nit, 256, 0, s.st>>>(G, items, s.tiles.p, s.nwall_tiles, s.cl_cen.p, s.cl_rad.p, ext.p, mw,
+                                                 smask.p);
+      EB_LAUNCH_CHECK();
+      k_bary_sum_near<<<near_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, smask.p, mw, pnear.p);
+      EB_LAUNCH_CHECK();
+      // strengths without the bodies' rigid parts (see k_stress_rigid), the
+      // near lists of this mask, their strain and that of the expansions
+      ClLists& lists = s.cl_stress;
+      k_prep<<<pr.M + 1, 256, 0, s.st>>>(G, d_den, s.ws.p, s.sq64.p, s.sq32.p, s.d_w.ensure(pr.ntot), s.sigdotn.p, 1);
+      EB_LAUNCH_CHECK();
+      build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand);
+      const ClView L = cl_view(s, lists);
+      const int parts = near_parts(nit);
+      s.partial.ensure((size_t)(parts + 1) * pr.N);
+      k_cl_near64<true, true><<<dim3(nit, parts), 256, 0, s.st>>>(G, L, items, s.tiles.p, 0, s.sq64.p, smask.p, mw,
+                                                                  pr.nout, s.partial.p);
+      EB_LAUNCH_CHECK();
+      if (s.cl_expand) {
+        k_cl_form<<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p,
+                                             s.cl_sing ? d_den : nullptr, s.cl_mp.p, s.cl_lam.p);
+        EB_LAUNCH_CHECK();
+        k_cl_shift_strain<<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,
+                                                                     s.cl_lam.p, s.partial.p + (size_t)parts * pr.N);
+        EB_LAUNCH_CHECK();
+      }
+      k_stress_assemble<<<nblk((long long)nb * COMBINE_G, 256), 256, 0, s.st>>>(
+          G, d_den, L, s.tiles.p, s.cl_sing, pnear.p, s.partial.p, parts + (s.cl_expand ? 1 : 0), eself.p, d_tau, d_E);
+      EB_LAUNCH_CHECK();
+      return;
+    }
+    k_stress_wall_dist<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.ensure(nb));
+    EB_LAUNCH_CHECK();
+    k_stress_near_mask<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.p, ext.p, mw, smask.p);
+    EB_LAUNCH_CHECK();
+    k_bary_sum_near<<<near_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, smask.p, mw, pnear.p);
     EB_LAUNCH_CHECK();
     const int nsplit = s.nsplit;
     part.ensure((size_t)nsplit * 3 * nb);
@@ -787,7 +932,6 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     EB_LAUNCH_CHECK();
     k_stress_final<<<nblk(nb, 256), 256, 0, s.st>>>(G, d_den, pnear.p, 1, part.p, nsplit, 1, eself.p, d_tau, d_E);
     EB_LAUNCH_CHECK();
-    EB_CK(cudaStreamSynchronize(s.st));   // the task list goes out of scope
   } else {
     const int nsplit = s.nsplit;
     part.ensure((size_t)nsplit * 3 * nb);

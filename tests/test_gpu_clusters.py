@@ -47,3 +47,21 @@ def test_clusters_match_direct_sum(lib, oracle, M, n, nout, kw, mode):
         # rigid part before a wall of 64 nodes put it 3e-11 and 3e-10 off, whatever the far field
         ref = oracle.matvec(g, den, mode=mode)
         assert rel(a[0], ref) < max(1e-11, 1.5 * rel(b, ref))
+
+
+@pytest.mark.parametrize("M,n,nout", [(1, 64, 130), (17, 128, 1020), (17, 128, 1026), (12, 258, 514), (40, 66, 770),
+                                      (30, 256, 2050)])
+def test_stress_by_clusters_matches_all_barycentric(lib, M, n, nout):
+    """On a density that the nodes resolve (modes up to n/10, decaying) the
+    stress by clusters and the all-barycentric one agree to the 1e-10 asked of
+    the hybrid evaluation elsewhere."""
+    g = packing(M, n, nout)
+    rng = np.random.default_rng(n)
+    th, tw = (2 * np.pi * np.arange(k) / k for k in (n, nout))
+    k = np.arange(1, n // 10 + 1)
+    f = lambda t: (rng.standard_normal(len(k)) / k ** 2) @ np.cos(np.outer(k, t) + rng.uniform(0, 6.3, (len(k), 1)))
+    den = np.concatenate([f(tw), f(tw)] + [f(th) for _ in range(2 * M)] + [rng.standard_normal(3 * M)])
+    tau, E = stokes.shear_stress(g, den)
+    tau_b, E_b = stokes.shear_stress(g, den, stress_all_bary=1)
+    assert rel(tau, tau_b) < 1e-10
+    assert rel(E, E_b) < 1e-10
