@@ -165,8 +165,8 @@ k_cl_lists(GeoDev G, int ntile, int nwt, int tile0, const int4* __restrict__ til
     pw += __shfl_xor_sync(0xffffffffu, pw, o);
     pb += __shfl_xor_sync(0xffffffffu, pb, o);
   }
-  if (lane == 0 && pw) atomicAdd(pairs, pw);
-  if (lane == 0 && pb) atomicAdd(pairs + 1, pb);
+  if (pairs && lane == 0 && pw) atomicAdd(pairs, pw);
+  if (pairs && lane == 0 && pb) atomicAdd(pairs + 1, pb);
 }
 
 // Multipoles of cluster blockIdx.x + tile0: mp[t][0..31] = a_k, [32..63] = x_k,
@@ -654,10 +654,10 @@ static inline ClView cl_view(const State& s, const ClLists& L) {
 }
 
 // Lists of the target clusters from tile0 on (mask as k_cl_lists takes it).
-static inline void build_lists(State& s, ClLists& L, int tile0, const unsigned* mask, int mw, int mask0, bool expand) {
+// pairs: see k_cl_lists, or nullptr.
+static inline void build_lists(State& s, ClLists& L, int tile0, const unsigned* mask, int mw, int mask0, bool expand,
+                               unsigned long long* pairs) {
   const size_t T = s.ntile;
-  unsigned long long* pairs = L.pairs.ensure(2);
-  EB_CK(cudaMemsetAsync(pairs, 0, 2 * sizeof(unsigned long long), s.st));
   const size_t smem = mask ? 32 * (size_t)mw * sizeof(int) : 0;
   k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(s.geo(), s.ntile, s.nwall_tiles, tile0, s.tiles.p, s.cl_cen.p,
                                                         s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),

@@ -1406,33 +1406,22 @@ __device__ __forceinline__ void node_fields(const GeoDev& G, const double* __res
 // both sums.  The first three fields are real and cost half a complex one:
 // 36 FP64 operations per pair.  One CTA per (curve, 32 nodes j), a node per
 // lane; the NEAR_W warps split the sources and meet in shared memory in a
-// fixed order; work = nullptr takes every curve.  Bound by the FP64 pipe for
+// fixed order.  cnt: curves with cnt[c] = 0 are skipped (nullptr: none); the
+// fields of a curve start at 5 times its first node.  Bound by the FP64 pipe for
 // long curves and by the latency of a
 // warp's chain of sources for short ones, which the split shortens 8-fold.
 // 8.7 us for 3 bodies of 64 nodes near a wall of 256 (one thread per node and
 // two weights: 66.4 us), 155 us for all curves of 400 bodies of 256 nodes and a
 // wall of 4096 (1081 us).
 __global__ void __launch_bounds__(NEAR_NT)
-k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
-        const int* __restrict__ src_curve, const long long* __restrict__ bd_off,
-        const double* __restrict__ dker_wall, const double* __restrict__ dker_body,
+k_bdval(GeoDev G, const double* __restrict__ den, const int* __restrict__ cnt, const double* __restrict__ dker_wall, const double* __restrict__ dker_body,
         double2* __restrict__ bd) {
   __shared__ double2 sz[NEAR_TK], sdz[NEAR_TK], s01[NEAR_TK], s3[NEAR_TK], s4[NEAR_TK];
   __shared__ double s2[NEAR_TK];
   __shared__ double red[NEAR_W / 2][10][32];
-  int c, j0;
-  long long off;
-  if (work) {
-    const int s = work[blockIdx.x].x;
-    j0 = work[blockIdx.x].y;
-    c = src_curve[s];
-    off = bd_off[s];
-  } else {   // every curve, the wall first, its fields at 5 times its first node
-    const int nwb = (G.nout + NEAR_T - 1) / NEAR_T, per = (G.n + NEAR_T - 1) / NEAR_T, r = (int)blockIdx.x - nwb;
-    c = r < 0 ? 0 : 1 + r / per;
-    j0 = NEAR_T * (r < 0 ? (int)blockIdx.x : r % per);
-    off = 5LL * curve_start(G, c);
-  }
+  const int nwb = (G.nout + NEAR_T - 1) / NEAR_T, per = (G.n + NEAR_T - 1) / NEAR_T, r = (int)blockIdx.x - nwb;
+  const int c = r < 0 ? 0 : 1 + r / per, j0 = NEAR_T * (r < 0 ? (int)blockIdx.x : r % per);
+  if (cnt && cnt[c] == 0) return;
   const int start = curve_start(G, c), len = curve_len(G, c);
   const double* __restrict__ dk = (c == 0) ? dker_wall : dker_body;
   const double h = EB_TWOPI / len;
@@ -1484,7 +1473,7 @@ k_bdval(GeoDev G, const double* __restrict__ den, const int2* __restrict__ work,
   }
   near_reduce(S, red);
   if (wid >= 5 || j0 + lane >= len) return;   // warp q writes field q
-  const long long at = off + (long long)wid * len + j0 + lane;
+  const long long at = 5LL * start + (long long)wid * len + j0 + lane;
   double2 Sq = make_double2(0, 0), fq = make_double2(0, 0);
 #pragma unroll
   for (int q = 0; q < 5; ++q)
@@ -1688,20 +1677,18 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
   return r;
 }
 
-// Near-pair list evaluation: CTA = (source s, pairs [p0, p1) of at most NEAR_T),
+// Near-pair list evaluation: CTA = (source curve, pairs [p0, p1) of at most NEAR_T),
 // one lane per (target, source curve) pair.  Output: (ux, uy) per pair.
 __global__ void __launch_bounds__(NEAR_NT)
-k_bary_list(GeoDev G, const int4* __restrict__ work, const int* __restrict__ src_curve,
-            const long long* __restrict__ bd_off, const double2* __restrict__ bd,
+k_bary_list(GeoDev G, const int4* __restrict__ work, const double2* __restrict__ bd,
             const int* __restrict__ pair_tgt, const double2* __restrict__ txy, double2* __restrict__ out) {
   __shared__ BaryTile T;
   const int4 wk = work[blockIdx.x];
-  const int s = wk.x, p0 = wk.y, p1 = wk.z;
-  const int c = src_curve[s];
+  const int c = wk.x, p0 = wk.y, p1 = wk.z;
   const int p = p0 + (threadIdx.x & 31);
   const bool act = p < p1;
   const double2 zt = txy[pair_tgt[act ? p : p1 - 1]];
-  DLPVal r = bary_eval<1>(T, G, c, bd + bd_off[s], zt, act);
+  DLPVal r = bary_eval<1>(T, G, c, bd + 5LL * curve_start(G, c), zt, act);
   if (act && threadIdx.x < 32) out[p] = make_double2(r.ux, r.uy);
 }
 
@@ -1720,7 +1707,7 @@ constexpr int SR_CHUNK = 256;
 constexpr int COMBINE_G = 4;
 __global__ void __launch_bounds__(256)
 k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ partial, int nsplit,
-          const int* __restrict__ tptr, const int* __restrict__ tpairs, const double2* __restrict__ pair_out,
+          const int2* __restrict__ tl, const int* __restrict__ tpairs, const double2* __restrict__ pair_out,
           const double* __restrict__ sigdotn, const double2* __restrict__ selfp, ClView L,
           const int4* __restrict__ tiles, double* __restrict__ vel) {
   __shared__ double4 sc[SR_CHUNK];   // cx, cy, stokeslet x, stokeslet y
@@ -1739,8 +1726,9 @@ k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ 
     double2 v = selfp[gc];
     ux += v.x; uy += v.y;
   }
-  if (tptr) {
-    for (int e = tptr[gc] + sub; e < tptr[gc + 1]; e += COMBINE_G) {
+  if (tl) {
+    const int2 r = tl[gc];
+    for (int e = r.x + sub; e < r.x + r.y; e += COMBINE_G) {
       double2 v = pair_out[tpairs[e]];
       ux += v.x; uy += v.y;
     }

@@ -2,6 +2,7 @@
 // C ABI entry points that replace the reference's libstokes.so.
 #include "state.h"
 #include "cluster.cuh"
+#include "near.cuh"
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -69,129 +70,6 @@ static std::vector<double> spectral_kernel(int n) {
   return d;
 }
 
-static void build_near(State& s, const std::vector<double2>& hxy, const std::vector<double>& hsp,
-                       const std::vector<double2>& hcen, const std::vector<double>& hrb) {
-  const Problem& pr = s.pr;
-  const int n = pr.n, M = pr.M, nout = pr.nout, N = pr.N;
-  const double TWOPI = 8.0 * std::atan(1.0);
-  Near& nr = s.near;
-  // matvec_DLP_fmmbary's wall length scale: 'lw' is an implicitly typed
-  // INTEGER there (stokesSolver.f:705-709), so each partial sum truncates and
-  // the mean is an integer division.
-  long long lw = 0;
-  for (int k = 0; k < nout; ++k) lw = (long long)((double)lw + hsp[k]);
-  lw = lw / nout;
-  nr.lw = lw;
-  nr.wall_bodies.clear();
-
-  std::vector<int> pc, pt;   // (source curve, target node) in the reference's order
-  if (pr.P.ibary == 1 && pr.P.ifmm != 0) {
-    const double alpha1 = 4.0, alpha2 = 4.0, bw = pr.P.wall_b;
-    for (int b = 0; b < M; ++b) {   // :711-816
-      double dsum = hrb[b] + alpha2 * (double)lw * TWOPI / nout;
-      double dsum2 = bw - dsum;
-      if (std::fabs(hcen[b].y) >= dsum2) {
-        nr.wall_bodies.push_back(b);
-        for (int k = 0; k < n; ++k) {
-          int g = nout + b * n + k;
-          if (std::fabs(hxy[g].y) >= dsum2) { pc.push_back(0); pt.push_back(g); }
-        }
-        double r = bw - std::fabs(hcen[b].y) + 2.0 * hrb[b];
-        for (int j = 0; j < nout; ++j) {
-          double dx = hcen[b].x - hxy[j].x, dy = hcen[b].y - hxy[j].y;
-          if (dx * dx + dy * dy <= r * r) { pc.push_back(1 + b); pt.push_back(j); }
-        }
-      }
-    }
-    for (int sb = 0; sb < M; ++sb) {   // :838-926
-      for (int t = 0; t < M; ++t) {
-        if (t == sb) continue;
-        double dx = hcen[sb].x - hcen[t].x, dy = hcen[sb].y - hcen[t].y;
-        double d2 = dx * dx + dy * dy;
-        double rsum = hrb[sb] + hrb[t] + alpha1 * (hrb[sb] + hrb[t]) * TWOPI / n;
-        if (d2 <= rsum * rsum) {
-          for (int k = 0; k < n; ++k) {
-            int g = nout + t * n + k;
-            double ex = hcen[sb].x - hxy[g].x, ey = hcen[sb].y - hxy[g].y;
-            if (ex * ex + ey * ey <= rsum * rsum) { pc.push_back(1 + sb); pt.push_back(g); }
-          }
-        }
-      }
-    }
-  } else if (pr.P.ibary == 1) {
-    // matvec_DLP_bary (:1128-1516): every pair of distinct curves.
-    for (int g = nout; g < N; ++g) { pc.push_back(0); pt.push_back(g); }
-    for (int sb = 0; sb < M; ++sb) {
-      for (int g = 0; g < N; ++g) {
-        if (g >= nout && (g - nout) / n == sb) continue;
-        pc.push_back(1 + sb); pt.push_back(g);
-      }
-    }
-  }
-  const long long P = (long long)pc.size();
-  nr.npairs = P;
-  nr.mw = (M + 1 + 31) / 32;
-  if (P == 0) { nr.nsrc = 0; nr.n_bd_work = nr.n_bary_work = 0; return; }
-  // group by source curve, stable
-  std::vector<long long> cnt(M + 2, 0);
-  for (long long p = 0; p < P; ++p) cnt[pc[p] + 1]++;
-  for (int c = 0; c <= M; ++c) cnt[c + 1] += cnt[c];
-  std::vector<int> order(P);
-  {
-    std::vector<long long> pos(cnt.begin(), cnt.end() - 1);
-    for (long long p = 0; p < P; ++p) order[pos[pc[p]]++] = (int)p;
-  }
-  nr.h_src_curve.clear(); nr.h_src_ptr.clear(); nr.h_pair_tgt.assign(P, 0);
-  std::vector<long long> hbdoff;
-  std::vector<int2> hbdw;
-  std::vector<int4> hbw;
-  long long bdtot = 0;
-  for (int c = 0; c <= M; ++c) {
-    if (cnt[c + 1] == cnt[c]) continue;
-    int sidx = (int)nr.h_src_curve.size();
-    nr.h_src_curve.push_back(c);
-    nr.h_src_ptr.push_back((int)cnt[c]);
-    int len = c == 0 ? nout : n;
-    hbdoff.push_back(bdtot);
-    bdtot += 5LL * len;
-    for (int j0 = 0; j0 < len; j0 += NEAR_T) hbdw.push_back(make_int2(sidx, j0));
-    for (long long p0 = cnt[c]; p0 < cnt[c + 1]; p0 += NEAR_T)
-      hbw.push_back(make_int4(sidx, (int)p0, (int)std::min<long long>(p0 + NEAR_T, cnt[c + 1]), 0));
-  }
-  nr.h_src_ptr.push_back((int)P);
-  for (long long q = 0; q < P; ++q) nr.h_pair_tgt[q] = pt[order[q]];
-  nr.nsrc = (int)nr.h_src_curve.size();
-  nr.bd_total = bdtot;
-  nr.n_bd_work = (int)hbdw.size();
-  nr.n_bary_work = (int)hbw.size();
-  // per-target list of pair slots (pairs are now in grouped order)
-  std::vector<int> tptr(N + 1, 0), tpairs(P);
-  for (long long q = 0; q < P; ++q) tptr[nr.h_pair_tgt[q] + 1]++;
-  for (int g = 0; g < N; ++g) tptr[g + 1] += tptr[g];
-  {
-    std::vector<int> pos(tptr.begin(), tptr.end() - 1);
-    for (long long q = 0; q < P; ++q) tpairs[pos[nr.h_pair_tgt[q]]++] = (int)q;
-  }
-  std::vector<unsigned> mask((size_t)N * nr.mw, 0u);
-  for (long long q = 0; q < P; ++q) {
-    int g = nr.h_pair_tgt[q];
-    int c = pc[order[q]];
-    mask[(size_t)g * nr.mw + (c >> 5)] |= 1u << (c & 31);
-  }
-  cudaStream_t st = s.st;
-  h2d(nr.src_curve.ensure(nr.nsrc), nr.h_src_curve.data(), nr.nsrc, st);
-  h2d(nr.pair_tgt.ensure(P), nr.h_pair_tgt.data(), P, st);
-  h2d(nr.tptr.ensure(N + 1), tptr.data(), N + 1, st);
-  h2d(nr.tpairs.ensure(P), tpairs.data(), P, st);
-  h2d(nr.bd_off.ensure(nr.nsrc), hbdoff.data(), nr.nsrc, st);
-  h2d(nr.bd_work.ensure(hbdw.size()), hbdw.data(), hbdw.size(), st);
-  h2d(nr.bary_work.ensure(hbw.size()), hbw.data(), hbw.size(), st);
-  h2d(nr.mask.ensure(mask.size()), mask.data(), mask.size(), st);
-  s.bd.ensure(bdtot);
-  s.pair_out.ensure(P);
-  EB_CK(cudaStreamSynchronize(st));   // host vectors go out of scope
-}
-
 // Split-K of the far-field sums: about 8 (target block, tile range) CTAs per
 // SM, contiguous tile ranges of equal count.  With the kernel's resident CTAs
 // per SM known (resident > 0), the count is chosen within [want/2, 2 want]
@@ -223,50 +101,45 @@ static void upload_splits(State& s, DBuf<int>& buf, int ns, int t0, int t1) {
   EB_CK(cudaStreamSynchronize(s.st));   // sp goes out of scope
 }
 
+// Tiles, their split ranges and the target items of the cluster kernels: a
+// function of the sizes alone, kept while they stay the same.
 static void build_tiles(State& s) {
   const Problem& pr = s.pr;
+  if (s.lay_n == pr.n && s.lay_M == pr.M && s.lay_nout == pr.nout) {
+    s.partial.ensure((size_t)s.nsplit * pr.N);
+    return;
+  }
+  s.lay_n = -1;
   std::vector<int4> tl;
+  std::vector<int2> i32, i64;
   auto add = [&](int start, int len, int c, int ts) {
-    for (int o = 0; o < len; o += ts) tl.push_back(make_int4(start + o, std::min(ts, len - o), c, 0));
+    for (int o = 0; o < len; o += ts) {
+      const int t = (int)tl.size(), k = std::min(ts, len - o);
+      tl.push_back(make_int4(start + o, k, c, 0));
+      for (int q = 0; q < k; q += 32) i32.push_back(make_int2(t, q));   // (tile, first node in it)
+      for (int q = 0; q < k; q += 64) i64.push_back(make_int2(t, q));
+    }
   };
   add(0, pr.nout, 0, WALL_TS);
   s.nwall_tiles = (int)tl.size();
+  s.n_items32_wall = (int)i32.size();
+  s.n_items64_wall = (int)i64.size();
   for (int b = 0; b < pr.M; ++b) add(pr.nout + b * pr.n, pr.n, 1 + b, FAR_TS);
   s.ntile = (int)tl.size();
+  s.n_items32 = (int)i32.size();
+  s.n_items64 = (int)i64.size();
   h2d(s.tiles.ensure(tl.size()), tl.data(), tl.size(), s.st);
+  h2d(s.items32.ensure(i32.size()), i32.data(), i32.size(), s.st);
+  h2d(s.items64.ensure(i64.size()), i64.data(), i64.size(), s.st);
   // tile splits of the shear-stress and target sums (the far-field kernels
   // get theirs from plan_far, per launch shape)
   s.nsplit = far_split_count(pr.N, s.ntile, FAR_NT * FAR_TPT);
   upload_splits(s, s.split_ptr, s.nsplit, 0, s.ntile);
   s.partial.ensure((size_t)s.nsplit * pr.N);
-  // target items of the cluster kernels: (tile, first node in it)
-  std::vector<int2> i32, i64;
-  for (int t = 0; t < s.ntile; ++t) {
-    for (int o = 0; o < tl[t].y; o += 32) i32.push_back(make_int2(t, o));
-    for (int o = 0; o < tl[t].y; o += 64) i64.push_back(make_int2(t, o));
-    if (t == s.nwall_tiles - 1) {
-      s.n_items32_wall = (int)i32.size();
-      s.n_items64_wall = (int)i64.size();
-    }
-  }
-  s.n_items32 = (int)i32.size();
-  s.n_items64 = (int)i64.size();
-  h2d(s.items32.ensure(i32.size()), i32.data(), i32.size(), s.st);
-  h2d(s.items64.ensure(i64.size()), i64.data(), i64.size(), s.st);
-  // pairs of distinct curves and of distinct wall nodes, less the near-masked
-  // ones (counted per launch)
-  long long same = (long long)pr.M * pr.n * (pr.n - 1);
-  long long masked = 0, masked_wall = 0;
-  for (int q = 0; q < s.near.nsrc; ++q) {
-    int c = s.near.h_src_curve[q];
-    long long m = (long long)(s.near.h_src_ptr[q + 1] - s.near.h_src_ptr[q]) * (c == 0 ? pr.nout : pr.n);
-    masked += m;
-    if (c == 0) masked_wall += m;
-  }
-  s.far64_pairs = (long long)pr.N * (pr.N - 1) - same - masked;
-  s.farw_pairs = (long long)pr.nout * (pr.N - 1) - masked_wall;
-  s.far32_pairs = s.far64_pairs - s.farw_pairs;
-  EB_CK(cudaStreamSynchronize(s.st));
+  EB_CK(cudaStreamSynchronize(s.st));   // host vectors go out of scope
+  s.lay_n = pr.n;
+  s.lay_M = pr.M;
+  s.lay_nout = pr.nout;
 }
 
 // ---------------------------------------------------------------------------
@@ -423,7 +296,7 @@ constexpr double kTuneMinPairs = 2e8;
 // deleted.  Kinds 0 and 2 (accurate and fast FP64) sum every tile; kind 1
 // (FP32) the body tiles, and the mixed operator adds the wall tiles in the
 // kind-0 shape.
-static void plan_far(State& s) {
+static void plan_far(State& s, bool tune) {
   const Problem& pr = s.pr;
   // the FP32 kernel sums the body tiles; the wall's tiles (first nwall_tiles)
   // always run in FP64 (their densities carry fields that cancel against the
@@ -442,7 +315,6 @@ static void plan_far(State& s) {
       }
     }
   s.partial.ensure((size_t)std::max(maxs, max32 + maxw) * pr.N);
-  const bool tune = (double)pr.N * (double)pr.N >= kTuneMinPairs;
   const bool cached = s.tune_N == pr.N && s.tune_ntile == s.ntile && s.tune_masked == masked;
   bool zeroed = false;
   for (int kind = 0; kind < kFarKinds; ++kind) {
@@ -511,7 +383,7 @@ constexpr int kExpandNodes = 3200;
 // 18.3 us in 5.
 int near_parts(int items) { return std::max(1, std::min(8, (2 * g_num_sms + items - 1) / items)); }
 
-// Decides how the current problem's far field is summed and builds the lists.
+// Decides how the current problem's far field is summed.
 // The direct sum over split tile ranges (launch_far) stays for a forced launch
 // shape and for more tiles than the lists are built for.
 static void plan_clusters(State& s) {
@@ -520,10 +392,10 @@ static void plan_clusters(State& s) {
   s.cl_active = s.cl_ready && s.force_shape[0] < 0 && s.force_shape[1] < 0 && s.force_shape[2] < 0;
   s.cl_expand = s.cl_ready && pr.N >= kExpandNodes;
   s.cl_sing = s.cl_expand && pr.n <= FAR_TS;   // a body in several clusters has no centre among theirs
-  if (!s.cl_ready) return;
   k_cl_geom<<<nblk(s.ntile, 4), 128, 0, s.st>>>(s.geo(), s.ntile, s.tiles.p, s.cl_cen.ensure(s.ntile),
                                                s.cl_rad.ensure(s.ntile));
   EB_LAUNCH_CHECK();
+  if (!s.cl_ready) return;
   s.cl_parts64 = near_parts(s.n_items32);
   s.cl_parts32 = near_parts(s.n_items64);
   s.partial.ensure((size_t)(s.cl_parts64 + s.cl_parts32 + 1) * pr.N);
@@ -531,15 +403,6 @@ static void plan_clusters(State& s) {
     s.cl_mp.ensure((size_t)s.ntile * CL_MP);
     s.cl_lam.ensure(s.ntile);
   }
-  if (!s.cl_active) return;
-  const bool masked = s.near.npairs > 0;
-  build_lists(s, s.cl, 0, masked ? s.near.mask.p : nullptr, s.near.mw, 0, s.cl_expand);
-  unsigned long long pairs[2] = {0, 0};
-  d2h(pairs, s.cl.pairs.p, 2, s.st);
-  EB_CK(cudaStreamSynchronize(s.st));
-  s.farw_pairs = (long long)pairs[0];
-  s.far32_pairs = (long long)pairs[1];
-  s.far64_pairs = s.farw_pairs + s.far32_pairs;
 }
 
 // FP64 near-list sums (wall_only: of the wall's clusters) into cl_parts64 slots.
@@ -598,6 +461,58 @@ static void launch_wall_coupling(State& s, double2* out) {
   EB_LAUNCH_CHECK();
 }
 
+// Near mask, input checks, near and far lists and the pair lists, with one
+// synchronisation (the sizes and the checks' outcome).
+static void build_near(State& s) {
+  const Problem& pr = s.pr;
+  Near& nr = s.near;
+  const GeoDev G = s.geo();
+  cudaStream_t st = s.st;
+  const int mode = pr.P.ibary != 1 ? 0 : (pr.P.ifmm != 0 ? 1 : 2);
+  nr.mw = (pr.M + 1 + 31) / 32;
+  NearInfo* info = reinterpret_cast<NearInfo*>(nr.info.ensure(sizeof(NearInfo)));
+  k_near_head<<<1, 256, 0, st>>>(G, pr.P.wall_b, info, nr.reach.ensure(std::max(pr.M, 1)),
+                                 nr.wflag.ensure(std::max(pr.M, 1)), nr.cnt.ensure(pr.M + 1), nr.fill.ensure(pr.M + 1));
+  EB_LAUNCH_CHECK();
+  k_near_mask<<<s.n_items32, 256, 0, st>>>(G, mode, pr.P.wall_a, pr.P.wall_b, pr.P.wall_order, s.items32.p, s.tiles.p,
+                                           s.cl_cen.p, s.cl_rad.p, nr.reach.p, nr.wflag.p, nr.mw,
+                                           nr.mask.ensure((size_t)pr.N * nr.mw), nr.tl.ensure(pr.N), nr.cnt.p, info);
+  EB_LAUNCH_CHECK();
+  if (mode) {
+    k_near_scan<<<1, 1024, 0, st>>>(pr.M + 1, pr.nout, nr.cnt.p, nr.ptr.ensure(pr.M + 1), nr.wptr.ensure(pr.M + 1),
+                                    info);
+    EB_LAUNCH_CHECK();
+  }
+  if (s.cl_active) build_lists(s, s.cl, 0, mode ? nr.mask.p : nullptr, nr.mw, 0, s.cl_expand, info->cl);
+  NearInfo hinfo;
+  d2h(&hinfo, info, 1, st);
+  EB_CK(cudaStreamSynchronize(st));
+  const NearInfo* h = &hinfo;
+  if (h->flags & 1) throw Error(EROSION_BAD_INPUT, "non-finite node coordinates");
+  if (h->flags & 2) throw Error(EROSION_BAD_INPUT, "degenerate wall geometry");
+  if (h->flags & 4) throw Error(EROSION_BAD_INPUT, "a body node lies on or outside the wall");
+  if (h->pairs > INT32_MAX) throw Error(EROSION_BAD_INPUT, "too many barycentric pairs");
+  nr.lw = h->lw;
+  nr.rules = mode == 1;
+  nr.npairs = h->pairs;
+  nr.n_bary_work = h->work;
+  // pairs of distinct curves and of distinct wall nodes, less the near-masked
+  // ones; by clusters those of the near lists
+  const long long wall_masked = h->wall_pairs * pr.nout, body_masked = (h->pairs - h->wall_pairs) * pr.n;
+  const long long wall = (long long)pr.nout * (pr.N - 1) - wall_masked;
+  const long long body = (long long)pr.M * pr.n * (pr.N - pr.n) - body_masked;
+  s.farw_pairs = s.cl_active ? (long long)h->cl[0] : wall;
+  s.far32_pairs = s.cl_active ? (long long)h->cl[1] : body;
+  s.far64_pairs = s.farw_pairs + s.far32_pairs;
+  if (nr.npairs == 0) return;
+  k_near_fill<<<s.n_items32, 256, 0, st>>>(pr.M + 1, s.items32.p, s.tiles.p, nr.mw, nr.mask.p, nr.tl.p, nr.cnt.p,
+                                           nr.ptr.p, nr.wptr.p, nr.fill.p, nr.pair_tgt.ensure(nr.npairs),
+                                           nr.tpairs.ensure(nr.npairs), nr.bary_work.ensure(nr.n_bary_work));
+  EB_LAUNCH_CHECK();
+  s.bd.ensure(5LL * pr.N);
+  s.pair_out.ensure(nr.npairs);
+}
+
 void setup_problem(State& s, const Problem& in, const double* d_xx, const double* d_yy) {
   const auto t_start = std::chrono::steady_clock::now();
   Problem pr = in;
@@ -612,6 +527,7 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   pr.ntot = 2LL * pr.N + 3LL * pr.M;
   s.pr = pr;
   s.geo_valid = false;
+  s.near.rules = false;
   cudaStream_t st = s.st;
   if (s.dker_wall_n != pr.nout) {
     auto d = spectral_kernel(pr.nout);
@@ -643,25 +559,8 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
     k_body_stats<<<pr.M, 256, 0, st>>>(pr.n, pr.nout, s.xy.p, s.sp.p, s.cen.p, s.rb.p);
     EB_LAUNCH_CHECK();
   }
-  std::vector<double2> hxy(N), hcen(pr.M);
-  std::vector<double> hsp(pr.nout), hrb(pr.M);
-  d2h(hxy.data(), s.xy.p, N, st);
-  d2h(hsp.data(), s.sp.p, pr.nout, st);
-  d2h(hcen.data(), s.cen.p, pr.M, st);
-  d2h(hrb.data(), s.rb.p, pr.M, st);
-  EB_CK(cudaStreamSynchronize(st));
-  for (int g = 0; g < N; ++g)
-    if (!std::isfinite(hxy[g].x) || !std::isfinite(hxy[g].y)) throw Error(EROSION_BAD_INPUT, "non-finite node coordinates");
-  for (int k = 0; k < pr.nout; ++k)
-    if (!(hsp[k] > 0) || !std::isfinite(hsp[k])) throw Error(EROSION_BAD_INPUT, "degenerate wall geometry");
-  // Every body node must lie strictly inside the superellipse wall.
-  for (int g = pr.nout; g < N; ++g) {
-    double fx = std::pow(std::fabs(hxy[g].x) / pr.P.wall_a, pr.P.wall_order);
-    double fy = std::pow(std::fabs(hxy[g].y) / pr.P.wall_b, pr.P.wall_order);
-    if (!(fx + fy < 1.0)) throw Error(EROSION_BAD_INPUT, "a body node lies on or outside the wall");
-  }
-  build_near(s, hxy, hsp, hcen, hrb);
   build_tiles(s);
+  plan_clusters(s);
   s.src32.ensure(N);
   s.sq32.ensure(N);
   s.tgt32.ensure(N);
@@ -671,9 +570,9 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   k_geom32<<<s.ntile, 256, 0, st>>>(s.ntile, s.tiles.p, s.xy.p, s.nrm.p, s.tile_c.p, s.src32.p, s.tgt32.p,
                                      s.anchor.p);
   EB_LAUNCH_CHECK();
+  build_near(s);
   harvest_far_timing(s);
-  plan_far(s);
-  plan_clusters(s);
+  if (!s.cl_active) plan_far(s, (double)pr.N * (double)pr.N >= kTuneMinPairs);
   setup_preconditioner(s);
   s.geo_valid = true;
   s.setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
@@ -985,14 +884,13 @@ void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
     EB_LAUNCH_CHECK();
   }
   if (nr.npairs > 0) {
-    k_bdval<<<nr.n_bd_work, NEAR_NT, 0, st>>>(G, d_den, nr.bd_work.p, nr.src_curve.p, nr.bd_off.p, s.dker_wall.p,
-                                            s.dker_body.p, s.bd.p);
+    k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, st>>>(
+        G, d_den, nr.cnt.p, s.dker_wall.p, s.dker_body.p, s.bd.p);
     EB_LAUNCH_CHECK();
-    k_bary_list<<<nr.n_bary_work, NEAR_NT, 0, st>>>(G, nr.bary_work.p, nr.src_curve.p, nr.bd_off.p, s.bd.p,
-                                                    nr.pair_tgt.p, s.xy.p, s.pair_out.p);
+    k_bary_list<<<nr.n_bary_work, NEAR_NT, 0, st>>>(G, nr.bary_work.p, s.bd.p, nr.pair_tgt.p, s.xy.p, s.pair_out.p);
     EB_LAUNCH_CHECK();
   }
-  k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tptr.p : nullptr,
+  k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tl.p : nullptr,
                                              nr.npairs ? nr.tpairs.p : nullptr, s.pair_out.p, s.sigdotn.p,
                                              s.selfsum.p, s.cl_active && s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel);
   EB_LAUNCH_CHECK();
@@ -1370,8 +1268,8 @@ void release_state_buffers(State& s) {
   DBuf<double2>* d2s[] = {&s.xy, &s.nrm, &s.dz, &s.cen, &s.d1tmp, &s.ws, &s.partial, &s.bd, &s.pair_out};
   s.sq64.release();
   for (auto* b : d2s) b->release();
-  s.near.src_curve.release(); s.near.pair_tgt.release(); s.near.tptr.release(); s.near.tpairs.release();
-  s.near.bd_off.release(); s.near.bd_work.release(); s.near.bary_work.release(); s.near.mask.release();
+  s.near.release();
+  s.lay_n = -1;
   s.tiles.release(); s.split_ptr.release();
   s.vcap = 0;
   s.zcap = 0;
@@ -1653,6 +1551,16 @@ int erosion_set_far_shape(int32_t kind, int32_t shape) {
 int erosion_get_far_shapes(int32_t* shape, int32_t* desc, float* ms, int32_t* num_shapes) {
   State& s = state();
   std::lock_guard<std::mutex> lk(s.mu);
+  // the sums by clusters use none of these shapes, so a problem that is summed
+  // so is timed when it is asked for
+  if (s.geo_valid && s.cl_active && (double)s.pr.N * (double)s.pr.N >= kTuneMinPairs) {
+    try {
+      plan_far(s, true);
+    } catch (const Error& e) {
+      set_status(e.code, e.what());
+      return e.code;
+    }
+  }
   for (int kind = 0; kind < kFarKinds; ++kind) {
     const int nsh = far_num_shapes(kind);
     if (shape) shape[kind] = s.far_shape[kind];
@@ -1674,10 +1582,18 @@ int64_t erosion_near_info(int64_t* lw, int64_t* wall_bodies, int64_t* near_pairs
   State& s = state();
   std::lock_guard<std::mutex> lk(s.mu);
   if (lw) *lw = s.near.lw;
-  if (wall_bodies)
-    for (size_t i = 0; i < s.near.wall_bodies.size(); ++i) wall_bodies[i] = s.near.wall_bodies[i];
+  int64_t count = 0;
+  if (s.near.rules && s.near.wflag.p && s.pr.M > 0) {
+    std::vector<int> f(s.pr.M);
+    if (cudaMemcpy(f.data(), s.near.wflag.p, f.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) f.clear();
+    for (size_t b = 0; b < f.size(); ++b)
+      if (f[b]) {
+        if (wall_bodies) wall_bodies[count] = (int64_t)b;
+        ++count;
+      }
+  }
   if (near_pairs) *near_pairs = s.near.npairs;
-  return (int64_t)s.near.wall_bodies.size();
+  return count;
 }
 
 void erosion_release(void) {

@@ -85,21 +85,24 @@ struct Problem {
   erosion_params P{};
 };
 
-// Near-field bookkeeping of one geometry.
+// Near-field bookkeeping of one geometry (near.cuh).
 struct Near {
   long long lw = 0;
-  std::vector<long long> wall_bodies;
-  int nsrc = 0;              // source curves with at least one pair
+  bool rules = false;        // the near-wall rules were applied (wflag is valid)
   long long npairs = 0;
   int mw = 0;                // mask words per target
-  int n_bd_work = 0, n_bary_work = 0;
-  long long bd_total = 0;    // complex entries of the boundary-value buffer
-  std::vector<int> h_src_curve, h_src_ptr, h_pair_tgt;
-  DBuf<int> src_curve, pair_tgt, tptr, tpairs;
-  DBuf<long long> bd_off;
-  DBuf<int2> bd_work;
+  int n_bary_work = 0;
+  DBuf<int> cnt, ptr, wptr, fill, wflag;   // per source curve: pairs, offsets, counters; per body: near the wall
+  DBuf<double2> reach;
+  DBuf<int> pair_tgt, tpairs;
+  DBuf<int2> tl;
   DBuf<int4> bary_work;
   DBuf<unsigned> mask;
+  DBuf<unsigned char> info;  // NearInfo
+  void release() {
+    cnt.release(); ptr.release(); wptr.release(); fill.release(); wflag.release(); reach.release();
+    pair_tgt.release(); tpairs.release(); tl.release(); bary_work.release(); mask.release(); info.release();
+  }
 };
 
 // Near and far lists of the clusters (ClView in kernels.cuh).
@@ -107,9 +110,8 @@ struct ClLists {
   DBuf<int> near, far;
   DBuf<int4> cnt;
   DBuf<double> lnd;
-  DBuf<unsigned long long> pairs;
   void release() {
-    near.release(); far.release(); cnt.release(); lnd.release(); pairs.release();
+    near.release(); far.release(); cnt.release(); lnd.release();
   }
 };
 
@@ -136,6 +138,7 @@ struct State {
   // far field
   DBuf<int4> tiles;
   DBuf<int> split_ptr, split_ptr32, split_ptr64t, split_ptr64f, split_ptrw, split_tune;
+  int lay_n = -1, lay_M = -1, lay_nout = -1;   // sizes that tiles, items and splits were built for
   int nsplit = 0, nsplit32 = 0, nsplit64t = 0, nsplit64f = 0, nsplitw = 0, ntile = 0;
   long long far64_pairs = 0, farw_pairs = 0;   // pairs per full FP64 / wall-source launch
   // far-field launch shapes: index into the candidate lists of kernels.cuh

@@ -730,7 +730,7 @@ static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all) {
   const Problem& pr = s.pr;
   bd_all.ensure(5LL * pr.nout + 5LL * pr.n * pr.M);
   k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, s.st>>>(
-      s.geo(), d_den, nullptr, nullptr, nullptr, s.dker_wall.p, s.dker_body.p, bd_all.p);
+      s.geo(), d_den, nullptr, s.dker_wall.p, s.dker_body.p, bd_all.p);
   EB_LAUNCH_CHECK();
 }
 
@@ -896,7 +896,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       ClLists& lists = s.cl_stress;
       k_prep<<<pr.M + 1, 256, 0, s.st>>>(G, d_den, s.ws.p, s.sq64.p, s.sq32.p, s.d_w.ensure(pr.ntot), s.sigdotn.p, 1);
       EB_LAUNCH_CHECK();
-      build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand);
+      build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand, nullptr);
       const ClView L = cl_view(s, lists);
       const int parts = near_parts(nit);
       s.partial.ensure((size_t)(parts + 1) * pr.N);
