@@ -28,12 +28,13 @@
 //
 // Accuracy.  Clusters are separated when R <= theta (|D| - R') and R' <= theta
 // (|D| - R), theta = 1/3: cutting both series after CL_P = 32 terms leaves
-// 3^-32 = 5e-16 of the cluster's field, FP64 rounding.  Measured against a
+// 3^-32 = 5e-16 of the cluster's field, FP64 rounding; wider pairs keep fewer
+// terms to the same bound (cl_class).  Measured against a
 // direct sum in FP64, the operator on 400 bodies x 256 nodes is as far from
 // the 64-bit value as the direct kernels are (their geometry's rounding).
 //
-// Cost.  Per pair of clusters 4 x 32 x 32 multiply-adds and ~40% around them,
-// against 256 x 256 x ~18 operations for the pairs of two bodies.
+// Cost.  Per pair of clusters 4 x p x p multiply-adds, p = 8..32, and about as
+// many operations around them, against 256 x 256 x ~18 operations for the pairs of two bodies.
 #pragma once
 #include "state.h"
 #include "kernels.cuh"
@@ -42,7 +43,7 @@ namespace {
 
 constexpr int CL_P = 32;                 // terms of an expansion
 constexpr double CL_THETA = 1.0 / 3.0;   // separation
-constexpr int CL_MP = 3 * CL_P;          // multipole record of a cluster: a_k, x_k, k a_(k-1)
+constexpr int CL_MP = 3 * CL_P;          // multipole record of a cluster: a_k, x_k, k a_(k-1) / R
 constexpr int CL_MAX_TILES = 4096;       // above this the lists (tiles^2 entries) are not built
 
 struct BinomTable {
@@ -83,27 +84,49 @@ k_cl_geom(GeoDev G, int ntile, const int4* __restrict__ tiles, double2* __restri
   }
 }
 
+// Orders of the expansions.  A pair of separated clusters needs the p terms for
+// which its own ratio theta = max(R/(|D| - R'), R'/(|D| - R)) has theta^p <=
+// 3^-32: 32 at theta = 1/3, 8 at 1/81.  The far list of a cluster is sorted by
+// class of order; most pairs of a packing are far apart (400 bodies in the 2 x 1
+// channel: 92% need 16 terms or fewer), and the work of a pair goes with p^2.
+constexpr int CL_NCLS = 5;
+
+// Class of a pair at centre distance D: 0..4 of ascending order, CL_NCLS near.
+__device__ __forceinline__ int cl_class(double D, double rs, double rt) {
+  // theta up to which 8, 12, 16, 24 and 32 terms reach 3^-32
+  constexpr double th[CL_NCLS] = {1.0 / 81.0, 0.0534, 1.0 / 9.0, 0.2311, CL_THETA};
+  const double a = D - rt, b = D - rs;
+#pragma unroll
+  for (int c = 0; c < CL_NCLS; ++c)
+    if (rs <= th[c] * a && rt <= th[c] * b) return c;
+  return CL_NCLS;
+}
+
 // The lists of target cluster blockIdx.x + tile0.  mask: bit c of node i's row
 // (node index less mask0) marks the source curves that another rule evaluates
 // at that node; a cluster pair with any marked node stays in the near list.
 // expand = 0 puts every cluster there.  A body's own clusters are in neither
 // list (k_self64); the wall's are, its own pairs included.  pairs[0], pairs[1]
-// += node pairs of the near lists with wall and with body sources, unmasked.
+// += node pairs of the near lists with wall and with body sources, unmasked
+// (nullptr: not counted).
 __global__ void __launch_bounds__(256)
-k_cl_lists(GeoDev G, int ntile, int nwt, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
+k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
            const double* __restrict__ rad, const unsigned* __restrict__ mask, int mw, int mask0, int expand,
-           int* __restrict__ near, int* __restrict__ far, double* __restrict__ lnd, int4* __restrict__ cnt,
-           unsigned long long* __restrict__ pairs) {
+           int* __restrict__ near, int* __restrict__ far, double* __restrict__ lnd, int2* __restrict__ ncnt,
+           int* __restrict__ fcls, unsigned long long* __restrict__ pairs) {
   extern __shared__ int marked[];   // marked nodes of this cluster per source curve
-  __shared__ int wn[8], wf[8];
+  constexpr int NC = CL_NCLS + 1;   // the near list is the last category
+  __shared__ int tot[NC], wall[NC], at[NC], wcnt[8][NC];
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
   const double2 ct = cen[t];
   const double rt = rad[t];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (mask) {
+  if (threadIdx.x < NC) tot[threadIdx.x] = wall[threadIdx.x] = 0;
+  if (mask)
     for (int c = threadIdx.x; c < 32 * mw; c += blockDim.x) marked[c] = 0;
-    __syncthreads();
+  __syncthreads();
+  if (mask) {
     for (int e = threadIdx.x; e < T.y * mw; e += blockDim.x) {
       const int w = e % mw;
       unsigned m = mask[(size_t)(T.x - mask0) * mw + e];
@@ -114,63 +137,84 @@ k_cl_lists(GeoDev G, int ntile, int nwt, int tile0, const int4* __restrict__ til
     }
     __syncthreads();
   }
-  int n0 = 0, f0 = 0;   // entries so far
-  int4 c4 = make_int4(0, 0, 0, 0);
+  double D = 0.0;
+  auto category = [&](int s) {
+    if (s >= ntile) return -1;
+    const int4 S = tiles[s];
+    if (S.z > 0 && S.z == T.z) return -1;
+    D = sqrt(cabs2(csub(ct, cen[s])));
+    if (!expand || (mask && marked[S.z])) return CL_NCLS;
+    return cl_class(D, rad[s], rt);
+  };
+  // sizes
   unsigned long long pw = 0, pb = 0;
   for (int s0 = 0; s0 < ntile; s0 += 256) {
-    const int s = s0 + threadIdx.x;
-    bool isn = false, isf = false;
-    double ld = 0.0;
-    if (s < ntile) {
+    const int s = s0 + threadIdx.x, c = category(s);
+    const bool sw = s < ntile && tiles[s].z == 0;
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const unsigned b = __ballot_sync(0xffffffffu, c == q), bw = __ballot_sync(0xffffffffu, c == q && sw);
+      if (lane == 0 && b) atomicAdd(&tot[q], __popc(b));
+      if (lane == 0 && bw) atomicAdd(&wall[q], __popc(bw));
+    }
+    if (c == CL_NCLS) {
       const int4 S = tiles[s];
-      if (S.z == 0 || S.z != T.z) {
-        const int mk = mask ? marked[S.z] : 0;
-        const double2 d = csub(ct, cen[s]);
-        const double D = sqrt(cabs2(d)), rs = rad[s];
-        isf = expand && mk == 0 && rs <= CL_THETA * (D - rt) && rt <= CL_THETA * (D - rs);
-        isn = !isf;
-        if (isf) ld = log(D);
-        if (isn) {
-          const unsigned long long p = (unsigned long long)(T.y - mk) * S.y - (s == t ? T.y : 0);
-          if (S.z == 0) pw += p;
-          else pb += p;
-        }
+      const unsigned long long p =
+          (unsigned long long)(T.y - (mask ? marked[S.z] : 0)) * S.y - (s == t ? T.y : 0);
+      if (S.z == 0) pw += p;
+      else pb += p;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int o = 0;
+    int* f = fcls + (size_t)t * (2 * CL_NCLS + 1);
+    for (int q = 0; q < CL_NCLS; ++q) {
+      at[q] = f[q] = o;
+      f[CL_NCLS + 1 + q] = o + wall[q];
+      o += tot[q];
+    }
+    f[CL_NCLS] = o;
+    at[CL_NCLS] = 0;
+    ncnt[t] = make_int2(wall[CL_NCLS], tot[CL_NCLS]);
+  }
+  // places: ascending within a category, so the wall's clusters come first
+  for (int s0 = 0; s0 < ntile; s0 += 256) {
+    const int s = s0 + threadIdx.x, c = category(s);
+    unsigned mine = 0;
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const unsigned b = __ballot_sync(0xffffffffu, c == q);
+      if (c == q) mine = b;
+      if (lane == 0) wcnt[wid][q] = __popc(b);
+    }
+    __syncthreads();
+    if (c >= 0) {
+      int o = at[c] + __popc(mine & ((1u << lane) - 1u));
+      for (int w = 0; w < wid; ++w) o += wcnt[w][c];
+      if (c == CL_NCLS) {
+        near[(size_t)t * ntile + o] = s;
+      } else {
+        far[(size_t)t * ntile + o] = s;
+        lnd[(size_t)t * ntile + o] = log(D);
       }
     }
-    const unsigned bn = __ballot_sync(0xffffffffu, isn), bf = __ballot_sync(0xffffffffu, isf);
-    if (lane == 0) { wn[wid] = __popc(bn); wf[wid] = __popc(bf); }
     __syncthreads();
-    int on = n0, of = f0, tn = 0, tf = 0;
-    for (int w = 0; w < 8; ++w) {
-      if (w < wid) { on += wn[w]; of += wf[w]; }
-      tn += wn[w];
-      tf += wf[w];
-    }
-    const unsigned below = (1u << lane) - 1u;
-    const int in = on + __popc(bn & below), jf = of + __popc(bf & below);
-    if (isn) near[(size_t)t * ntile + in] = s;
-    if (isf) { far[(size_t)t * ntile + jf] = s; lnd[(size_t)t * ntile + jf] = ld; }
-    if (s == nwt) { c4.x = in; c4.z = jf; }   // entries before the first body cluster
-    n0 += tn;
-    f0 += tf;
+    if (threadIdx.x < NC)
+      for (int w = 0; w < 8; ++w) at[threadIdx.x] += wcnt[w][threadIdx.x];
     __syncthreads();
   }
-  // exactly one thread saw s == nwt; without body clusters nobody did
-  if (ntile == nwt) {
-    c4.x = n0;
-    c4.z = f0;
-  }
-  if (threadIdx.x == nwt % 256) cnt[t] = make_int4(c4.x, n0, c4.z, f0);
+  if (!pairs) return;
   for (int o = 16; o > 0; o >>= 1) {
     pw += __shfl_xor_sync(0xffffffffu, pw, o);
     pb += __shfl_xor_sync(0xffffffffu, pb, o);
   }
-  if (pairs && lane == 0 && pw) atomicAdd(pairs, pw);
-  if (pairs && lane == 0 && pb) atomicAdd(pairs + 1, pb);
+  if (lane == 0 && pw) atomicAdd(pairs, pw);
+  if (lane == 0 && pb) atomicAdd(pairs + 1, pb);
 }
 
 // Multipoles of cluster blockIdx.x + tile0: mp[t][0..31] = a_k, [32..63] = x_k,
-// [64..95] = k a_(k-1) (entry 0: 2 q R L of the stokeslet), lam[t] = -2 q L.
+// [64..95] = k a_(k-1) / R (entry 0: 2 q L of the stokeslet), lam[t] = -2 q L.
 // den: the density the stokeslets and rotlets are read from (nullptr: none).
 // Warp w sums the powers 4w..4w+3 over all nodes, a node per lane: 11 complex
 // products a node instead of a chain of 32, then the lanes meet in a fixed
@@ -238,7 +282,7 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
   double2 x = kb[k], d = make_double2(0, 0);
   if (k > 0) {
     x = make_double2(fma(-(double)k, ke[k - 1].x, x.x), fma(-(double)k, ke[k - 1].y, x.y));
-    d = cscale(ka[k - 1], k);
+    d = cscale(ka[k - 1], k * iR);
   } else {
     double2 L = make_double2(0, 0);
     double xi = 0.0;
@@ -248,7 +292,7 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
     }
     const double q2 = 1.0 / EB_TWOPI;   // 2 q
     x.y += 4.0 * xi;
-    d = cscale(L, q2 * R);
+    d = cscale(L, q2);
     lam[t] = cscale(L, -q2);
   }
   double2* o = mp + (size_t)t * CL_MP;
@@ -261,45 +305,44 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
 // lane/4, column lane%4; b: row lane%4, column lane/4; c: row lane/4, columns
 // 2 (lane%4) and the next.
 __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
 }
 
 // The local expansion of the far list of cluster t: loc[0][l] = alpha_l,
-// loc[1][l] = those of chi, valid for all threads on return.  wall_only: only
-// the wall's clusters as sources.  Every warp takes two sources at a time;
-// their phi and chi, real and imaginary, are the 8 columns of the product with
-// the 32 x 32 binomials that a warp holds in registers (a lane 32 of them).
-// Each lane forms its own operand: its component of the scaled multipole of
-// the order k it holds, the power of R/D by recurrence from k to k + 4.  The
-// products stay in registers until they are scaled by (-R'/D)^l and added to
-// the lane's sums, which the warps combine at the end in a fixed order.
+// loc[1][l] = those of chi, valid for all threads on return.  Every warp takes
+// two sources at a time; their phi and chi, real and imaginary, are the 8
+// columns of the product with the binomials, which sit in shared memory in the
+// order a lane reads them.  Each lane forms its own operand: its component of
+// the scaled multipole of the order k it holds, the power of R/D by recurrence
+// from k to k + 4.  The products stay in registers until they are scaled by
+// (-R'/D)^l and added to the lane's sums, which the warps combine at the end in
+// a fixed order.  Bound by the FP64 pipe, which the tensor-core products share:
+// of ~450 operations per lane for two sources of order 32, 256 are products.
+// All far pairs at order 32 took 180 us at 400 bodies x 256 nodes (236 us with
+// the binomials in 64 registers and half the warps), by classes 87 us.
 struct ClShared {
+  double P[CL_P * CL_P];
   double2 red[8][CL_P][2];
   double2 loc[2][CL_P];
 };
 
-__device__ __forceinline__ void cl_shift(const ClView& L, int t, bool wall_only, const double2* __restrict__ mp,
-                                         const double2* __restrict__ lam, ClShared& sh) {
+// The entries [i0, i1) of the far list with 8 LT local and 4 KT multipole terms.
+template <int LT, int KT>
+__device__ __forceinline__ void cl_shift_run(const ClView& L, int t, int i0, int i1, const double2* __restrict__ mp,
+                                             const double2* __restrict__ lam, const double* P, double (&ax)[4],
+                                             double (&ay)[4]) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int4 c4 = L.cnt[t];
-  const int nf = wall_only ? c4.z : c4.w;
   const double2 ct = L.cen[t];
   const double rt = L.rad[t];
   const int* __restrict__ far = L.far + (size_t)t * L.T;
   const double* __restrict__ lnd = L.lnd + (size_t)t * L.T;
   const int kq = lane & 3, bsrc = lane >> 4, bfn = (lane >> 3) & 1, bri = (lane >> 2) & 1;
   const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
-  double P[4][8];
-#pragma unroll
-  for (int lt = 0; lt < 4; ++lt)
-#pragma unroll
-    for (int kt = 0; kt < 8; ++kt) P[lt][kt] = kBinom.c[8 * lt + row][4 * kt + kq];
-  double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
-  for (int i = 2 * wid; i < nf; i += 16) {
-    const bool vb = i + bsrc < nf;
-    const int s = far[min(i + bsrc, nf - 1)];
+  for (int i = i0 + 2 * wid; i < i1; i += 16) {
+    const bool vb = i + bsrc < i1;
+    const int s = far[min(i + bsrc, i1 - 1)];
     const double2 D = csub(ct, L.cen[s]);
     const double R = L.rad[s];
     const double id2 = rcp_raw64(cabs2(D));
@@ -308,26 +351,28 @@ __device__ __forceinline__ void cl_shift(const ClView& L, int t, bool wall_only,
     double2 g = vb ? rho : make_double2(0, 0);                 // (R/D)^k / D, k = kq
     if (kq & 1) g = cmul(g, q1);
     if (kq & 2) g = cmul(g, q2);
-    const double2 kap = bfn ? cscale(make_double2(D.x, -D.y), 1.0 / R) : make_double2(0, 0);
+    const double2 kap = bfn ? make_double2(D.x, -D.y) : make_double2(0, 0);
     const double2* __restrict__ m = mp + (size_t)s * CL_MP;
     const double2* __restrict__ mb = m + bfn * CL_P;
-    double c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+    double c0[LT], c1[LT];
 #pragma unroll
-    for (int kt = 0; kt < 8; ++kt) {
+    for (int lt = 0; lt < LT; ++lt) c0[lt] = c1[lt] = 0.0;
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
       const int k = 4 * kt + kq;
       double2 y = mb[k];
       const double2 d = m[2 * CL_P + k];
       cfma2(y.x, y.y, kap, d);
       const double b = bri ? fma(y.x, g.y, y.y * g.x) : fma(y.x, g.x, -y.y * g.y);
 #pragma unroll
-      for (int lt = 0; lt < 4; ++lt) mma_f64(c0[lt], c1[lt], P[lt][kt], b);
-      g = cmul(g, q4);
+      for (int lt = 0; lt < LT; ++lt) mma_f64(c0[lt], c1[lt], P[(lt * 8 + kt) * 32 + lane], b);
+      if (kt + 1 < KT) g = cmul(g, q4);
     }
     // scale by (-R'/D)^l of the lane's own source
     const int from = csrc << 4;
     const double2 r1 = make_double2(__shfl_sync(0xffffffffu, rho.x, from), __shfl_sync(0xffffffffu, rho.y, from));
     const int sc = __shfl_sync(0xffffffffu, s, from);
-    const bool vc = i + csrc < nf;
+    const bool vc = i + csrc < i1;
     const double2 p1 = cscale(r1, -rt), p2 = cmul(p1, p1), p4 = cmul(p2, p2), p8 = cmul(p4, p4);
     double2 pw = vc ? make_double2(1.0, 0.0) : make_double2(0, 0);
     if (row & 1) pw = cmul(pw, p1);
@@ -335,15 +380,44 @@ __device__ __forceinline__ void cl_shift(const ClView& L, int t, bool wall_only,
     if (row & 4) pw = cmul(pw, p4);
     double2 lm = lam[sc];
     if (cfn) lm.y = -lm.y;
-    const double l0 = lnd[min(i + csrc, nf - 1)] - cfn;
+    const double l0 = lnd[min(i + csrc, i1 - 1)] - cfn;
 #pragma unroll
-    for (int lt = 0; lt < 4; ++lt) {
+    for (int lt = 0; lt < LT; ++lt) {
       const int l = 8 * lt + row;
       const double f = l == 0 ? l0 : -1.0 / l;
       cfma2(ax[lt], ay[lt], make_double2(fma(lm.x, f, c0[lt]), fma(lm.y, f, c1[lt])), pw);
-      pw = cmul(pw, p8);
+      if (lt + 1 < LT) pw = cmul(pw, p8);
     }
   }
+}
+
+// wall_only: only the wall's clusters as sources, to single precision (half the
+// terms, 3^-16 of a cluster's field): the preconditioner's coupling.  strain:
+// one class more, for the derivative.
+enum ClUse { CL_VELOCITY, CL_STRAIN, CL_WALL32 };
+
+template <int USE>
+__device__ __forceinline__ void cl_shift(const ClView& L, int t, const double2* __restrict__ mp,
+                                         const double2* __restrict__ lam, ClShared& sh) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
+  for (int e = threadIdx.x; e < CL_P * CL_P; e += blockDim.x) {
+    const int ln = e & 31, kt = (e >> 5) & 7, lt = e >> 8;
+    sh.P[e] = kBinom.c[8 * lt + (ln >> 2)][4 * kt + (ln & 3)];
+  }
+  __syncthreads();
+  double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
+  const int* __restrict__ f = L.fcls + (size_t)t * (2 * CL_NCLS + 1);
+  constexpr int E = USE == CL_WALL32 ? CL_NCLS + 1 : 1;   // ends of the wall's entries, or of all
+#define EB_RUN(C, LT, KT) cl_shift_run<LT, KT>(L, t, f[C], f[C + E], mp, lam, sh.P, ax, ay)
+  if constexpr (USE == CL_WALL32) {
+    EB_RUN(0, 1, 1); EB_RUN(1, 1, 2); EB_RUN(2, 1, 2); EB_RUN(3, 2, 3); EB_RUN(4, 2, 4);
+  } else if constexpr (USE == CL_STRAIN) {
+    EB_RUN(0, 2, 3); EB_RUN(1, 2, 4); EB_RUN(2, 3, 6); EB_RUN(3, 4, 8); EB_RUN(4, 4, 8);
+  } else {
+    EB_RUN(0, 1, 2); EB_RUN(1, 2, 3); EB_RUN(2, 2, 4); EB_RUN(3, 3, 6); EB_RUN(4, 4, 8);
+  }
+#undef EB_RUN
 #pragma unroll
   for (int lt = 0; lt < 4; ++lt) {
     ax[lt] += __shfl_xor_sync(0xffffffffu, ax[lt], 2);
@@ -352,23 +426,24 @@ __device__ __forceinline__ void cl_shift(const ClView& L, int t, bool wall_only,
   }
   __syncthreads();
   if (threadIdx.x < 2 * CL_P) {
-    const int l = threadIdx.x >> 1, f = threadIdx.x & 1;
-    double2 v = sh.red[0][l][f];
+    const int l = threadIdx.x >> 1, fn = threadIdx.x & 1;
+    double2 v = sh.red[0][l][fn];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) v = cadd(v, sh.red[w][l][f]);
-    sh.loc[f][l] = v;
+    for (int w = 1; w < 8; ++w) v = cadd(v, sh.red[w][l][fn]);
+    sh.loc[fn][l] = v;
   }
   __syncthreads();
 }
 
 // The separated sources' velocity at the nodes of cluster blockIdx.x + tile0.
-__global__ void __launch_bounds__(256)
-k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, int wall_only,
-           const double2* __restrict__ mp, const double2* __restrict__ lam, double2* __restrict__ out) {
+template <int USE>
+__global__ void __launch_bounds__(256, 2)
+k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ mp,
+           const double2* __restrict__ lam, double2* __restrict__ out) {
   __shared__ ClShared sh;
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
-  cl_shift(L, t, wall_only != 0, mp, lam, sh);
+  cl_shift<USE>(L, t, mp, lam, sh);
   const double2 c = L.cen[t];
   const double iR = 1.0 / L.rad[t];
   for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
@@ -392,13 +467,13 @@ k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, int wa
 // derivative and by |D|/R' against that field's own gradient: 1e-13.  With the
 // near lists' strain 626 us at 400 bodies x 256 nodes, where the trapezoid sum
 // over every pair took 30.8 ms.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 k_cl_shift_strain(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ mp,
                   const double2* __restrict__ lam, double2* __restrict__ out) {
   __shared__ ClShared sh;
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
-  cl_shift(L, t, false, mp, lam, sh);
+  cl_shift<CL_STRAIN>(L, t, mp, lam, sh);
   const double2 c = L.cen[t];
   const double iR = 1.0 / L.rad[t];
   for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
@@ -449,7 +524,7 @@ k_cl_near64(GeoDev G, ClView L, const int2* __restrict__ items, const int4* __re
   const bool act = it.y + lane < T.y;
   const int i = T.x + (act ? it.y + lane : T.y - 1);
   const double2 p = G.xy[i];
-  const int4 c4 = L.cnt[it.x];
+  const int2 c4 = L.ncnt[it.x];
   const int nt = wall_only ? c4.x : c4.y;
   const int ne = (int)((long long)nt * (blockIdx.y + 1) / gridDim.y);
   const int* __restrict__ near = L.near + (size_t)it.x * L.T;
@@ -546,7 +621,7 @@ k_cl_near32(GeoDev G, ClView L, const int2* __restrict__ items, const int4* __re
   const int i0 = T.x + min(k0, T.y - 1), i1 = T.x + min(k1, T.y - 1);
   const double2 an = anchor[i0];   // one cluster: one anchor
   const float2 o0 = tgt[i0], o1 = tgt[i1];
-  const int4 c4 = L.cnt[it.x];
+  const int2 c4 = L.ncnt[it.x];
   const int n0 = wall_only ? 0 : c4.x, nt = (wall_only ? c4.x : c4.y) - n0;
   const int ne = n0 + (int)((long long)nt * (blockIdx.y + 1) / gridDim.y);
   const int* __restrict__ near = L.near + (size_t)it.x * L.T;
@@ -648,7 +723,8 @@ static inline ClView cl_view(const State& s, const ClLists& L) {
   v.rad = s.cl_rad.p;
   v.near = L.near.p;
   v.far = L.far.p;
-  v.cnt = L.cnt.p;
+  v.ncnt = L.ncnt.p;
+  v.fcls = L.fcls.p;
   v.lnd = L.lnd.p;
   return v;
 }
@@ -659,10 +735,9 @@ static inline void build_lists(State& s, ClLists& L, int tile0, const unsigned* 
                                unsigned long long* pairs) {
   const size_t T = s.ntile;
   const size_t smem = mask ? 32 * (size_t)mw * sizeof(int) : 0;
-  k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(s.geo(), s.ntile, s.nwall_tiles, tile0, s.tiles.p, s.cl_cen.p,
-                                                        s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),
-                                                        L.far.ensure(T * T), L.lnd.ensure(T * T), L.cnt.ensure(T),
-                                                        pairs);
+  k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(
+      s.geo(), s.ntile, tile0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),
+      L.far.ensure(T * T), L.lnd.ensure(T * T), L.ncnt.ensure(T), L.fcls.ensure(T * (2 * CL_NCLS + 1)), pairs);
   EB_LAUNCH_CHECK();
 }
 

@@ -44,17 +44,19 @@ __device__ __forceinline__ void near_reduce(double (&v)[NV], double (*red)[NR][3
   __syncthreads();
 }
 
-// Lists of the target clusters.  near/far: row t holds the source clusters in
-// ascending order (the wall's first), T entries apart; cnt[t] = (wall entries
-// of near, entries of near, wall entries of far, entries of far); lnd: log |D|
-// of the far entries.
+// Lists of the target clusters.  near/far: row t holds the source clusters, T
+// entries apart, the near ones in ascending order (the wall's first), the far
+// ones by class of expansion order and ascending within a class.  ncnt[t] = (wall
+// entries, entries) of near; fcls[t]: the far list's class starts and its end, then
+// the end of every class's wall entries; lnd: log |D| of the far entries.
 struct ClView {
   int T = 0;
   const double2* __restrict__ cen = nullptr;
   const double* __restrict__ rad = nullptr;
   const int* __restrict__ near = nullptr;
   const int* __restrict__ far = nullptr;
-  const int4* __restrict__ cnt = nullptr;
+  const int2* __restrict__ ncnt = nullptr;
+  const int* __restrict__ fcls = nullptr;
   const double* __restrict__ lnd = nullptr;
 };
 
@@ -1744,7 +1746,7 @@ k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ 
   };
   if (L.T > 0) {   // the bodies of the node's near list and its own; the others came with the expansions
     const int t = tile_of(G, gc), own = tiles[t].z;
-    const int4 c4 = L.cnt[t];
+    const int2 c4 = L.ncnt[t];
     for (int e = c4.x - 1 + sub; e < c4.y; e += COMBINE_G) {
       const int c = e < c4.x ? own : tiles[L.near[(size_t)t * L.T + e]].z;
       if (c > 0)

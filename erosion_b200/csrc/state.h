@@ -107,11 +107,11 @@ struct Near {
 
 // Near and far lists of the clusters (ClView in kernels.cuh).
 struct ClLists {
-  DBuf<int> near, far;
-  DBuf<int4> cnt;
+  DBuf<int> near, far, fcls;
+  DBuf<int2> ncnt;
   DBuf<double> lnd;
   void release() {
-    near.release(); far.release(); cnt.release(); lnd.release();
+    near.release(); far.release(); fcls.release(); ncnt.release(); lnd.release();
   }
 };
 

@@ -588,7 +588,7 @@ k_stress_assemble(GeoDev G, const double* __restrict__ den, ClView L, const int4
   };
   if (sing) {
     const int t = tile_of(G, g), own = tiles[t].z;
-    const int4 c4 = L.cnt[t];
+    const int2 c4 = L.ncnt[t];
     for (int e = c4.x - 1 + sub; e < c4.y; e += COMBINE_G)
       singular((e < c4.x ? own : tiles[L.near[(size_t)t * L.T + e]].z) - 1);
   } else {
