@@ -1107,6 +1107,202 @@ k_gj_inv32_blocked(int m, int pb, float* __restrict__ B, int* __restrict__ bad) 
   }
 }
 
+// The same inversion with the panel's rows in registers and the update as a
+// register-tiled product: the form in use while a thread's rows of a panel fit
+// (invert_fp32).  A thread owns rows tid + 512 q of the panel; a pivot costs two
+// block synchronisations (the search's 16 warp maxima; the pivot row and the
+// row it changes places with through shared memory) and PB fused operations
+// per row.  The panel's swaps reach the other columns at once: thread 0 plays
+// them on an index array, and every thread then reads the pivot rows of its
+// columns (into W) and the rows they displaced from where they were.  The
+// update, m x m x PB multiply-adds, runs in warp tiles of 32 x 64 with 8 x 8 per
+// lane.  The final column order is applied in one pass.  Bound by the FP32 pipe
+// (136 M multiply-adds per 515 x 515 matrix, 0.55 ms on one SM) and the pivots'
+// chain: 100 such matrices take 3.2 ms, 200 6.0 ms, where the form above took
+// 14.6 and 29.6 ms; 259 x 259 0.58 ms (2.49 ms).
+// Shared memory: 2 PB mp floats (mp = m rounded up to 64) + 2 m ints.
+template <int PB, int R>
+__global__ void __launch_bounds__(512)
+k_gj_inv32_tiled(int m, int mp, float* __restrict__ B, int* __restrict__ bad) {
+  extern __shared__ __align__(16) float gjt[];
+  float* PT = gjt;                       // PB x mp: panel column k of row i at PT[k * mp + i]
+  float* W = gjt + (size_t)PB * mp;      // PB x mp: the pivot rows
+  int* piv = (int*)(W + (size_t)PB * mp);
+  int* map = piv + m;
+  __shared__ unsigned ru[2][16];
+  __shared__ int ri[2][16];
+  __shared__ __align__(16) float prow[2][PB], krow[2][PB];
+  __shared__ int srcw[PB], dstd[PB], srcd[PB], nd;
+  float* A = B + (size_t)blockIdx.x * m * m;
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < m; i += 512) map[i] = i;
+  for (int k0 = 0; k0 < m; k0 += PB) {
+    const int kb = min(PB, m - k0);
+    float a[R][PB];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int r = tid + 512 * q;
+#pragma unroll
+      for (int k = 0; k < PB; ++k) a[q][k] = r < m && k < kb ? A[(size_t)r * m + k0 + k] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < PB; ++k) {
+      if (k >= kb) break;
+      const int kk = k0 + k, f = k & 1;
+      // pivot: the largest |a|, the lowest row among equals (NaN never)
+      unsigned u = 0;
+      int bi = 0x7fffffff;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int r = tid + 512 * q;
+        const float v = fabsf(a[q][k]);
+        const unsigned b = r >= kk && r < m && v == v ? __float_as_uint(v) : 0u;
+        if (b > u) { u = b; bi = r; }
+      }
+      const unsigned wu = __reduce_max_sync(0xffffffffu, u);
+      const int wi = __reduce_min_sync(0xffffffffu, u == wu && wu ? bi : 0x7fffffff);
+      if (lane == 0) { ru[f][wid] = wu; ri[f][wid] = wi; }
+      __syncthreads();
+      const unsigned cu = lane < 16 ? ru[f][lane] : 0u;
+      const int ci = lane < 16 ? ri[f][lane] : 0x7fffffff;
+      const unsigned bu = __reduce_max_sync(0xffffffffu, cu);
+      int p = __reduce_min_sync(0xffffffffu, cu == bu && bu ? ci : 0x7fffffff);
+      if (!bu) {
+        p = kk;
+        if (tid == 0) bad[blockIdx.x] = 1;
+      }
+      if (tid == 0) piv[kk] = p;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int r = tid + 512 * q;
+        if (r == p)
+#pragma unroll
+          for (int j = 0; j < PB; ++j) prow[f][j] = a[q][j];
+        if (r == kk)
+#pragma unroll
+          for (int j = 0; j < PB; ++j) krow[f][j] = a[q][j];
+      }
+      __syncthreads();
+      const float d = 1.f / prow[f][k];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int r = tid + 512 * q;
+        if (r == p && p != kk)
+#pragma unroll
+          for (int j = 0; j < PB; ++j) a[q][j] = krow[f][j];
+        const bool pivot = r == kk;
+        const float g = pivot ? 0.f : a[q][k];
+#pragma unroll
+        for (int j = 0; j < PB; ++j) {
+          const float v = j == k ? d : prow[f][j] * d;
+          const float t = j == k ? 0.f : a[q][j];
+          a[q][j] = pivot ? v : fmaf(-g, v, t);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int r = tid + 512 * q;
+      if (r < m)
+#pragma unroll
+        for (int k = 0; k < PB; ++k) PT[(size_t)k * mp + r] = a[q][k];
+    }
+    for (int e = tid; e < PB * (mp - m); e += 512) PT[(size_t)(e / (mp - m)) * mp + m + e % (mp - m)] = 0.f;
+    if (tid == 0) {
+      for (int k = 0; k < kb; ++k) {
+        const int kk = k0 + k, p = piv[kk], t = map[kk];
+        map[kk] = map[p];
+        map[p] = t;
+      }
+      int n = 0;
+      for (int k = 0; k < kb; ++k) {
+        const int p = piv[k0 + k];
+        srcw[k] = map[k0 + k];
+        if (p >= k0 + kb && map[p] != p) {
+          dstd[n] = p;
+          srcd[n] = map[p];
+          map[p] = p;
+          ++n;
+        }
+      }
+      nd = n;
+      for (int k = 0; k < kb; ++k) map[k0 + k] = k0 + k;
+    }
+    __syncthreads();
+    for (int j = tid; j < mp; j += 512) {
+      const bool col = j < m && (j < k0 || j >= k0 + kb);
+      float x[PB];
+#pragma unroll
+      for (int k = 0; k < PB; ++k) x[k] = col && k < kb ? A[(size_t)srcw[k] * m + j] : 0.f;
+#pragma unroll
+      for (int k = 0; k < PB; ++k) W[(size_t)k * mp + j] = x[k];
+      if (col) {
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+          if (k < nd) x[k] = A[(size_t)srcd[k] * m + j];
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+          if (k < nd) A[(size_t)dstd[k] * m + j] = x[k];
+      }
+    }
+    __syncthreads();
+    const int ct = mp / 64, tiles = ((m + 31) / 32) * ct;
+    for (int t = wid; t < tiles; t += 16) {
+      const int i0 = 32 * (t / ct) + 8 * (lane >> 3), j0 = 64 * (t % ct) + (lane & 7);
+      float c[8][8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = i0 + r;
+        const bool rd = i < m && (i < k0 || i >= k0 + kb);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) c[r][s] = rd && j0 + 8 * s < m ? A[(size_t)i * m + j0 + 8 * s] : 0.f;
+      }
+#pragma unroll 4
+      for (int k = 0; k < PB; ++k) {
+        const float4 u0 = *reinterpret_cast<const float4*>(PT + (size_t)k * mp + i0);
+        const float4 u1 = *reinterpret_cast<const float4*>(PT + (size_t)k * mp + i0 + 4);
+        const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+        float v[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = W[(size_t)k * mp + j0 + 8 * s];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+          for (int s = 0; s < 8; ++s) c[r][s] = fmaf(u[r], v[s], c[r][s]);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = i0 + r;
+        if (i >= m) break;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const int j = j0 + 8 * s;
+          if (j < m && (j < k0 || j >= k0 + kb)) A[(size_t)i * m + j] = c[r][s];
+        }
+      }
+    }
+    for (int i = tid; i < m; i += 512)
+      for (int k = 0; k < kb; ++k) A[(size_t)i * m + k0 + k] = PT[(size_t)k * mp + i];
+    __syncthreads();
+  }
+  // the row swaps undone as column swaps, last first: column j comes from map[j]
+  if (tid == 0)
+    for (int k = m - 1; k >= 0; --k) {
+      const int p = piv[k], t = map[k];
+      map[k] = map[p];
+      map[p] = t;
+    }
+  __syncthreads();
+  float* rowbuf = gjt + (size_t)wid * mp;   // 16 rows <= 2 PB mp floats
+  for (int i = wid; i < m; i += 16) {
+    float* row = A + (size_t)i * m;
+    for (int j = lane; j < m; j += 32) rowbuf[j] = row[j];
+    __syncwarp();
+    for (int j = lane; j < m; j += 32) row[j] = rowbuf[map[j]];
+    __syncwarp();
+  }
+}
+
 // z_b = B_b^{-1} t_b for every body.  t is gathered from v (the body part of
 // the unknown vector) less the wall coupling A_bw z_wall, given as ntw
 // partial sums per body node (slot q at tw + q * tw_stride, body-major); z is

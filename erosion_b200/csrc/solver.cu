@@ -688,10 +688,28 @@ bool choose_initial_guess(State& s, const double* d_b, double* d_x, bool have_x,
 }
 
 // In-place inversion of count m x m FP32 matrices (one CTA each), a zero
-// pivot flagged in bad[matrix].  Blocked Gauss-Jordan with the widest panel
-// whose shared-memory working set (2 m pb + m floats, m ints) fits; the
-// unblocked kernel past that.
+// pivot flagged in bad[matrix].  The register-tiled Gauss-Jordan up to 1500
+// rows; past that the blocked one with the widest panel whose shared-memory
+// working set (2 m pb + m floats, m ints) fits, then the unblocked kernel.
 static void invert_fp32(State& s, float* B, int m, int count, int* bad) {
+  // panels of 32 while they fit beside the pivot rows in shared memory, of 16
+  // up to 1500 rows
+  const int mp = (m + 63) / 64 * 64;
+  auto tiled = [&](int pb) { return 2 * (size_t)pb * mp * sizeof(float) + 2 * (size_t)m * sizeof(int); };
+  if (m <= 1024 && tiled(32) <= 200 * 1024) {
+    const void* fn = m <= 512 ? (const void*)k_gj_inv32_tiled<32, 1> : (const void*)k_gj_inv32_tiled<32, 2>;
+    allow_max_dynamic_smem(fn);
+    if (m <= 512) k_gj_inv32_tiled<32, 1><<<count, 512, tiled(32), s.st>>>(m, mp, B, bad);
+    else k_gj_inv32_tiled<32, 2><<<count, 512, tiled(32), s.st>>>(m, mp, B, bad);
+    EB_LAUNCH_CHECK();
+    return;
+  }
+  if (m <= 1536 && tiled(16) <= 200 * 1024) {
+    allow_max_dynamic_smem((const void*)k_gj_inv32_tiled<16, 3>);
+    k_gj_inv32_tiled<16, 3><<<count, 512, tiled(16), s.st>>>(m, mp, B, bad);
+    EB_LAUNCH_CHECK();
+    return;
+  }
   int pb = 32;
   auto gj_smem = [m](int b) { return (2 * (size_t)m * b + m) * sizeof(float) + (size_t)m * sizeof(int); };
   while (pb > 4 && gj_smem(pb) > 200 * 1024) pb /= 2;
