@@ -1898,7 +1898,8 @@ k_bary_list(GeoDev G, const int4* __restrict__ work, const double2* __restrict__
 // COMBINE_G consecutive threads share one node: they split the partial-sum
 // slots, the near pairs and the bodies of the stokeslet/rotlet sum, and their
 // sums meet by warp shuffles (launch nblk(N * COMBINE_G, 256) CTAs of 256).
-// L.T = 0: every body's stokeslet and rotlet is summed here (a logarithm and a
+// kp (may be nullptr): the Arnoldi column count, which the operator's last
+// launch advances.  L.T = 0: every body's stokeslet and rotlet is summed here (a logarithm and a
 // division each, 206 us at 400 bodies x 256 nodes), otherwise those of the
 // cluster's near list and the node's own body.
 constexpr int SR_CHUNK = 256;
@@ -1907,10 +1908,11 @@ __global__ void __launch_bounds__(256)
 k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ partial, int nsplit,
           const int2* __restrict__ tl, const int* __restrict__ tpairs, const double2* __restrict__ pair_out,
           const double* __restrict__ sigdotn, const double2* __restrict__ selfp, ClView L,
-          const int4* __restrict__ tiles, double* __restrict__ vel) {
+          const int4* __restrict__ tiles, double* __restrict__ vel, int* __restrict__ kp) {
   __shared__ double4 sc[SR_CHUNK];   // cx, cy, stokeslet x, stokeslet y
   __shared__ double sr[SR_CHUNK];    // rotlet
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (kp && tid == 0) *kp += 1;
   const int g = (int)(tid / COMBINE_G), sub = (int)(tid % COMBINE_G);
   const bool act = g < G.N;
   const int gc = act ? g : G.N - 1;

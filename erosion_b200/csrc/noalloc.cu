@@ -229,7 +229,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
       EB_LAUNCH_CHECK();
     }
     k_combine<<<nblk((long long)N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, partial, nsplit, nullptr, nullptr, nullptr,
-                                                                  sigdotn, selfsum, ClView{}, nullptr, d_vel);
+                                                                  sigdotn, selfsum, ClView{}, nullptr, d_vel, nullptr);
     EB_LAUNCH_CHECK();
     set_status(EROSION_OK, "");
     return EROSION_OK;

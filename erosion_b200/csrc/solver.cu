@@ -3,6 +3,7 @@
 #include "state.h"
 #include "cluster.cuh"
 #include "near.cuh"
+#include "krylov.cuh"
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -405,6 +406,30 @@ static void plan_clusters(State& s) {
   }
 }
 
+// Stream of branch b (0..2) of an operator's independent launches.
+static cudaStream_t branch(State& s, int b) { return s.forked ? s.br[b] : s.st; }
+
+// Runs f with the library stream of the state replaced by st.
+template <class F>
+static void on_stream(State& s, cudaStream_t st, F&& f) {
+  const cudaStream_t main = s.st;
+  s.st = st;
+  f();
+  s.st = main;
+}
+
+static void fork(State& s, int ev, std::initializer_list<int> to) {
+  if (!s.forked) return;
+  EB_CK(cudaEventRecord(s.ev_fork[ev], s.st));
+  for (int b : to) EB_CK(cudaStreamWaitEvent(s.br[b], s.ev_fork[ev], 0));
+}
+
+static void join(State& s, int b) {
+  if (!s.forked) return;
+  EB_CK(cudaEventRecord(s.ev_join[b], s.br[b]));
+  EB_CK(cudaStreamWaitEvent(s.st, s.ev_join[b], 0));
+}
+
 // FP64 near-list sums (wall_only: of the wall's clusters) into cl_parts64 slots.
 static void launch_near64(State& s, bool wall_only, double2* out) {
   const Near& nr = s.near;
@@ -449,16 +474,21 @@ static void launch_wall_coupling(State& s, double2* out) {
   const GeoDev G = s.geo();
   const ClView L = cl_view(s, s.cl);
   const int nit = s.n_items64 - s.n_items64_wall;
-  k_cl_near32<false><<<nit, 256, 0, s.st>>>(G, L, s.items64.p + s.n_items64_wall, s.tiles.p, 1, s.src32.p, s.tgt32.p,
+  fork(s, 1, {0});
+  k_cl_near32<false><<<nit, 256, 0, branch(s, 0)>>>(G, L, s.items64.p + s.n_items64_wall, s.tiles.p, 1, s.src32.p, s.tgt32.p,
                                             s.anchor.p, s.tile_c.p, s.pc_sq32.p, nullptr, 0, out);
   EB_LAUNCH_CHECK();
-  if (!s.cl_expand) return;
+  if (!s.cl_expand) {
+    join(s, 0);
+    return;
+  }
   k_cl_form<<<s.nwall_tiles, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.pc_sq64.p, nullptr, s.cl_mp.p,
                                              s.cl_lam.p);
   EB_LAUNCH_CHECK();
   k_cl_shift<CL_WALL32><<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,
                                                                    s.cl_lam.p, out + s.pr.N);
   EB_LAUNCH_CHECK();
+  join(s, 0);
 }
 
 // Near mask, input checks, near and far lists and the pair lists, with one
@@ -528,6 +558,7 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   s.pr = pr;
   s.geo_valid = false;
   s.near.rules = false;
+  drop_steps(s);   // captured for the previous problem
   cudaStream_t st = s.st;
   if (s.dker_wall_n != pr.nout) {
     auto d = spectral_kernel(pr.nout);
@@ -867,15 +898,16 @@ void harvest_far_timing(State& s) {
   if (s.far_pending) {
     EB_CK(cudaEventSynchronize(s.ef1));   // complete already on every path that calls this
     EB_CK(cudaEventElapsedTime(&ms, s.ef0, s.ef1));
-    if (s.far_kind == 1) s.stats.ms_far32 += ms;
-    else if (s.far_kind == 2) s.stats.ms_far64f += ms;
-    else s.stats.ms_far += ms;
+    if (s.far_kind == 1) { s.stats.ms_far32 += ms; s.timed_far32++; }
+    else if (s.far_kind == 2) { s.stats.ms_far64f += ms; s.timed_far64f++; }
+    else { s.stats.ms_far += ms; s.timed_far++; }
     s.far_pending = false;
   }
   if (s.farw_pending) {
     EB_CK(cudaEventSynchronize(s.ew1));
     EB_CK(cudaEventElapsedTime(&ms, s.ew0, s.ew1));
     s.stats.ms_farw += ms;
+    s.timed_farw++;
     s.farw_pending = false;
   }
 }
@@ -892,77 +924,79 @@ int far_slots(const State& s, int prec) {
   return prec == 1 ? s.nsplit32 + s.nsplitw : (prec == 2 ? s.nsplit64f : s.nsplit64t);
 }
 
-void operator_post(State& s, const double* d_den, double* d_vel, int nsplit) {
+void far_field(State& s, const double* d_den, int kind, bool timed) {
+  const Problem& pr = s.pr;
+  const size_t N = pr.N;
+  auto mark = [&](cudaEvent_t e) {
+    if (timed) EB_CK(cudaEventRecord(e, s.st));
+  };
+  if (s.cl_active) {
+    on_stream(s, branch(s, 0), [&] {
+      mark(s.ef0);
+      if (kind != 1) launch_near64(s, false, s.partial.p);
+      else launch_near32(s, s.partial.p);
+      mark(s.ef1);
+      if (kind == 1) {   // the wall's sources stay FP64
+        mark(s.ew0);
+        launch_near64(s, true, s.partial.p + s.cl_parts32 * N);
+        mark(s.ew1);
+        if (timed) s.farw_pending = true;
+      }
+    });
+    if (s.cl_expand) launch_expansions(s, d_den, s.partial.p + (far_slots(s, kind) - 1) * N);
+    if (timed) {
+      s.far_kind = kind;
+      s.far_pending = true;
+    }
+    return;
+  }
+  const int n1 = kind == 1 ? s.nsplit32 : (kind == 2 ? s.nsplit64f : s.nsplit64t);
+  if (n1 > 0) {
+    mark(s.ef0);
+    launch_far(s, kind, s.far_shape[kind],
+               kind == 1 ? s.split_ptr32.p : (kind == 2 ? s.split_ptr64f.p : s.split_ptr64t.p), n1, s.partial.p);
+    mark(s.ef1);
+    if (timed) {
+      s.far_kind = kind;
+      s.far_pending = true;
+    }
+  }
+  if (kind == 1) {
+    // wall sources in FP64, into the partial slots after the FP32 ones
+    mark(s.ew0);
+    const int wk = pr.P.fast_fp64 ? 2 : 0;
+    launch_far(s, wk, s.far_shape[wk], s.split_ptrw.p, s.nsplitw, s.partial.p + (size_t)n1 * N);
+    mark(s.ew1);
+    if (timed) s.farw_pending = true;
+  }
+}
+
+void operator_post(State& s, const double* d_den, double* d_vel, int nsplit, int* kp) {
   const Problem& pr = s.pr;
   const GeoDev G = s.geo();
   const Near& nr = s.near;
-  cudaStream_t st = s.st;
   if (pr.M > 0) {
-    k_self64<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, st>>>(G, s.ws.p, s.selfsum.p);
+    k_self64<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, branch(s, 2)>>>(G, s.ws.p, s.selfsum.p);
     EB_LAUNCH_CHECK();
   }
   if (nr.npairs > 0) {
+    const cudaStream_t st = branch(s, 1);
     k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, st>>>(
         G, d_den, nr.cnt.p, s.dker_wall.p, s.dker_body.p, s.bd.p);
     EB_LAUNCH_CHECK();
     k_bary_list<<<nr.n_bary_work, NEAR_NT, 0, st>>>(G, nr.bary_work.p, s.bd.p, nr.pair_tgt.p, s.xy.p, s.pair_out.p);
     EB_LAUNCH_CHECK();
   }
-  k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tl.p : nullptr,
-                                             nr.npairs ? nr.tpairs.p : nullptr, s.pair_out.p, s.sigdotn.p,
-                                             s.selfsum.p, s.cl_active && s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel);
+  for (int b = 0; b < 3; ++b) join(s, b);
+  k_combine<<<nblk((long long)pr.N * COMBINE_G, 256), 256, 0, s.st>>>(
+      G, d_den, s.partial.p, nsplit, nr.npairs ? nr.tl.p : nullptr, nr.npairs ? nr.tpairs.p : nullptr, s.pair_out.p,
+      s.sigdotn.p, s.selfsum.p, s.cl_active && s.cl_sing ? cl_view(s, s.cl) : ClView{}, s.tiles.p, d_vel, kp);
   EB_LAUNCH_CHECK();
 }
 
-// The far field of a prepared density into the partial slots, its launches
-// bracketed by the timing events (ef: body sources or all, ew: the wall's
-// sources of the mixed operator).
-static void far_field(State& s, const double* d_den, int kind) {
+// Counts one operator application of the given kind.
+static void count_operator(State& s, int kind) {
   const Problem& pr = s.pr;
-  cudaStream_t st = s.st;
-  const size_t N = pr.N;
-  if (s.cl_active) {
-    EB_CK(cudaEventRecord(s.ef0, st));
-    if (kind != 1) launch_near64(s, false, s.partial.p);
-    else launch_near32(s, s.partial.p);
-    EB_CK(cudaEventRecord(s.ef1, st));
-    if (kind == 1) {   // the wall's sources stay FP64
-      EB_CK(cudaEventRecord(s.ew0, st));
-      launch_near64(s, true, s.partial.p + s.cl_parts32 * N);
-      EB_CK(cudaEventRecord(s.ew1, st));
-      s.farw_pending = true;
-    }
-    if (s.cl_expand) launch_expansions(s, d_den, s.partial.p + (far_slots(s, kind) - 1) * N);
-    s.far_kind = kind;
-    s.far_pending = true;
-    return;
-  }
-  const int n1 = kind == 1 ? s.nsplit32 : (kind == 2 ? s.nsplit64f : s.nsplit64t);
-  if (n1 > 0) {
-    EB_CK(cudaEventRecord(s.ef0, st));
-    launch_far(s, kind, s.far_shape[kind],
-               kind == 1 ? s.split_ptr32.p : (kind == 2 ? s.split_ptr64f.p : s.split_ptr64t.p), n1, s.partial.p);
-    EB_CK(cudaEventRecord(s.ef1, st));
-    s.far_kind = kind;
-    s.far_pending = true;
-  }
-  if (kind == 1) {
-    // wall sources in FP64, into the partial slots after the FP32 ones
-    EB_CK(cudaEventRecord(s.ew0, st));
-    const int wk = pr.P.fast_fp64 ? 2 : 0;
-    launch_far(s, wk, s.far_shape[wk], s.split_ptrw.p, s.nsplitw, s.partial.p + (size_t)n1 * pr.N);
-    EB_CK(cudaEventRecord(s.ew1, st));
-    s.farw_pending = true;
-  }
-}
-
-void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
-  harvest_far_timing(s);
-  const Problem& pr = s.pr;
-  cudaStream_t st = s.st;
-  operator_prep(s, d_den, d_vel);
-  const int kind = prec == 1 ? 1 : (prec == 2 ? 2 : 0);
-  far_field(s, d_den, kind);
   if (kind == 1) {
     s.stats.matvecs_fp32++;
     if (pr.M > 0) s.stats.far32_launches++;
@@ -972,11 +1006,19 @@ void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
   } else {
     s.stats.far_launches++;
   }
-  operator_post(s, d_den, d_vel, far_slots(s, prec));
   s.stats.matvecs++;
   s.stats.far32_pairs = s.far32_pairs;
   s.stats.far64_pairs = s.far64_pairs;
   s.stats.farw_pairs = s.farw_pairs;
+}
+
+void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
+  harvest_far_timing(s);
+  operator_prep(s, d_den, d_vel);
+  const int kind = prec == 1 ? 1 : (prec == 2 ? 2 : 0);
+  far_field(s, d_den, kind, true);
+  operator_post(s, d_den, d_vel, far_slots(s, prec));
+  count_operator(s, kind);
 }
 
 void build_rhs(State& s, double* d_rhs) {
@@ -1027,6 +1069,138 @@ static double* pinned(State& s, size_t n) {
   return s.h_pinned;
 }
 
+// ---------------------------------------------------------------------------
+// One Arnoldi step (krylov.cuh) and its captured graphs.
+
+// Column bound of the graph that serves step ll (ll basis vectors).
+static int step_bound(int ll) {
+  int b = 64;
+  while (b < ll) b *= 2;
+  return std::min(b, CGS_MAX);
+}
+
+static size_t step_tile(int bound) { return (size_t)bound * 34 * sizeof(double); }
+
+static void step_buffers(State& s, long long N, long long cols) {
+  if (!s.br[0]) {
+    for (auto& b : s.br) EB_CK(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
+    for (auto* e : {&s.ev_fork[0], &s.ev_fork[1], &s.ev_join[0], &s.ev_join[1], &s.ev_join[2], &s.ev_step[0],
+                    &s.ev_step[1]})
+      EB_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    allow_max_dynamic_smem((const void*)k_cgs_update_dot);
+  }
+  if (!s.k_host) EB_CK(cudaMallocHost((void**)&s.k_host, 2 * (size_t)(CGS_MAX + 2) * sizeof(double)));
+  int R;
+  const int nb = std::max(dot_blocks(N, &R), 4 * g_num_sms);
+  const double* before[] = {s.k_cur.p, s.k_w.p, s.k_h1.p, s.k_h2.p, s.k_np.p, s.part.p, s.pc_z.p};
+  s.k_cur.ensure(N);
+  s.k_w.ensure(N);
+  s.k_h1.ensure(CGS_MAX + 1);
+  s.k_h2.ensure(CGS_MAX + 1);
+  s.k_np.ensure(4 * g_num_sms);
+  s.k_count.ensure(1);
+  s.pc_z.ensure(N);
+  s.part.ensure((size_t)std::min<long long>(cols, CGS_MAX) * nb);
+  const double* after[] = {s.k_cur.p, s.k_w.p, s.k_h1.p, s.k_h2.p, s.k_np.p, s.part.p, s.pc_z.p};
+  if (!std::equal(before, before + 7, after)) drop_steps(s);
+}
+
+// Launches one step for up to `bound` columns: the (preconditioned) operator
+// applied to k_cur, and the Gram-Schmidt launches.
+static void launch_step(State& s, long long N, long long ldv, int bound, int prec, bool timed, double* host) {
+  const double* den = s.k_cur.p;
+  const int* kp = s.k_count.p;
+  if (s.pc_active) {
+    apply_preconditioner(s, s.k_cur.p, s.pc_z.p);
+    den = s.pc_z.p;
+  }
+  operator_prep(s, den, s.k_w.p);
+  fork(s, 0, {0, 1, 2});
+  far_field(s, den, prec == 1 ? 1 : (prec == 2 ? 2 : 0), timed);
+  operator_post(s, den, s.k_w.p, far_slots(s, prec), s.k_count.p);
+  cudaStream_t st = s.st;
+  int R;
+  const int nb = dot_blocks(N, &R);
+  const int ny = std::max(1, std::min((bound + 31) / 32, (2 * g_num_sms + nb - 1) / nb));
+  k_cgs_dot<<<dim3(nb, ny), 256, R * sizeof(double), st>>>(s.V.p, ldv, kp, s.k_w.p, N, R, s.part.p);
+  EB_LAUNCH_CHECK();
+  const unsigned nred = nblk(bound, 8);
+  k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, 0, s.k_h1.p);
+  EB_LAUNCH_CHECK();
+  // as many CTAs as are resident with the chunk's block of V in shared memory
+  const size_t tile = step_tile(bound);
+  const int chunks = (int)nblk(N, CGS_ROWS), per_sm = std::max(1, std::min(4, (int)((220 * 1024) / (tile + 4096))));
+  if (tile <= 220 * 1024) {
+    const int g = std::min(chunks, per_sm * g_num_sms);
+    k_cgs_update_dot<<<g, 256, tile, st>>>(s.V.p, ldv, kp, s.k_h1.p, s.k_w.p, N, s.part.p);
+    EB_LAUNCH_CHECK();
+    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, g, kp, 0, s.k_h2.p);
+    EB_LAUNCH_CHECK();
+  } else {   // more columns than fit: the update and the product by themselves
+    k_vh_dk<<<nblk(N, 256), 256, 0, st>>>(s.V.p, ldv, kp, s.k_h1.p, -1.0, s.k_w.p, N);
+    EB_LAUNCH_CHECK();
+    k_cgs_dot<<<dim3(nb, ny), 256, R * sizeof(double), st>>>(s.V.p, ldv, kp, s.k_w.p, N, R, s.part.p);
+    EB_LAUNCH_CHECK();
+    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, 0, s.k_h2.p);
+    EB_LAUNCH_CHECK();
+  }
+  const int gn = std::min(chunks, 4 * g_num_sms);
+  k_cgs_update_norm<<<gn, 256, 0, st>>>(s.V.p, ldv, kp, s.k_h2.p, s.k_w.p, N, s.k_np.p);
+  EB_LAUNCH_CHECK();
+  k_cgs_finish<<<std::min(nblk(N, 256), (unsigned)(4 * g_num_sms)), 256, 0, st>>>(
+      s.V.p, s.Z.p, ldv, kp, s.k_h1.p, s.k_h2.p, s.k_np.p, gn, s.k_w.p, s.pc_active ? s.pc_z.p : nullptr, s.k_cur.p, N,
+      host, CGS_MAX + 2);
+  EB_LAUNCH_CHECK();
+}
+
+void drop_steps(State& s) {
+  for (auto& g : s.steps) cudaGraphExecDestroy(g.exec);
+  s.steps.clear();
+}
+
+// The same step as a graph, its independent launches on branches, captured on
+// first use.
+static void replay_step(State& s, long long N, long long ldv, int bound, int prec, double* host) {
+  for (size_t i = 0; i < s.steps.size(); ++i)
+    if (s.steps[i].V != s.V.p || s.steps[i].part != s.part.p || (s.pc_active && s.steps[i].Z != s.Z.p)) {   // moved
+      EB_CK(cudaStreamSynchronize(s.st));
+      drop_steps(s);
+      break;
+    }
+  for (auto& g : s.steps)
+    if (g.bound == bound && g.prec == prec) {
+      EB_CK(cudaGraphLaunch(g.exec, s.st));
+      g_launches += g.launches;
+      return;
+    }
+  const long long l0 = g_launches;
+  EB_CK(cudaStreamBeginCapture(s.st, cudaStreamCaptureModeRelaxed));
+  cudaGraph_t graph = nullptr;
+  s.forked = true;
+  try {
+    launch_step(s, N, ldv, bound, prec, false, host);
+  } catch (...) {
+    s.forked = false;
+    cudaStreamEndCapture(s.st, &graph);
+    if (graph) cudaGraphDestroy(graph);
+    throw;
+  }
+  s.forked = false;
+  EB_CK(cudaStreamEndCapture(s.st, &graph));
+  State::StepGraph g;
+  g.launches = g_launches - l0;
+  g.bound = bound;
+  g.prec = prec;
+  g.V = s.V.p;
+  g.Z = s.Z.p;
+  g.part = s.part.p;
+  const cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
+  cudaGraphDestroy(graph);
+  EB_CK(err);
+  s.steps.push_back(g);
+  EB_CK(cudaGraphLaunch(g.exec, s.st));
+}
+
 // One GMRES run with the semantics of SLATEC DGMRES as solveBIE calls it
 // (stokesSolver.f:481-497, gmres_routines.f): no restart, MAXL = min(maxl, N),
 // stop when the Givens estimate rho <= abs_tol, least squares by DHELS, x += V y.
@@ -1061,30 +1235,94 @@ static int gmres_cycle(State& s, double* d_r, double* d_x, long long maxl_in, do
   double prod = 1.0, rho = r0nrm;
   long long lgmr = 0;
   int iflag = -1;
-  double* hdev = s.hdev.ensure((size_t)MAXL + 2);
-  double* hs = s.ydev.ensure((size_t)MAXL + 2);
-  double* hp = pinned(s, 2 * (size_t)MAXL + 4);
-  for (long long ll = 1; ll <= MAXL; ++ll) {
-    lgmr = ll;
-    if (ll + 1 > s.vcap) {
-      long long nc = std::min<long long>(MAXL + 1, std::max<long long>(2 * s.vcap, ll + 1));
-      s.V.grow_keep((size_t)nc * ldv, (size_t)ll * ldv, st);
+  auto reserve = [&](long long cols) {   // room for cols basis vectors, and as many preconditioned ones less one
+    if (cols > s.vcap) {
+      const long long nc = std::min<long long>(MAXL + 1, std::max<long long>(2 * s.vcap, cols));
+      s.V.grow_keep((size_t)nc * ldv, (size_t)s.vcap * ldv, st);
       s.vcap = nc;
     }
+    if (s.pc_active && cols - 1 > s.zcap) {
+      const long long nc = std::min<long long>(MAXL, std::max<long long>(2 * s.zcap, std::max<long long>(cols - 1, 64)));
+      s.Z.grow_keep((size_t)nc * ldv, (size_t)s.zcap * ldv, st);
+      s.zcap = nc;
+    }
+  };
+  // mixed precision: the fast FP64 operator while the residual is large, the
+  // FP32 far field once it is below relax_abs
+  auto precision_at = [&](double r) { return relax_abs > 0.0 ? (r <= relax_abs ? 1 : (s.pr.P.fast_fp64 ? 2 : 0)) : 0; };
+  // Column ll of the Hessenberg matrix (col[0..ll], the last entry |w|^2):
+  // DHEQR's update of the last column (gmres_routines.f:1148).  False when the
+  // cycle ends.
+  auto hessenberg = [&](long long ll, const double* h) {
+    lgmr = ll;
+    std::vector<double> col(h, h + ll + 1);
+    col[ll] = std::sqrt(col[ll]);
+    for (long long i = 0; i <= ll; ++i)
+      if (!std::isfinite(col[i])) { iflag = 3; return false; }
+    for (long long kk = 1; kk <= ll - 1; ++kk) {
+      double c = Q[2 * (kk - 1)], sn = Q[2 * (kk - 1) + 1];
+      double t1 = col[kk - 1], t2 = col[kk];
+      col[kk - 1] = c * t1 - sn * t2;
+      col[kk] = sn * t1 + c * t2;
+    }
+    double t1 = col[ll - 1], t2 = col[ll], c, sn;
+    if (t2 == 0.0) { c = 1; sn = 0; }
+    else if (std::fabs(t2) >= std::fabs(t1)) { double t = t1 / t2; sn = -1.0 / std::sqrt(1.0 + t * t); c = -sn * t; }
+    else { double t = t2 / t1; c = 1.0 / std::sqrt(1.0 + t * t); sn = -c * t; }
+    Q.push_back(c); Q.push_back(sn);
+    col[ll - 1] = c * t1 - sn * t2;
+    HES.push_back(col);
+    if (col[ll - 1] == 0.0) { iflag = 2; return false; }
+    prod = prod * sn;
+    rho = std::fabs(prod * r0nrm);
+    if (rho <= abs_tol) { iflag = 0; return false; }
+    if (ll == MAXL) { iflag = (rho < r0nrm) ? 1 : 2; return false; }
+    return true;
+  };
+  // Steps up to CGS_MAX columns.  The first of a cycle is launched as it is,
+  // with its far field timed; the others replay a captured graph.  While the
+  // precision of the next step is known it is launched before this one's column
+  // has been looked at, so that the GPU does not wait for the host; a step in
+  // flight when the cycle ends writes a column that nobody reads.
+  const long long last = std::min<long long>(MAXL, CGS_MAX);
+  bool running = true;
+  {
+    step_buffers(s, N, last);
+    double* host = s.k_host;
+    EB_CK(cudaMemsetAsync(s.k_count.p, 0, sizeof(int), st));
+    EB_CK(cudaMemcpyAsync(s.k_cur.p, s.V.p, N * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    long long launched = 0;
+    int kind[2] = {0, 0};
+    auto launch = [&](long long ll) {
+      const int prec = precision_at(rho);
+      reserve(ll + 1);
+      kind[ll & 1] = prec;
+      harvest_far_timing(s);
+      if (ll == 1) launch_step(s, N, ldv, step_bound(1), prec, true, host);
+      else replay_step(s, N, ldv, step_bound((int)ll), prec, host);
+      EB_CK(cudaEventRecord(s.ev_step[ll & 1], st));
+      launched = ll;
+    };
+    for (long long ll = 1; ll <= last && running; ++ll) {
+      if (launched < ll) launch(ll);
+      const bool settled = relax_abs <= 0.0 || kind[ll & 1] == 1;   // rho only falls
+      if (ll < last && settled && ll > 1) launch(ll + 1);
+      EB_CK(cudaEventSynchronize(s.ev_step[ll & 1]));
+      count_operator(s, kind[ll & 1]);
+      running = hessenberg(ll, host + (size_t)(ll & 1) * (CGS_MAX + 2));
+    }
+  }
+  // Longer cycles (the unpreconditioned solve of hundreds of bodies): one launch
+  // per product and update, whatever the column count.
+  for (long long ll = CGS_MAX + 1; ll <= MAXL && running; ++ll) {
+    double* hdev = s.hdev.ensure((size_t)MAXL + 2);
+    double* hs = s.ydev.ensure((size_t)MAXL + 2);
+    double* hp = pinned(s, 2 * (size_t)MAXL + 4);
+    reserve(ll + 1);
     double* V = s.V.p;
     double* vnew = V + ll * ldv;
-    // mixed precision: the fast FP64 operator while the residual is large,
-    // the FP32 far field once it is below relax_abs
-    const int prec = relax_abs > 0.0 ? (rho <= relax_abs ? 1 : (s.pr.P.fast_fp64 ? 2 : 0)) : 0;
+    const int prec = precision_at(rho);
     if (s.pc_active) {
-      // flexible GMRES: keep z_k = P^{-1} v_k so that x = x0 + Z y is exactly
-      // consistent with the Arnoldi relation A Z = V H whatever the
-      // preconditioner's rounding
-      if (ll > s.zcap) {
-        long long nc = std::min<long long>(MAXL, std::max<long long>(2 * s.zcap, std::max<long long>(ll, 64)));
-        s.Z.grow_keep((size_t)nc * ldv, (size_t)(ll - 1) * ldv, st);
-        s.zcap = nc;
-      }
       double* zk = s.Z.p + (ll - 1) * ldv;
       apply_preconditioner(s, V + (ll - 1) * ldv, zk);
       apply_operator(s, zk, vnew, prec);
@@ -1103,33 +1341,10 @@ static int gmres_cycle(State& s, double* d_r, double* d_x, long long maxl_in, do
     d2h(hp + MAXL + 2, hs, (size_t)k, st);
     EB_CK(cudaStreamSynchronize(st));
     harvest_far_timing(s);
-    const double snormw = std::sqrt(hp[k]);
-    std::vector<double> col(ll + 1);
-    for (int i = 0; i < k; ++i) col[i] = hp[i] + hp[MAXL + 2 + i];
-    col[ll] = snormw;
-    bool finite = std::isfinite(snormw);
-    for (int i = 0; i < k && finite; ++i) finite = std::isfinite(col[i]);
-    if (!finite) { iflag = 3; break; }
-    // DHEQR (gmres_routines.f:1148), update of the last column.
-    for (long long kk = 1; kk <= ll - 1; ++kk) {
-      double c = Q[2 * (kk - 1)], sn = Q[2 * (kk - 1) + 1];
-      double t1 = col[kk - 1], t2 = col[kk];
-      col[kk - 1] = c * t1 - sn * t2;
-      col[kk] = sn * t1 + c * t2;
-    }
-    double t1 = col[ll - 1], t2 = col[ll], c, sn;
-    if (t2 == 0.0) { c = 1; sn = 0; }
-    else if (std::fabs(t2) >= std::fabs(t1)) { double t = t1 / t2; sn = -1.0 / std::sqrt(1.0 + t * t); c = -sn * t; }
-    else { double t = t2 / t1; c = 1.0 / std::sqrt(1.0 + t * t); sn = -c * t; }
-    Q.push_back(c); Q.push_back(sn);
-    col[ll - 1] = c * t1 - sn * t2;
-    HES.push_back(col);
-    if (col[ll - 1] == 0.0) { iflag = 2; break; }
-    prod = prod * sn;
-    rho = std::fabs(prod * r0nrm);
-    if (rho <= abs_tol) { iflag = 0; break; }
-    if (ll == MAXL) { iflag = (rho < r0nrm) ? 1 : 2; break; }
-    k_scale<<<nblk(N, 256), 256, 0, st>>>(vnew, 1.0 / snormw, N);
+    for (int i = 0; i < k; ++i) hp[i] += hp[MAXL + 2 + i];
+    running = hessenberg(ll, hp);
+    if (!running) break;
+    k_scale<<<nblk(N, 256), 256, 0, st>>>(vnew, 1.0 / std::sqrt(hp[k]), N);
     EB_LAUNCH_CHECK();
   }
   *iters = lgmr;
@@ -1286,6 +1501,8 @@ void release_state_buffers(State& s) {
   DBuf<double2>* d2s[] = {&s.xy, &s.nrm, &s.dz, &s.cen, &s.d1tmp, &s.ws, &s.partial, &s.bd, &s.pair_out};
   s.sq64.release();
   for (auto* b : d2s) b->release();
+  drop_steps(s);
+  s.k_cur.release(); s.k_w.release(); s.k_h1.release(); s.k_h2.release(); s.k_np.release(); s.k_count.release();
   s.near.release();
   s.lay_n = -1;
   s.tiles.release(); s.split_ptr.release();
@@ -1362,6 +1579,9 @@ int solve_device_impl(State& s, double* d_den, bool x0_zero, int64_t* nits) {
     for (int q = 0; q < 3; ++q) s.stats.guess_residual[q] = gr[q];
     record_setup_stats(s);
   }
+  harvest_far_timing(s);
+  s.stats.ms_far = s.stats.ms_far32 = s.stats.ms_farw = s.stats.ms_far64f = 0.0;
+  s.timed_far = s.timed_far32 = s.timed_farw = s.timed_far64f = 0;
   EB_CK(cudaEventRecord(s.e0, s.st));
   double* rhs = s.d_rhs.ensure(pr.ntot);
   build_rhs(s, rhs);
@@ -1382,6 +1602,14 @@ int solve_device_impl(State& s, double* d_den, bool x0_zero, int64_t* nits) {
   EB_CK(cudaEventRecord(s.e1, s.st));
   EB_CK(cudaEventSynchronize(s.e1));
   harvest_far_timing(s);
+  // the launches inside replayed graphs take the mean of the timed ones
+  auto scale = [](double& t, long long launches, long long timed) {
+    if (timed > 0) t *= (double)launches / (double)timed;
+  };
+  scale(s.stats.ms_far, s.stats.far_launches, s.timed_far);
+  scale(s.stats.ms_far32, s.stats.far32_launches, s.timed_far32);
+  scale(s.stats.ms_farw, s.stats.farw_launches, s.timed_farw);
+  scale(s.stats.ms_far64f, s.stats.far64f_launches, s.timed_far64f);
   float ms = 0;
   EB_CK(cudaEventElapsedTime(&ms, s.e0, s.e1));
   s.stats.ms_total = ms;

@@ -201,6 +201,22 @@ struct State {
 
   // Krylov
   DBuf<double> V, Z, part, hdev, ydev;
+  // Arnoldi steps by captured graphs (gmres_cycle): the vector to apply the
+  // operator to, its image, dot products, column count, and the branches of a step
+  DBuf<double> k_cur, k_w, k_h1, k_h2, k_np;
+  DBuf<int> k_count;
+  cudaStream_t br[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t ev_fork[2] = {nullptr, nullptr}, ev_join[3] = {nullptr, nullptr, nullptr}, ev_step[2] = {nullptr, nullptr};
+  double* k_host = nullptr; // pinned: two slots of CGS_MAX + 2, a column of the Hessenberg matrix each
+  bool forked = false;      // the operator's independent launches go to br
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    long long launches = 0;
+    int bound = 0, prec = 0;
+    const double *V = nullptr, *Z = nullptr, *part = nullptr;
+  };
+  std::vector<StepGraph> steps;   // of the current set-up
+  long long timed_far = 0, timed_farw = 0, timed_far32 = 0, timed_far64f = 0;   // launches with event times
   long long vcap = 0;   // vectors held by V
   long long zcap = 0;   // vectors held by Z (preconditioned basis, flexible GMRES)
   double* h_pinned = nullptr;
@@ -245,7 +261,9 @@ void apply_operator(State& s, const double* d_den, double* d_vel, int prec = 0);
 // assembly.
 void operator_prep(State& s, const double* d_den, double* d_vel);
 int far_slots(const State& s, int prec);
-void operator_post(State& s, const double* d_den, double* d_vel, int nsplit);
+void operator_post(State& s, const double* d_den, double* d_vel, int nsplit, int* kp = nullptr);
+// Destroys the captured Arnoldi steps (a set-up or a buffer they refer to changed).
+void drop_steps(State& s);
 void build_rhs(State& s, double* d_rhs);
 // GMRES (SLATEC DGMRES semantics, CGS2 Arnoldi); returns EROSION_* status.
 int gmres_solve(State& s, const double* d_b, double* d_x, bool x0_zero, long long maxl, double tol,
@@ -272,6 +290,9 @@ void setup_preconditioner(State& s);
 void record_setup_stats(State& s);
 // z = P^{-1} v (device vectors of length ntot).
 void apply_preconditioner(State& s, const double* v, double* z);
+// The far field of a prepared density into the partial slots (kind 0 FP64, 1 mixed,
+// 2 fast FP64), timed: its launches bracketed by events for the statistics.
+void far_field(State& s, const double* d_den, int kind, bool timed);
 double device_norm(State& s, const double* d_v, long long n);
 // Adds the last far-field launch's event time to stats.ms_far (after a sync).
 void harvest_far_timing(State& s);
