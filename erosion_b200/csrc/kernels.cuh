@@ -232,81 +232,87 @@ __device__ __forceinline__ double4 pair_tensor64(double2 nn, double2 v) {
   return make_double4(nn.x * v.x, nn.x * v.y + nn.y * v.x, nn.y * v.y, 0.0);
 }
 
+// The first ceil(nout/256) CTAs take 256 wall nodes each (sigdotn: their parts of
+// the integral), the others a body; a body's eight sums (the constraint rows',
+// and about the node mean the moments that give the centroid, the rotation and
+// its norm) are one reduction.  Bound by latency: 5.0 us at 100 bodies x 256
+// nodes and 2048 wall nodes, 5.5 us at 200 x 256 and 4096 (the wall in one CTA
+// and a reduction per sum: 15.0 and 28.2 us).
 __global__ void __launch_bounds__(256) k_prep(GeoDev G, const double* __restrict__ den,
                                               double2* __restrict__ ws, double4* __restrict__ sq64,
                                               float4* __restrict__ sq32, double* __restrict__ vel,
                                               double* __restrict__ sigdotn, int split_rigid) {
-  __shared__ double sh[32];
-  const int c = blockIdx.x;
-  const int start = curve_start(G, c), len = curve_len(G, c);
-  if (c == 0) {
-    double a0 = 0;
-    for (int j = threadIdx.x; j < len; j += blockDim.x) {
-      int g = start + j;
-      double sx = den[ix_of(G, g)], sy = den[iy_of(G, g)];
-      double wg = G.w[g];
-      double2 v = make_double2(wg * sx, wg * sy);
+  __shared__ double sh[8][8], tot[8];
+  const int nwb = (G.nout + 255) / 256, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  auto reduce = [&]() {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double v = warp_sum(a[q]);
+      if (lane == 0) sh[wid][q] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+      double v = sh[0][lane];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) v += sh[w][lane];
+      tot[lane] = v;
+    }
+    __syncthreads();
+  };
+  if ((int)blockIdx.x < nwb) {
+    const int g = blockIdx.x * 256 + threadIdx.x;
+    if (g < G.nout) {
+      const double sx = den[g], sy = den[G.nout + g], wg = G.w[g];
+      const double2 v = make_double2(wg * sx, wg * sy), nn = G.nrm[g];
       ws[g] = v;
-      double2 nn = G.nrm[g];
       sq64[g] = pair_tensor64(nn, v);
       sq32[g] = pair_tensor32(nn, v);
-      a0 += (nn.x * sx + nn.y * sy) * G.sp[g];
+      a[0] = (nn.x * sx + nn.y * sy) * G.sp[g];
     }
-    a0 = block_sum<256>(a0, sh);
-    if (threadIdx.x == 0) *sigdotn = a0 * (EB_TWOPI / len);
+    reduce();
+    if (threadIdx.x == 0) sigdotn[blockIdx.x] = tot[0] * (EB_TWOPI / G.nout);
     return;
   }
-  // pass 1: constraint sums and the weighted means
-  double a0 = 0, a1 = 0, a2 = 0, s0 = 0, sxw = 0, syw = 0;
-  for (int j = threadIdx.x; j < len; j += blockDim.x) {
-    int g = start + j;
-    double sx = den[ix_of(G, g)], sy = den[iy_of(G, g)];
-    double s = G.sp[g];
-    double2 p = G.xy[g];
-    a0 += sx * s;
-    a1 += sy * s;
-    a2 += (sx * p.y - sy * p.x) * s;
-    s0 += s;
-    sxw += s * p.x;
-    syw += s * p.y;
+  const int b = blockIdx.x - nwb, n = G.n, start = G.nout + b * n;
+  const double* __restrict__ sxp = den + 2LL * G.nout + 2LL * n * b;
+  const double* __restrict__ syp = sxp + n;
+  const double2 c = G.cen[b];
+  for (int j = threadIdx.x; j < n; j += 256) {
+    const double sx = sxp[j], sy = syp[j], s = G.sp[start + j];
+    const double2 p = G.xy[start + j];
+    const double dx = p.x - c.x, dy = p.y - c.y;
+    a[0] += sx * s;
+    a[1] += sy * s;
+    a[2] += (sx * p.y - sy * p.x) * s;
+    a[3] += s;
+    a[4] += s * dx;
+    a[5] += s * dy;
+    a[6] += s * (dx * sy - dy * sx);
+    a[7] += s * (dx * dx + dy * dy);
   }
-  a0 = block_sum<256>(a0, sh);
-  a1 = block_sum<256>(a1, sh);
-  a2 = block_sum<256>(a2, sh);
-  s0 = block_sum<256>(s0, sh);
-  sxw = block_sum<256>(sxw, sh);
-  syw = block_sum<256>(syw, sh);
-  if (threadIdx.x == 0) {
-    int b = c - 1;
-    vel[ic_of(G, b, 0)] = (-a0) / EB_TWOPI * (EB_TWOPI / len) + den[ic_of(G, b, 0)];
-    vel[ic_of(G, b, 1)] = (-a1) / EB_TWOPI * (EB_TWOPI / len) + den[ic_of(G, b, 1)];
-    vel[ic_of(G, b, 2)] = (-a2) / EB_TWOPI * (EB_TWOPI / len) + den[ic_of(G, b, 2)];
+  reduce();
+  if (threadIdx.x < 3) {
+    const long long r = ic_of(G, b, threadIdx.x);
+    vel[r] = (-tot[threadIdx.x]) / EB_TWOPI * (EB_TWOPI / n) + den[r];
   }
-  const double xb = sxw / s0, yb = syw / s0;
-  // pass 2: rotation coefficient about (xb, yb); phi3 = (-(y - yb), x - xb)
-  double r0 = 0, r1 = 0;
-  for (int j = threadIdx.x; j < len; j += blockDim.x) {
-    int g = start + j;
-    double sx = den[ix_of(G, g)], sy = den[iy_of(G, g)];
-    double s = G.sp[g];
-    double2 p = G.xy[g];
-    double fx = -(p.y - yb), fy = p.x - xb;
-    r0 += s * (fx * sx + fy * sy);
-    r1 += s * (fx * fx + fy * fy);
+  double t1 = 0.0, t2 = 0.0, t3 = 0.0, xb = 0.0, yb = 0.0;
+  if (split_rigid) {
+    xb = tot[4] / tot[3];
+    yb = tot[5] / tot[3];
+    const double r0 = tot[6] - xb * tot[1] + yb * tot[0], r1 = tot[7] - tot[3] * (xb * xb + yb * yb);
+    t1 = tot[0] / tot[3];
+    t2 = tot[1] / tot[3];
+    t3 = r1 > 0 ? r0 / r1 : 0.0;
+    xb += c.x;
+    yb += c.y;
   }
-  r0 = block_sum<256>(r0, sh);
-  r1 = block_sum<256>(r1, sh);
-  double t1 = a0 / s0, t2 = a1 / s0, t3 = r1 > 0 ? r0 / r1 : 0.0;
-  if (!split_rigid) t1 = t2 = t3 = 0.0;
-  for (int j = threadIdx.x; j < len; j += blockDim.x) {
-    int g = start + j;
-    double sx = den[ix_of(G, g)], sy = den[iy_of(G, g)];
-    double2 p = G.xy[g];
-    double wg = G.w[g];
+  for (int j = threadIdx.x; j < n; j += 256) {
+    const int g = start + j;
+    const double sx = sxp[j], sy = syp[j], wg = G.w[g];
+    const double2 p = G.xy[g], nn = G.nrm[g];
     ws[g] = make_double2(wg * sx, wg * sy);
-    double rx = sx - t1 + t3 * (p.y - yb), ry = sy - t2 - t3 * (p.x - xb);
-    double2 v = make_double2(wg * rx, wg * ry);
-    const double2 nn = G.nrm[g];
+    const double2 v = make_double2(wg * (sx - t1 + t3 * (p.y - yb)), wg * (sy - t2 - t3 * (p.x - xb)));
     sq64[g] = pair_tensor64(nn, v);
     sq32[g] = pair_tensor32(nn, v);
   }
@@ -349,20 +355,17 @@ __device__ __forceinline__ double rcp_newton(double r2) {
 }
 
 // The FP64 hardware reciprocal estimate (rcp.approx.ftz.f64, a coarse
-// approximation formed from the upper half of the operand) refined by
-// Newton-Raphson steps y <- y + y (1 - r2 y) in FP64.  Each step squares the
-// relative error; NSTEP = 2 takes the estimate below FP64 rounding, NSTEP = 1
-// leaves a relative error of the order of the square of the estimate's.
+// approximation formed from the upper half of the operand, ~1e-6 off) refined in
+// FP64 with e = 1 - r2 y: NSTEP = 1 by the Newton-Raphson step y + y e, which
+// squares the relative error; NSTEP = 2 by y + y (e + e^2), which cubes it, below
+// FP64 rounding, in three operations where two Newton-Raphson steps take four.
 // r2 > 0 in the double's normal range (0 for r2 = 0, as rcp_or_zero).
 template <int NSTEP>
 __device__ __forceinline__ double rcp_newton64(double r2) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-#pragma unroll
-  for (int k = 0; k < NSTEP; ++k) {
-    const double e = fma(-r2, y, 1.0);
-    y = fma(y, e, y);
-  }
+  const double e = fma(-r2, y, 1.0);
+  y = fma(y, NSTEP == 2 ? fma(e, e, e) : e, y);
   return r2 > 0.0 ? y : 0.0;
 }
 
@@ -370,10 +373,8 @@ __device__ __forceinline__ double rcp_newton64(double r2) {
 __device__ __forceinline__ double rcp_raw64(double r2) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-  double e = fma(-r2, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-r2, y, 1.0);
-  return fma(y, e, y);
+  const double e = fma(-r2, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 // One Newton-Raphson step from the FP32 estimate: relative error ~2^-46
@@ -1306,7 +1307,8 @@ k_gj_inv32_tiled(int m, int mp, float* __restrict__ B, int* __restrict__ bad) {
 // z_b = B_b^{-1} t_b for every body.  t is gathered from v (the body part of
 // the unknown vector) less the wall coupling A_bw z_wall, given as ntw
 // partial sums per body node (slot q at tw + q * tw_stride, body-major); z is
-// scattered into the same layout.  CTA = (body, 256-row chunk), warp per row.
+// scattered into the same layout.  A warp takes four rows at a time.  Bound by reading the inverses ((2n + 3)^2 floats per body):
+// 26.5 us at 100 bodies x 256 nodes (4.0 TB/s), 50 us at 200.
 __global__ void __launch_bounds__(256)
 k_pc_apply_bodies(GeoDev G, const float* __restrict__ Binv, const double* __restrict__ v,
                   const double2* __restrict__ tw, long long tw_stride, int ntw, double* __restrict__ z) {
@@ -1331,14 +1333,30 @@ k_pc_apply_bodies(GeoDev G, const float* __restrict__ Binv, const double* __rest
   }
   __syncthreads();
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = blockIdx.y * 8 + wid; r < m; r += gridDim.y * 8) {
+  for (int r = 4 * (blockIdx.y * 8 + wid); r < m; r += gridDim.y * 32) {
     const float* __restrict__ row = Binv + ((size_t)b * m + r) * m;
-    float acc = 0.f;
-    for (int c = lane; c < m; c += 32) acc = fmaf(__ldg(row + c), tv[c], acc);
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      if (r < 2 * n) z[sb + r] = (double)acc;
-      else z[cbk + (r - 2 * n)] = (double)acc;
+    const int nr = min(4, m - r);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (nr == 4) {
+#pragma unroll 4
+      for (int c = lane; c < m; c += 32) {
+        const float t = tv[c];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fmaf(__ldg(row + (size_t)q * m + c), t, acc[q]);
+      }
+    } else {
+      for (int c = lane; c < m; c += 32)
+        for (int q = 0; q < 4; ++q)
+          if (q < nr) acc[q] = fmaf(__ldg(row + (size_t)q * m + c), tv[c], acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane < nr) {
+      const double v = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
+      const int i = r + lane;
+      if (i < 2 * n) z[sb + i] = v;
+      else z[cbk + (i - 2 * n)] = v;
     }
   }
 }
@@ -1983,7 +2001,8 @@ k_combine(GeoDev G, const double* __restrict__ den, const double2* __restrict__ 
   ux -= 0.5 * sx;
   uy -= 0.5 * sy;
   if (gc < G.nout) {
-    const double sg = *sigdotn;
+    double sg = 0.0;
+    for (int q = 0; q < (G.nout + 255) / 256; ++q) sg += sigdotn[q];
     ux += sg * nn.x;
     uy += sg * nn.y;
   }

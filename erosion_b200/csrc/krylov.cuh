@@ -7,7 +7,7 @@
 //   k_dot_reduce_dk      h1 = their sums
 //   k_cgs_update_dot     w -= V h1, and part = V^T w from the same reading of V
 //   k_dot_reduce_dk      h2
-//   k_cgs_update_norm    w -= V h2, and parts of |w|^2
+//   k_cgs_update_norm    w -= V h2, and parts of |w|^2 (k_cgs_vh_norm for long w)
 //   k_cgs_finish         V[k] = w/|w| (and the buffers the next step reads), the
 //                        column h1 + h2, |w|^2 to the host
 //
@@ -119,6 +119,31 @@ k_cgs_update_norm(const double* __restrict__ V, long long ldv, const int* __rest
     nn = warp_sum(nn);
     if (lane == 0) npart[blockIdx.x] = nn;
   }
+}
+
+// The same update with a row per thread (k_vh_dk), for long vectors.
+__global__ void __launch_bounds__(256)
+k_cgs_vh_norm(const double* __restrict__ V, long long ldv, const int* __restrict__ kp, const double* __restrict__ h,
+              double* __restrict__ w, long long n, double* __restrict__ npart) {
+  __shared__ double sh[CGS_MAX], red[32];
+  const int k = *kp;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  for (int t = threadIdx.x; t < k; t += 256) sh[t] = h[t];
+  __syncthreads();
+  double x = 0.0;
+  if (i < n) {
+    const double* __restrict__ vp = V + i;
+    double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int j = 0;
+    for (; j + 7 < k; j += 8)   // eight independent loads in flight
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = fma(__ldg(vp + (long long)(j + q) * ldv), sh[j + q], a[q]);
+    for (; j < k; ++j) a[0] = fma(__ldg(vp + (long long)j * ldv), sh[j], a[0]);
+    x = w[i] - (((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));
+    w[i] = x;
+  }
+  const double s = block_sum<256>(x * x, red);
+  if (threadIdx.x == 0) npart[blockIdx.x] = s;
 }
 
 // Every CTA sums the parts of |w|^2 in the same order.  z (may be nullptr): the

@@ -188,7 +188,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     double2* ws = cv.take<double2>(N);
     double4* sq64 = cv.take<double4>(N);
     float4* sq32 = cv.take<float4>(N);
-    double* sigdotn = cv.take<double>(1);
+    double* sigdotn = cv.take<double>(nblk(nout, 256));
     int4* tiles = cv.take<int4>(ntile);
     double2* selfsum = cv.take<double2>(N);
     // split-K of the far field as the host-side operator chooses it, capped by
@@ -219,7 +219,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
       k_body_stats<<<M, 256, 0, st>>>(n, nout, xy, sp, cen, rb);
       EB_LAUNCH_CHECK();
     }
-    k_prep<<<M + 1, 256, 0, st>>>(G, d_den, ws, sq64, sq32, d_vel, sigdotn, 0);
+    k_prep<<<M + nblk(nout, 256), 256, 0, st>>>(G, d_den, ws, sq64, sq32, d_vel, sigdotn, 0);
     EB_LAUNCH_CHECK();
     k_far64<false, FAR_NT, FAR_TPT, 0><<<dim3((unsigned)TB, (unsigned)nsplit), FAR_NT, 0, st>>>(
         G, sq64, tiles, split_ptr, nullptr, 0, partial);

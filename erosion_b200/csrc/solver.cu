@@ -379,10 +379,11 @@ static void plan_far(State& s, bool tune) {
 // expansions are two launches more.
 constexpr int kExpandNodes = 3200;
 
-// Parts of the near lists: about two CTAs per SM from items CTAs, at most 8.
+// Parts of the near lists: about four CTAs per SM from items CTAs, at most 8.
 // 10 bodies x 128 nodes and 1024 wall nodes (72 items): 31.5 us in one part,
-// 18.3 us in 5.
-int near_parts(int items) { return std::max(1, std::min(8, (2 * g_num_sms + items - 1) / items)); }
+// 20.4 us in 5, 17.1 us in 8, 16.0 us in 12 (and 3 us more in larger assemblies);
+// 100 x 256, FP32 (464 items): 39.8 us in one part, 33.7 us in 2, 33.3 us in 4.
+int near_parts(int items) { return std::max(1, std::min(8, (4 * g_num_sms + items - 1) / items)); }
 
 // Decides how the current problem's far field is summed.
 // The direct sum over split tile ranges (launch_far) stays for a forced launch
@@ -577,7 +578,7 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   s.xy.ensure(N); s.nrm.ensure(N); s.dz.ensure(N); s.d1tmp.ensure(N);
   s.sp.ensure(N); s.cur.ensure(N); s.w.ensure(N);
   s.cen.ensure(std::max(pr.M, 1)); s.rb.ensure(std::max(pr.M, 1));
-  s.ws.ensure(N); s.sq64.ensure(N); s.sigdotn.ensure(1);
+  s.ws.ensure(N); s.sq64.ensure(N); s.sigdotn.ensure(nblk(pr.nout, 256));
   k_wall_nodes<<<nblk(pr.nout, 256), 256, 0, st>>>(pr.nout, pr.P.wall_a, pr.P.wall_b, pr.P.wall_order, s.wx.p, s.wy.p);
   EB_LAUNCH_CHECK();
   const GeomIn gin{s.wx.p, s.wy.p, d_xx, d_yy, s.dker_wall.p, s.dker_body.p, pr.nout, pr.n};
@@ -914,8 +915,8 @@ void harvest_far_timing(State& s) {
 
 void operator_prep(State& s, const double* d_den, double* d_vel) {
   const Problem& pr = s.pr;
-  k_prep<<<pr.M + 1, 256, 0, s.st>>>(s.geo(), d_den, s.ws.p, s.sq64.p, s.sq32.p, d_vel, s.sigdotn.p,
-                                      pr.P.ibary == 1);
+  k_prep<<<pr.M + nblk(pr.nout, 256), 256, 0, s.st>>>(s.geo(), d_den, s.ws.p, s.sq64.p, s.sq32.p, d_vel, s.sigdotn.p,
+                                                     pr.P.ibary == 1);
   EB_LAUNCH_CHECK();
 }
 
@@ -1079,6 +1080,13 @@ static int step_bound(int ll) {
   return std::min(b, CGS_MAX);
 }
 
+// Unknowns from which a thread owns a row of the update: its CTA then reads 2 KB
+// of a column at a time, and the two passes over V are no slower than the
+// fused one's 256-byte pieces.  55,596 unknowns (k = 240): fused 19.8 and 16.4
+// us, by rows 31.6 and 16.8 us; 107,392 (k = 165): 31.7 and 29.0 us, by rows
+// 33.8 and 17.4 us.
+constexpr long long kRowPerThread = 75000;
+
 static size_t step_tile(int bound) { return (size_t)bound * 34 * sizeof(double); }
 
 static void step_buffers(State& s, long long N, long long cols) {
@@ -1097,7 +1105,7 @@ static void step_buffers(State& s, long long N, long long cols) {
   s.k_w.ensure(N);
   s.k_h1.ensure(CGS_MAX + 1);
   s.k_h2.ensure(CGS_MAX + 1);
-  s.k_np.ensure(4 * g_num_sms);
+  s.k_np.ensure(std::max<long long>(4 * g_num_sms, nblk(N, 256)));
   s.k_count.ensure(1);
   s.pc_z.ensure(N);
   s.part.ensure((size_t)std::min<long long>(cols, CGS_MAX) * nb);
@@ -1130,13 +1138,13 @@ static void launch_step(State& s, long long N, long long ldv, int bound, int pre
   // as many CTAs as are resident with the chunk's block of V in shared memory
   const size_t tile = step_tile(bound);
   const int chunks = (int)nblk(N, CGS_ROWS), per_sm = std::max(1, std::min(4, (int)((220 * 1024) / (tile + 4096))));
-  if (tile <= 220 * 1024) {
+  if (tile <= 220 * 1024 && N < kRowPerThread) {
     const int g = std::min(chunks, per_sm * g_num_sms);
     k_cgs_update_dot<<<g, 256, tile, st>>>(s.V.p, ldv, kp, s.k_h1.p, s.k_w.p, N, s.part.p);
     EB_LAUNCH_CHECK();
     k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, g, kp, 0, s.k_h2.p);
     EB_LAUNCH_CHECK();
-  } else {   // more columns than fit: the update and the product by themselves
+  } else {   // the update and the product by themselves
     k_vh_dk<<<nblk(N, 256), 256, 0, st>>>(s.V.p, ldv, kp, s.k_h1.p, -1.0, s.k_w.p, N);
     EB_LAUNCH_CHECK();
     k_cgs_dot<<<dim3(nb, ny), 256, R * sizeof(double), st>>>(s.V.p, ldv, kp, s.k_w.p, N, R, s.part.p);
@@ -1144,8 +1152,13 @@ static void launch_step(State& s, long long N, long long ldv, int bound, int pre
     k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, 0, s.k_h2.p);
     EB_LAUNCH_CHECK();
   }
-  const int gn = std::min(chunks, 4 * g_num_sms);
-  k_cgs_update_norm<<<gn, 256, 0, st>>>(s.V.p, ldv, kp, s.k_h2.p, s.k_w.p, N, s.k_np.p);
+  int gn = std::min(chunks, 4 * g_num_sms);
+  if (N >= kRowPerThread) {
+    gn = (int)nblk(N, 256);
+    k_cgs_vh_norm<<<gn, 256, 0, st>>>(s.V.p, ldv, kp, s.k_h2.p, s.k_w.p, N, s.k_np.p);
+  } else {
+    k_cgs_update_norm<<<gn, 256, 0, st>>>(s.V.p, ldv, kp, s.k_h2.p, s.k_w.p, N, s.k_np.p);
+  }
   EB_LAUNCH_CHECK();
   k_cgs_finish<<<std::min(nblk(N, 256), (unsigned)(4 * g_num_sms)), 256, 0, st>>>(
       s.V.p, s.Z.p, ldv, kp, s.k_h1.p, s.k_h2.p, s.k_np.p, gn, s.k_w.p, s.pc_active ? s.pc_z.p : nullptr, s.k_cur.p, N,

@@ -894,7 +894,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       // strengths without the bodies' rigid parts (see k_stress_rigid), the
       // near lists of this mask, their strain and that of the expansions
       ClLists& lists = s.cl_stress;
-      k_prep<<<pr.M + 1, 256, 0, s.st>>>(G, d_den, s.ws.p, s.sq64.p, s.sq32.p, s.d_w.ensure(pr.ntot), s.sigdotn.p, 1);
+      k_prep<<<pr.M + nblk(pr.nout, 256), 256, 0, s.st>>>(G, d_den, s.ws.p, s.sq64.p, s.sq32.p, s.d_w.ensure(pr.ntot), s.sigdotn.p, 1);
       EB_LAUNCH_CHECK();
       build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand, nullptr);
       const ClView L = cl_view(s, lists);
