@@ -1768,23 +1768,40 @@ __device__ double2 bary_coincident(const GeoDev& G, int start, int len, const do
 // the sources, and the sums meet in near_reduce, so that every thread returns
 // the result of its lane.  The curve is read in passes over its shared-memory
 // tiles (value, first and second derivative, :5190-5228 / :5468-5525); a curve
-// of at most NEAR_TK nodes is staged once for all of them.  Bound by the FP64
-// pipe with many targets and by a warp's chain of sources with few: against one
-// thread per target and a correctly rounded division, the near pairs of 3
-// bodies x 64 nodes take 11.8 us (69.6), of 400 x 256 28.7 us (78.1), and the
-// gradients of the latter's shear stress 454 us (2200).
+// of at most NEAR_TK nodes is staged once for all of them.
+// With e = v_0 - x v_1 - y v_2 of the first three fields (zt = x + iy) the results
+// are, for the values v, their first derivatives v' and second v'',
+//   ux = Re(e' + v_3), uy = -Im e' + Re v_4,
+//   u1x = Re(e'' - v_1' + v_3'),  u1y = -Im(e'' + v_3') - Re v_2',
+//   u2x = -Im(e'' - v_1') + Re v_4',  u2y = -Re e'' + Im(v_2' - v_4'),
+// and e obeys the same formulas as a field, so it takes the place of v_0 (and
+// without the gradient of v_0, v_1 and v_2): 71 FP64 operations per source and
+// target, 143 with the gradient.  Bound by the FP64 pipe with many targets and by
+// a warp's chain of sources with few: against one thread per target and
+// correctly rounded divisions, the near pairs of 3 bodies x 64 nodes take 10.5 us
+// (69.6), of 400 x 256 25.0 us (78.1), the gradients of the latter's shear stress
+// 461 us (2200), and of 3200 targets against 50 x 128 + 1024 nodes 329 us (577).
 template <int NDER>
-__device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* __restrict__ bdc, double2 zt,
-                            bool act) {
+__device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* __restrict__ bdc,
+                                            double2 zt, bool act) {
   const int start = curve_start(G, c), len = curve_len(G, c);
   const bool ext = c != 0, whole = len <= NEAR_TK;
   const int wid = threadIdx.x >> 5;
+  constexpr int NF = NDER == 2 ? 5 : 3;   // fields: e, (v_1, v_2,) v_3, v_4
   double2 a = make_double2(0, 0);
   if (ext) a = G.cen[c - 1];
+  // the fields of staged source kk
+  auto field = [&](int kk, int q) {
+    if (q == 0) {
+      const double2 b0 = T.b[0][kk], b1 = T.b[1][kk], b2 = T.b[2][kk];
+      return make_double2(fma(-zt.x, b1.x, fma(-zt.y, b2.x, b0.x)), fma(-zt.x, b1.y, fma(-zt.y, b2.y, b0.y)));
+    }
+    return T.b[NDER == 2 ? q : q + 2][kk];
+  };
   // Pass 1: values.
-  double v1[12];   // the denominator, then the five numerators
+  double v1[2 + 2 * NF];   // the denominator, then the numerators
 #pragma unroll
-  for (int q = 0; q < 12; ++q) v1[q] = 0.0;
+  for (int q = 0; q < 2 + 2 * NF; ++q) v1[q] = 0.0;
   for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
     bary_load_tile(T, G, start, len, k0, bdc, ext, a);
     const int kt = min(NEAR_TK, len - k0);
@@ -1795,20 +1812,20 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
       v1[0] += c1.x;
       v1[1] += c1.y;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) cfma2(v1[2 + 2 * q], v1[3 + 2 * q], T.b[q][kk], c1);
+      for (int q = 0; q < NF; ++q) cfma2(v1[2 + 2 * q], v1[3 + 2 * q], field(kk, q), c1);
     }
   }
   near_reduce(v1, T.red);
   const double2 den = make_double2(v1[0], v1[1]);
-  double2 u[5];
+  double2 u[NF];
   {
     const double2 dd = ext ? make_double2(den.x, den.y - EB_TWOPI) : den;
     const double2 di = cinv(dd);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) u[q] = cmul(make_double2(v1[2 + 2 * q], v1[3 + 2 * q]), di);
+    for (int q = 0; q < NF; ++q) u[q] = cmul(make_double2(v1[2 + 2 * q], v1[3 + 2 * q]), di);
   }
-  // Pass 2: first derivative (of all five fields when the gradient is asked for).
-  constexpr int ND = NDER == 2 ? 5 : 3;
+  // Pass 2: first derivative (of e alone without the gradient).
+  constexpr int ND = NDER == 2 ? 5 : 1;
   double v2[2 + 2 * ND];
 #pragma unroll
   for (int q = 0; q < 2 + 2 * ND; ++q) v2[q] = 0.0;
@@ -1820,22 +1837,23 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
 #pragma unroll 2
     for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
       const double2 d = csub(T.z[kk], zt);
-      const double2 inv = bary_inv(d);
+      const double r2 = cabs2(d), ir = rcp_raw64(r2);
+      const double2 inv = make_double2(d.x * ir, -d.y * ir);
       const double2 c1 = cmul(T.dz[kk], inv);
       if (ext) {
         cfma2(v2[0], v2[1], c1, T.za[kk]);
-        if (cabs2(d) <= 1e-20) { coinc = true; continue; }
+        if (r2 <= 1e-20) { coinc = true; continue; }
       }
       const double2 c2 = cmul(c1, inv);
 #pragma unroll
-      for (int q = 0; q < ND; ++q) cfma2(v2[2 + 2 * q], v2[3 + 2 * q], csub(T.b[q][kk], u[q]), c2);
+      for (int q = 0; q < ND; ++q) cfma2(v2[2 + 2 * q], v2[3 + 2 * q], csub(field(kk, q), u[q]), c2);
     }
   }
   if (ext) {
     // a warp adds the branch of the coincident nodes in its own share
     if (coinc && act) {
 #pragma unroll 1
-      for (int q = 0; q < ND; ++q) {
+      for (int q = 0; q < 5; ++q) {
         double2 tmp1 = make_double2(0, 0), tmp2 = make_double2(0, 0), add = make_double2(0, 0);
         for (int k = 0; k < len; ++k) {
           const double2 d = csub(G.xy[start + k], zt);
@@ -1843,28 +1861,28 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
           if (kk >= kt * wid / NEAR_W && kk < kt * (wid + 1) / NEAR_W && cabs2(d) <= 1e-20)
             add = cadd(add, bary_coincident(G, start, len, bdc, q, k, zt, a, tmp1, tmp2));
         }
+        const double f = q == 0 ? 1.0 : q == 1 ? -zt.x : -zt.y;   // e = v_0 - x v_1 - y v_2
+        if (q < 3) { v2[2] += f * add.x; v2[3] += f * add.y; }
 #pragma unroll
-        for (int p = 0; p < ND; ++p)
+        for (int p = 1; p < ND; ++p)
           if (p == q) { v2[2 + 2 * p] += add.x; v2[3 + 2 * p] += add.y; }
       }
     }
   }
   near_reduce(v2, T.red);
-  double2 du[5];
+  double2 du[ND];
   double2 fac;
   if (ext) fac = cinv(cmul(csub(zt, a), make_double2(v2[0], v2[1])));
   else fac = cinv(den);
 #pragma unroll
   for (int q = 0; q < ND; ++q) du[q] = cmul(make_double2(v2[2 + 2 * q], v2[3 + 2 * q]), fac);
   DLPVal r;
-  r.ux = du[0].x - zt.x * du[1].x - zt.y * du[2].x + u[3].x;
-  r.uy = -du[0].y + zt.x * du[1].y + zt.y * du[2].y + u[4].x;
+  r.ux = du[0].x + u[NF - 2].x;
+  r.uy = -du[0].y + u[NF - 1].x;
   r.u1x = r.u1y = r.u2x = r.u2y = 0.0;
   if constexpr (NDER == 2) {
-    // Pass 3: second derivative.
-    double v3[10];
-#pragma unroll
-    for (int q = 0; q < 10; ++q) v3[q] = 0.0;
+    // Pass 3: second derivative of e.
+    double v3[2] = {0.0, 0.0};
     for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
       if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
       const int kt = min(NEAR_TK, len - k0);
@@ -1874,21 +1892,16 @@ __device__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* 
         const double2 d = csub(T.z[kk], zt);
         const double2 inv = bary_inv(d);
         const double2 c3 = cmul(cmul(cmul(T.dz[kk], inv), inv), inv);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          const double2 t = csub(csub(T.b[q][kk], u[q]), cmul(du[q], d));
-          cfma2(v3[2 * q], v3[2 * q + 1], t, c3);
-        }
+        const double2 t = csub(csub(field(kk, 0), u[0]), cmul(du[0], d));
+        cfma2(v3[0], v3[1], t, c3);
       }
     }
     near_reduce(v3, T.red);
-    double2 dd[5];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) dd[q] = cscale(cmul(make_double2(v3[2 * q], v3[2 * q + 1]), fac), 2.0);
-    r.u1x = dd[0].x - du[1].x - zt.x * dd[1].x - zt.y * dd[2].x + du[3].x;
-    r.u1y = -dd[0].y + zt.x * dd[1].y - du[2].x + zt.y * dd[2].y - du[3].y;
-    r.u2x = -dd[0].y + du[1].y + zt.x * dd[1].y + zt.y * dd[2].y + du[4].x;
-    r.u2y = -dd[0].x + zt.x * dd[1].x + du[2].y + zt.y * dd[2].x - du[4].y;
+    const double2 e = cscale(cmul(make_double2(v3[0], v3[1]), fac), 2.0);
+    r.u1x = e.x - du[1].x + du[3].x;
+    r.u1y = -e.y - du[2].x - du[3].y;
+    r.u2x = -e.y + du[1].y + du[4].x;
+    r.u2y = -e.x + du[2].y - du[4].y;
   }
   return r;
 }

@@ -12,29 +12,31 @@ __device__ __forceinline__ long long bd_all_off(const GeoDev& G, int c) {
   return c == 0 ? 0LL : 5LL * G.nout + 5LL * (c - 1) * G.n;
 }
 
-// Barycentric Stokes DLP (NDER = 2: with gradient) of the source curves
-// [split_c[y], split_c[y+1]) at the targets of this CTA's task, skipping the
-// task's own curve.  Partial sums per split: out[(y*6 + q)*ntar + t] with
+// Barycentric Stokes DLP with gradient of the source curves of part blockIdx.y
+// of gridDim.y at 32 targets: CTA blockIdx.x takes targets 32 blockIdx.x.. of all
+// ntar, or with bodies = 1 (the targets are the body nodes) 32 nodes of one body,
+// skipping that body's curve.  Partial sums per part: out[(y*6 + q)*ntar + t] with
 // q = ux, uy, u1x, u1y, u2x, u2y.
-template <int NDER>
-__global__ void __launch_bounds__(NEAR_NT)
-k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const int4* __restrict__ tasks,
-           const double2* __restrict__ txy, const int* __restrict__ split_c, int ntar, double* __restrict__ out) {
+__global__ void __launch_bounds__(NEAR_NT, 2)
+k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const double2* __restrict__ txy, int bodies, int ntar,
+           double* __restrict__ out) {
   __shared__ BaryTile T;
-  const int4 tk = tasks[blockIdx.x];
-  const int split = blockIdx.y;
-  const int t = tk.x + (threadIdx.x & 31);
-  const bool act = t < tk.y;
-  const double2 zt = txy[act ? t : tk.y - 1];
+  const int per = bodies ? (G.n + NEAR_T - 1) / NEAR_T : 0, b = bodies ? blockIdx.x / per : -1;
+  const int t0 = bodies ? b * G.n + NEAR_T * (blockIdx.x - b * per) : NEAR_T * blockIdx.x;
+  const int t1 = bodies ? min((b + 1) * G.n, t0 + NEAR_T) : min(ntar, t0 + NEAR_T);
+  const int t = t0 + (threadIdx.x & 31);
+  const bool act = t < t1;
+  const double2 zt = txy[act ? t : t1 - 1];
   double a[6] = {0, 0, 0, 0, 0, 0};
-  for (int c = split_c[split]; c < split_c[split + 1]; ++c) {
-    if (c == tk.z) continue;
-    DLPVal r = bary_eval<NDER>(T, G, c, bd_all + bd_all_off(G, c), zt, act);
+  const int nc = G.M + 1, c1 = (int)((long long)nc * (blockIdx.y + 1) / gridDim.y);
+  for (int c = (int)((long long)nc * blockIdx.y / gridDim.y); c < c1; ++c) {
+    if (c == b + 1 && bodies) continue;
+    DLPVal r = bary_eval<2>(T, G, c, bd_all + bd_all_off(G, c), zt, act);
     a[0] += r.ux; a[1] += r.uy; a[2] += r.u1x; a[3] += r.u1y; a[4] += r.u2x; a[5] += r.u2y;
   }
   if (act && threadIdx.x < 32) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) out[((size_t)split * 6 + q) * ntar + t] = a[q];
+    for (int q = 0; q < 6; ++q) out[((size_t)blockIdx.y * 6 + q) * ntar + t] = a[q];
   }
 }
 
@@ -337,7 +339,7 @@ k_stress_near_items(GeoDev G, const int2* __restrict__ items, const int4* __rest
 // visits fewer curves that only some of its nodes need than with 128, and the
 // warps share each curve's nodes (bary_eval).  out[q * nb + i], q as
 // k_bary_sum (one split).
-__global__ void __launch_bounds__(NEAR_NT)
+__global__ void __launch_bounds__(NEAR_NT, 2)
 k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const unsigned* __restrict__ mask, int mw,
                 double* __restrict__ out) {
   __shared__ BaryTile T;
@@ -617,109 +619,135 @@ k_stress_assemble(GeoDev G, const double* __restrict__ den, ClView L, const int4
   }
 }
 
-// Trapezoid pressure (always) and velocity/vorticity (ibary = 0) at targets
-// from every node (:3170-3197, :3225-3255).  out[(split*4 + q)*ntar + t],
-// q = u, v, p, w.
+// Trapezoid pressure (always) and velocity/vorticity (VEL: ibary = 0) at targets
+// from every node (:3170-3197, :3225-3255).  CTA = 32 targets, one per lane, and
+// part blockIdx.y of the source tiles; its 8 warps split a tile's sources.
+// out[(part*4 + q)*ntar + t], q = u, v, p, w.  Bound by the FP64 pipe: 3200
+// targets and 7424 nodes 47 us (a thread per target, three divisions a pair,
+// 132 us).
+template <bool VEL>
 __global__ void __launch_bounds__(256)
-k_qoi_trap(GeoDev G, const double* __restrict__ den, const int4* __restrict__ tiles,
-           const int* __restrict__ split_ptr, int ntar, const double2* __restrict__ txy, int velocity,
-           double* __restrict__ out) {
-  __shared__ double2 sxy[FAR_TS], sn[FAR_TS], ss[FAR_TS];
-  __shared__ double sw[FAR_TS];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+k_qoi_trap(GeoDev G, const double* __restrict__ den, const int4* __restrict__ tiles, int ntile, int ntar,
+           const double2* __restrict__ txy, double* __restrict__ out) {
+  __shared__ double4 sg[FAR_TS];   // x, y, nx, ny
+  __shared__ double4 sd[FAR_TS];   // w sigma, w n.sigma
+  __shared__ double red[NEAR_W / 2][4][32];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = 32 * blockIdx.x + lane;
   const bool act = t < ntar;
   const double2 p = txy[act ? t : ntar - 1];
-  double u = 0, v = 0, pr = 0, w = 0;
-  const int split = blockIdx.y;
-  for (int ti = split_ptr[split]; ti < split_ptr[split + 1]; ++ti) {
-    const int4 T = tiles[ti];
+  double a[4] = {0, 0, 0, 0};
+  int ti = (int)((long long)ntile * blockIdx.y / gridDim.y);
+  const int te = (int)((long long)ntile * (blockIdx.y + 1) / gridDim.y);
+  while (ti < te) {
+    // consecutive tiles are consecutive nodes: take as many as fit
+    const int g0 = tiles[ti].x;
+    int len = 0;
     __syncthreads();
-    if (threadIdx.x < T.y) {
-      int gs = T.x + threadIdx.x;
-      sxy[threadIdx.x] = G.xy[gs];
-      sn[threadIdx.x] = G.nrm[gs];
-      ss[threadIdx.x] = make_double2(den[ix_of(G, gs)], den[iy_of(G, gs)]);
-      sw[threadIdx.x] = G.w[gs];
+    while (ti < te && len + tiles[ti].y <= FAR_TS) len += tiles[ti++].y;
+    if ((int)threadIdx.x < len) {
+      const int g = g0 + threadIdx.x;
+      const double2 q = G.xy[g], nn = G.nrm[g];
+      const double wg = G.w[g], sx = wg * den[ix_of(G, g)], sy = wg * den[iy_of(G, g)];
+      sg[threadIdx.x] = make_double4(q.x, q.y, nn.x, nn.y);
+      sd[threadIdx.x] = make_double4(sx, sy, nn.x * sx + nn.y * sy, 0.0);
     }
     __syncthreads();
-    for (int j = 0; j < T.y; ++j) {
-      const double2 q = sxy[j], nn = sn[j], s = ss[j];
-      double rx = p.x - q.x, ry = p.y - q.y;
-      double rho2 = rx * rx + ry * ry;
-      double rdotn = rx * nn.x + ry * nn.y;
-      double rdotden = rx * s.x + ry * s.y;
-      double dendotn = nn.x * s.x + nn.y * s.y;
-      double wg = sw[j];
-      pr += (2.0 * rdotn * rdotden / rho2 / rho2 - dendotn / rho2) * wg;
-      if (velocity) {
-        double routn = -rx * nn.y + ry * nn.x;
-        double routden = -rx * s.y + ry * s.x;
-        u += rdotn / rho2 * rdotden / rho2 * rx * wg;
-        v += rdotn / rho2 * rdotden / rho2 * ry * wg;
-        w += (rdotden * routn + rdotn * routden) / (rho2 * rho2) * wg;
+    const int kb = len * (wid + 1) / NEAR_W;
+#pragma unroll 2
+    for (int j = len * wid / NEAR_W; j < kb; ++j) {
+      const double4 q = sg[j], s = sd[j];
+      const double rx = p.x - q.x, ry = p.y - q.y;
+      const double i2 = rcp_raw64(fma(rx, rx, ry * ry));
+      const double rdn = fma(rx, q.z, ry * q.w), rds = fma(rx, s.x, ry * s.y);
+      const double m = rdn * rds * i2 * i2;
+      a[2] += fma(2.0, m, -s.z * i2);
+      if (VEL) {
+        const double rn = fma(-rx, q.w, ry * q.z), rs = fma(-rx, s.y, ry * s.x);
+        a[0] = fma(m, rx, a[0]);
+        a[1] = fma(m, ry, a[1]);
+        a[3] = fma(fma(rds, rn, rdn * rs), i2 * i2, a[3]);
       }
     }
   }
-  if (act) {
-    out[((size_t)split * 4 + 0) * ntar + t] = u;
-    out[((size_t)split * 4 + 1) * ntar + t] = v;
-    out[((size_t)split * 4 + 2) * ntar + t] = pr;
-    out[((size_t)split * 4 + 3) * ntar + t] = w;
+  __syncthreads();
+  near_reduce(a, red);
+  if (act && wid == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[((size_t)blockIdx.y * 4 + q) * ntar + t] = a[q];
   }
 }
 
 // Final assembly at targets: barycentric velocity and vorticity (:3199-3212,
 // :3257-3270), stokeslets/rotlets (:3275-3298), and zeroing of targets that
-// classifyPointsOld (:4420-4500) puts inside a body (:3301-3309).
-__global__ void __launch_bounds__(128)
+// classifyPointsOld (:4420-4500) puts inside a body (:3301-3309): the nearest
+// body node (first minimum in body-major order) decides the side through the
+// sign of (x_t - x_k).n_k.  CTA = 32 targets, one per lane; the warps split the
+// bodies and the nodes, in order, and meet in order.  3200 targets, 6400 body
+// nodes: 52 us (a thread per target 265 us).
+__global__ void __launch_bounds__(256)
 k_qoi_final(GeoDev G, const double* __restrict__ den, int ntar, const double2* __restrict__ txy,
             const double* __restrict__ ptrap, int ns1, const double* __restrict__ pbary, int ns2, int ibary,
             double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ po, double* __restrict__ wo) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntar) return;
-  double u = 0, v = 0, pr = 0, w = 0;
-  for (int s = 0; s < ns1; ++s) {
-    u += ptrap[((size_t)s * 4 + 0) * ntar + t];
-    v += ptrap[((size_t)s * 4 + 1) * ntar + t];
-    pr += ptrap[((size_t)s * 4 + 2) * ntar + t];
-    w += ptrap[((size_t)s * 4 + 3) * ntar + t];
-  }
-  if (ibary) {
-    for (int s = 0; s < ns2; ++s) {
+  __shared__ double red[NEAR_W / 2][4][32];
+  __shared__ double dm[NEAR_W][32];
+  __shared__ int di[NEAR_W][32];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = 32 * blockIdx.x + lane;
+  const bool act = t < ntar;
+  const int tc = act ? t : ntar - 1;
+  const double2 p = txy[tc];
+  double a[4] = {0, 0, 0, 0};   // u, v, p, w
+  for (int s = wid; s < ns1; s += NEAR_W)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] += ptrap[((size_t)s * 4 + q) * ntar + tc];
+  if (ibary)
+    for (int s = wid; s < ns2; s += NEAR_W) {
       const double* P = pbary + (size_t)s * 6 * ntar;
-      u += P[t];
-      v += P[(size_t)ntar + t];
-      w += P[4 * (size_t)ntar + t] - P[3 * (size_t)ntar + t];
+      a[0] += P[tc];
+      a[1] += P[(size_t)ntar + tc];
+      a[3] += P[4 * (size_t)ntar + tc] - P[3 * (size_t)ntar + tc];
     }
+  for (int b = wid; b < G.M; b += NEAR_W) {
+    const double2 cc = G.cen[b];
+    const double s1 = den[ic_of(G, b, 0)], s2 = den[ic_of(G, b, 1)], rot = den[ic_of(G, b, 2)];
+    const double rx = p.x - cc.x, ry = p.y - cc.y;
+    const double rho2 = rx * rx + ry * ry, rd = rx * s1 + ry * s2;
+    const double ir = 1.0 / rho2, lg = log(rho2);
+    a[0] += 0.5 / EB_TWOPI * (-0.5 * lg * s1 + rd * ir * rx) + rot * ry * ir;
+    a[1] += 0.5 / EB_TWOPI * (-0.5 * lg * s2 + rd * ir * ry) - rot * rx * ir;
+    a[2] += 1.0 / EB_TWOPI * rd * ir;
+    a[3] += (ry * s1 - rx * s2) * ir / EB_TWOPI;
   }
-  const double2 p = txy[t];
+  near_reduce(a, red);
+  const int nb = G.n * G.M;
+  double dmin = 1e10;
+  int ind = 0;
+  const int hi = (int)((long long)nb * (wid + 1) / NEAR_W);
+#pragma unroll 4
+  for (int i = (int)((long long)nb * wid / NEAR_W); i < hi; ++i) {
+    const double2 q = G.xy[G.nout + i];
+    const double d2 = (p.x - q.x) * (p.x - q.x) + (p.y - q.y) * (p.y - q.y);
+    if (d2 < dmin) { dmin = d2; ind = i; }
+  }
+  dm[wid][lane] = dmin;
+  di[wid][lane] = ind;
+  __syncthreads();
+  if (wid != 0 || !act) return;
   if (G.M > 0) {
-    for (int b = 0; b < G.M; ++b) {
-      const double2 cc = G.cen[b];
-      const double s1 = den[ic_of(G, b, 0)], s2 = den[ic_of(G, b, 1)], rot = den[ic_of(G, b, 2)];
-      const double rx = p.x - cc.x, ry = p.y - cc.y;
-      const double rho2 = rx * rx + ry * ry, rd = rx * s1 + ry * s2;
-      u += 0.5 / EB_TWOPI * (-0.5 * log(rho2) * s1 + rd / rho2 * rx);
-      v += 0.5 / EB_TWOPI * (-0.5 * log(rho2) * s2 + rd / rho2 * ry);
-      pr += 1.0 / EB_TWOPI * rd / rho2;
-      w += (ry * s1 - rx * s2) / rho2 / EB_TWOPI;
-      u += rot * ry / rho2;
-      v -= rot * rx / rho2;
-    }
-    // classifyPointsOld: nearest body node (first minimum in body-major
-    // order) decides the side through the sign of (x_t - x_k).n_k.
-    double dmin = 1e10;
-    int ind = 0;
-    for (int i = 0; i < G.n * G.M; ++i) {
-      const double2 q = G.xy[G.nout + i];
-      const double d2 = (p.x - q.x) * (p.x - q.x) + (p.y - q.y) * (p.y - q.y);
-      if (d2 < dmin) { dmin = d2; ind = i; }
-    }
+    for (int w = 1; w < NEAR_W; ++w)
+      if (dm[w][lane] < dmin) { dmin = dm[w][lane]; ind = di[w][lane]; }
     const double2 q = G.xy[G.nout + ind], nn = G.nrm[G.nout + ind];
     const double vdn = (p.x - q.x) * nn.x + (p.y - q.y) * nn.y;
-    if (!(vdn < 0.0)) { u = 0; v = 0; pr = 0; w = 0; }
+    if (!(vdn < 0.0)) a[0] = a[1] = a[2] = a[3] = 0.0;
   }
-  uo[t] = u; vo[t] = v; po[t] = pr; wo[t] = w;
+  uo[t] = a[0];
+  vo[t] = a[1];
+  po[t] = a[2];
+  wo[t] = a[3];
+}
+
+__global__ void k_pack(int n, const double* __restrict__ x, const double* __restrict__ y, double2* __restrict__ xy) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) xy[i] = make_double2(x[i], y[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -820,12 +848,9 @@ k_pressure_final(GeoDev G, const double* __restrict__ den, const double* __restr
   out[t] = acc;
 }
 
-static int source_splits(int ntasks, int ncurves, std::vector<int>& sc) {
-  int want = std::max(1, (4 * eb_num_sms() + ntasks - 1) / std::max(ntasks, 1));
-  int S = std::max(1, std::min(want, ncurves));
-  sc.resize(S + 1);
-  for (int q = 0; q <= S; ++q) sc[q] = (int)((long long)q * ncurves / S);
-  return S;
+// Parts of the source curves for ntasks CTAs of targets: about four CTAs per SM.
+static int source_splits(int ntasks, int ncurves) {
+  return std::max(1, std::min((4 * eb_num_sms() + ntasks - 1) / std::max(ntasks, 1), ncurves));
 }
 
 void body_pressure(State& s, const double* d_den, double* d_p) {
@@ -848,29 +873,18 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
   if (nb == 0) return;
   static DBuf<double> eself, part;
   static DBuf<double2> bd_all;
-  static DBuf<int4> d_tasks;
-  static DBuf<int> d_sc;
   eself.ensure(3LL * nb);
   k_stress_self<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, s.st>>>(G, d_den, s.dker_body.p, eself.p);
   EB_LAUNCH_CHECK();
   const int bary = pr.P.ibary == 1;
   if (bary && pr.P.stress_all_bary) {   // every pair barycentric, as the reference evaluates it
     bdval_all(s, d_den, bd_all);
-    std::vector<int4> tasks;
-    for (int b = 0; b < pr.M; ++b)
-      for (int k0 = 0; k0 < pr.n; k0 += NEAR_T)
-        tasks.push_back(make_int4(b * pr.n + k0, b * pr.n + std::min(pr.n, k0 + NEAR_T), 1 + b, 0));
-    std::vector<int> sc;
-    const int nsplit = source_splits((int)tasks.size(), pr.M + 1, sc);
-    h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
-    h2d(d_sc.ensure(sc.size()), sc.data(), sc.size(), s.st);
+    const int tasks = pr.M * (int)nblk(pr.n, NEAR_T), nsplit = source_splits(tasks, pr.M + 1);
     part.ensure((size_t)nsplit * 6 * nb);
-    dim3 grid((unsigned)tasks.size(), nsplit);
-    k_bary_sum<2><<<grid, NEAR_NT, 0, s.st>>>(G, bd_all.p, d_tasks.p, s.xy.p + pr.nout, d_sc.p, nb, part.p);
+    k_bary_sum<<<dim3(tasks, nsplit), NEAR_NT, 0, s.st>>>(G, bd_all.p, s.xy.p + pr.nout, 1, nb, part.p);
     EB_LAUNCH_CHECK();
     k_stress_final<<<nblk(nb, 256), 256, 0, s.st>>>(G, d_den, part.p, nsplit, nullptr, 0, 1, eself.p, d_tau, d_E);
     EB_LAUNCH_CHECK();
-    EB_CK(cudaStreamSynchronize(s.st));
   } else if (bary) {   // barycentric near pairs, trapezoid elsewhere
     static DBuf<double> wall_d2h;
     static DBuf<double2> ext;
@@ -950,42 +964,27 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
   if (ntar == 0) return;
   static DBuf<double2> txy, bd_all;
   static DBuf<double> ptrap, pbary;
-  static DBuf<int4> d_tasks;
-  static DBuf<int> d_sc;
   txy.ensure(ntar);
-  {
-    std::vector<double> hx(ntar), hy(ntar);
-    d2h(hx.data(), d_xt, ntar, s.st);
-    d2h(hy.data(), d_yt, ntar, s.st);
-    EB_CK(cudaStreamSynchronize(s.st));
-    std::vector<double2> h(ntar);
-    for (long long t = 0; t < ntar; ++t) h[t] = make_double2(hx[t], hy[t]);
-    h2d(txy.p, h.data(), ntar, s.st);
-    EB_CK(cudaStreamSynchronize(s.st));
-  }
-  const int ibary = pr.P.ibary == 1;
-  ptrap.ensure((size_t)s.nsplit * 4 * ntar);
-  dim3 g1(nblk(ntar, 256), s.nsplit);
-  k_qoi_trap<<<g1, 256, 0, s.st>>>(G, d_den, s.tiles.p, s.split_ptr.p, (int)ntar, txy.p, !ibary, ptrap.p);
+  k_pack<<<nblk(ntar, 256), 256, 0, s.st>>>((int)ntar, d_xt, d_yt, txy.p);
+  EB_LAUNCH_CHECK();
+  const int ibary = pr.P.ibary == 1, tasks = (int)nblk(ntar, NEAR_T);
+  const int ns1 = source_splits(tasks, std::min(s.ntile, 16));
+  ptrap.ensure((size_t)ns1 * 4 * ntar);
+  if (ibary)
+    k_qoi_trap<false><<<dim3(tasks, ns1), 256, 0, s.st>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
+  else
+    k_qoi_trap<true><<<dim3(tasks, ns1), 256, 0, s.st>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
   EB_LAUNCH_CHECK();
   int ns2 = 0;
   if (ibary) {
     bdval_all(s, d_den, bd_all);
-    std::vector<int4> tasks;
-    for (long long t0 = 0; t0 < ntar; t0 += NEAR_T)
-      tasks.push_back(make_int4((int)t0, (int)std::min<long long>(ntar, t0 + NEAR_T), -1, 0));
-    std::vector<int> sc;
-    ns2 = source_splits((int)tasks.size(), pr.M + 1, sc);
-    h2d(d_tasks.ensure(tasks.size()), tasks.data(), tasks.size(), s.st);
-    h2d(d_sc.ensure(sc.size()), sc.data(), sc.size(), s.st);
+    ns2 = source_splits(tasks, pr.M + 1);
     pbary.ensure((size_t)ns2 * 6 * ntar);
-    dim3 g2((unsigned)tasks.size(), ns2);
-    k_bary_sum<2><<<g2, NEAR_NT, 0, s.st>>>(G, bd_all.p, d_tasks.p, txy.p, d_sc.p, (int)ntar, pbary.p);
+    k_bary_sum<<<dim3(tasks, ns2), NEAR_NT, 0, s.st>>>(G, bd_all.p, txy.p, 0, (int)ntar, pbary.p);
     EB_LAUNCH_CHECK();
-    EB_CK(cudaStreamSynchronize(s.st));
   }
-  k_qoi_final<<<nblk(ntar, 128), 128, 0, s.st>>>(G, d_den, (int)ntar, txy.p, ptrap.p, s.nsplit, pbary.p, ns2, ibary,
-                                                  d_u, d_v, d_p, d_w);
+  k_qoi_final<<<tasks, 256, 0, s.st>>>(G, d_den, (int)ntar, txy.p, ptrap.p, ns1, pbary.p, ns2, ibary, d_u, d_v, d_p,
+                                       d_w);
   EB_LAUNCH_CHECK();
 }
 
