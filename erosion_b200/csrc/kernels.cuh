@@ -405,7 +405,7 @@ __device__ __forceinline__ double rcp_variant(double r2) {
 }
 
 // One CTA's share of the FP64 far field: targets of block bx, tiles of split
-// 'split'.  Shared by k_far64 and the ensemble kernel k_far64_batch.
+// 'split'.
 template <bool MASK, int NT, int TPT, int RCP>
 __device__ __forceinline__ void far64_cta(const GeoDev& G, const double4* __restrict__ sq,
                                           const int4* __restrict__ tiles, const int* __restrict__ split_ptr,
@@ -534,7 +534,7 @@ __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float t) {
 constexpr int F32_CHUNK = EROSION_F32_CHUNK;
 
 // One CTA's share of the FP32 far field (targets of block bx, tiles of split
-// 'split'); shared by k_far32 and the ensemble kernel k_far32_batch.
+// 'split').
 template <bool MASK, int NT, int TPT, int U>
 __device__ __forceinline__ void far32_cta(int N, int nout, int n, const float4* __restrict__ src,
                                           const float2* __restrict__ tgt, const double2* __restrict__ anchor,
@@ -647,84 +647,6 @@ k_far32(int N, int nout, int n, const float4* __restrict__ src, const float2* __
   __shared__ float2 s_q2[F32_TS];
   far32_cta<MASK, NT, TPT, U>(N, nout, n, src, tgt, anchor, tile_c, sq32, tiles, split_ptr, mask, mw, partial,
                            blockIdx.x, blockIdx.y, s_pos, s_q1, s_q2);
-}
-
-// ---------------------------------------------------------------------------
-// Ensemble far field: ONE persistent launch covers the far field of every
-// geometry of an ensemble.  Work item = (geometry, target block, tile split);
-// items are numbered job by job (FarJob*.item0) and CTAs stride over them.
-struct FarJob64 {
-  GeoDev G;
-  const double4* sq;
-  const int4* tiles;
-  const int* split_ptr;
-  const unsigned* mask;   // nullptr: no near masking
-  int mw;
-  double2* partial;
-  int nbx, nsplit;
-  long long item0;
-};
-
-struct FarJob32 {
-  int N, nout, n;
-  const float4* src;
-  const float2* tgt;
-  const double2* anchor;
-  const double2* tile_c;
-  const float4* sq32;
-  const int4* tiles;
-  const int* split_ptr;
-  const unsigned* mask;
-  int mw;
-  double2* partial;
-  int nbx, nsplit;
-  long long item0;
-};
-
-template <class Job>
-__device__ __forceinline__ int find_job(const Job* __restrict__ jobs, int njobs, long long item) {
-  int lo = 0, hi = njobs - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].item0 <= item) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-template <int NT, int TPT, int RCP>
-__global__ void __launch_bounds__(NT, 512 / NT)
-k_far64_batch(const FarJob64* __restrict__ jobs, int njobs, long long nitems) {
-  __shared__ double4 sg[FAR_TS];
-  __shared__ double sw[FAR_TS];
-  for (long long item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const FarJob64 J = jobs[find_job(jobs, njobs, item)];
-    const int local = (int)(item - J.item0);
-    const int bx = local % J.nbx, q = local / J.nbx;
-    if (J.mask) far64_cta<true, NT, TPT, RCP>(J.G, J.sq, J.tiles, J.split_ptr, J.mask, J.mw, J.partial, bx, q, sg, sw);
-    else far64_cta<false, NT, TPT, RCP>(J.G, J.sq, J.tiles, J.split_ptr, nullptr, 0, J.partial, bx, q, sg, sw);
-    __syncthreads();
-  }
-}
-
-template <int NT, int TPT, int U, int MINB>
-__global__ void __launch_bounds__(NT, MINB)
-k_far32_batch(const FarJob32* __restrict__ jobs, int njobs, long long nitems) {
-  __shared__ float4 s_pos[F32_TS];
-  __shared__ float4 s_q1[F32_TS];
-  __shared__ float2 s_q2[F32_TS];
-  for (long long item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const FarJob32 J = jobs[find_job(jobs, njobs, item)];
-    const int local = (int)(item - J.item0);
-    const int bx = local % J.nbx, q = local / J.nbx;
-    if (J.mask)
-      far32_cta<true, NT, TPT, U>(J.N, J.nout, J.n, J.src, J.tgt, J.anchor, J.tile_c, J.sq32, J.tiles, J.split_ptr,
-                               J.mask, J.mw, J.partial, bx, q, s_pos, s_q1, s_q2);
-    else
-      far32_cta<false, NT, TPT, U>(J.N, J.nout, J.n, J.src, J.tgt, J.anchor, J.tile_c, J.sq32, J.tiles, J.split_ptr,
-                                nullptr, 0, J.partial, bx, q, s_pos, s_q1, s_q2);
-    __syncthreads();
-  }
 }
 
 // Launch shapes the autotuner chooses from (threads per CTA, targets per
@@ -2171,28 +2093,6 @@ __global__ void k_copy(const double* __restrict__ a, double* __restrict__ out, l
 // Arnoldi steps whose column count lives in device memory (*kp), so that one
 // captured CUDA graph serves every iteration of a GMRES cycle.
 
-// out = V[:, *kp + off]
-__global__ void k_col_get(const double* __restrict__ V, long long ldv, const int* __restrict__ kp, int off,
-                          double* __restrict__ out, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = V[(long long)(*kp + off) * ldv + i];
-}
-
-// V[:, *kp + off] = in (times *scale when scale is given)
-__global__ void k_col_put(double* __restrict__ V, long long ldv, const int* __restrict__ kp, int off,
-                          const double* __restrict__ in, const double* __restrict__ scale, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) V[(long long)(*kp + off) * ldv + i] = scale ? in[i] * *scale : in[i];
-}
-
-// part[j][b] = partial dot of columns j < *kp with w over the rows of block b
-__global__ void __launch_bounds__(256)
-k_dot_part_dk(const double* __restrict__ V, long long ldv, const int* __restrict__ kp, const double* __restrict__ w,
-              long long n, int R, double* __restrict__ part) {
-  extern __shared__ double swv[];
-  dot_cols_cta(V, ldv, *kp, w, n, R, part, swv);
-}
-
 // h[j] = sum_b part[j][b] for j < *kp (+ koff); one warp per j, grid-stride.
 __global__ void k_dot_reduce_dk(const double* __restrict__ part, int nb, const int* __restrict__ kp, int koff,
                                 double* __restrict__ h) {
@@ -2238,53 +2138,6 @@ k_vh_dk(const double* __restrict__ V, long long ldv, const int* __restrict__ kp,
     }
   }
   if (i < n) w[i] += sign * acc;
-}
-
-// The Givens step of one Arnoldi iteration on the device (DHEQR,
-// gmres_routines.f:1148, last column).  Column k = *kp of the Hessenberg
-// matrix is h1[0..k-1] + h2[0..k-1] (the two Gram-Schmidt passes) with
-// subdiagonal sqrt(*hn); the previous rotations (cs[2i], cs[2i+1]) are applied,
-// a new rotation zeroes the subdiagonal, the column is stored packed in R
-// (column k-1 at offset (k-1)k/2), prod <- prod * s and rho = |prod r0|.
-// scale <- 1/sqrt(hn) for the next basis vector.  st: 0 running, 2 breakdown
-// (zero diagonal), 3 non-finite.  One thread.
-__global__ void k_givens_step(const int* __restrict__ kp, const double* __restrict__ h1,
-                              const double* __restrict__ h2, const double* __restrict__ hn, double* __restrict__ cs,
-                              double* __restrict__ R, double* __restrict__ prod, const double* __restrict__ r0,
-                              double* __restrict__ rho, double* __restrict__ scale, int* __restrict__ st) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int k = *kp;
-  double* col = R + (size_t)(k - 1) * k / 2;
-  const double snormw = sqrt(*hn);
-  bool finite = isfinite(snormw);
-  for (int i = 0; i < k; ++i) {
-    col[i] = h1[i] + h2[i];
-    finite = finite && isfinite(col[i]);
-  }
-  if (!finite) { *st = 3; return; }
-  for (int kk = 0; kk < k - 1; ++kk) {
-    const double c = cs[2 * kk], sn = cs[2 * kk + 1];
-    const double t1 = col[kk], t2 = col[kk + 1];
-    col[kk] = c * t1 - sn * t2;
-    col[kk + 1] = sn * t1 + c * t2;
-  }
-  const double t1 = col[k - 1], t2 = snormw;
-  double c, sn;
-  if (t2 == 0.0) { c = 1.0; sn = 0.0; }
-  else if (fabs(t2) >= fabs(t1)) { const double t = t1 / t2; sn = -1.0 / sqrt(1.0 + t * t); c = -sn * t; }
-  else { const double t = t2 / t1; c = 1.0 / sqrt(1.0 + t * t); sn = -c * t; }
-  cs[2 * (k - 1)] = c;
-  cs[2 * (k - 1) + 1] = sn;
-  col[k - 1] = c * t1 - sn * t2;
-  if (col[k - 1] == 0.0) { *st = 2; return; }
-  *prod *= sn;
-  *rho = fabs(*prod * *r0);
-  *scale = snormw > 0.0 ? 1.0 / snormw : 0.0;
-  *st = 0;
-}
-
-__global__ void k_inc(int* kp) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *kp += 1;
 }
 
 }  // namespace

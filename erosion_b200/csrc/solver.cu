@@ -16,6 +16,7 @@ State& state() {
 }
 
 std::atomic<long long> g_launches{0};
+thread_local long long t_launches = 0;
 
 thread_local int t_status = EROSION_OK;
 thread_local std::string t_err;
@@ -28,12 +29,20 @@ static int g_num_sms = 148;
 int eb_num_sms() { return g_num_sms; }
 
 void allow_max_dynamic_smem(const void* fn) {
+  // once per kernel and device: the driver call takes milliseconds while other
+  // threads launch
+  static std::mutex mu;
+  static std::vector<std::pair<int, const void*>> done;
+  std::lock_guard<std::mutex> lk(mu);
   int dev = 0, optin = 0;
   EB_CK(cudaGetDevice(&dev));
+  for (const auto& d : done)
+    if (d.first == dev && d.second == fn) return;
   EB_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   cudaFuncAttributes fa;
   EB_CK(cudaFuncGetAttributes(&fa, fn));   // the cap excludes the kernel's static shared memory
   EB_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+  done.emplace_back(dev, fn);
 }
 
 void ensure_init(State& s) {
@@ -46,16 +55,33 @@ void ensure_init(State& s) {
   cudaDeviceProp prop;
   EB_CK(cudaGetDeviceProperties(&prop, s.device));
   g_num_sms = prop.multiProcessorCount;
+  init_state(s, s.device);
+}
+
+void init_state(State& s, int device) {
+  if (s.init) return;
+  s.device = device;
   EB_CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
-  EB_CK(cudaEventCreate(&s.e0));
-  EB_CK(cudaEventCreate(&s.e1));
-  EB_CK(cudaEventCreate(&s.ef0));
-  EB_CK(cudaEventCreate(&s.ef1));
-  EB_CK(cudaEventCreate(&s.ew0));
-  EB_CK(cudaEventCreate(&s.ew1));
-  EB_CK(cudaEventCreate(&s.et0));
-  EB_CK(cudaEventCreate(&s.et1));
+  for (auto* e : {&s.e0, &s.e1, &s.ef0, &s.ef1, &s.ew0, &s.ew1, &s.et0, &s.et1}) EB_CK(cudaEventCreate(e));
   s.init = true;
+}
+
+void destroy_state(State& s) {
+  drop_steps(s);
+  for (auto* e : {&s.e0, &s.e1, &s.ef0, &s.ef1, &s.ew0, &s.ew1, &s.et0, &s.et1, &s.ev_fork[0], &s.ev_fork[1],
+                  &s.ev_join[0], &s.ev_join[1], &s.ev_join[2], &s.ev_step[0], &s.ev_step[1]}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
+  for (auto* t : {&s.br[0], &s.br[1], &s.br[2], &s.st}) {
+    if (*t) cudaStreamDestroy(*t);
+    *t = nullptr;
+  }
+  if (s.k_host) cudaFreeHost(s.k_host);
+  if (s.h_pinned) cudaFreeHost(s.h_pinned);
+  s.k_host = s.h_pinned = nullptr;
+  s.h_pinned_cap = 0;
+  s.init = false;
 }
 
 // The circulant matrix of fourierDiff (stokesSolver.f:348-388) for even n:
@@ -559,7 +585,7 @@ void setup_problem(State& s, const Problem& in, const double* d_xx, const double
   s.pr = pr;
   s.geo_valid = false;
   s.near.rules = false;
-  drop_steps(s);   // captured for the previous problem
+  stale_steps(s);   // captured for the previous problem
   cudaStream_t st = s.st;
   if (s.dker_wall_n != pr.nout) {
     auto d = spectral_kernel(pr.nout);
@@ -1075,7 +1101,7 @@ static double* pinned(State& s, size_t n) {
 
 // Column bound of the graph that serves step ll (ll basis vectors).
 static int step_bound(int ll) {
-  int b = 64;
+  int b = 256;
   while (b < ll) b *= 2;
   return std::min(b, CGS_MAX);
 }
@@ -1110,7 +1136,7 @@ static void step_buffers(State& s, long long N, long long cols) {
   s.pc_z.ensure(N);
   s.part.ensure((size_t)std::min<long long>(cols, CGS_MAX) * nb);
   const double* after[] = {s.k_cur.p, s.k_w.p, s.k_h1.p, s.k_h2.p, s.k_np.p, s.part.p, s.pc_z.p};
-  if (!std::equal(before, before + 7, after)) drop_steps(s);
+  if (!std::equal(before, before + 7, after)) stale_steps(s);
 }
 
 // Launches one step for up to `bound` columns: the (preconditioned) operator
@@ -1171,22 +1197,24 @@ void drop_steps(State& s) {
   s.steps.clear();
 }
 
+void stale_steps(State& s) {
+  for (auto& g : s.steps) g.stale = true;
+}
+
 // The same step as a graph, its independent launches on branches, captured on
 // first use.
 static void replay_step(State& s, long long N, long long ldv, int bound, int prec, double* host) {
-  for (size_t i = 0; i < s.steps.size(); ++i)
-    if (s.steps[i].V != s.V.p || s.steps[i].part != s.part.p || (s.pc_active && s.steps[i].Z != s.Z.p)) {   // moved
-      EB_CK(cudaStreamSynchronize(s.st));
-      drop_steps(s);
-      break;
-    }
-  for (auto& g : s.steps)
-    if (g.bound == bound && g.prec == prec) {
-      EB_CK(cudaGraphLaunch(g.exec, s.st));
-      g_launches += g.launches;
-      return;
-    }
-  const long long l0 = g_launches;
+  State::StepGraph* g = nullptr;
+  for (auto& q : s.steps)
+    if (q.bound == bound && q.prec == prec) g = &q;
+  if (g && (g->V != s.V.p || g->part != s.part.p || (s.pc_active && g->Z != s.Z.p))) g->stale = true;   // moved
+  if (g && !g->stale) {
+    EB_CK(cudaGraphLaunch(g->exec, s.st));
+    g_launches += g->launches;
+    t_launches += g->launches;
+    return;
+  }
+  const long long l0 = t_launches;
   EB_CK(cudaStreamBeginCapture(s.st, cudaStreamCaptureModeRelaxed));
   cudaGraph_t graph = nullptr;
   s.forked = true;
@@ -1200,18 +1228,35 @@ static void replay_step(State& s, long long N, long long ldv, int bound, int pre
   }
   s.forked = false;
   EB_CK(cudaStreamEndCapture(s.st, &graph));
-  State::StepGraph g;
-  g.launches = g_launches - l0;
-  g.bound = bound;
-  g.prec = prec;
-  g.V = s.V.p;
-  g.Z = s.Z.p;
-  g.part = s.part.p;
-  const cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
+  // the graph of the previous set-up usually has the same nodes: updating it is
+  // several times cheaper than instantiating another and destroying it
+  if (g) {
+    cudaGraphExecUpdateResultInfo info;
+    if (cudaGraphExecUpdate(g->exec, graph, &info) != cudaSuccess) {
+      (void)cudaGetLastError();
+      cudaGraphExecDestroy(g->exec);
+      g->exec = nullptr;
+    }
+  } else {
+    s.steps.emplace_back();
+    g = &s.steps.back();
+    g->bound = bound;
+    g->prec = prec;
+  }
+  cudaError_t err = cudaSuccess;
+  if (!g->exec) err = cudaGraphInstantiate(&g->exec, graph, 0);
   cudaGraphDestroy(graph);
-  EB_CK(err);
-  s.steps.push_back(g);
-  EB_CK(cudaGraphLaunch(g.exec, s.st));
+  if (err != cudaSuccess) {
+    s.steps.erase(s.steps.begin() + (g - s.steps.data()));
+    EB_CK(err);
+  }
+  g->launches = t_launches - l0;
+  g->V = s.V.p;
+  g->Z = s.Z.p;
+  g->part = s.part.p;
+  g->stale = false;
+  s.captures++;
+  EB_CK(cudaGraphLaunch(g->exec, s.st));
 }
 
 // One GMRES run with the semantics of SLATEC DGMRES as solveBIE calls it
@@ -1231,7 +1276,9 @@ static int gmres_cycle(State& s, double* d_r, double* d_x, long long maxl_in, do
   if (MAXL > N) MAXL = N;
   *iters = 0;
   cudaStream_t st = s.st;
-  long long cap0 = std::min<long long>(MAXL + 1, 64);
+  // first basis: 64 columns, or what 32 MB hold, up to 512 (a growth copies the
+  // basis and its cudaFree waits for the whole device)
+  const long long cap0 = std::min<long long>(MAXL + 1, std::max<long long>(64, std::min<long long>(512, (4LL << 20) / ldv)));
   if ((long long)(s.V.cap / ldv) < cap0) s.V.ensure((size_t)cap0 * ldv);
   s.vcap = (long long)(s.V.cap / ldv);
   s.zcap = (long long)(s.Z.cap / ldv);
@@ -1255,7 +1302,7 @@ static int gmres_cycle(State& s, double* d_r, double* d_x, long long maxl_in, do
       s.vcap = nc;
     }
     if (s.pc_active && cols - 1 > s.zcap) {
-      const long long nc = std::min<long long>(MAXL, std::max<long long>(2 * s.zcap, std::max<long long>(cols - 1, 64)));
+      const long long nc = std::min<long long>(MAXL, std::max<long long>(2 * s.zcap, std::max<long long>(cols - 1, cap0)));
       s.Z.grow_keep((size_t)nc * ldv, (size_t)s.zcap * ldv, st);
       s.zcap = nc;
     }

@@ -16,6 +16,7 @@
 namespace eb {
 
 extern std::atomic<long long> g_launches;
+extern thread_local long long t_launches;   // those of the calling thread
 
 struct Error : std::runtime_error {
   int code;
@@ -32,6 +33,7 @@ struct Error : std::runtime_error {
 #define EB_LAUNCH_CHECK()  \
   do {                     \
     ++::eb::g_launches;    \
+    ++::eb::t_launches;    \
     EB_CK(cudaGetLastError()); \
   } while (0)
 
@@ -213,9 +215,11 @@ struct State {
     cudaGraphExec_t exec = nullptr;
     long long launches = 0;
     int bound = 0, prec = 0;
+    bool stale = false;     // of an earlier set-up: to be updated before its next use
     const double *V = nullptr, *Z = nullptr, *part = nullptr;
   };
-  std::vector<StepGraph> steps;   // of the current set-up
+  std::vector<StepGraph> steps;
+  long long captures = 0;         // graphs captured so far
   long long timed_far = 0, timed_farw = 0, timed_far32 = 0, timed_far64f = 0;   // launches with event times
   long long vcap = 0;   // vectors held by V
   long long zcap = 0;   // vectors held by Z (preconditioned basis, flexible GMRES)
@@ -249,6 +253,10 @@ void allow_max_dynamic_smem(const void* fn);
 // takes no lock and one thread's call never overwrites another's outcome.
 void set_status(int code, const std::string& msg);
 void ensure_init(State& s);
+// Streams and events of a state on the current device (no-op when it has them), and
+// their end; the buffers are release_state_buffers'.
+void init_state(State& s, int device);
+void destroy_state(State& s);
 
 // Geometry + near lists + far-field tiles for (xx, yy) already on the device.
 void setup_problem(State& s, const Problem& pr, const double* d_xx, const double* d_yy);
@@ -262,8 +270,10 @@ void apply_operator(State& s, const double* d_den, double* d_vel, int prec = 0);
 void operator_prep(State& s, const double* d_den, double* d_vel);
 int far_slots(const State& s, int prec);
 void operator_post(State& s, const double* d_den, double* d_vel, int nsplit, int* kp = nullptr);
-// Destroys the captured Arnoldi steps (a set-up or a buffer they refer to changed).
+// The captured Arnoldi steps: their end, and their invalidation (a set-up or a buffer
+// they refer to changed).
 void drop_steps(State& s);
+void stale_steps(State& s);
 void build_rhs(State& s, double* d_rhs);
 // GMRES (SLATEC DGMRES semantics, CGS2 Arnoldi); returns EROSION_* status.
 int gmres_solve(State& s, const double* d_b, double* d_x, bool x0_zero, long long maxl, double tol,

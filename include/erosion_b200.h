@@ -164,7 +164,9 @@ typedef struct {
   double est_residual;      /* GMRES estimate rho/||b|| at exit                    */
   double true_residual;     /* ||b - A x||/||b|| (FP64 operator) when requested    */
   double ms_total;          /* device time of the solve                            */
-  double ms_far;            /* device time inside the FP64 far-field kernel        */
+  double ms_far;            /* device time inside the FP64 far-field kernel (here and
+                               below: launches inside replayed graphs are counted
+                               at the mean of the timed ones)                      */
   int64_t far_launches;     /* FP64 far-field kernel launches                      */
   int64_t near_pairs;       /* (target node, source curve) barycentric pairs       */
   double ms_far32;          /* device time inside the FP32 far-field kernel        */
@@ -215,29 +217,27 @@ void erosion_get_solve_stats(erosion_solve_stats* s);
  * another (2*npts*nbods + 3*nbods + 2*nouter each; initial guess in, solution
  * out), nits[g] receives each geometry's GMRES iterations.  Every geometry is
  * solved with the method erosion_solve applies for the same parameters (one
- * erosion_params for all); the geometries advance together, one Arnoldi
- * iteration per round: the far field of all of them is one persistent launch
- * per precision and the rest of a round replays one captured CUDA graph.
+ * erosion_params for all), on streams of its own, from a pool of up to 16 host
+ * threads; the GPU works on as many geometries at a time.
  * Returns EROSION_OK or the first non-OK status of a geometry. */
 int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* npts, const int64_t* nbods,
                         const int64_t* nouter, const double* xx, const double* yy, double* density, int64_t* nits);
 
 typedef struct {
   int64_t geometries;
-  int64_t rounds;            /* lockstep Arnoldi rounds (graph replays)            */
+  int64_t rounds;            /* GMRES iterations of the geometry that took most    */
   int64_t iterations;        /* GMRES iterations summed over the geometries        */
-  int64_t graph_captures;    /* round graphs captured (pattern or buffer changes)   */
+  int64_t graph_captures;    /* Arnoldi steps captured (or updated) as graphs      */
   double ms_total;           /* device time of the whole ensemble solve            */
-  double pairs64_per_round;  /* FP64 far-field pairs of the last captured round     */
-  double pairs32_per_round;  /* FP32 far-field pairs of the last captured round     */
-  double pairs64_total;      /* FP64 far-field pairs over all rounds               */
-  double pairs32_total;      /* FP32 far-field pairs over all rounds               */
+  double pairs64_per_round;  /* FP64 far-field pairs of one iteration of each geometry */
+  double pairs32_per_round;  /* FP32 far-field pairs of one iteration of each geometry */
+  double pairs64_total;      /* FP64 far-field pairs over all iterations           */
+  double pairs32_total;      /* FP32 far-field pairs over all iterations           */
   double max_true_residual;  /* largest final residual over the geometries         */
-  int64_t shape64, shape32;  /* ensemble launch shapes (indices as erosion_get_far_shapes) */
-  float tune_ms[8];          /* timed candidates: [0..3] FP64, [4..7] FP32 (0 = not timed) */
+  int64_t shape64, shape32;  /* 0: the geometries are summed by clusters           */
+  float tune_ms[8];          /* 0                                                  */
   double setup_host_ms;      /* host wall time of the members' set-ups (geometry,
-                                near lists, tiles, preconditioners, initial residuals),
-                                run on a pool of host threads                      */
+                                near lists, preconditioners) on the host threads   */
 } erosion_batch_stats;
 
 void erosion_get_batch_stats(erosion_batch_stats* s);
@@ -446,7 +446,7 @@ double erosion_peak_tflops(int32_t precision);
  * times every candidate on the geometry at hand the first time a problem of
  * that size is set up (problems above 2e8 node pairs) and keeps the fastest.
  * The shapes are those of the direct sum over every pair, which runs when one
- * is forced, in ensembles and for more than 4096 clusters (wall arcs of 32
+ * is forced and for more than 4096 clusters (wall arcs of 32
  * nodes and bodies of up to 256); otherwise the far field is summed by clusters.
  * erosion_set_far_shape(kind, shape) forces candidate 'shape' (kind 0 = the
  * accurate FP64 kernel, 1 = the FP32 kernel, 2 = the fast FP64 kernel of the
