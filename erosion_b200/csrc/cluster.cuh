@@ -46,6 +46,14 @@ constexpr double CL_THETA = 1.0 / 3.0;   // separation
 constexpr int CL_MP = 3 * CL_P;          // multipole record of a cluster: a_k, x_k, k a_(k-1) / R
 constexpr int CL_MAX_TILES = 4096;       // above this the lists (tiles^2 entries) are not built
 
+// Nodes from which the separated clusters act through expansions; below, every
+// cluster pair is summed directly.  Near lists, expansions and assembly with
+// and without them, FP64 (mixed): 2304 nodes 24.0 and 23.0 us (28.2 and 21.7),
+// 3072 nodes 29.9 and 34.8 us (32.7 and 28.8), 3584 nodes 29.0 and 47.2 us
+// (32.1 and 33.0), 8704 nodes 44.7 and 160.7 us (43.7 and 109.8); the
+// expansions are two launches more.
+constexpr int kExpandNodes = 3200;
+
 struct BinomTable {
   double c[CL_P][CL_P];   // c[l][k] = C(k + l, l)
   constexpr BinomTable() : c{} {

@@ -330,8 +330,6 @@ __global__ void __launch_bounds__(256) k_prep(GeoDev G, const double* __restrict
 // crosses a curve, so the mask test is one bit per tile and target.  blockIdx.y
 // selects a contiguous range of tiles (split-K); partial sums are reduced in a
 // fixed order by k_combine.
-__device__ __forceinline__ double rcp_or_zero(double r2) { return r2 > 0.0 ? __drcp_rn(r2) : 0.0; }
-
 // 1/r2 for r2 > 0 by Newton-Raphson: the FP32 hardware reciprocal estimate
 // (relative error ~2^-23), refined twice by y <- y + y (1 - r2 y) in FP64
 // (quadratic convergence: ~2^-46, then below FP64 rounding).  Not correctly
@@ -359,7 +357,7 @@ __device__ __forceinline__ double rcp_newton(double r2) {
 // FP64 with e = 1 - r2 y: NSTEP = 1 by the Newton-Raphson step y + y e, which
 // squares the relative error; NSTEP = 2 by y + y (e + e^2), which cubes it, below
 // FP64 rounding, in three operations where two Newton-Raphson steps take four.
-// r2 > 0 in the double's normal range (0 for r2 = 0, as rcp_or_zero).
+// r2 > 0 in the double's normal range (0 for r2 = 0).
 template <int NSTEP>
 __device__ __forceinline__ double rcp_newton64(double r2) {
   double y;
@@ -389,16 +387,14 @@ __device__ __forceinline__ double rcp_newton1(double r2) {
   return r2 > 0.0 ? y : 0.0;
 }
 
-// 1/r2 by variant: 0 correctly rounded division, 1 FP32 estimate + 2 Newton
-// steps, 3 FP64 estimate + 2 Newton steps (both at FP64 rounding: the
-// accurate FP64 operator); 2 FP32 estimate + 1 step, 4 FP64 estimate + 1 step
+// 1/r2 by variant: 1 FP32 estimate + 2 Newton steps, 3 FP64 estimate + a cubic
+// step (both at FP64 rounding: the accurate FP64 operator); 2 FP32 estimate + 1 step, 4 FP64 estimate + 1 step
 // (relative error ~1e-14 and ~1e-12 per pair: the fast FP64 operator that the
 // mixed-precision solve applies while its residual is still large, where an
 // operator error far above FP64 rounding is harmless).
 template <int RCP>
 __device__ __forceinline__ double rcp_variant(double r2) {
-  if constexpr (RCP == 0) return rcp_or_zero(r2);
-  else if constexpr (RCP == 1) return rcp_newton(r2);
+  if constexpr (RCP == 1) return rcp_newton(r2);
   else if constexpr (RCP == 2) return rcp_newton1(r2);
   else if constexpr (RCP == 3) return rcp_newton64<2>(r2);
   else return rcp_newton64<1>(r2);

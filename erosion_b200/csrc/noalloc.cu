@@ -23,16 +23,17 @@
 // cudaGetSymbolAddress (host code cannot use the array's name as a device
 // pointer) and queries the SM count; make that first call before capturing
 // any stream.  The computation is the one erosion_matvec performs with
-// ibary = 0 and precision = 0 (geometry from spectral derivatives, far field
-// with the split-K partial sums, self-curve sums, jump, stokeslets/rotlets,
-// constraint rows and the rank-one wall term), by the same kernels.
+// ibary = 0 and precision = 0 (geometry from spectral derivatives, far field by
+// clusters, the bodies' self sums, jump, stokeslets/rotlets, constraint rows and
+// the rank-one wall term), by the same kernels.
 #include <mutex>
 
 #include "state.h"
-#include "kernels.cuh"
+#include "cluster.cuh"
 
 namespace {
 
+static_assert(WALL_TS == 32 && FAR_TS % 32 == 0, "items of 32 nodes");
 constexpr int NA_MAX_NODES = 32768;
 constexpr int NA_MAX_BODIES = 128;
 constexpr int NA_MAX_NPTS = 512;
@@ -40,16 +41,15 @@ constexpr int NA_MAX_NOUT = 4096;
 constexpr size_t NA_SCRATCH_BYTES = size_t(24) << 20;
 constexpr int NA_MAX_DEVICES = 64;
 
-// Per-layout tables the host-side operator builds on the CPU: tiles of the
-// far-field sum, their split-K ranges (same order and contents as build_tiles
-// in solver.cu) and the two circulant derivative
-// kernels d[m] = (1/2)(-1)^m cot(pi m/n) (fourierDiff, stokesSolver.f:348-388).
-__global__ void k_na_layout(int nout, int n, int M, int nsplit, int4* __restrict__ tiles,
-                            int* __restrict__ split_ptr, double* __restrict__ dker_w,
-                            double* __restrict__ dker_b) {
+// Per-layout tables the host-side operator builds on the CPU: tiles and target
+// items of the far-field sum (same order and contents as build_tiles in
+// solver.cu) and the two circulant derivative kernels d[m] = (1/2)(-1)^m
+// cot(pi m/n) (fourierDiff, stokesSolver.f:348-388).
+__global__ void k_na_layout(int nout, int n, int M, int4* __restrict__ tiles, int2* __restrict__ items,
+                            double* __restrict__ dker_w, double* __restrict__ dker_b) {
   const int nwt = (nout + WALL_TS - 1) / WALL_TS;
-  const int tpb = M > 0 ? (n + FAR_TS - 1) / FAR_TS : 0;
-  const int ntile = nwt + M * tpb;
+  const int tpb = M > 0 ? (n + FAR_TS - 1) / FAR_TS : 0, ipb = M > 0 ? (n + 31) / 32 : 0;
+  const int ntile = nwt + M * tpb, nitem = nwt + M * ipb;
   for (int t = threadIdx.x; t < ntile; t += blockDim.x) {
     if (t < nwt) {
       const int o = t * WALL_TS;
@@ -59,7 +59,14 @@ __global__ void k_na_layout(int nout, int n, int M, int nsplit, int4* __restrict
       tiles[t] = make_int4(nout + b * n + o, min(FAR_TS, n - o), 1 + b, 0);
     }
   }
-  for (int q = threadIdx.x; q <= nsplit; q += blockDim.x) split_ptr[q] = (int)((long long)q * ntile / nsplit);
+  for (int t = threadIdx.x; t < nitem; t += blockDim.x) {
+    if (t < nwt) {   // a wall tile is one item
+      items[t] = make_int2(t, 0);
+    } else {
+      const int r = t - nwt, b = r / ipb, o = (r % ipb) * 32;
+      items[t] = make_int2(nwt + b * tpb + o / FAR_TS, o % FAR_TS);
+    }
+  }
   for (int m = threadIdx.x; m < nout + n; m += blockDim.x) {
     const int len = m < nout ? nout : n, k = m < nout ? m : m - nout;
     double d = 0.0;
@@ -190,22 +197,30 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     float4* sq32 = cv.take<float4>(N);
     double* sigdotn = cv.take<double>(nblk(nout, 256));
     int4* tiles = cv.take<int4>(ntile);
+    const int nitem = nwt + (M > 0 ? M * (int)nblk(n, 32) : 0);
+    int2* items = cv.take<int2>(nitem);
     double2* selfsum = cv.take<double2>(N);
-    // split-K of the far field as the host-side operator chooses it, capped by
-    // the room left in the array
-    const int TB = (int)nblk(N, FAR_NT * FAR_TPT);
-    int nsplit = std::max(1, std::min((int)std::ceil(8.0 * nd.sms / TB), ntile));
-    const size_t room = NA_SCRATCH_BYTES - cv.off - 2 * 256 - (size_t)(ntile + 1) * sizeof(int);
-    nsplit = std::max(1, std::min<int>(nsplit, (int)(room / ((size_t)N * sizeof(double2)))));
-    int* split_ptr = cv.take<int>(nsplit + 1);
-    double2* partial = cv.take<double2>((size_t)nsplit * N);
+    // the far field by clusters (cluster.cuh): at most 350 tiles here, 2 MB of lists
+    const size_t T2 = (size_t)ntile * ntile;
+    double2* ccen = cv.take<double2>(ntile);
+    double* crad = cv.take<double>(ntile);
+    int* near = cv.take<int>(T2);
+    int* far = cv.take<int>(T2);
+    double* lnd = cv.take<double>(T2);
+    int2* ncnt = cv.take<int2>(ntile);
+    int* fcls = cv.take<int>((size_t)ntile * (2 * CL_NCLS + 1));
+    const bool expand = N >= kExpandNodes, sing = expand && n <= FAR_TS;
+    double2* mp = cv.take<double2>(expand ? (size_t)ntile * CL_MP : 1);
+    double2* lam = cv.take<double2>(ntile);
+    const int parts = near_parts(nitem);
+    double2* partial = cv.take<double2>((size_t)(parts + 1) * N);
     if (cv.off > NA_SCRATCH_BYTES) throw Error(EROSION_BAD_INPUT, "erosion_matvec_noalloc: scratch layout");
 
     GeoDev G;
     G.n = n; G.M = M; G.nout = nout; G.N = N; G.ntot = ntot;
     G.xy = xy; G.nrm = nrm; G.sp = sp; G.cur = cur; G.w = w; G.dz = dz; G.cen = cen; G.rb = rb;
 
-    k_na_layout<<<1, 256, 0, st>>>(nout, n, M, nsplit, tiles, split_ptr, dker_w, dker_b);
+    k_na_layout<<<1, 1024, 0, st>>>(nout, n, M, tiles, items, dker_w, dker_b);
     EB_LAUNCH_CHECK();
     k_wall_nodes<<<nblk(nout, 256), 256, 0, st>>>(nout, p->wall_a, p->wall_b, p->wall_order, wx, wy);
     EB_LAUNCH_CHECK();
@@ -221,15 +236,28 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     }
     k_prep<<<M + nblk(nout, 256), 256, 0, st>>>(G, d_den, ws, sq64, sq32, d_vel, sigdotn, 0);
     EB_LAUNCH_CHECK();
-    k_far64<false, FAR_NT, FAR_TPT, 0><<<dim3((unsigned)TB, (unsigned)nsplit), FAR_NT, 0, st>>>(
-        G, sq64, tiles, split_ptr, nullptr, 0, partial);
+    k_cl_geom<<<nblk(ntile, 4), 128, 0, st>>>(G, ntile, tiles, ccen, crad);
     EB_LAUNCH_CHECK();
+    k_cl_lists<<<ntile, 256, 0, st>>>(G, ntile, 0, tiles, ccen, crad, nullptr, 0, 0, expand, near, far, lnd, ncnt, fcls,
+                                      nullptr);
+    EB_LAUNCH_CHECK();
+    ClView L;
+    L.T = ntile;
+    L.cen = ccen; L.rad = crad; L.near = near; L.far = far; L.ncnt = ncnt; L.fcls = fcls; L.lnd = lnd;
+    k_cl_near64<false, false><<<dim3(nitem, parts), 256, 0, st>>>(G, L, items, tiles, 0, sq64, nullptr, 0, 0, partial);
+    EB_LAUNCH_CHECK();
+    if (expand) {
+      k_cl_form<<<ntile, 256, 0, st>>>(G, 0, tiles, ccen, crad, sq64, sing ? d_den : nullptr, mp, lam);
+      EB_LAUNCH_CHECK();
+      k_cl_shift<CL_VELOCITY><<<ntile, 256, 0, st>>>(G, L, 0, tiles, mp, lam, partial + (size_t)parts * N);
+      EB_LAUNCH_CHECK();
+    }
     if (M > 0) {
       k_self64<<<M * nblk(n, 32), NEAR_NT, 0, st>>>(G, ws, selfsum);
       EB_LAUNCH_CHECK();
     }
-    k_combine<<<nblk((long long)N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, partial, nsplit, nullptr, nullptr, nullptr,
-                                                                  sigdotn, selfsum, ClView{}, nullptr, d_vel, nullptr);
+    k_combine<<<nblk((long long)N * COMBINE_G, 256), 256, 0, st>>>(G, d_den, partial, parts + expand, nullptr, nullptr, nullptr,
+                                                                  sigdotn, selfsum, sing ? L : ClView{}, tiles, d_vel, nullptr);
     EB_LAUNCH_CHECK();
     set_status(EROSION_OK, "");
     return EROSION_OK;

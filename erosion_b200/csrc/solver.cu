@@ -397,14 +397,6 @@ static void plan_far(State& s, bool tune) {
 // ---------------------------------------------------------------------------
 // The far field by clusters.
 
-// Nodes from which the separated clusters act through expansions; below, every
-// cluster pair is summed directly.  Near lists, expansions and assembly with
-// and without them, FP64 (mixed): 2304 nodes 24.0 and 23.0 us (28.2 and 21.7),
-// 3072 nodes 29.9 and 34.8 us (32.7 and 28.8), 3584 nodes 29.0 and 47.2 us
-// (32.1 and 33.0), 8704 nodes 44.7 and 160.7 us (43.7 and 109.8); the
-// expansions are two launches more.
-constexpr int kExpandNodes = 3200;
-
 // Parts of the near lists: about four CTAs per SM from items CTAs, at most 8.
 // 10 bodies x 128 nodes and 1024 wall nodes (72 items): 31.5 us in one part,
 // 20.4 us in 5, 17.1 us in 8, 16.0 us in 12 (and 3 us more in larger assemblies);

@@ -65,3 +65,20 @@ def test_stress_by_clusters_matches_all_barycentric(lib, M, n, nout):
     tau_b, E_b = stokes.shear_stress(g, den, stress_all_bary=1)
     assert rel(tau, tau_b) < 1e-10
     assert rel(E, E_b) < 1e-10
+
+
+@pytest.mark.parametrize("M,n,nout", [(2, 16, 16), (17, 128, 1020), (17, 128, 1026), (12, 258, 514), (128, 34, 770)])
+def test_noalloc_by_clusters(lib, M, n, nout):
+    """erosion_matvec_noalloc keeps its clusters, lists and expansions in its
+    fixed memory; both operators sum the same terms in another order."""
+    import ctypes
+    import torch
+    g = packing(M, n, nout)
+    den = np.random.default_rng(M).standard_normal(g.ntot)
+    x, y, d = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (g.xx, g.yy, den))
+    v = torch.empty_like(d)
+    p = stokes.params_for(g, ibary=0)
+    st = torch.cuda.current_stream()
+    assert lib.erosion_matvec_noalloc(ctypes.byref(p), g.n, g.M, g.nout, x.data_ptr(), y.data_ptr(), d.data_ptr(),
+                                      v.data_ptr(), st.cuda_stream) == 0
+    assert rel(v.cpu().numpy(), stokes.matvec(g, den, ibary=0)) < 1e-11
