@@ -1,6 +1,7 @@
 // Device kernels of the boundary operator, its geometry and the Krylov
 // solver.  Launch wrappers live in solver.cu.
 #pragma once
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 // Internal linkage: the translation units that include this header each get
@@ -41,6 +42,30 @@ __device__ __forceinline__ void near_reduce(double (&v)[NV], double (*red)[NR][3
     for (int w = 1; w < H; ++w) t += red[w][q][lane];
     v[q] = t;
   }
+  __syncthreads();
+}
+
+// v[q] (the same in every warp) summed over the CL CTAs of the cluster, in rank order;
+// all threads of all CTAs receive the sums.  red as near_reduce's.
+template <int CL, int NV, int NR>
+__device__ __forceinline__ void cluster_reduce(double (&v)[NV], double (*red)[NR][32]) {
+  static_assert(NV <= NR && NEAR_W >= 4, "reduction buffer");
+  const auto cl = cooperative_groups::this_cluster();
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (wid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[0][q][lane] = v[q];
+  }
+  cl.sync();
+  for (int q = wid; q < NV; q += NEAR_W) {
+    double t = 0.0;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) t += *cl.map_shared_rank(&red[0][q][lane], r);
+    red[1][q][lane] = t;
+  }
+  cl.sync();   // every CTA has read red[0]
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = red[1][q][lane];
   __syncthreads();
 }
 
@@ -1697,13 +1722,20 @@ __device__ double2 bary_coincident(const GeoDev& G, int start, int len, const do
 // target, 143 with the gradient.  Bound by the FP64 pipe with many targets and by
 // a warp's chain of sources with few: against one thread per target and
 // correctly rounded divisions, the near pairs of 3 bodies x 64 nodes take 10.5 us
-// (69.6), of 400 x 256 25.0 us (78.1), the gradients of the latter's shear stress
-// 461 us (2200), and of 3200 targets against 50 x 128 + 1024 nodes 329 us (577).
-template <int NDER>
+// (69.6), of 400 x 256 25.0 us (78.1), and of 3200 targets against 50 x 128 + 1024 nodes 329 us (577).
+// CL > 1 (the wall's curve only): the CTAs of a cluster of CL hold the same targets,
+// take a share of the nodes each and add their sums through distributed shared memory.
+template <int NDER, int CL = 1>
 __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* __restrict__ bdc,
                                             double2 zt, bool act) {
   const int start = curve_start(G, c), len = curve_len(G, c);
-  const bool ext = c != 0, whole = len <= NEAR_TK;
+  int lo = 0, hi = len;   // this CTA's share
+  if constexpr (CL > 1) {
+    const int rank = (int)cooperative_groups::this_cluster().block_rank();
+    lo = (int)((long long)len * rank / CL);
+    hi = (int)((long long)len * (rank + 1) / CL);
+  }
+  const bool ext = CL == 1 && c != 0, whole = hi - lo <= NEAR_TK;
   const int wid = threadIdx.x >> 5;
   constexpr int NF = NDER == 2 ? 5 : 3;   // fields: e, (v_1, v_2,) v_3, v_4
   double2 a = make_double2(0, 0);
@@ -1720,9 +1752,9 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
   double v1[2 + 2 * NF];   // the denominator, then the numerators
 #pragma unroll
   for (int q = 0; q < 2 + 2 * NF; ++q) v1[q] = 0.0;
-  for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
+  for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
     bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-    const int kt = min(NEAR_TK, len - k0);
+    const int kt = min(NEAR_TK, hi - k0);
     const int kb = kt * (wid + 1) / NEAR_W;
 #pragma unroll 2
     for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
@@ -1734,6 +1766,7 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
     }
   }
   near_reduce(v1, T.red);
+  if constexpr (CL > 1) cluster_reduce<CL>(v1, T.red);
   const double2 den = make_double2(v1[0], v1[1]);
   double2 u[NF];
   {
@@ -1748,9 +1781,9 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
 #pragma unroll
   for (int q = 0; q < 2 + 2 * ND; ++q) v2[q] = 0.0;
   bool coinc = false;
-  for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
+  for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
     if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-    const int kt = min(NEAR_TK, len - k0);
+    const int kt = min(NEAR_TK, hi - k0);
     const int kb = kt * (wid + 1) / NEAR_W;
 #pragma unroll 2
     for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
@@ -1788,6 +1821,7 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
     }
   }
   near_reduce(v2, T.red);
+  if constexpr (CL > 1) cluster_reduce<CL>(v2, T.red);
   double2 du[ND];
   double2 fac;
   if (ext) fac = cinv(cmul(csub(zt, a), make_double2(v2[0], v2[1])));
@@ -1801,9 +1835,9 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
   if constexpr (NDER == 2) {
     // Pass 3: second derivative of e.
     double v3[2] = {0.0, 0.0};
-    for (int k0 = 0; k0 < len; k0 += NEAR_TK) {
+    for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
       if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-      const int kt = min(NEAR_TK, len - k0);
+      const int kt = min(NEAR_TK, hi - k0);
       const int kb = kt * (wid + 1) / NEAR_W;
 #pragma unroll 2
       for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
@@ -1815,6 +1849,7 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
       }
     }
     near_reduce(v3, T.red);
+  if constexpr (CL > 1) cluster_reduce<CL>(v3, T.red);
     const double2 e = cscale(cmul(make_double2(v3[0], v3[1]), fac), 2.0);
     r.u1x = e.x - du[1].x + du[3].x;
     r.u1y = -e.y - du[2].x - du[3].y;

@@ -207,10 +207,24 @@ k_stress_wall_dist(GeoDev G, double* __restrict__ d2h) {
 }
 
 // Per body: radius of the smallest centroid-centred disc holding its nodes,
-// and its node spacing (mean speed x 2 pi / n).
+// and its node spacing (mean speed x 2 pi / n); per wall cluster (nwt of them, 8 to a
+// CTA behind the bodies') the distance from its centre within which its nodes' near
+// targets lie.  Clears the count of k_stress_wall's list.
 __global__ void __launch_bounds__(256)
-k_body_extent(GeoDev G, double2* __restrict__ ext) {
+k_body_extent(GeoDev G, const int4* __restrict__ tiles, const double* __restrict__ rad, int nwt,
+              double2* __restrict__ ext, int* __restrict__ wcount) {
   __shared__ double red[32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *wcount = 0;
+  if ((int)blockIdx.x >= G.M) {
+    const int t = 8 * ((int)blockIdx.x - G.M) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= nwt) return;
+    const int4 W = tiles[t];
+    double hm = lane < W.y ? G.sp[W.x + lane] * (EB_TWOPI / G.nout) : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) hm = fmax(hm, __shfl_xor_sync(0xffffffffu, hm, o));
+    if (lane == 0) ext[G.M + t] = make_double2(rad[t] + STRESS_NEAR_H * hm, 0.0);
+    return;
+  }
   const int b = blockIdx.x;
   const double2 c = G.cen[b];
   double r = 0.0;
@@ -229,15 +243,28 @@ k_body_extent(GeoDev G, double2* __restrict__ ext) {
   }
 }
 
+// Appends the lanes' nodes i with take set to the list of k_stress_wall (all lanes of a
+// warp call it).
+__device__ __forceinline__ void wall_list_add(bool take, int i, int* __restrict__ wcount, int* __restrict__ wlist) {
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  if (!m) return;
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(wcount, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (take) wlist[at + __popc(m & ((1u << lane) - 1u))] = i;
+}
+
 // Near mask of the stress: bit c of mask[i * mw + c/32] is set when body node
 // i lies within STRESS_NEAR_H node spacings of source curve c (its own body
 // excluded): for the wall from k_stress_wall_dist, for a body by its bounding
 // disc.
 __global__ void __launch_bounds__(256)
 k_stress_near_mask(GeoDev G, const double* __restrict__ wall_d2h, const double2* __restrict__ ext, int mw,
-                   unsigned* __restrict__ mask) {
+                   unsigned* __restrict__ mask, int* __restrict__ wcount, int* __restrict__ wlist) {
   const int nb = G.n * G.M;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  wall_list_add(i < nb && wall_d2h[i] <= STRESS_NEAR_H * STRESS_NEAR_H, i, wcount, wlist);
   if (i >= nb) return;
   const int own = 1 + i / G.n;
   const double2 p = G.xy[G.nout + i];
@@ -267,12 +294,14 @@ k_stress_near_mask(GeoDev G, const double* __restrict__ wall_d2h, const double2*
 // of a body cluster, one per lane).  A curve or wall cluster is tested node by
 // node only when its disc, widened by STRESS_NEAR_H of its spacings, reaches
 // the disc of the item's cluster; the warps share the words of the mask and the
-// wall's clusters.  7.1 us at 37 bodies x 200 nodes and 55 us at 400 x 256
-// (every node against every body and wall node: 35 and 334 us).
+// wall's clusters, whose reach k_body_extent has left behind the bodies' extents.
+// 4.8 us at 37 bodies x 200 nodes and 15 us at 400 x 256 (every warp measuring every
+// wall cluster's spacing: 7.1 and 55 us; every node against every body and wall node:
+// 35 and 334 us).
 __global__ void __launch_bounds__(256)
 k_stress_near_items(GeoDev G, const int2* __restrict__ items, const int4* __restrict__ tiles, int nwt,
                     const double2* __restrict__ cen, const double* __restrict__ rad, const double2* __restrict__ ext,
-                    int mw, unsigned* __restrict__ mask) {
+                    int mw, unsigned* __restrict__ mask, int* __restrict__ wcount, int* __restrict__ wlist) {
   __shared__ unsigned wall[8][32];
   const int2 it = items[blockIdx.x];
   const int4 T = tiles[it.x];
@@ -282,21 +311,24 @@ k_stress_near_items(GeoDev G, const int2* __restrict__ items, const int4* __rest
   const double rt = rad[it.x];
   const double hs = EB_TWOPI / G.nout;
   unsigned nearw = 0u;
-  for (int t = wid; t < nwt; t += 8) {
-    const int4 W = tiles[t];
-    const double hl = lane < W.y ? G.sp[W.x + lane] * hs : 0.0;
-    const double2 xl = G.xy[W.x + min(lane, W.y - 1)];
-    double hm = hl;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) hm = fmax(hm, __shfl_xor_sync(0xffffffffu, hm, o));
-    const double reach = rt + rad[t] + STRESS_NEAR_H * hm;
-    if (cabs2(csub(ct, cen[t])) > reach * reach * 1.0001) continue;
-    const double ih2 = 1.0 / (hl * hl);
-    for (int j = 0; j < W.y; ++j) {
-      const double wx = __shfl_sync(0xffffffffu, xl.x, j), wy = __shfl_sync(0xffffffffu, xl.y, j);
-      const double w2 = __shfl_sync(0xffffffffu, ih2, j);
-      const double dx = p.x - wx, dy = p.y - wy;
-      if ((dx * dx + dy * dy) * w2 <= STRESS_NEAR_H * STRESS_NEAR_H) nearw = 1u;
+  for (int t0 = 0; t0 < nwt; t0 += 256) {   // neighbouring clusters to different warps
+    const int tl = t0 + 8 * lane + wid;
+    bool cand = false;
+    if (tl < nwt) {
+      const double reach = rt + ext[G.M + tl].x;
+      cand = cabs2(csub(ct, cen[tl])) <= reach * reach * 1.0001;
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, cand); todo; todo &= todo - 1u) {
+      const int4 W = tiles[t0 + 8 * (__ffs(todo) - 1) + wid];
+      const double hl = lane < W.y ? G.sp[W.x + lane] * hs : 0.0;
+      const double2 xl = G.xy[W.x + min(lane, W.y - 1)];
+      const double ih2 = 1.0 / (hl * hl);
+      for (int j = 0; j < W.y; ++j) {
+        const double wx = __shfl_sync(0xffffffffu, xl.x, j), wy = __shfl_sync(0xffffffffu, xl.y, j);
+        const double w2 = __shfl_sync(0xffffffffu, ih2, j);
+        const double dx = p.x - wx, dy = p.y - wy;
+        if ((dx * dx + dy * dy) * w2 <= STRESS_NEAR_H * STRESS_NEAR_H) nearw = 1u;
+      }
     }
   }
   wall[wid][lane] = nearw;
@@ -327,15 +359,16 @@ k_stress_near_items(GeoDev G, const int2* __restrict__ items, const int4* __rest
 #pragma unroll
       for (int v = 0; v < 8; ++v) any |= wall[v][lane];
       bits |= any;
+      wall_list_add(any != 0u && it.y + lane < T.y, i, wcount, wlist);
     }
     if (it.y + lane < T.y) mask[(size_t)i * mw + w] = bits;
   }
 }
 
-// Barycentric Stokes DLP gradient of the near source curves only: CTA =
+// Barycentric Stokes DLP gradient of the near source bodies only: CTA =
 // NEAR_T nodes of one body, one per lane of every warp; the CTA visits,
-// in curve order, every curve that is near for at least one of its nodes, and a
-// node keeps the value only for the curves near to it.  With 32 nodes a CTA
+// in order, every body that is near for at least one of its nodes, and a
+// node keeps the value only for the bodies near to it.  With 32 nodes a CTA
 // visits fewer curves that only some of its nodes need than with 128, and the
 // warps share each curve's nodes (bary_eval).  out[q * nb + i], q as
 // k_bary_sum (one split).
@@ -351,7 +384,8 @@ k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const unsigned* __
   const double2 zt = G.xy[G.nout + tc];
   double a[6] = {0, 0, 0, 0, 0, 0};
   for (int w = 0; w < mw; ++w) {
-    const unsigned my = act ? mask[(size_t)tc * mw + w] : 0u;
+    unsigned my = act ? mask[(size_t)tc * mw + w] : 0u;
+    if (w == 0) my &= ~1u;   // the wall: k_stress_wall
     unsigned bits = __reduce_or_sync(0xffffffffu, my);   // the same in every warp
     while (bits) {
       const int q = __ffs(bits) - 1;
@@ -367,6 +401,33 @@ k_bary_sum_near(GeoDev G, const double2* __restrict__ bd_all, const unsigned* __
 #pragma unroll
     for (int q = 0; q < 6; ++q) out[(size_t)q * nb + t] = a[q];
   }
+}
+
+// Adds the wall's to out of k_bary_sum_near, for the nodes near to it (wlist, *wcount of
+// them in any order): a cluster of STRESS_CL CTAs takes 32 of them at a time, its CTAs
+// 1/STRESS_CL of the wall's nodes each.  Bound by the FP64 pipe.  Within
+// k_bary_sum_near a CTA near the wall had the whole wall in one chain, for a third of
+// its lanes on average, and the chip was half idle: both together took 463 us at 400 bodies
+// x 256 nodes and a wall of 4096 and 69 us at 37 x 200, this takes 235 and 16 us and the
+// bodies' 88 and 47 us.
+constexpr int STRESS_CL = 8;
+__global__ void __cluster_dims__(STRESS_CL, 1, 1) __launch_bounds__(NEAR_NT, 2)
+k_stress_wall(GeoDev G, const double2* __restrict__ bd_all, const int* __restrict__ wcount,
+              const int* __restrict__ wlist, double* __restrict__ out) {
+  __shared__ BaryTile T;
+  const int nb = G.n * G.M, cnt = *wcount;
+  for (int p0 = 32 * (blockIdx.x / STRESS_CL); p0 < cnt; p0 += 32 * (gridDim.x / STRESS_CL)) {
+    const int p = p0 + (threadIdx.x & 31);
+    const bool act = p < cnt;
+    const int t = wlist[act ? p : cnt - 1];
+    const DLPVal r = bary_eval<2, STRESS_CL>(T, G, 0, bd_all + bd_all_off(G, 0), G.xy[G.nout + t], act);
+    if (act && threadIdx.x < 32 && blockIdx.x % STRESS_CL == 0) {
+      const double v[6] = {r.ux, r.uy, r.u1x, r.u1y, r.u2x, r.u2y};
+#pragma unroll
+      for (int q = 0; q < 6; ++q) out[(size_t)q * nb + t] += v[q];
+    }
+  }
+  cooperative_groups::this_cluster().sync();   // no CTA's shared memory goes before the others have read it
 }
 
 // Per body: the speed-weighted rigid part of its density, sigma_rigid(x) =
@@ -891,8 +952,14 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     static DBuf<unsigned> smask;
     static DBuf<double> pnear;
     const int mw = (pr.M + 1 + 31) / 32;
-    k_body_extent<<<pr.M, 256, 0, s.st>>>(G, ext.ensure(pr.M));
+    static DBuf<int> wlist;   // the nodes near the wall, their count at [nb]
+    wlist.ensure((size_t)nb + 1);
+    const int nwt = s.cl_ready ? s.nwall_tiles : 0;
+    k_body_extent<<<pr.M + nblk(nwt, 8), 256, 0, s.st>>>(G, s.tiles.p, s.cl_rad.p, nwt, ext.ensure(pr.M + nwt),
+                                                         wlist.p + nb);
     EB_LAUNCH_CHECK();
+    const unsigned wall_ctas =
+        STRESS_CL * std::max(1u, std::min(nblk(nb, 32), (unsigned)(2 * eb_num_sms() / STRESS_CL)));
     smask.ensure((size_t)nb * mw);
     pnear.ensure(6LL * nb);
     bdval_all(s, d_den, bd_all);
@@ -901,9 +968,11 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       const int2* items = s.items32.p + s.n_items32_wall;
       const int nit = s.n_items32 - s.n_items32_wall;
       k_stress_near_items<<<nit, 256, 0, s.st>>>(G, items, s.tiles.p, s.nwall_tiles, s.cl_cen.p, s.cl_rad.p, ext.p, mw,
-                                                 smask.p);
+                                                 smask.p, wlist.p + nb, wlist.p);
       EB_LAUNCH_CHECK();
       k_bary_sum_near<<<near_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, smask.p, mw, pnear.p);
+      EB_LAUNCH_CHECK();
+      k_stress_wall<<<wall_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, wlist.p + nb, wlist.p, pnear.p);
       EB_LAUNCH_CHECK();
       // strengths without the bodies' rigid parts (see k_stress_rigid), the
       // near lists of this mask, their strain and that of the expansions
@@ -932,9 +1001,11 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     }
     k_stress_wall_dist<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.ensure(nb));
     EB_LAUNCH_CHECK();
-    k_stress_near_mask<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.p, ext.p, mw, smask.p);
+    k_stress_near_mask<<<nblk(nb, 256), 256, 0, s.st>>>(G, wall_d2h.p, ext.p, mw, smask.p, wlist.p + nb, wlist.p);
     EB_LAUNCH_CHECK();
     k_bary_sum_near<<<near_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, smask.p, mw, pnear.p);
+    EB_LAUNCH_CHECK();
+    k_stress_wall<<<wall_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, wlist.p + nb, wlist.p, pnear.p);
     EB_LAUNCH_CHECK();
     const int nsplit = s.nsplit;
     part.ensure((size_t)nsplit * 3 * nb);
