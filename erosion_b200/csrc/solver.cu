@@ -1107,14 +1107,17 @@ constexpr long long kRowPerThread = 75000;
 
 static size_t step_tile(int bound) { return (size_t)bound * 34 * sizeof(double); }
 
+void ensure_branches(State& s) {
+  if (s.br[0]) return;
+  for (auto& b : s.br) EB_CK(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
+  for (auto* e : {&s.ev_fork[0], &s.ev_fork[1], &s.ev_join[0], &s.ev_join[1], &s.ev_join[2], &s.ev_step[0],
+                  &s.ev_step[1]})
+    EB_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+}
+
 static void step_buffers(State& s, long long N, long long cols) {
-  if (!s.br[0]) {
-    for (auto& b : s.br) EB_CK(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
-    for (auto* e : {&s.ev_fork[0], &s.ev_fork[1], &s.ev_join[0], &s.ev_join[1], &s.ev_join[2], &s.ev_step[0],
-                    &s.ev_step[1]})
-      EB_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    allow_max_dynamic_smem((const void*)k_cgs_update_dot);
-  }
+  ensure_branches(s);
+  allow_max_dynamic_smem((const void*)k_cgs_update_dot);
   if (!s.k_host) EB_CK(cudaMallocHost((void**)&s.k_host, 2 * (size_t)(CGS_MAX + 2) * sizeof(double)));
   int R;
   const int nb = std::max(dot_blocks(N, &R), 4 * g_num_sms);

@@ -241,6 +241,8 @@ struct State {
 
 State& state();
 int eb_num_sms();
+// Creates the branch streams and their events.
+void ensure_branches(State& s);
 // Parts of the near lists for a launch of that many items.
 int near_parts(int items);
 // Raises a kernel's dynamic shared-memory cap to the device's opt-in maximum

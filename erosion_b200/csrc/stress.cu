@@ -815,10 +815,10 @@ __global__ void k_pack(int n, const double* __restrict__ x, const double* __rest
 // Host side.
 
 // Boundary values of all curves (wall first, then every body).
-static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all) {
+static void bdval_all(State& s, const double* d_den, DBuf<double2>& bd_all, cudaStream_t st) {
   const Problem& pr = s.pr;
   bd_all.ensure(5LL * pr.nout + 5LL * pr.n * pr.M);
-  k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, s.st>>>(
+  k_bdval<<<nblk(pr.nout, NEAR_T) + (unsigned)pr.M * nblk(pr.n, NEAR_T), NEAR_NT, 0, st>>>(
       s.geo(), d_den, nullptr, s.dker_wall.p, s.dker_body.p, bd_all.p);
   EB_LAUNCH_CHECK();
 }
@@ -935,11 +935,23 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
   static DBuf<double> eself, part;
   static DBuf<double2> bd_all;
   eself.ensure(3LL * nb);
-  k_stress_self<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, s.st>>>(G, d_den, s.dker_body.p, eself.p);
-  EB_LAUNCH_CHECK();
   const int bary = pr.P.ibary == 1;
+  // By clusters, a branch takes the bodies' own strain, the boundary values and the
+  // barycentric sums, the library stream the near lists and the expansions: neither
+  // half fills the chip with its last CTAs and its short launches.  A call at 400 bodies
+  // x 256 nodes takes 1.80 ms, 2.05 with one after the other; at 37 x 200 0.33 and 0.41.
+  const bool branch = bary && !pr.P.stress_all_bary && s.cl_ready;
+  cudaStream_t side = s.st;
+  if (branch) {
+    ensure_branches(s);
+    side = s.br[0];
+    EB_CK(cudaEventRecord(s.ev_fork[0], s.st));
+    EB_CK(cudaStreamWaitEvent(side, s.ev_fork[0], 0));
+  }
+  k_stress_self<<<pr.M * nblk(pr.n, 32), NEAR_NT, 0, side>>>(G, d_den, s.dker_body.p, eself.p);
+  EB_LAUNCH_CHECK();
   if (bary && pr.P.stress_all_bary) {   // every pair barycentric, as the reference evaluates it
-    bdval_all(s, d_den, bd_all);
+    bdval_all(s, d_den, bd_all, s.st);
     const int tasks = pr.M * (int)nblk(pr.n, NEAR_T), nsplit = source_splits(tasks, pr.M + 1);
     part.ensure((size_t)nsplit * 6 * nb);
     k_bary_sum<<<dim3(tasks, nsplit), NEAR_NT, 0, s.st>>>(G, bd_all.p, s.xy.p + pr.nout, 1, nb, part.p);
@@ -962,7 +974,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
         STRESS_CL * std::max(1u, std::min(nblk(nb, 32), (unsigned)(2 * eb_num_sms() / STRESS_CL)));
     smask.ensure((size_t)nb * mw);
     pnear.ensure(6LL * nb);
-    bdval_all(s, d_den, bd_all);
+    bdval_all(s, d_den, bd_all, side);
     const unsigned near_ctas = pr.M * nblk(pr.n, NEAR_T);
     if (s.cl_ready) {
       const int2* items = s.items32.p + s.n_items32_wall;
@@ -970,10 +982,13 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       k_stress_near_items<<<nit, 256, 0, s.st>>>(G, items, s.tiles.p, s.nwall_tiles, s.cl_cen.p, s.cl_rad.p, ext.p, mw,
                                                  smask.p, wlist.p + nb, wlist.p);
       EB_LAUNCH_CHECK();
-      k_bary_sum_near<<<near_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, smask.p, mw, pnear.p);
+      EB_CK(cudaEventRecord(s.ev_fork[1], s.st));
+      EB_CK(cudaStreamWaitEvent(side, s.ev_fork[1], 0));
+      k_bary_sum_near<<<near_ctas, NEAR_NT, 0, side>>>(G, bd_all.p, smask.p, mw, pnear.p);
       EB_LAUNCH_CHECK();
-      k_stress_wall<<<wall_ctas, NEAR_NT, 0, s.st>>>(G, bd_all.p, wlist.p + nb, wlist.p, pnear.p);
+      k_stress_wall<<<wall_ctas, NEAR_NT, 0, side>>>(G, bd_all.p, wlist.p + nb, wlist.p, pnear.p);
       EB_LAUNCH_CHECK();
+      EB_CK(cudaEventRecord(s.ev_join[0], side));
       // strengths without the bodies' rigid parts (see k_stress_rigid), the
       // near lists of this mask, their strain and that of the expansions
       ClLists& lists = s.cl_stress;
@@ -994,6 +1009,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
                                                                      s.cl_lam.p, s.partial.p + (size_t)parts * pr.N);
         EB_LAUNCH_CHECK();
       }
+      EB_CK(cudaStreamWaitEvent(s.st, s.ev_join[0], 0));
       k_stress_assemble<<<nblk((long long)nb * COMBINE_G, 256), 256, 0, s.st>>>(
           G, d_den, L, s.tiles.p, s.cl_sing, pnear.p, s.partial.p, parts + (s.cl_expand ? 1 : 0), eself.p, d_tau, d_E);
       EB_LAUNCH_CHECK();
@@ -1048,7 +1064,7 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
   EB_LAUNCH_CHECK();
   int ns2 = 0;
   if (ibary) {
-    bdval_all(s, d_den, bd_all);
+    bdval_all(s, d_den, bd_all, s.st);
     ns2 = source_splits(tasks, pr.M + 1);
     pbary.ensure((size_t)ns2 * 6 * ntar);
     k_bary_sum<<<dim3(tasks, ns2), NEAR_NT, 0, s.st>>>(G, bd_all.p, txy.p, 0, (int)ntar, pbary.p);
