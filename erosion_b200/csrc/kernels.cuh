@@ -1722,7 +1722,7 @@ __device__ double2 bary_coincident(const GeoDev& G, int start, int len, const do
 // target, 143 with the gradient.  Bound by the FP64 pipe with many targets and by
 // a warp's chain of sources with few: against one thread per target and
 // correctly rounded divisions, the near pairs of 3 bodies x 64 nodes take 10.5 us
-// (69.6), of 400 x 256 25.0 us (78.1), and of 3200 targets against 50 x 128 + 1024 nodes 329 us (577).
+// (69.6), of 400 x 256 25.0 us (78.1), and of 3200 targets against 50 x 128 + 1024 nodes 325 us (577).
 // CL > 1 (the wall's curve only): the CTAs of a cluster of CL hold the same targets,
 // take a share of the nodes each and add their sums through distributed shared memory.
 template <int NDER, int CL = 1>

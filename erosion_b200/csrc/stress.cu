@@ -28,8 +28,14 @@ k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const double2* __restri
   const bool act = t < t1;
   const double2 zt = txy[act ? t : t1 - 1];
   double a[6] = {0, 0, 0, 0, 0, 0};
-  const int nc = G.M + 1, c1 = (int)((long long)nc * (blockIdx.y + 1) / gridDim.y);
-  for (int c = (int)((long long)nc * blockIdx.y / gridDim.y); c < c1; ++c) {
+  // parts of about as many nodes each: part y starts at the first curve with N y / gridDim.y
+  // nodes or more before it
+  auto first = [&](int y) {
+    const long long at = (long long)G.N * y / gridDim.y;
+    return at == 0 ? 0 : at <= G.nout ? 1 : 1 + (int)((at - G.nout + G.n - 1) / G.n);
+  };
+  const int c1 = blockIdx.y + 1 == gridDim.y ? G.M + 1 : first(blockIdx.y + 1);
+  for (int c = first(blockIdx.y); c < c1; ++c) {
     if (c == b + 1 && bodies) continue;
     DLPVal r = bary_eval<2>(T, G, c, bd_all + bd_all_off(G, c), zt, act);
     a[0] += r.ux; a[1] += r.uy; a[2] += r.u1x; a[3] += r.u1y; a[4] += r.u2x; a[5] += r.u2y;
@@ -738,20 +744,47 @@ k_qoi_trap(GeoDev G, const double* __restrict__ den, const int4* __restrict__ ti
   }
 }
 
+// Nearest body node of 32 targets (one per lane), the first minimum in body-major
+// order, among part blockIdx.y of the nodes: the warps split them, in order, and meet
+// in order.  dist[part*ntar + t], idx[...].
+__global__ void __launch_bounds__(256)
+k_qoi_nearest(GeoDev G, int ntar, const double2* __restrict__ txy, double* __restrict__ dist, int* __restrict__ idx) {
+  __shared__ double dm[NEAR_W][32];
+  __shared__ int di[NEAR_W][32];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = 32 * blockIdx.x + lane;
+  const double2 p = txy[min(t, ntar - 1)];
+  const long long nb = (long long)G.n * G.M, parts = (long long)NEAR_W * gridDim.y, w0 = (long long)NEAR_W * blockIdx.y + wid;
+  double dmin = 1e10;
+  int ind = 0;
+  const int hi = (int)(nb * (w0 + 1) / parts);
+#pragma unroll 4
+  for (int i = (int)(nb * w0 / parts); i < hi; ++i) {
+    const double2 q = G.xy[G.nout + i];
+    const double d2 = (p.x - q.x) * (p.x - q.x) + (p.y - q.y) * (p.y - q.y);
+    if (d2 < dmin) { dmin = d2; ind = i; }
+  }
+  dm[wid][lane] = dmin;
+  di[wid][lane] = ind;
+  __syncthreads();
+  if (wid != 0 || t >= ntar) return;
+  for (int w = 1; w < NEAR_W; ++w)
+    if (dm[w][lane] < dmin) { dmin = dm[w][lane]; ind = di[w][lane]; }
+  dist[(size_t)blockIdx.y * ntar + t] = dmin;
+  idx[(size_t)blockIdx.y * ntar + t] = ind;
+}
+
 // Final assembly at targets: barycentric velocity and vorticity (:3199-3212,
 // :3257-3270), stokeslets/rotlets (:3275-3298), and zeroing of targets that
 // classifyPointsOld (:4420-4500) puts inside a body (:3301-3309): the nearest
-// body node (first minimum in body-major order) decides the side through the
+// body node (npart candidates of k_qoi_nearest, in order) decides the side through the
 // sign of (x_t - x_k).n_k.  CTA = 32 targets, one per lane; the warps split the
-// bodies and the nodes, in order, and meet in order.  3200 targets, 6400 body
-// nodes: 52 us (a thread per target 265 us).
+// bodies.  8 us at 3200 targets and 50 bodies (with the nearest nodes searched by the same
+// 100 CTAs: 52 us).
 __global__ void __launch_bounds__(256)
 k_qoi_final(GeoDev G, const double* __restrict__ den, int ntar, const double2* __restrict__ txy,
             const double* __restrict__ ptrap, int ns1, const double* __restrict__ pbary, int ns2, int ibary,
-            double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ po, double* __restrict__ wo) {
+            const double* __restrict__ dist, const int* __restrict__ idx, int npart, double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ po, double* __restrict__ wo) {
   __shared__ double red[NEAR_W / 2][4][32];
-  __shared__ double dm[NEAR_W][32];
-  __shared__ int di[NEAR_W][32];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, t = 32 * blockIdx.x + lane;
   const bool act = t < ntar;
   const int tc = act ? t : ntar - 1;
@@ -779,23 +812,14 @@ k_qoi_final(GeoDev G, const double* __restrict__ den, int ntar, const double2* _
     a[3] += (ry * s1 - rx * s2) * ir / EB_TWOPI;
   }
   near_reduce(a, red);
-  const int nb = G.n * G.M;
-  double dmin = 1e10;
-  int ind = 0;
-  const int hi = (int)((long long)nb * (wid + 1) / NEAR_W);
-#pragma unroll 4
-  for (int i = (int)((long long)nb * wid / NEAR_W); i < hi; ++i) {
-    const double2 q = G.xy[G.nout + i];
-    const double d2 = (p.x - q.x) * (p.x - q.x) + (p.y - q.y) * (p.y - q.y);
-    if (d2 < dmin) { dmin = d2; ind = i; }
-  }
-  dm[wid][lane] = dmin;
-  di[wid][lane] = ind;
-  __syncthreads();
   if (wid != 0 || !act) return;
   if (G.M > 0) {
-    for (int w = 1; w < NEAR_W; ++w)
-      if (dm[w][lane] < dmin) { dmin = dm[w][lane]; ind = di[w][lane]; }
+    double dmin = dist[t];
+    int ind = idx[t];
+    for (int w = 1; w < npart; ++w) {
+      const double d = dist[(size_t)w * ntar + t];
+      if (d < dmin) { dmin = d; ind = idx[(size_t)w * ntar + t]; }
+    }
     const double2 q = G.xy[G.nout + ind], nn = G.nrm[G.nout + ind];
     const double vdn = (p.x - q.x) * nn.x + (p.y - q.y) * nn.y;
     if (!(vdn < 0.0)) a[0] = a[1] = a[2] = a[3] = 0.0;
@@ -914,6 +938,18 @@ static int source_splits(int ntasks, int ncurves) {
   return std::max(1, std::min((4 * eb_num_sms() + ntasks - 1) / std::max(ntasks, 1), ncurves));
 }
 
+// The same for k_bary_sum, two CTAs of which an SM holds: the parts, up to eight CTAs per
+// SM, with the least time in whole waves of them.  3200 targets (100 CTAs) against 50
+// x 128 + 1024 nodes: 11 parts (3.7 waves) 325 us, 6 (2.03 waves) 382 us.
+static int bary_splits(int ntasks, int ncurves) {
+  const long long slots = 2 * eb_num_sms();
+  int best = 1;
+  auto waves = [&](int p) { return ((long long)ntasks * p + slots - 1) / slots; };
+  for (int p = 2; p <= ncurves && (long long)ntasks * p <= 4 * slots; ++p)
+    if (waves(p) * best < waves(best) * p) best = p;
+  return best;
+}
+
 void body_pressure(State& s, const double* d_den, double* d_p) {
   const Problem& pr = s.pr;
   const GeoDev G = s.geo();
@@ -952,7 +988,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
   EB_LAUNCH_CHECK();
   if (bary && pr.P.stress_all_bary) {   // every pair barycentric, as the reference evaluates it
     bdval_all(s, d_den, bd_all, s.st);
-    const int tasks = pr.M * (int)nblk(pr.n, NEAR_T), nsplit = source_splits(tasks, pr.M + 1);
+    const int tasks = pr.M * (int)nblk(pr.n, NEAR_T), nsplit = bary_splits(tasks, pr.M + 1);
     part.ensure((size_t)nsplit * 6 * nb);
     k_bary_sum<<<dim3(tasks, nsplit), NEAR_NT, 0, s.st>>>(G, bd_all.p, s.xy.p + pr.nout, 1, nb, part.p);
     EB_LAUNCH_CHECK();
@@ -1057,21 +1093,34 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
   const int ibary = pr.P.ibary == 1, tasks = (int)nblk(ntar, NEAR_T);
   const int ns1 = source_splits(tasks, std::min(s.ntile, 16));
   ptrap.ensure((size_t)ns1 * 4 * ntar);
-  if (ibary)
-    k_qoi_trap<false><<<dim3(tasks, ns1), 256, 0, s.st>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
-  else
-    k_qoi_trap<true><<<dim3(tasks, ns1), 256, 0, s.st>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
-  EB_LAUNCH_CHECK();
+  // the trapezoid sums and the nearest nodes on a branch beside the barycentric sums: of
+  // the call at 3200 targets, 50 x 128 + 1024 nodes 65 us
+  ensure_branches(s);
+  const cudaStream_t side = s.br[0];
+  EB_CK(cudaEventRecord(s.ev_fork[0], s.st));
+  EB_CK(cudaStreamWaitEvent(side, s.ev_fork[0], 0));
   int ns2 = 0;
   if (ibary) {
     bdval_all(s, d_den, bd_all, s.st);
-    ns2 = source_splits(tasks, pr.M + 1);
+    ns2 = bary_splits(tasks, pr.M + 1);
     pbary.ensure((size_t)ns2 * 6 * ntar);
     k_bary_sum<<<dim3(tasks, ns2), NEAR_NT, 0, s.st>>>(G, bd_all.p, txy.p, 0, (int)ntar, pbary.p);
     EB_LAUNCH_CHECK();
+    k_qoi_trap<false><<<dim3(tasks, ns1), 256, 0, side>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
+  } else {
+    k_qoi_trap<true><<<dim3(tasks, ns1), 256, 0, side>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
   }
-  k_qoi_final<<<tasks, 256, 0, s.st>>>(G, d_den, (int)ntar, txy.p, ptrap.p, ns1, pbary.p, ns2, ibary, d_u, d_v, d_p,
-                                       d_w);
+  EB_LAUNCH_CHECK();
+  const int parts = near_parts(tasks);
+  static DBuf<double> ndist;
+  static DBuf<int> nidx;
+  k_qoi_nearest<<<dim3(tasks, parts), 256, 0, side>>>(G, (int)ntar, txy.p, ndist.ensure((size_t)parts * ntar),
+                                                      nidx.ensure((size_t)parts * ntar));
+  EB_LAUNCH_CHECK();
+  EB_CK(cudaEventRecord(s.ev_join[0], side));
+  EB_CK(cudaStreamWaitEvent(s.st, s.ev_join[0], 0));
+  k_qoi_final<<<tasks, 256, 0, s.st>>>(G, d_den, (int)ntar, txy.p, ptrap.p, ns1, pbary.p, ns2, ibary, ndist.p, nidx.p,
+                                       parts, d_u, d_v, d_p, d_w);
   EB_LAUNCH_CHECK();
 }
 
