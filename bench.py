@@ -18,8 +18,8 @@ flushed (a 256 MiB write) before every timed step.  The body count is fixed
 over the timed window: the step dt is chosen so that no body erodes away, and
 should one be deleted all the same the state is restored to the window's
 starting state before the next step (counted in `config.restores`).  The
-far-field launch shapes are tuned during the warm-up and then frozen, so no
-tuning runs inside a timed region.  `plain_fp64` is one step of the
+far field's launches follow from the sizes: no tuning runs inside a timed
+region.  `plain_fp64` is one step of the
 reference's algorithm on the GPU (FP64 operator, no preconditioner, zero
 initial guess) from the same starting state.
 """
@@ -64,18 +64,6 @@ WORKLOADS = {
                     "{128,256,512}, porosity U[0.5,0.8], 2048 wall nodes", dt=None, dt_config=None),
 }
 METRIC = "erosion steps/s at 1e-8 residual"
-
-# DRAM bytes per node and far-field launch (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch divided by the node count N) from the ncu
-# captures of k_far32 and the fast k_far64 on the 400-body channel (N =
-# 106,496; one operator application with pinned launch shapes).  A launch
-# reads each source and target record once (N x 64 B) and each target's row
-# of the near mask once (N x 4 B per 32 curves: 52 B at 401 curves).  The
-# accurate k_far64 and the wall-source launch read the same records as the
-# fast k_far64 and carry its figure.
-TRAFFIC_BYTES_PER_NODE = {"k_far32": (11398144 + 16384) / 106496, "k_far64_fast": 10671360 / 106496,
-                          "k_far64": 10671360 / 106496, "k_far64_wall_sources": 10671360 / 106496}
-
 
 # Plain FP64 GMRES iterations per erosion step (unpreconditioned, zero initial
 # guess: the reference's algorithm) on the seeded workloads, as the plain_fp64
@@ -567,17 +555,18 @@ class Stepper:
 
 
 def kernel_roofline(s0, s1, N, curves, peak64, peak32, ms_timed):
-    """Per far-field kernel: launches, time, pairs per launch, achieved
-    TFLOP/s (20 flops per pair), fraction of the measured FMA peak of its pipe
-    and the DRAM bytes per launch (ncu figure per node x N) beside the
-    algorithmic bytes (64 B per node record plus the node's near-mask row,
-    4 B per 32 curves)."""
+    """Per near-list kernel of the far field: launches, time (of the timed ones,
+    scaled to all: the others replay captured steps), pairs of its lists per
+    launch, achieved TFLOP/s (20 flops per pair), fraction of the measured FMA
+    peak of its pipe and the algorithmic bytes (64 B per node record plus the
+    node's near-mask row, 4 B per 32 curves).  The pairs of separated clusters
+    act through expansions and are not counted."""
     algorithmic = N * (64 + 4 * ((curves + 31) // 32))
     kernels = {}
-    spec = (("k_far64", "ms_far", "far_launches", "far64_pairs", peak64),
-            ("k_far64_fast", "ms_far64f", "far64f_launches", "far64_pairs", peak64),
-            ("k_far64_wall_sources", "ms_farw", "farw_launches", "farw_pairs", peak64),
-            ("k_far32", "ms_far32", "far32_launches", "far32_pairs", peak32))
+    spec = (("k_cl_near64", "ms_far", "far_launches", "far64_pairs", peak64),
+            ("k_cl_near64_relaxed", "ms_far64f", "far64f_launches", "far64_pairs", peak64),
+            ("k_cl_near64_wall_sources", "ms_farw", "farw_launches", "farw_pairs", peak64),
+            ("k_cl_near32", "ms_far32", "far32_launches", "far32_pairs", peak32))
     for name, kms, kn, kp, peak in spec:
         ms = s1[kms] - s0[kms]
         nl = s1[kn] - s0[kn]
@@ -588,7 +577,6 @@ def kernel_roofline(s0, s1, N, curves, peak64, peak32, ms_timed):
         kernels[name] = {"launches": nl, "ms_total": ms, "ms_avg": ms / nl, "pairs_per_launch": pairs,
                          "achieved_tflops": a, "peak_tflops": peak, "frac": a / peak,
                          "share_of_timed": ms / ms_timed,
-                         "traffic_bytes_per_launch": TRAFFIC_BYTES_PER_NODE[name] * N,
                          "algorithmic_bytes_per_launch": algorithmic}
     return kernels
 
@@ -615,12 +603,6 @@ def run_steps(args, world, rank, local, dist):
     M_start0 = S.M
     for _ in range(args.warmup):
         S.step(p)
-    # freeze the launch shapes the warm-up tuned
-    shapes = _lib.far_shapes()
-    L.erosion_set_far_shape(0, shapes["fp64"]["index"])
-    L.erosion_set_far_shape(1, shapes["fp32"]["index"])
-    if "fp64_fast" in shapes:
-        L.erosion_set_far_shape(2, shapes["fp64_fast"]["index"])
     S.snapshot()
     M0 = S.M
     torch.cuda.synchronize()
@@ -658,23 +640,22 @@ def run_steps(args, world, rank, local, dist):
     peak32 = max(peak32_scalar, peak32_packed)
     kernels = kernel_roofline(s0, s1, N, M0 + 1, peak64, peak32, ms)
     dom = max(kernels, key=lambda k: kernels[k]["ms_total"]) if kernels else None
-    roofline = {"bound": ("fp32" if dom == "k_far32" else "fp64") if dom else None,
+    roofline = {"bound": ("fp32" if dom == "k_cl_near32" else "fp64") if dom else None,
                 "achieved": kernels[dom]["achieved_tflops"] if dom else None,
                 "peak": kernels[dom]["peak_tflops"] if dom else None, "unit": "TFLOP/s",
                 "frac": kernels[dom]["frac"] if dom else None,
-                "traffic": kernels[dom]["traffic_bytes_per_launch"] if dom else None, "kernel": dom,
-                "algorithmic": "20 flops per source-target pair; pairs per launch: k_far64 (accurate FP64) and "
-                               "k_far64_fast (the mixed solve's FP64 phase) = node pairs of distinct curves less the "
-                               "barycentric near pairs (self-curve pairs run in k_self64); in the mixed operator's "
-                               "FP32 phase k_far32 takes the body-source pairs and k_far64_wall_sources the "
-                               "wall-source pairs",
+                "traffic": None, "kernel": dom,
+                "algorithmic": "20 flops per source-target pair; pairs per launch: those of the near lists less the "
+                               "barycentric near pairs (self-curve pairs run in k_self64, separated clusters act "
+                               "through expansions): k_cl_near64 (accurate FP64) and k_cl_near64_relaxed (the mixed "
+                               "solve's FP64 phase) all of them; in the mixed operator's FP32 phase k_cl_near32 takes "
+                               "the body sources and k_cl_near64_wall_sources the wall's",
                 "peak_source": "of measured: FMA loop on this GPU (erosion_peak_tflops), vector pipe; FP32 = max of "
                                "scalar and packed two-lane FMA",
-                "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum per launch of the ncu captures of "
-                                  "k_far32 and the fast k_far64 on the 400-body channel, per node, times N",
+                "traffic_source": "not captured per launch: the node records of a launch stay in L2",
                 "peaks_measured_tflops": {"fp64": peak64, "fp32_scalar": peak32_scalar,
                                           "fp32_packed": peak32_packed},
-                "launch_shapes": shapes, "kernels": kernels}
+                "kernels": kernels}
     mv = sum(sum(st["matvecs"]) for st in per_step)
     mv32 = sum(sum(st["matvecs_fp32"]) for st in per_step)
 
@@ -736,8 +717,6 @@ def run_steps(args, world, rank, local, dist):
                          "the timed window's starting state",
                  "speedup_of_value": value / pv,
                  "speedup_of_e2e": (e2e["value"] / pv) if e2e else None}
-    L.erosion_set_far_shape(0, -1)
-    L.erosion_set_far_shape(1, -1)
 
     if rank == 0:
         cpu = None
@@ -761,13 +740,13 @@ def run_steps(args, world, rank, local, dist):
                           "fixpdrop": 0, "tol": 1e-8,
                           "precision": "fp64" if args.precision == 0 else "mixed", "warm_start": args.warm_start,
                           "precond": "block Gauss-Seidel" if args.precond else "none",
-                          "launch_shapes": "tuned in the warm-up, frozen for the timed regions",
                           "parallelism": "replicas" if world > 1 else "single GPU",
                           "l2": "flushed (256 MiB write) before every step"},
                "gmres_iterations_per_step": float(np.mean(iters)) if iters else 0.0,
                "gmres_iterations_per_solve": [i for st in per_step for i in st["gmres_iterations"]],
                "far_field_launches": {"total": mv, "fp32": mv32, "fp32_share": mv32 / mv if mv else None},
                "pair_interactions_per_s": pairs_per_s,
+               "pair_interactions_note": "node pairs that the operator stands for, most of them through expansions",
                "gmres_solves_per_s": 2 * value,
                "step_breakdown_ms": {k: float(np.mean([s[k] for s in per_step])) for k in
                                      ("ms_solve", "ms_stress", "ms_thetalen", "ms_total", "ms_setup",

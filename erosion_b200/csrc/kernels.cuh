@@ -533,14 +533,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float t) {
-  float s = hi + t;
-  float bp = s - hi;
-  float e = (hi - (s - bp)) + (t - bp);
-  hi = s;
-  lo += e;
-}
-
 // Sources per FP32 partial sum of k_far32: the running FP32 sum of a target is
 // added to its FP64 accumulator after every F32_CHUNK sources, so the rounding
 // error of the plain FP32 accumulation grows with the chunk length instead of

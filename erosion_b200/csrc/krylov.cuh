@@ -15,7 +15,7 @@
 // update read it four times) for long vectors and by latency for short ones:
 // the splits over rows and columns keep a warp's chain of loads short.  n =
 // 4638, k = 180: 17 us for the step, with one launch per operation 52 us; n =
-// 55,596, k = 240: 72 us (102 us).
+// 55,596, k = 240: 65 us (102 us).
 #pragma once
 #include "kernels.cuh"
 

@@ -1670,14 +1670,6 @@ int solve_device_impl(State& s, double* d_den, bool x0_zero, int64_t* nits) {
   EB_CK(cudaEventRecord(s.e1, s.st));
   EB_CK(cudaEventSynchronize(s.e1));
   harvest_far_timing(s);
-  // the launches inside replayed graphs take the mean of the timed ones
-  auto scale = [](double& t, long long launches, long long timed) {
-    if (timed > 0) t *= (double)launches / (double)timed;
-  };
-  scale(s.stats.ms_far, s.stats.far_launches, s.timed_far);
-  scale(s.stats.ms_far32, s.stats.far32_launches, s.timed_far32);
-  scale(s.stats.ms_farw, s.stats.farw_launches, s.timed_farw);
-  scale(s.stats.ms_far64f, s.stats.far64f_launches, s.timed_far64f);
   float ms = 0;
   EB_CK(cudaEventElapsedTime(&ms, s.e0, s.e1));
   s.stats.ms_total = ms;
@@ -1710,7 +1702,18 @@ void erosion_default_params(erosion_params* p) {
 int erosion_last_status(void) { return t_status; }
 const char* erosion_last_error(void) { return t_err.c_str(); }
 
-void erosion_get_solve_stats(erosion_solve_stats* out) { *out = state().stats; }
+void erosion_get_solve_stats(erosion_solve_stats* out) {
+  const State& s = state();
+  *out = s.stats;
+  // the launches inside replayed graphs take the mean of the timed ones
+  auto scale = [](double& t, long long launches, long long timed) {
+    if (timed > 0) t *= (double)launches / (double)timed;
+  };
+  scale(out->ms_far, out->far_launches, s.timed_far);
+  scale(out->ms_far32, out->far32_launches, s.timed_far32);
+  scale(out->ms_farw, out->farw_launches, s.timed_farw);
+  scale(out->ms_far64f, out->far64f_launches, s.timed_far64f);
+}
 
 int erosion_solve(const erosion_params* p, int64_t npts, int64_t nbods, int64_t nouter, const double* xx,
                   const double* yy, double* density, int64_t* nits) {

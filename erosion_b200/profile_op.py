@@ -1,13 +1,12 @@
-"""One application of the boundary operator on a named workload, with the
-far-field launch shapes pinned: the small, fixed sequence of launches a
-kernel profiler captures.
+"""One application of the boundary operator on a named workload: the small,
+fixed sequence of launches a kernel profiler captures.
 
     python -m erosion_b200.profile_op [--workload c3] [--precision 1]
-                                      [--shape64 0] [--shape32 0] [--shape64f 0] [--reps 1]
+                                      [--shape64 -1] [--shape32 -1] [--shape64f -1] [--reps 1]
 
 precision: 0 accurate FP64 far field, 1 mixed (FP32 body sources, FP64 wall
-sources), 2 the fast FP64 far field.  The density is seeded random.  With
-pinned shapes the set-up launches no autotuner timing.
+sources), 2 the fast FP64 far field.  The density is seeded random.  A shape of
+0 or more pins the direct far-field sum of that kind (every pair, no clusters).
 """
 from __future__ import annotations
 
@@ -22,9 +21,9 @@ def main(argv=None):
     ap = argparse.ArgumentParser()
     ap.add_argument("--workload", default="c3")
     ap.add_argument("--precision", type=int, default=1)
-    ap.add_argument("--shape64", type=int, default=0)
-    ap.add_argument("--shape32", type=int, default=0)
-    ap.add_argument("--shape64f", type=int, default=0)
+    ap.add_argument("--shape64", type=int, default=-1)
+    ap.add_argument("--shape32", type=int, default=-1)
+    ap.add_argument("--shape64f", type=int, default=-1)
     ap.add_argument("--reps", type=int, default=1)
     args = ap.parse_args(argv)
     L = _lib.load()
