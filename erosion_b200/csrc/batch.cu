@@ -141,6 +141,7 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
       Member& mb = *B.m[g];
       State& s = mb.s;
       init_state(s, lib.device);
+      s.pc_valid = false;   // the inverses it holds are of another call's geometry
       Problem pr;
       pr.P = P;
       pr.n = (int)npts[g]; pr.M = (int)nbods[g]; pr.nout = (int)nouter[g];

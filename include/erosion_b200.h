@@ -127,7 +127,8 @@ typedef struct {
                            stages and time steps of an erosion run, whose shapes
                            change little).  Flexible GMRES meets the same
                            tolerance with any fixed preconditioner; only the
-                           iteration count can change                            */
+                           iteration count can change.  erosion_solve_batch
+                           rebuilds them in every call                           */
   int32_t stress_all_bary; /* shear stress with ibary = 1: 0 (default) evaluates
                            another curve by the barycentric formulas only at body
                            nodes within 12 of its node spacings and by the
