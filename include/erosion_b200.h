@@ -220,7 +220,9 @@ void erosion_get_solve_stats(erosion_solve_stats* s);
  * solved with the method erosion_solve applies for the same parameters (one
  * erosion_params for all), on streams of its own, from a pool of up to 16 host
  * threads; the GPU works on as many geometries at a time.
- * Returns EROSION_OK or the first non-OK status of a geometry. */
+ * Returns EROSION_OK or the first non-OK status of a geometry.  Geometries that
+ * reach maxl or stall still return their densities; on any other error (bad
+ * input, a non-finite value, a CUDA error) density and nits stay as they were. */
 int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* npts, const int64_t* nbods,
                         const int64_t* nouter, const double* xx, const double* yy, double* density, int64_t* nits);
 

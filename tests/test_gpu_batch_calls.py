@@ -1,9 +1,12 @@
 """What one erosion_solve_batch call leaves for the next: nothing of an earlier ensemble's
-geometry reaches a later one."""
+geometry reaches a later one; and for its caller: a call that fails leaves the densities as
+they were."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from erosion_b200 import geometry as G, stokes
+from erosion_b200 import _lib, geometry as G, stokes
 
 pytestmark = pytest.mark.gpu
 
@@ -25,3 +28,20 @@ def test_inverses_are_not_kept_between_calls(lib):
     assert n_after.tolist() == n_fresh.tolist()
     for a, f in zip(after, fresh):
         assert np.array_equal(a, f)
+
+
+def test_failed_call_leaves_the_densities(lib):
+    """A geometry that fails in its solve (a guess that is not finite) fails the call; the
+    others' densities stay the caller's guesses, as its own does."""
+    ens = ensemble(50)
+    den = np.concatenate([np.full(ens[0].ntot, 1e-3), np.full(ens[1].ntot, np.nan)])
+    kept = den.copy()
+    nits = np.full(2, -1, np.int64)
+    size = [np.array(v, np.int64) for v in ([g.n for g in ens], [g.M for g in ens], [g.nout for g in ens])]
+    xx, yy = (np.concatenate([getattr(g, k) for g in ens]) for k in ("xx", "yy"))
+    p = stokes.params_for(ens[0], tol=1e-8)
+    rc = lib.erosion_solve_batch(ctypes.byref(p), 2, *[v.ctypes.data_as(_lib.PI64) for v in size], _lib.ptr(xx),
+                                 _lib.ptr(yy), _lib.ptr(den), nits.ctypes.data_as(_lib.PI64))
+    assert rc == _lib.EROSION_BREAKDOWN
+    assert np.array_equal(den, kept, equal_nan=True)
+    assert nits.tolist() == [-1, -1]
