@@ -48,7 +48,7 @@ Batch& batch() {
 }
 
 void destroy_member(Member& mb) {
-  if (mb.s.st) cudaStreamSynchronize(mb.s.st);
+  settle(mb.s);
   release_state_buffers(mb.s);
   destroy_state(mb.s);
   mb.x.release();
@@ -203,13 +203,11 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
     set_status(worst, worst == EROSION_OK ? "" : "a geometry of the ensemble did not converge");
     return worst;
   } catch (const Error& e) {
-    for (auto& mb : batch().m)
-      if (mb->s.st) cudaStreamSynchronize(mb->s.st);
+    for (auto& mb : batch().m) settle(mb->s);
     set_status(e.code, e.what());
     return e.code;
   } catch (const std::exception& e) {
-    for (auto& mb : batch().m)
-      if (mb->s.st) cudaStreamSynchronize(mb->s.st);
+    for (auto& mb : batch().m) settle(mb->s);
     set_status(EROSION_CUDA_ERROR, e.what());
     return EROSION_CUDA_ERROR;
   }

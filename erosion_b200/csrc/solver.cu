@@ -428,15 +428,6 @@ static void plan_clusters(State& s) {
 // Stream of branch b (0..2) of an operator's independent launches.
 static cudaStream_t branch(State& s, int b) { return s.forked ? s.br[b] : s.st; }
 
-// Runs f with the library stream of the state replaced by st.
-template <class F>
-static void on_stream(State& s, cudaStream_t st, F&& f) {
-  const cudaStream_t main = s.st;
-  s.st = st;
-  f();
-  s.st = main;
-}
-
 static void fork(State& s, int ev, std::initializer_list<int> to) {
   if (!s.forked) return;
   EB_CK(cudaEventRecord(s.ev_fork[ev], s.st));
@@ -1039,17 +1030,14 @@ void apply_operator(State& s, const double* d_den, double* d_vel, int prec) {
   // side by side, as in the captured steps, where they take longer than the ten event
   // calls: 480 -> 426 us a call at 100 bodies x 256 nodes, 1150 -> 1080 at 400, no
   // difference at 3 x 64
-  s.forked = s.cl_active && s.cl_expand;
-  if (s.forked) ensure_branches(s);
-  try {
+  const bool branches = s.cl_active && s.cl_expand;
+  if (branches) ensure_branches(s);
+  {
+    const Scoped<bool> forked(s.forked, branches);
     fork(s, 0, {0, 1, 2});
     far_field(s, d_den, kind, true);
     operator_post(s, d_den, d_vel, far_slots(s, prec));
-  } catch (...) {
-    s.forked = false;
-    throw;
   }
-  s.forked = false;
   count_operator(s, kind);
 }
 
@@ -1119,6 +1107,12 @@ static int step_bound(int ll) {
 constexpr long long kRowPerThread = 75000;
 
 static size_t step_tile(int bound) { return (size_t)bound * 34 * sizeof(double); }
+
+void settle(State& s) {
+  if (s.st) cudaStreamSynchronize(s.st);
+  for (auto& b : s.br)
+    if (b) cudaStreamSynchronize(b);
+}
 
 void ensure_branches(State& s) {
   if (s.br[0]) return;
@@ -1225,16 +1219,15 @@ static void replay_step(State& s, long long N, long long ldv, int bound, int pre
   const long long l0 = t_launches;
   EB_CK(cudaStreamBeginCapture(s.st, cudaStreamCaptureModeRelaxed));
   cudaGraph_t graph = nullptr;
-  s.forked = true;
   try {
+    const Scoped<bool> forked(s.forked, true);
     launch_step(s, N, ldv, bound, prec, false, host);
   } catch (...) {
-    s.forked = false;
-    cudaStreamEndCapture(s.st, &graph);
+    cudaStreamEndCapture(s.st, &graph);   // ends the branches' part of it too
     if (graph) cudaGraphDestroy(graph);
+    (void)cudaGetLastError();             // the broken capture's own error is not the next launch's
     throw;
   }
-  s.forked = false;
   EB_CK(cudaStreamEndCapture(s.st, &graph));
   // the graph of the previous set-up usually has the same nodes: updating it is
   // several times cheaper than instantiating another and destroying it
@@ -1609,9 +1602,11 @@ int guarded(F&& f) {
                                                             : (rc == EROSION_BREAKDOWN ? "GMRES stalled" : "error")));
     return rc;
   } catch (const Error& e) {
+    settle(s);
     set_status(e.code, e.what());
     return e.code;
   } catch (const std::exception& e) {
+    settle(s);
     set_status(EROSION_CUDA_ERROR, e.what());
     return EROSION_CUDA_ERROR;
   }

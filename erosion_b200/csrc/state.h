@@ -240,6 +240,30 @@ struct State {
 };
 
 State& state();
+
+// Sets v while it lives; the old value comes back however the scope is left.
+template <class T>
+struct Scoped {
+  T& v;
+  T old;
+  Scoped(T& ref, T value) : v(ref), old(ref) { v = value; }
+  ~Scoped() { v = old; }
+  Scoped(const Scoped&) = delete;
+  Scoped& operator=(const Scoped&) = delete;
+};
+
+// Runs f with the library stream of the state replaced by st.  A failed launch in f throws:
+// the stream comes back with it, or the next call would run, and destroy_state end, a branch
+// in its place.
+template <class F>
+void on_stream(State& s, cudaStream_t st, F&& f) {
+  const Scoped<cudaStream_t> keep(s.st, st);
+  f();
+}
+
+// Waits for what a failed call left in flight on the state's streams: its branches are
+// joined by nothing, and the next call uses the same buffers.
+void settle(State& s);
 int eb_num_sms();
 // Creates the branch streams and their events.
 void ensure_branches(State& s);

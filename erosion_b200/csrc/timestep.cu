@@ -702,9 +702,11 @@ int guarded3(F&& f) {
     set_status(rc, "");
     return rc;
   } catch (const Error& e) {
+    settle(s);
     set_status(e.code, e.what());
     return e.code;
   } catch (const std::exception& e) {
+    settle(s);
     set_status(EROSION_CUDA_ERROR, e.what());
     return EROSION_CUDA_ERROR;
   }
