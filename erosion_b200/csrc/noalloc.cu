@@ -212,7 +212,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     const bool expand = N >= kExpandNodes, sing = expand && n <= FAR_TS;
     double2* mp = cv.take<double2>(expand ? (size_t)ntile * CL_MP : 1);
     double2* lam = cv.take<double2>(ntile);
-    const int parts = near_parts(nitem);
+    const int parts = near_parts(nitem, nd.sms);
     double2* partial = cv.take<double2>((size_t)(parts + 1) * N);
     if (cv.off > NA_SCRATCH_BYTES) throw Error(EROSION_BAD_INPUT, "erosion_matvec_noalloc: scratch layout");
 

@@ -397,12 +397,6 @@ static void plan_far(State& s, bool tune) {
 // ---------------------------------------------------------------------------
 // The far field by clusters.
 
-// Parts of the near lists: about four CTAs per SM from items CTAs, at most 8.
-// 10 bodies x 128 nodes and 1024 wall nodes (72 items): 31.5 us in one part,
-// 20.4 us in 5, 17.1 us in 8, 16.0 us in 12 (and 3 us more in larger assemblies);
-// 100 x 256, FP32 (464 items): 39.8 us in one part, 33.7 us in 2, 33.3 us in 4.
-int near_parts(int items) { return std::max(1, std::min(8, (4 * g_num_sms + items - 1) / items)); }
-
 // Decides how the current problem's far field is summed.
 // The direct sum over split tile ranges (launch_far) stays for a forced launch
 // shape and for more tiles than the lists are built for.
@@ -416,8 +410,8 @@ static void plan_clusters(State& s) {
                                                s.cl_rad.ensure(s.ntile));
   EB_LAUNCH_CHECK();
   if (!s.cl_ready) return;
-  s.cl_parts64 = near_parts(s.n_items32);
-  s.cl_parts32 = near_parts(s.n_items64);
+  s.cl_parts64 = near_parts(s.n_items32, g_num_sms);
+  s.cl_parts32 = near_parts(s.n_items64, g_num_sms);
   s.partial.ensure((size_t)(s.cl_parts64 + s.cl_parts32 + 1) * pr.N);
   if (s.cl_expand) {
     s.cl_mp.ensure((size_t)s.ntile * CL_MP);

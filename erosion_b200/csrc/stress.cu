@@ -1032,7 +1032,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       EB_LAUNCH_CHECK();
       build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand, nullptr);
       const ClView L = cl_view(s, lists);
-      const int parts = near_parts(nit);
+      const int parts = near_parts(nit, eb_num_sms());
       s.partial.ensure((size_t)(parts + 1) * pr.N);
       k_cl_near64<true, true><<<dim3(nit, parts), 256, 0, s.st>>>(G, L, items, s.tiles.p, 0, s.sq64.p, smask.p, mw,
                                                                   pr.nout, s.partial.p);
@@ -1111,7 +1111,7 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
     k_qoi_trap<true><<<dim3(tasks, ns1), 256, 0, side>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
   }
   EB_LAUNCH_CHECK();
-  const int parts = near_parts(tasks);
+  const int parts = near_parts(tasks, eb_num_sms());
   static DBuf<double> ndist;
   static DBuf<int> nidx;
   k_qoi_nearest<<<dim3(tasks, parts), 256, 0, side>>>(G, (int)ntar, txy.p, ndist.ensure((size_t)parts * ntar),
