@@ -26,8 +26,10 @@ struct NearInfo {
 // The wall length scale 'lw' of matvec_DLP_fmmbary, an implicitly typed INTEGER
 // there (:705-709): lw = (lw + |z'_k|) truncated at every node, then an integer
 // division.  Truncating every |z'_k| gives the same sum unless a fraction is so
-// close to 1 that the addition may round up: the 1/256 of the nodes around one
-// is then summed in order (at the wall's flat sides |z'| is 1 to 1e-13).  Per body:
+// close to 1 that the addition may round up, within half an ulp of the running sum (at
+// most 1.2e-16 of it; the margin allows for nodes at 1/80 of the mean speed): the 1/256
+// of the nodes around one is then summed in order (at the wall's flat sides |z'| is 1 to
+// 1e-13).  Per body:
 // near the wall (:711-730) or not, the |y| from which its nodes are, and the
 // radius within which wall nodes are.
 __global__ void __launch_bounds__(256)
@@ -53,7 +55,7 @@ k_near_head(GeoDev G, double bw, NearInfo* __restrict__ info, double2* __restric
       bad = 1;
     } else if (v < 1e15) {
       const long long f = (long long)v;
-      if (v - (double)f > 1.0 - 1e-9) e = 1;
+      if (v - (double)f > 1.0 - (1e-9 + 1e-14 * G.nout * v)) e = 1;
       s += f;
     } else {
       e = 1;
