@@ -27,30 +27,32 @@
 // pairs: FP64 tensor-core work (mma m8n8k4).
 //
 // Accuracy.  Clusters are separated when R <= theta (|D| - R') and R' <= theta
-// (|D| - R), theta = 1/3: cutting both series after CL_P = 32 terms leaves
-// 3^-32 = 5e-16 of the cluster's field, FP64 rounding; wider pairs keep fewer
-// terms to the same bound (cl_class).  Measured against a
-// direct sum in FP64, the operator on 400 bodies x 256 nodes is as far from
-// the 64-bit value as the direct kernels are (their geometry's rounding).
+// (|D| - R); phi's series then converge like theta^p.  The terms k a_(k-1) and, in
+// the evaluation, phi' put a factor p / theta on the first one that is cut, so p
+// terms carry pairs up to a theta whose cut is 5e-16 (FP64 rounding) of a source's
+// field |A|/r, or of its strain |A|/r^2, measured over positions, directions and radii
+// of the two clusters: 0.373 and 0.337 for CL_P = 40 (cl_class has the others').
+// By theta^p alone (32 terms at 1/3, 8 at 1/81) the cut was 2e-14 to 9e-14 of the
+// field and 1e-12 of the strain.
 //
-// Cost.  Per pair of clusters 4 x p x p multiply-adds, p = 8..32, and about as
-// many operations around them, against 256 x 256 x ~18 operations for the pairs of two bodies.
+// Cost.  Per pair of clusters 4 multiply-adds per local and multipole term, 16 x 12 to
+// 40 x 40 of them, and about as many operations around them, against 256 x 256 x ~18
+// operations for the pairs of two bodies.
 #pragma once
 #include "state.h"
 #include "kernels.cuh"
 
 namespace {
 
-constexpr int CL_P = 32;                 // terms of an expansion
-constexpr double CL_THETA = 1.0 / 3.0;   // separation
+constexpr int CL_P = 40;                 // terms of an expansion
 constexpr int CL_MP = 3 * CL_P;          // multipole record of a cluster: a_k, x_k, k a_(k-1) / R
 constexpr int CL_MAX_TILES = 4096;       // above this the lists (tiles^2 entries) are not built
 
 // Nodes from which the separated clusters act through expansions; below, every
 // cluster pair is summed directly.  Near lists, expansions and assembly with
-// and without them, FP64 (mixed): 2304 nodes 24.0 and 23.0 us (28.2 and 21.7),
-// 3072 nodes 29.9 and 34.8 us (32.7 and 28.8), 3584 nodes 29.0 and 47.2 us
-// (32.1 and 33.0), 8704 nodes 44.7 and 160.7 us (43.7 and 109.8); the
+// and without them, FP64 (mixed): 2304 nodes 24.8 and 20.5 us (30.4 and 19.1),
+// 3072 nodes 29.2 and 28.7 us (34.7 and 27.3), 3584 nodes 32.0 and 33.5 us
+// (36.2 and 32.5), 8704 nodes 54.7 and 140.6 us (47.4 and 89.2); the
 // expansions are two launches more.
 constexpr int kExpandNodes = 3200;
 
@@ -92,34 +94,42 @@ k_cl_geom(GeoDev G, int ntile, const int4* __restrict__ tiles, double2* __restri
   }
 }
 
-// Orders of the expansions.  A pair of separated clusters needs the p terms for
-// which its own ratio theta = max(R/(|D| - R'), R'/(|D| - R)) has theta^p <=
-// 3^-32: 32 at theta = 1/3, 8 at 1/81.  The far list of a cluster is sorted by
-// class of order; most pairs of a packing are far apart (400 bodies in the 2 x 1
-// channel: 92% need 16 terms or fewer), and the work of a pair goes with p^2.
+// Orders of the expansions.  A pair of separated clusters with theta = max(R/(|D| -
+// R'), R'/(|D| - R)) takes the local x multipole terms that keep its cut below 5e-16:
+//   terms            16 x 12   16 x 16   24 x 24   32 x 32   40 x 40
+//   velocity, theta   0.036     0.085     0.195     0.293     0.373
+//   strain, theta     0.0286    0.068     0.167     0.26      0.337
+// The far list of a cluster is sorted by class of order; most pairs of a packing are
+// far apart (400 bodies in the 2 x 1 channel: 90% need 16 terms), and the work of a pair
+// goes with the product.  The last class pays: with 32 terms at most the near lists of 400
+// bodies x 256 nodes take in 168 M pairs instead of 115 M.  Finer steps (8 x 12 at 0.0098,
+// 24 x 20 at 0.14) changed the time of a mixed step by 0.2% at most.
 constexpr int CL_NCLS = 5;
 
 // Class of a pair at centre distance D: 0..4 of ascending order, CL_NCLS near.
-__device__ __forceinline__ int cl_class(double D, double rs, double rt) {
-  // theta up to which 8, 12, 16, 24 and 32 terms reach 3^-32
-  constexpr double th[CL_NCLS] = {1.0 / 81.0, 0.0534, 1.0 / 9.0, 0.2311, CL_THETA};
+// strain: for the derivative.
+__device__ __forceinline__ int cl_class(double D, double rs, double rt, int strain) {
+  constexpr double vel[CL_NCLS] = {0.036, 0.085, 0.195, 0.293, 0.373};
+  constexpr double str[CL_NCLS] = {0.0286, 0.068, 0.167, 0.26, 0.337};
   const double a = D - rt, b = D - rs;
 #pragma unroll
-  for (int c = 0; c < CL_NCLS; ++c)
-    if (rs <= th[c] * a && rt <= th[c] * b) return c;
+  for (int c = 0; c < CL_NCLS; ++c) {
+    const double th = strain ? str[c] : vel[c];
+    if (rs <= th * a && rt <= th * b) return c;
+  }
   return CL_NCLS;
 }
 
 // The lists of target cluster blockIdx.x + tile0.  mask: bit c of node i's row
 // (node index less mask0) marks the source curves that another rule evaluates
 // at that node; a cluster pair with any marked node stays in the near list.
-// expand = 0 puts every cluster there.  A body's own clusters are in neither
+// expand = 0 puts every cluster there; strain: see cl_class.  A body's own clusters are in neither
 // list (k_self64); the wall's are, its own pairs included.  pairs[0], pairs[1]
 // += node pairs of the near lists with wall and with body sources, unmasked
 // (nullptr: not counted).
 __global__ void __launch_bounds__(256)
 k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
-           const double* __restrict__ rad, const unsigned* __restrict__ mask, int mw, int mask0, int expand,
+           const double* __restrict__ rad, const unsigned* __restrict__ mask, int mw, int mask0, int expand, int strain,
            int* __restrict__ near, int* __restrict__ far, double* __restrict__ lnd, int2* __restrict__ ncnt,
            int* __restrict__ fcls, unsigned long long* __restrict__ pairs) {
   extern __shared__ int marked[];   // marked nodes of this cluster per source curve
@@ -152,7 +162,7 @@ k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const
     if (S.z > 0 && S.z == T.z) return -1;
     D = sqrt(cabs2(csub(ct, cen[s])));
     if (!expand || (mask && marked[S.z])) return CL_NCLS;
-    return cl_class(D, rad[s], rt);
+    return cl_class(D, rad[s], rt, strain);
   };
   // sizes
   unsigned long long pw = 0, pb = 0;
@@ -221,19 +231,20 @@ k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const
   if (lane == 0 && pb) atomicAdd(pairs + 1, pb);
 }
 
-// Multipoles of cluster blockIdx.x + tile0: mp[t][0..31] = a_k, [32..63] = x_k,
-// [64..95] = k a_(k-1) / R (entry 0: 2 q L of the stokeslet), lam[t] = -2 q L.
+// The first 8 NP multipoles of cluster blockIdx.x + tile0: mp[t][0..39] = a_k, [40..79]
+// = x_k, [80..119] = k a_(k-1) / R (entry 0: 2 q L of the stokeslet), lam[t] = -2 q L.
 // den: the density the stokeslets and rotlets are read from (nullptr: none).
-// Warp w sums the powers 4w..4w+3 over all nodes, a node per lane: 11 complex
-// products a node instead of a chain of 32, then the lanes meet in a fixed
-// tree.  Bound by latency (a few hundred FP64 operations per thread).
+// Warp w sums the powers NP w .. NP w + NP - 1 over all nodes, a node per lane: 15
+// complex products a node (NP = 5) instead of a chain of 40, then the lanes meet in a
+// fixed tree.  Bound by latency (a few hundred FP64 operations per thread).
+template <int NP>
 __global__ void __launch_bounds__(256)
 k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
           const double* __restrict__ rad, const double4* __restrict__ sq, const double* __restrict__ den,
           double2* __restrict__ mp, double2* __restrict__ lam) {
   __shared__ double2 sA[FAR_TS], sT[FAR_TS];
   __shared__ double sB[FAR_TS];
-  __shared__ double2 ka[CL_P], ke[CL_P], kb[CL_P];
+  __shared__ double2 ka[8 * NP], ke[8 * NP], kb[8 * NP];
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
   const double2 c = cen[t];
@@ -246,17 +257,18 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
   }
   __syncthreads();
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double a[4][6];
+  double a[NP][6];
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < NP; ++q)
 #pragma unroll
     for (int v = 0; v < 6; ++v) a[q][v] = 0.0;
   for (int j = lane; j < T.y; j += 32) {
     const double2 A = sA[j], tj = sT[j];
     const double B = sB[j];
-    double2 p = make_double2(1.0, 0.0);   // t^(4 wid)
-    double2 tp = cmul(tj, tj);
-    tp = cmul(tp, tp);
+    double2 p = make_double2(1.0, 0.0);   // t^(NP wid)
+    double2 tp = tj;
+#pragma unroll
+    for (int q = 1; q < NP; ++q) tp = cmul(tp, tj);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       if ((wid >> b) & 1) p = cmul(p, tp);
@@ -264,7 +276,7 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
     }
     const double2 At = cmul(A, make_double2(tj.x, -tj.y));
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < NP; ++q) {
       cfma2(a[q][0], a[q][1], A, p);
       cfma2(a[q][2], a[q][3], At, p);
       a[q][4] = fma(B, p.x, a[q][4]);
@@ -273,20 +285,20 @@ k_cl_form(GeoDev G, int tile0, const int4* __restrict__ tiles, const double2* __
     }
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < NP; ++q)
 #pragma unroll
     for (int v = 0; v < 6; ++v) a[q][v] = warp_sum(a[q][v]);
   if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ka[4 * wid + q] = make_double2(a[q][0], a[q][1]);
-      ke[4 * wid + q] = make_double2(a[q][2], a[q][3]);
-      kb[4 * wid + q] = make_double2(a[q][4], a[q][5]);
+    for (int q = 0; q < NP; ++q) {
+      ka[NP * wid + q] = make_double2(a[q][0], a[q][1]);
+      ke[NP * wid + q] = make_double2(a[q][2], a[q][3]);
+      kb[NP * wid + q] = make_double2(a[q][4], a[q][5]);
     }
   }
   __syncthreads();
   const int k = threadIdx.x;
-  if (k >= CL_P) return;
+  if (k >= 8 * NP) return;
   double2 x = kb[k], d = make_double2(0, 0);
   if (k > 0) {
     x = make_double2(fma(-(double)k, ke[k - 1].x, x.x), fma(-(double)k, ke[k - 1].y, x.y));
@@ -327,28 +339,29 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double
 // from k to k + 4.  The products stay in registers until they are scaled by
 // (-R'/D)^l and added to the lane's sums, which the warps combine at the end in
 // a fixed order.  Bound by the FP64 pipe, which the tensor-core products share:
-// of ~450 operations per lane for two sources of order 32, 256 are products.
-// All far pairs at order 32 took 180 us at 400 bodies x 256 nodes (236 us with
-// the binomials in 64 registers and half the warps), by classes 87 us.
+// of ~450 operations per lane for two sources of 32 x 32 terms, 256 are products.
+// The velocity at 400 bodies x 256 nodes takes 101 us, at 200 x 256 67 us, at
+// 100 x 256 27 us (all pairs with 32 x 32 terms took 180 us at the first).
 struct ClShared {
   double P[CL_P * CL_P];
   double2 red[8][CL_P][2];
   double2 loc[2][CL_P];
 };
 
-// The entries [i0, i1) of the far list with 8 LT local and 4 KT multipole terms.
-template <int LT, int KT>
-__device__ __forceinline__ void cl_shift_run(const ClView& L, int t, int i0, int i1, const double2* __restrict__ mp,
-                                             const double2* __restrict__ lam, const double* P, double (&ax)[4],
-                                             double (&ay)[4]) {
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// The entries [i0, i1) of the far list with 8 LT local and 4 KT multipole terms; w: which of
+// the eight warps this one is here.
+template <int LT, int KT, int NL>
+__device__ __forceinline__ void cl_shift_run(const ClView& L, int t, int i0, int i1, int w,
+                                             const double2* __restrict__ mp, const double2* __restrict__ lam,
+                                             const double* P, double (&ax)[NL], double (&ay)[NL]) {
+  const int lane = threadIdx.x & 31;
   const double2 ct = L.cen[t];
   const double rt = L.rad[t];
   const int* __restrict__ far = L.far + (size_t)t * L.T;
   const double* __restrict__ lnd = L.lnd + (size_t)t * L.T;
   const int kq = lane & 3, bsrc = lane >> 4, bfn = (lane >> 3) & 1, bri = (lane >> 2) & 1;
   const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
-  for (int i = i0 + 2 * wid; i < i1; i += 16) {
+  for (int i = i0 + 2 * w; i < i1; i += 16) {
     const bool vb = i + bsrc < i1;
     const int s = far[min(i + bsrc, i1 - 1)];
     const double2 D = csub(ct, L.cen[s]);
@@ -373,7 +386,7 @@ __device__ __forceinline__ void cl_shift_run(const ClView& L, int t, int i0, int
       cfma2(y.x, y.y, kap, d);
       const double b = bri ? fma(y.x, g.y, y.y * g.x) : fma(y.x, g.x, -y.y * g.y);
 #pragma unroll
-      for (int lt = 0; lt < LT; ++lt) mma_f64(c0[lt], c1[lt], P[(lt * 8 + kt) * 32 + lane], b);
+      for (int lt = 0; lt < LT; ++lt) mma_f64(c0[lt], c1[lt], P[(lt * (CL_P / 4) + kt) * 32 + lane], b);
       if (kt + 1 < KT) g = cmul(g, q4);
     }
     // scale by (-R'/D)^l of the lane's own source
@@ -399,41 +412,47 @@ __device__ __forceinline__ void cl_shift_run(const ClView& L, int t, int i0, int
   }
 }
 
-// wall_only: only the wall's clusters as sources, to single precision (half the
-// terms, 3^-16 of a cluster's field): the preconditioner's coupling.  strain:
-// one class more, for the derivative.
-enum ClUse { CL_VELOCITY, CL_STRAIN, CL_WALL32 };
+// CL_WALL32: only the wall's clusters as sources, to single precision (a cut of 8e-8 of a
+// source's field, an ulp being 1.2e-7): the preconditioner's coupling.
+enum ClUse { CL_ALL, CL_WALL32 };
+
+// Local terms that a use fills.
+constexpr int cl_terms(int use) { return use == CL_WALL32 ? 24 : CL_P; }
 
 template <int USE>
 __device__ __forceinline__ void cl_shift(const ClView& L, int t, const double2* __restrict__ mp,
                                          const double2* __restrict__ lam, ClShared& sh) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
-  for (int e = threadIdx.x; e < CL_P * CL_P; e += blockDim.x) {
-    const int ln = e & 31, kt = (e >> 5) & 7, lt = e >> 8;
+  constexpr int NL = cl_terms(USE) / 8;
+  for (int e = threadIdx.x; e < NL * 8 * CL_P; e += blockDim.x) {
+    const int ln = e & 31, kt = (e >> 5) % (CL_P / 4), lt = (e >> 5) / (CL_P / 4);
     sh.P[e] = kBinom.c[8 * lt + (ln >> 2)][4 * kt + (ln & 3)];
   }
   __syncthreads();
-  double ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
+  double ax[NL] = {}, ay[NL] = {};
   const int* __restrict__ f = L.fcls + (size_t)t * (2 * CL_NCLS + 1);
   constexpr int E = USE == CL_WALL32 ? CL_NCLS + 1 : 1;   // ends of the wall's entries, or of all
-#define EB_RUN(C, LT, KT) cl_shift_run<LT, KT>(L, t, f[C], f[C + E], mp, lam, sh.P, ax, ay)
+  // pairs of the classes before: the warps go on in turn instead of from the first in
+  // every class (a mixed step of 100 bodies 171 ms, 177; of 200 bodies 1.5% less)
+  int at = 0;
+#define EB_RUN(C, LT, KT)                                                                  \
+  cl_shift_run<LT, KT>(L, t, f[C], f[C + E], (wid - at) & 7, mp, lam, sh.P, ax, ay);       \
+  at += (f[C + E] - f[C] + 1) >> 1
   if constexpr (USE == CL_WALL32) {
-    EB_RUN(0, 1, 1); EB_RUN(1, 1, 2); EB_RUN(2, 1, 2); EB_RUN(3, 2, 3); EB_RUN(4, 2, 4);
-  } else if constexpr (USE == CL_STRAIN) {
-    EB_RUN(0, 2, 3); EB_RUN(1, 2, 4); EB_RUN(2, 3, 6); EB_RUN(3, 4, 8); EB_RUN(4, 4, 8);
+    EB_RUN(0, 1, 2); EB_RUN(1, 1, 2); EB_RUN(2, 2, 3); EB_RUN(3, 2, 4); EB_RUN(4, 3, 5);
   } else {
-    EB_RUN(0, 1, 2); EB_RUN(1, 2, 3); EB_RUN(2, 2, 4); EB_RUN(3, 3, 6); EB_RUN(4, 4, 8);
+    EB_RUN(0, 2, 3); EB_RUN(1, 2, 4); EB_RUN(2, 3, 6); EB_RUN(3, 4, 8); EB_RUN(4, 5, 10);
   }
 #undef EB_RUN
 #pragma unroll
-  for (int lt = 0; lt < 4; ++lt) {
+  for (int lt = 0; lt < NL; ++lt) {
     ax[lt] += __shfl_xor_sync(0xffffffffu, ax[lt], 2);
     ay[lt] += __shfl_xor_sync(0xffffffffu, ay[lt], 2);
     if (csrc == 0) sh.red[wid][8 * lt + row][cfn] = make_double2(ax[lt], ay[lt]);
   }
   __syncthreads();
-  if (threadIdx.x < 2 * CL_P) {
+  if (threadIdx.x < 16 * NL) {
     const int l = threadIdx.x >> 1, fn = threadIdx.x & 1;
     double2 v = sh.red[0][l][fn];
 #pragma unroll
@@ -449,6 +468,7 @@ __global__ void __launch_bounds__(256, 2)
 k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ mp,
            const double2* __restrict__ lam, double2* __restrict__ out) {
   __shared__ ClShared sh;
+  constexpr int TL = cl_terms(USE);
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
   cl_shift<USE>(L, t, mp, lam, sh);
@@ -456,9 +476,9 @@ k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const 
   const double iR = 1.0 / L.rad[t];
   for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
     const double2 w = cscale(csub(G.xy[T.x + j], c), iR);
-    double2 f = sh.loc[0][CL_P - 1], df = make_double2(0, 0), x = sh.loc[1][CL_P - 1];
+    double2 f = sh.loc[0][TL - 1], df = make_double2(0, 0), x = sh.loc[1][TL - 1];
 #pragma unroll 4
-    for (int l = CL_P - 2; l >= 0; --l) {
+    for (int l = TL - 2; l >= 0; --l) {
       df = cadd(cmul(df, w), f);
       f = cadd(cmul(f, w), sh.loc[0][l]);
       x = cadd(cmul(x, w), sh.loc[1][l]);
@@ -470,18 +490,16 @@ k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const 
 
 // The separated sources' strain at the nodes of cluster blockIdx.x + tile0:
 // du/d(conj z) = 1/4 [ -z conj(phi'') + conj(chi') ] = (E11 - E22)/2 + i E12, and
-// the field is free of divergence (E22 = -E11).  out[i] = (E11, E12).  The
-// cut of the series, 3^-32 of a cluster's field, grows by the 32 of the
-// derivative and by |D|/R' against that field's own gradient: 1e-13.  With the
-// near lists' strain 626 us at 400 bodies x 256 nodes, where the trapezoid sum
-// over every pair took 30.8 ms.
+// the field is free of divergence (E22 = -E11).  out[i] = (E11, E12).
+// 121 us at 400 bodies x 256 nodes, with the near lists' strain 530 us, where the
+// trapezoid sum over every pair took 30.8 ms.
 __global__ void __launch_bounds__(256, 2)
 k_cl_shift_strain(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ mp,
                   const double2* __restrict__ lam, double2* __restrict__ out) {
   __shared__ ClShared sh;
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
-  cl_shift<CL_STRAIN>(L, t, mp, lam, sh);
+  cl_shift<CL_ALL>(L, t, mp, lam, sh);
   const double2 c = L.cen[t];
   const double iR = 1.0 / L.rad[t];
   for (int j = threadIdx.x; j < T.y; j += blockDim.x) {
@@ -740,11 +758,11 @@ static inline ClView cl_view(const State& s, const ClLists& L) {
 // Lists of the target clusters from tile0 on (mask as k_cl_lists takes it).
 // pairs: see k_cl_lists, or nullptr.
 static inline void build_lists(State& s, ClLists& L, int tile0, const unsigned* mask, int mw, int mask0, bool expand,
-                               unsigned long long* pairs) {
+                               bool strain, unsigned long long* pairs) {
   const size_t T = s.ntile;
   const size_t smem = mask ? 32 * (size_t)mw * sizeof(int) : 0;
   k_cl_lists<<<(unsigned)(T - tile0), 256, smem, s.st>>>(
-      s.geo(), s.ntile, tile0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, mask, mw, mask0, expand, L.near.ensure(T * T),
+      s.geo(), s.ntile, tile0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, mask, mw, mask0, expand, strain, L.near.ensure(T * T),
       L.far.ensure(T * T), L.lnd.ensure(T * T), L.ncnt.ensure(T), L.fcls.ensure(T * (2 * CL_NCLS + 1)), pairs);
   EB_LAUNCH_CHECK();
 }

@@ -238,7 +238,7 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     EB_LAUNCH_CHECK();
     k_cl_geom<<<nblk(ntile, 4), 128, 0, st>>>(G, ntile, tiles, ccen, crad);
     EB_LAUNCH_CHECK();
-    k_cl_lists<<<ntile, 256, 0, st>>>(G, ntile, 0, tiles, ccen, crad, nullptr, 0, 0, expand, near, far, lnd, ncnt, fcls,
+    k_cl_lists<<<ntile, 256, 0, st>>>(G, ntile, 0, tiles, ccen, crad, nullptr, 0, 0, expand, 0, near, far, lnd, ncnt, fcls,
                                       nullptr);
     EB_LAUNCH_CHECK();
     ClView L;
@@ -247,9 +247,9 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     k_cl_near64<false, false><<<dim3(nitem, parts), 256, 0, st>>>(G, L, items, tiles, 0, sq64, nullptr, 0, 0, partial);
     EB_LAUNCH_CHECK();
     if (expand) {
-      k_cl_form<<<ntile, 256, 0, st>>>(G, 0, tiles, ccen, crad, sq64, sing ? d_den : nullptr, mp, lam);
+      k_cl_form<CL_P / 8><<<ntile, 256, 0, st>>>(G, 0, tiles, ccen, crad, sq64, sing ? d_den : nullptr, mp, lam);
       EB_LAUNCH_CHECK();
-      k_cl_shift<CL_VELOCITY><<<ntile, 256, 0, st>>>(G, L, 0, tiles, mp, lam, partial + (size_t)parts * N);
+      k_cl_shift<CL_ALL><<<ntile, 256, 0, st>>>(G, L, 0, tiles, mp, lam, partial + (size_t)parts * N);
       EB_LAUNCH_CHECK();
     }
     if (M > 0) {

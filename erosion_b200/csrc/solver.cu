@@ -465,10 +465,10 @@ static void launch_near32(State& s, double2* out) {
 // Expansions of every cluster and their sum over the far lists into out[N].
 static void launch_expansions(State& s, const double* d_den, double2* out) {
   const GeoDev G = s.geo();
-  k_cl_form<<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p, s.cl_sing ? d_den : nullptr,
+  k_cl_form<CL_P / 8><<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p, s.cl_sing ? d_den : nullptr,
                                        s.cl_mp.p, s.cl_lam.p);
   EB_LAUNCH_CHECK();
-  k_cl_shift<CL_VELOCITY><<<s.ntile, 256, 0, s.st>>>(G, cl_view(s, s.cl), 0, s.tiles.p, s.cl_mp.p, s.cl_lam.p, out);
+  k_cl_shift<CL_ALL><<<s.ntile, 256, 0, s.st>>>(G, cl_view(s, s.cl), 0, s.tiles.p, s.cl_mp.p, s.cl_lam.p, out);
   EB_LAUNCH_CHECK();
 }
 
@@ -486,7 +486,7 @@ static void launch_wall_coupling(State& s, double2* out) {
     join(s, 0);
     return;
   }
-  k_cl_form<<<s.nwall_tiles, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.pc_sq64.p, nullptr, s.cl_mp.p,
+  k_cl_form<3><<<s.nwall_tiles, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.pc_sq64.p, nullptr, s.cl_mp.p,
                                              s.cl_lam.p);
   EB_LAUNCH_CHECK();
   k_cl_shift<CL_WALL32><<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,
@@ -517,7 +517,7 @@ static void build_near(State& s) {
                                     info);
     EB_LAUNCH_CHECK();
   }
-  if (s.cl_active) build_lists(s, s.cl, 0, mode ? nr.mask.p : nullptr, nr.mw, 0, s.cl_expand, info->cl);
+  if (s.cl_active) build_lists(s, s.cl, 0, mode ? nr.mask.p : nullptr, nr.mw, 0, s.cl_expand, false, info->cl);
   NearInfo hinfo;
   d2h(&hinfo, info, 1, st);
   EB_CK(cudaStreamSynchronize(st));

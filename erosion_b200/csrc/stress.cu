@@ -1030,7 +1030,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
       ClLists& lists = s.cl_stress;
       k_prep<<<pr.M + nblk(pr.nout, 256), 256, 0, s.st>>>(G, d_den, s.ws.p, s.sq64.p, s.sq32.p, s.d_w.ensure(pr.ntot), s.sigdotn.p, 1);
       EB_LAUNCH_CHECK();
-      build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand, nullptr);
+      build_lists(s, lists, s.nwall_tiles, smask.p, mw, pr.nout, s.cl_expand, true, nullptr);
       const ClView L = cl_view(s, lists);
       const int parts = near_parts(nit, eb_num_sms());
       s.partial.ensure((size_t)(parts + 1) * pr.N);
@@ -1038,7 +1038,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
                                                                   pr.nout, s.partial.p);
       EB_LAUNCH_CHECK();
       if (s.cl_expand) {
-        k_cl_form<<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p,
+        k_cl_form<CL_P / 8><<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p,
                                              s.cl_sing ? d_den : nullptr, s.cl_mp.p, s.cl_lam.p);
         EB_LAUNCH_CHECK();
         k_cl_shift_strain<<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,

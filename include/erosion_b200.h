@@ -44,7 +44,7 @@ enum {
  * on entry and the solution on exit; nits receives the GMRES iterations.
  * ifmm is accepted for ABI compatibility: the far field is summed directly
  * between close clusters of nodes and through expansions cut at FP64 rounding
- * (5e-16 of a cluster's field) between separated ones.
+ * (5e-16 of a source's field) between separated ones.
  * ibary = 1 applies the barycentric near-singular corrections with the
  * selection rules of matvec_DLP_fmmbary (ifmm = 1) or to every pair of
  * distinct curves as matvec_DLP_bary does (ifmm = 0); ibary = 0 is the
