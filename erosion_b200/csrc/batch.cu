@@ -14,15 +14,12 @@
 // those of more geometries than the next call has are freed by it, all of them by
 // erosion_release.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
-#include <exception>
-#include <functional>
 #include <memory>
-#include <thread>
 #include <vector>
 
+#include "pool.h"
 #include "state.h"
 
 namespace eb {
@@ -55,28 +52,11 @@ void destroy_member(Member& mb) {
   mb.b.release();
 }
 
-// Runs f(0), ..., f(n - 1) on a pool of host threads, in the order of `order`; the
-// first exception is thrown again once all have ended.
-void on_pool(int device, const std::vector<int>& order, const std::function<void(int)>& f) {
-  const int n = (int)order.size();
-  const int threads = std::max(1, std::min<int>(n, std::min(16u, std::max(1u, std::thread::hardware_concurrency()))));
-  std::atomic<int> next{0};
-  std::atomic<bool> stop{false};
-  std::vector<std::exception_ptr> errs(threads);
-  std::vector<std::thread> pool;
-  for (int t = 0; t < threads; ++t)
-    pool.emplace_back([&, t] {
-      try {
-        EB_CK(cudaSetDevice(device));
-        for (int i; !stop && (i = next++) < n;) f(order[i]);
-      } catch (...) {
-        errs[t] = std::current_exception();
-        stop = true;
-      }
-    });
-  for (auto& th : pool) th.join();
-  for (auto& e : errs)
-    if (e) std::rethrow_exception(e);
+// Runs f for every geometry, in the order of `order`, on a pool of host threads.
+template <class F>
+void for_each(int device, const std::vector<int>& order, F&& f) {
+  const int threads = (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+  on_pool(threads, order, [device] { EB_CK(cudaSetDevice(device)); }, f);
 }
 
 }  // namespace ensemble
@@ -137,7 +117,7 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
     cudaStream_t st = lib.st;
     EB_CK(cudaEventRecord(B.a, st));
     const auto t_setup = std::chrono::steady_clock::now();
-    on_pool(lib.device, order, [&](int g) {
+    for_each(lib.device, order, [&](int g) {
       Member& mb = *B.m[g];
       State& s = mb.s;
       init_state(s, lib.device);
@@ -158,7 +138,7 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
     });
     B.stats.setup_host_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_setup).count();
-    on_pool(lib.device, order, [&](int g) {
+    for_each(lib.device, order, [&](int g) {
       Member& mb = *B.m[g];
       State& s = mb.s;
       const long long n = s.pr.ntot, maxl = std::min<long long>(P.maxl > 0 ? P.maxl : 10, n);
