@@ -1863,8 +1863,13 @@ int erosion_get_far_shapes(int32_t* shape, int32_t* desc, float* ms, int32_t* nu
     try {
       plan_far(s, true);
     } catch (const Error& e) {
+      settle(s);
       set_status(e.code, e.what());
       return e.code;
+    } catch (const std::exception& e) {
+      settle(s);
+      set_status(EROSION_CUDA_ERROR, e.what());
+      return EROSION_CUDA_ERROR;
     }
   }
   for (int kind = 0; kind < kFarKinds; ++kind) {
@@ -1889,14 +1894,17 @@ int64_t erosion_near_info(int64_t* lw, int64_t* wall_bodies, int64_t* near_pairs
   std::lock_guard<std::mutex> lk(s.mu);
   if (lw) *lw = s.near.lw;
   int64_t count = 0;
-  if (s.near.rules && s.near.wflag.p && s.pr.M > 0) {
-    std::vector<int> f(s.pr.M);
-    if (cudaMemcpy(f.data(), s.near.wflag.p, f.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) f.clear();
-    for (size_t b = 0; b < f.size(); ++b)
-      if (f[b]) {
-        if (wall_bodies) wall_bodies[count] = (int64_t)b;
-        ++count;
-      }
+  if (s.near.rules && s.near.wflag.p) {
+    int f[256];   // read in pieces: no allocation that could throw
+    for (int b0 = 0; b0 < s.pr.M; b0 += 256) {
+      const int k = std::min(256, s.pr.M - b0);
+      if (cudaMemcpy(f, s.near.wflag.p + b0, k * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) break;
+      for (int b = 0; b < k; ++b)
+        if (f[b]) {
+          if (wall_bodies) wall_bodies[count] = b0 + b;
+          ++count;
+        }
+    }
   }
   if (near_pairs) *near_pairs = s.near.npairs;
   return count;

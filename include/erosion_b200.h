@@ -117,10 +117,10 @@ typedef struct {
                            (reciprocal to ~1e-12 instead of FP64 rounding) while the
                            residual is above relax_tol and to the wall's sources
                            after, 0 the accurate one; true residuals always use
-                           the accurate one.  Only the direct sums of a forced
-                           launch shape (erosion_set_far_shape) and of the ensemble
-                           distinguish the two; the sums by clusters are always
-                           accurate                                               */
+                           the accurate one.  Only the direct sums (a forced launch
+                           shape, erosion_set_far_shape, or more than 4096
+                           clusters) distinguish the two; the sums by clusters
+                           are always accurate                                    */
   int32_t precond_refresh; /* block preconditioner: 0 or 1 rebuilds the body blocks
                            at every set-up; k > 1 keeps the previous inverses for up
                            to k - 1 further set-ups of the same size (consecutive
@@ -445,12 +445,12 @@ double erosion_peak_tflops(int32_t precision);
 
 /* Far-field launch shapes (extended API; the reference's FMM has no
  * counterpart).  Each far-field kernel has a list of candidate CTA shapes
- * (threads per CTA x targets per thread x variant); by default an autotuner
- * times every candidate on the geometry at hand the first time a problem of
- * that size is set up (problems above 2e8 node pairs) and keeps the fastest.
- * The shapes are those of the direct sum over every pair, which runs when one
- * is forced and for more than 4096 clusters (wall arcs of 32
- * nodes and bodies of up to 256); otherwise the far field is summed by clusters.
+ * (threads per CTA x targets per thread x variant).  They are the shapes of the
+ * direct sum over every pair, which runs when one is forced and for more than
+ * 4096 clusters (wall arcs of 32 nodes and bodies of up to 256); otherwise the far
+ * field is summed by clusters.  For the direct sum an autotuner times every
+ * candidate on the geometry at hand the first time a problem of that size is set
+ * up (problems above 2e8 node pairs) and keeps the fastest.
  * erosion_set_far_shape(kind, shape) forces candidate 'shape' (kind 0 = the
  * accurate FP64 kernel, 1 = the FP32 kernel, 2 = the fast FP64 kernel of the
  * mixed solve's early iterations) from the next set-up on; shape = -1
@@ -467,7 +467,10 @@ int erosion_set_far_shape(int32_t kind, int32_t shape);
  * kernel the unroll factor of the source loop plus 10 x the resident CTAs
  * per SM it is compiled for (its register budget).  ms[8*kind + i] = the
  * autotuner's time of candidate i in milliseconds (0 when not timed;
- * capacity 24).  Any pointer may be NULL. */
+ * capacity 24).  Any pointer may be NULL.  When the last problem was summed by
+ * clusters and has more than 2e8 node pairs, the call times the candidates on it
+ * first (milliseconds of GPU time, and device memory for their partial sums);
+ * otherwise it only reads. */
 int erosion_get_far_shapes(int32_t* shape, int32_t* desc, float* ms, int32_t* num_shapes);
 
 /* ------------------------------------------------------------------------

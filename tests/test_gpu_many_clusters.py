@@ -70,3 +70,16 @@ def test_stress(lib, lattice, density):
     tau_b, E_b = stokes.shear_stress(lattice, density, stress_all_bary=1)
     assert rel(tau, tau_b) < 1e-10
     assert rel(E, E_b) < 1e-10
+
+
+def test_near_wall_bodies(lib, lattice):
+    """The list of near-wall bodies comes back in pieces of 256: all of it, by the rule."""
+    g = lattice
+    stokes.matvec(g, np.zeros(g.ntot))
+    lw, bodies, _ = stokes.near_info(g.M)
+    speed = stokes.geometry(g)["speed"].reshape(g.M, N)
+    lim = g.wall[1] - (speed.mean(1) + 4 * lw * 2 * np.pi / NOUT)
+    y = g.yy.reshape(g.M, N).mean(1)
+    want = np.nonzero(np.abs(y) >= lim)[0]
+    assert 256 < len(want) < g.M and not (np.abs(np.abs(y) - lim) < 1e-9).any()
+    assert bodies == want.tolist()
