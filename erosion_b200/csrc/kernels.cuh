@@ -1717,9 +1717,11 @@ __device__ double2 bary_coincident(const GeoDev& G, int start, int len, const do
 // (69.6), of 400 x 256 25.0 us (78.1), and of 3200 targets against 50 x 128 + 1024 nodes 325 us (577).
 // CL > 1 (the wall's curve only): the CTAs of a cluster of CL hold the same targets,
 // take a share of the nodes each and add their sums through distributed shared memory.
-template <int NDER, int CL = 1>
+// SOLO: a warp has the curve to itself, staged by the caller from place `at` of the
+// tile on; nothing is shared, and each warp may have another curve.
+template <int NDER, int CL = 1, bool SOLO = false>
 __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c, const double2* __restrict__ bdc,
-                                            double2 zt, bool act) {
+                                            double2 zt, bool act, int at = 0) {
   const int start = curve_start(G, c), len = curve_len(G, c);
   int lo = 0, hi = len;   // this CTA's share
   if constexpr (CL > 1) {
@@ -1727,8 +1729,11 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
     lo = (int)((long long)len * rank / CL);
     hi = (int)((long long)len * (rank + 1) / CL);
   }
-  const bool ext = CL == 1 && c != 0, whole = hi - lo <= NEAR_TK;
+  const bool ext = CL == 1 && c != 0, whole = SOLO || hi - lo <= NEAR_TK;
   const int wid = threadIdx.x >> 5;
+  // this warp's part of kt staged sources
+  auto first = [&](int kt) { return SOLO ? at : kt * wid / NEAR_W; };
+  auto last = [&](int kt) { return SOLO ? at + kt : kt * (wid + 1) / NEAR_W; };
   constexpr int NF = NDER == 2 ? 5 : 3;   // fields: e, (v_1, v_2,) v_3, v_4
   double2 a = make_double2(0, 0);
   if (ext) a = G.cen[c - 1];
@@ -1745,11 +1750,10 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
 #pragma unroll
   for (int q = 0; q < 2 + 2 * NF; ++q) v1[q] = 0.0;
   for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
-    bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-    const int kt = min(NEAR_TK, hi - k0);
-    const int kb = kt * (wid + 1) / NEAR_W;
+    if (!SOLO) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
+    const int kt = min(NEAR_TK, hi - k0), kb = last(kt);
 #pragma unroll 2
-    for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
+    for (int kk = first(kt); kk < kb; ++kk) {
       const double2 c1 = cmul(T.dz[kk], bary_inv(csub(T.z[kk], zt)));
       v1[0] += c1.x;
       v1[1] += c1.y;
@@ -1757,7 +1761,7 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
       for (int q = 0; q < NF; ++q) cfma2(v1[2 + 2 * q], v1[3 + 2 * q], field(kk, q), c1);
     }
   }
-  near_reduce(v1, T.red);
+  if constexpr (!SOLO) near_reduce(v1, T.red);
   if constexpr (CL > 1) cluster_reduce<CL>(v1, T.red);
   const double2 den = make_double2(v1[0], v1[1]);
   double2 u[NF];
@@ -1775,10 +1779,9 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
   bool coinc = false;
   for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
     if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-    const int kt = min(NEAR_TK, hi - k0);
-    const int kb = kt * (wid + 1) / NEAR_W;
+    const int kt = min(NEAR_TK, hi - k0), kb = last(kt);
 #pragma unroll 2
-    for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
+    for (int kk = first(kt); kk < kb; ++kk) {
       const double2 d = csub(T.z[kk], zt);
       const double r2 = cabs2(d), ir = rcp_raw64(r2);
       const double2 inv = make_double2(d.x * ir, -d.y * ir);
@@ -1801,7 +1804,8 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
         for (int k = 0; k < len; ++k) {
           const double2 d = csub(G.xy[start + k], zt);
           const int kk = k % NEAR_TK, kt = min(NEAR_TK, len - (k - kk));
-          if (kk >= kt * wid / NEAR_W && kk < kt * (wid + 1) / NEAR_W && cabs2(d) <= 1e-20)
+          const bool mine = SOLO || (kk >= first(kt) && kk < last(kt));
+          if (mine && cabs2(d) <= 1e-20)
             add = cadd(add, bary_coincident(G, start, len, bdc, q, k, zt, a, tmp1, tmp2));
         }
         const double f = q == 0 ? 1.0 : q == 1 ? -zt.x : -zt.y;   // e = v_0 - x v_1 - y v_2
@@ -1812,7 +1816,7 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
       }
     }
   }
-  near_reduce(v2, T.red);
+  if constexpr (!SOLO) near_reduce(v2, T.red);
   if constexpr (CL > 1) cluster_reduce<CL>(v2, T.red);
   double2 du[ND];
   double2 fac;
@@ -1829,10 +1833,9 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
     double v3[2] = {0.0, 0.0};
     for (int k0 = lo; k0 < hi; k0 += NEAR_TK) {
       if (!whole) bary_load_tile(T, G, start, len, k0, bdc, ext, a);
-      const int kt = min(NEAR_TK, hi - k0);
-      const int kb = kt * (wid + 1) / NEAR_W;
+      const int kt = min(NEAR_TK, hi - k0), kb = last(kt);
 #pragma unroll 2
-      for (int kk = kt * wid / NEAR_W; kk < kb; ++kk) {
+      for (int kk = first(kt); kk < kb; ++kk) {
         const double2 d = csub(T.z[kk], zt);
         const double2 inv = bary_inv(d);
         const double2 c3 = cmul(cmul(cmul(T.dz[kk], inv), inv), inv);
@@ -1840,8 +1843,8 @@ __device__ __forceinline__ DLPVal bary_eval(BaryTile& T, const GeoDev& G, int c,
         cfma2(v3[0], v3[1], t, c3);
       }
     }
-    near_reduce(v3, T.red);
-  if constexpr (CL > 1) cluster_reduce<CL>(v3, T.red);
+    if constexpr (!SOLO) near_reduce(v3, T.red);
+    if constexpr (CL > 1) cluster_reduce<CL>(v3, T.red);
     const double2 e = cscale(cmul(make_double2(v3[0], v3[1]), fac), 2.0);
     r.u1x = e.x - du[1].x + du[3].x;
     r.u1y = -e.y - du[2].x - du[3].y;

@@ -12,11 +12,29 @@ __device__ __forceinline__ long long bd_all_off(const GeoDev& G, int c) {
   return c == 0 ? 0LL : 5LL * G.nout + 5LL * (c - 1) * G.n;
 }
 
+// Parts of the source curves of about as many nodes each: the first curve of part y, the
+// one with N y / parts nodes or more before it.
+__device__ __forceinline__ int part_first(const GeoDev& G, int y, int parts) {
+  const long long at = (long long)G.N * y / parts;
+  if (y == parts) return G.M + 1;
+  return at == 0 ? 0 : at <= G.nout ? 1 : 1 + (int)((at - G.nout + G.n - 1) / G.n);
+}
+
+// Longest body curve that a warp takes by itself (k_bary_sum): a stage of the tile holds
+// eight of them or more.  With eight warps sharing a curve's nodes the block sums after
+// each of the three passes cost more than the nodes do: 20,000 targets (60,000) against
+// 500 bodies of 8 nodes take 1.8 ms (4.2) by warps and 5.9 (14.5) shared, 1000 of 16 nodes
+// 5.2 (13.1) and 13.4 (33.1), 500 of 32 nodes 4.9 (12.5) and 8.9 (22.2); 100 targets against
+// the last 0.32 and 0.33.
+constexpr int SHORT_CURVE = NEAR_TK / NEAR_W;
+
 // Barycentric Stokes DLP with gradient of the source curves of part blockIdx.y
 // of gridDim.y at 32 targets: CTA blockIdx.x takes targets 32 blockIdx.x.. of all
 // ntar, or with bodies = 1 (the targets are the body nodes) 32 nodes of one body,
 // skipping that body's curve.  Partial sums per part: out[(y*6 + q)*ntar + t] with
-// q = ux, uy, u1x, u1y, u2x, u2y.
+// q = ux, uy, u1x, u1y, u2x, u2y.  SHORT: the bodies' curves are staged many at a time and
+// a warp takes every eighth.
+template <bool SHORT>
 __global__ void __launch_bounds__(NEAR_NT, 2)
 k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const double2* __restrict__ txy, int bodies, int ntar,
            double* __restrict__ out) {
@@ -24,26 +42,62 @@ k_bary_sum(GeoDev G, const double2* __restrict__ bd_all, const double2* __restri
   const int per = bodies ? (G.n + NEAR_T - 1) / NEAR_T : 0, b = bodies ? blockIdx.x / per : -1;
   const int t0 = bodies ? b * G.n + NEAR_T * (blockIdx.x - b * per) : NEAR_T * blockIdx.x;
   const int t1 = bodies ? min((b + 1) * G.n, t0 + NEAR_T) : min(ntar, t0 + NEAR_T);
-  const int t = t0 + (threadIdx.x & 31);
+  const int t = t0 + (threadIdx.x & 31), wid = threadIdx.x >> 5;
   const bool act = t < t1;
   const double2 zt = txy[act ? t : t1 - 1];
   double a[6] = {0, 0, 0, 0, 0, 0};
-  // parts of about as many nodes each: part y starts at the first curve with N y / gridDim.y
-  // nodes or more before it
-  auto first = [&](int y) {
-    const long long at = (long long)G.N * y / gridDim.y;
-    return at == 0 ? 0 : at <= G.nout ? 1 : 1 + (int)((at - G.nout + G.n - 1) / G.n);
-  };
-  const int c1 = blockIdx.y + 1 == gridDim.y ? G.M + 1 : first(blockIdx.y + 1);
-  for (int c = first(blockIdx.y); c < c1; ++c) {
-    if (c == b + 1 && bodies) continue;
-    DLPVal r = bary_eval<2>(T, G, c, bd_all + bd_all_off(G, c), zt, act);
+  auto add = [&](const DLPVal& r) {
     a[0] += r.ux; a[1] += r.uy; a[2] += r.u1x; a[3] += r.u1y; a[4] += r.u2x; a[5] += r.u2y;
+  };
+  int c = part_first(G, blockIdx.y, gridDim.y);
+  const int c1 = part_first(G, blockIdx.y + 1, gridDim.y);
+  if constexpr (SHORT) {
+    if (c == 0 && c1 > 0) {   // the wall by all warps; each holds the sum
+      const DLPVal r = bary_eval<2>(T, G, 0, bd_all, zt, act);
+      if (wid == 0) add(r);
+      c = 1;
+    }
+    const int stage = NEAR_TK / G.n / NEAR_W * NEAR_W;   // bodies staged at a time
+    for (; c < c1; c += stage) {
+      const int k = min(stage, c1 - c);
+      __syncthreads();
+      if ((int)threadIdx.x < k * G.n) {
+        const int e = threadIdx.x / G.n, j = threadIdx.x - e * G.n, g = curve_start(G, c) + (int)threadIdx.x;
+        const double2 z = G.xy[g];
+        const double2* __restrict__ bdc = bd_all + bd_all_off(G, c + e) + j;
+        T.z[threadIdx.x] = z;
+        T.dz[threadIdx.x] = G.dz[g];
+        T.za[threadIdx.x] = cinv(csub(z, G.cen[c + e - 1]));
+#pragma unroll
+        for (int q = 0; q < 5; ++q) T.b[q][threadIdx.x] = bdc[q * G.n];
+      }
+      __syncthreads();
+      for (int e = wid; e < k; e += NEAR_W)
+        if (c + e != b + 1 || !bodies)
+          add(bary_eval<2, 1, true>(T, G, c + e, bd_all + bd_all_off(G, c + e), zt, act, e * G.n));
+    }
+    __syncthreads();
+    near_reduce(a, T.red);
+  } else {
+    for (; c < c1; ++c)
+      if (c != b + 1 || !bodies) add(bary_eval<2>(T, G, c, bd_all + bd_all_off(G, c), zt, act));
   }
   if (act && threadIdx.x < 32) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) out[((size_t)blockIdx.y * 6 + q) * ntar + t] = a[q];
   }
+}
+
+// Launches k_bary_sum for tasks CTAs of targets and the parts of the curves.
+static void bary_sum(State& s, int tasks, int parts, const double2* bd_all, const double2* txy, int bodies, int ntar,
+                     double* out) {
+  const GeoDev G = s.geo();
+  const dim3 grid(tasks, parts);
+  if (G.M > 0 && G.n <= SHORT_CURVE)
+    k_bary_sum<true><<<grid, NEAR_NT, 0, s.st>>>(G, bd_all, txy, bodies, ntar, out);
+  else
+    k_bary_sum<false><<<grid, NEAR_NT, 0, s.st>>>(G, bd_all, txy, bodies, ntar, out);
+  EB_LAUNCH_CHECK();
 }
 
 // Self-interaction of each body for the deformation tensor: the odd-even
@@ -990,8 +1044,7 @@ void shear_stress(State& s, const double* d_den, double* d_tau, double* d_E) {
     bdval_all(s, d_den, bd_all, s.st);
     const int tasks = pr.M * (int)nblk(pr.n, NEAR_T), nsplit = bary_splits(tasks, pr.M + 1);
     part.ensure((size_t)nsplit * 6 * nb);
-    k_bary_sum<<<dim3(tasks, nsplit), NEAR_NT, 0, s.st>>>(G, bd_all.p, s.xy.p + pr.nout, 1, nb, part.p);
-    EB_LAUNCH_CHECK();
+    bary_sum(s, tasks, nsplit, bd_all.p, s.xy.p + pr.nout, 1, nb, part.p);
     k_stress_final<<<nblk(nb, 256), 256, 0, s.st>>>(G, d_den, part.p, nsplit, nullptr, 0, 1, eself.p, d_tau, d_E);
     EB_LAUNCH_CHECK();
   } else if (bary) {   // barycentric near pairs, trapezoid elsewhere
@@ -1104,8 +1157,7 @@ void qoi_targets(State& s, const double* d_den, long long ntar, const double* d_
     bdval_all(s, d_den, bd_all, s.st);
     ns2 = bary_splits(tasks, pr.M + 1);
     pbary.ensure((size_t)ns2 * 6 * ntar);
-    k_bary_sum<<<dim3(tasks, ns2), NEAR_NT, 0, s.st>>>(G, bd_all.p, txy.p, 0, (int)ntar, pbary.p);
-    EB_LAUNCH_CHECK();
+    bary_sum(s, tasks, ns2, bd_all.p, txy.p, 0, (int)ntar, pbary.p);
     k_qoi_trap<false><<<dim3(tasks, ns1), 256, 0, side>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
   } else {
     k_qoi_trap<true><<<dim3(tasks, ns1), 256, 0, side>>>(G, d_den, s.tiles.p, s.ntile, (int)ntar, txy.p, ptrap.p);
