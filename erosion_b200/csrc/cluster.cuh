@@ -126,7 +126,8 @@ __device__ __forceinline__ int cl_class(double D, double rs, double rt, int stra
 // expand = 0 puts every cluster there; strain: see cl_class.  A body's own clusters are in neither
 // list (k_self64); the wall's are, its own pairs included.  pairs[0], pairs[1]
 // += node pairs of the near lists with wall and with body sources, unmasked
-// (nullptr: not counted).
+// (nullptr: not counted).  With expand = 0, no mask and no count, cen, rad, far, lnd
+// and fcls are not touched.
 __global__ void __launch_bounds__(256)
 k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ cen,
            const double* __restrict__ rad, const unsigned* __restrict__ mask, int mw, int mask0, int expand, int strain,
@@ -137,6 +138,13 @@ k_cl_lists(GeoDev G, int ntile, int tile0, const int4* __restrict__ tiles, const
   __shared__ int tot[NC], wall[NC], at[NC], wcnt[8][NC];
   const int t = blockIdx.x + tile0;
   const int4 T = tiles[t];
+  if (!expand && !mask && !pairs) {   // every cluster but the own body's, in order
+    const int nwt = (G.nout + WALL_TS - 1) / WALL_TS, per = T.z > 0 ? (G.n + FAR_TS - 1) / FAR_TS : 0;
+    const int a = T.z > 0 ? nwt + (T.z - 1) * per : ntile;
+    for (int s = threadIdx.x; s < ntile - per; s += blockDim.x) near[(size_t)t * ntile + s] = s < a ? s : s + per;
+    if (threadIdx.x == 0) ncnt[t] = make_int2(nwt, ntile - per);
+    return;
+  }
   const double2 ct = cen[t];
   const double rt = rad[t];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
