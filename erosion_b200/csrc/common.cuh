@@ -48,11 +48,6 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-// a += b * c
-__device__ __forceinline__ void cfma(double2& a, double2 b, double2 c) {
-  a.x = fma(b.x, c.x, fma(-b.y, c.y, a.x));
-  a.y = fma(b.x, c.y, fma(b.y, c.x, a.y));
-}
 __device__ __forceinline__ double2 cinv(double2 a) {
   double d = 1.0 / fma(a.x, a.x, a.y * a.y);
   return make_double2(a.x * d, -a.y * d);

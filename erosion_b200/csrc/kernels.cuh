@@ -2119,10 +2119,10 @@ __global__ void k_copy(const double* __restrict__ a, double* __restrict__ out, l
 // Arnoldi steps whose column count lives in device memory (*kp), so that one
 // captured CUDA graph serves every iteration of a GMRES cycle.
 
-// h[j] = sum_b part[j][b] for j < *kp (+ koff); one warp per j, grid-stride.
-__global__ void k_dot_reduce_dk(const double* __restrict__ part, int nb, const int* __restrict__ kp, int koff,
+// h[j] = sum_b part[j][b] for j < *kp; one warp per j, grid-stride.
+__global__ void k_dot_reduce_dk(const double* __restrict__ part, int nb, const int* __restrict__ kp,
                                 double* __restrict__ h) {
-  const int k = *kp + koff;
+  const int k = *kp;
   const int lane = threadIdx.x & 31;
   for (int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); j < k; j += gridDim.x * (blockDim.x >> 5)) {
     double a = 0.0;

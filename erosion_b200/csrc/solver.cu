@@ -723,12 +723,12 @@ bool choose_initial_guess(State& s, const double* d_b, double* d_x, bool have_x,
 }
 
 // In-place inversion of count m x m FP32 matrices (one CTA each), a zero
-// pivot flagged in bad[matrix].  The register-tiled Gauss-Jordan up to 1500
+// pivot flagged in bad[matrix].  The register-tiled Gauss-Jordan up to 1472
 // rows; past that the blocked one with the widest panel whose shared-memory
 // working set (2 m pb + m floats, m ints) fits, then the unblocked kernel.
 static void invert_fp32(State& s, float* B, int m, int count, int* bad) {
-  // panels of 32 while they fit beside the pivot rows in shared memory, of 16
-  // up to 1500 rows
+  // panels of 32 while they fit beside the pivot rows in shared memory (768 rows), of
+  // 16 up to 1472
   const int mp = (m + 63) / 64 * 64;
   auto tiled = [&](int pb) { return 2 * (size_t)pb * mp * sizeof(float) + 2 * (size_t)m * sizeof(int); };
   if (m <= 1024 && tiled(32) <= 200 * 1024) {
@@ -1093,11 +1093,11 @@ static int step_bound(int ll) {
   return std::min(b, CGS_MAX);
 }
 
-// Unknowns from which a thread owns a row of the update: its CTA then reads 2 KB
-// of a column at a time, and the two passes over V are no slower than the
-// fused one's 256-byte pieces.  55,596 unknowns (k = 240): fused 19.8 and 16.4
-// us, by rows 31.6 and 16.8 us; 107,392 (k = 165): 31.7 and 29.0 us, by rows
-// 33.8 and 17.4 us.
+// Unknowns from which a thread owns a row of the updates, so that its CTA reads 2 KB of a
+// column at a time where the fused pass (k_cgs_update_dot, then k_cgs_update_norm) reads
+// 256-byte pieces.  One rule for both: at 55,596 unknowns (k = 240) fused 19.8 + 16.4 us,
+// by rows 31.6 + 16.8; at 107,392 (k = 165) 31.7 + 29.0 us, by rows 33.8 + 17.4, where
+// the first pass alone would still be the faster one fused.
 constexpr long long kRowPerThread = 75000;
 
 static size_t step_tile(int bound) { return (size_t)bound * 34 * sizeof(double); }
@@ -1155,7 +1155,7 @@ static void launch_step(State& s, long long N, long long ldv, int bound, int pre
   k_cgs_dot<<<dim3(nb, ny), 256, R * sizeof(double), st>>>(s.V.p, ldv, kp, s.k_w.p, N, R, s.part.p);
   EB_LAUNCH_CHECK();
   const unsigned nred = nblk(bound, 8);
-  k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, 0, s.k_h1.p);
+  k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, s.k_h1.p);
   EB_LAUNCH_CHECK();
   // as many CTAs as are resident with the chunk's block of V in shared memory
   const size_t tile = step_tile(bound);
@@ -1164,14 +1164,14 @@ static void launch_step(State& s, long long N, long long ldv, int bound, int pre
     const int g = std::min(chunks, per_sm * g_num_sms);
     k_cgs_update_dot<<<g, 256, tile, st>>>(s.V.p, ldv, kp, s.k_h1.p, s.k_w.p, N, s.part.p);
     EB_LAUNCH_CHECK();
-    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, g, kp, 0, s.k_h2.p);
+    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, g, kp, s.k_h2.p);
     EB_LAUNCH_CHECK();
   } else {   // the update and the product by themselves
     k_vh_dk<<<nblk(N, 256), 256, 0, st>>>(s.V.p, ldv, kp, s.k_h1.p, -1.0, s.k_w.p, N);
     EB_LAUNCH_CHECK();
     k_cgs_dot<<<dim3(nb, ny), 256, R * sizeof(double), st>>>(s.V.p, ldv, kp, s.k_w.p, N, R, s.part.p);
     EB_LAUNCH_CHECK();
-    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, 0, s.k_h2.p);
+    k_dot_reduce_dk<<<nred, 256, 0, st>>>(s.part.p, nb, kp, s.k_h2.p);
     EB_LAUNCH_CHECK();
   }
   int gn = std::min(chunks, 4 * g_num_sms);

@@ -293,10 +293,9 @@ void setup_problem(State& s, const Problem& pr, const double* d_xx, const double
 // vel = A den, device pointers.  prec 0: FP64 far field; 1: FP32 far field
 // between distinct curves + FP64 self-curve sums.
 void apply_operator(State& s, const double* d_den, double* d_vel, int prec = 0);
-// apply_operator in three parts, for callers that batch the far field of
-// several geometries into one launch: k_prep (strengths), then the far field
-// into s.partial (far_slots(s, prec) slots), then the self/near sums and the
-// assembly.
+// apply_operator in parts, as a captured step launches it: k_prep (strengths), then
+// far_field into s.partial (far_slots(s, prec) slots) beside the self and near sums of
+// operator_post, then its assembly.
 void operator_prep(State& s, const double* d_den, double* d_vel);
 int far_slots(const State& s, int prec);
 void operator_post(State& s, const double* d_den, double* d_vel, int nsplit, int* kp = nullptr);
