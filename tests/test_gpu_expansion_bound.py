@@ -1,7 +1,7 @@
 """The cut of the expansions by which separated clusters act, one source node at a time: the
 field of a single node with a unit density, at bodies 2.7 to 220 radii away (every class of
 order, close to its edge: distances 6 to 10% apart) and at the wall, against the pair term in 80
-bits.  The bound is the one the kernels state, 3^-32 of the node's field, and the
+bits.  The bound is the one the kernels state, 5e-16 of the node's field (3^-32), and the
 rounding of one expansion: 32 terms, so 32 eps for the velocity; 64 eps for the strain, the
 derivative of the same series.  (A field or a strain is measured by |w sigma|/r or |w sigma|/r^2, summed
 over the sources.)"""
