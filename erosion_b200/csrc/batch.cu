@@ -10,9 +10,9 @@
 // per round), in which every geometry waited for the slowest one's kernels and the
 // host: 12 geometries of 20-40 bodies x 128 nodes to 1e-11 took 440 ms in 422
 // rounds, and 110 ms here.  The members' buffers and captured steps stay for the
-// next call (allocating, capturing and freeing them took 100 ms and more of it);
-// those of more geometries than the next call has are freed by it, all of them by
-// erosion_release.
+// next call (allocating, capturing and freeing them took 100 ms and more of it), up to a
+// share of the device's memory; those of more geometries than the next call has are
+// freed by it, all of them by erosion_release.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -44,12 +44,32 @@ Batch& batch() {
   return B;
 }
 
-void destroy_member(Member& mb) {
+void release_buffers(Member& mb) {
   settle(mb.s);
   release_state_buffers(mb.s);
-  destroy_state(mb.s);
   mb.x.release();
   mb.b.release();
+}
+
+void destroy_member(Member& mb) {
+  release_buffers(mb);
+  destroy_state(mb.s);
+}
+
+// What the members keep for the next call is bounded by this share of the device's memory
+// (11 GB): the bases of many large geometries are freed when the call ends, those of 12
+// geometries of 40 bodies x 128 nodes (1.5 GB) stay.
+constexpr size_t kKeepShare = 16;
+
+void trim(Batch& B) {
+  size_t kept = 0;
+  for (auto& mb : B.m) {
+    kept += state_bytes(mb->s);
+    if (kept > eb_device_bytes() / kKeepShare) {
+      kept -= state_bytes(mb->s);
+      release_buffers(*mb);
+    }
+  }
 }
 
 // Runs f for every geometry, in the order of `order`, on a pool of host threads.
@@ -116,39 +136,42 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
     std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return size[i] > size[j]; });
     cudaStream_t st = lib.st;
     EB_CK(cudaEventRecord(B.a, st));
-    const auto t_setup = std::chrono::steady_clock::now();
-    for_each(lib.device, order, [&](int g) {
-      Member& mb = *B.m[g];
-      State& s = mb.s;
-      init_state(s, lib.device);
-      s.pc_valid = false;   // the inverses it holds are of another call's geometry
-      Problem pr;
-      pr.P = P;
-      pr.n = (int)npts[g]; pr.M = (int)nbods[g]; pr.nout = (int)nouter[g];
-      const size_t nb = (size_t)pr.n * pr.M;
-      double* dx = s.d_xx.ensure(std::max<size_t>(nb, 1));
-      double* dy = s.d_yy.ensure(std::max<size_t>(nb, 1));
-      h2d(dx, xx + node_offs[g], nb, s.st);
-      h2d(dy, yy + node_offs[g], nb, s.st);
-      setup_problem(s, pr, dx, dy);
-      h2d(mb.x.ensure(s.pr.ntot), density + den_offs[g], (size_t)s.pr.ntot, s.st);
-      build_rhs(s, mb.b.ensure(s.pr.ntot));
-      if (device_norm(s, mb.b.p, s.pr.ntot) == 0.0)
-        throw Error(EROSION_BAD_INPUT, "erosion_solve_batch: zero right-hand side");
-    });
-    B.stats.setup_host_ms =
-        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_setup).count();
-    for_each(lib.device, order, [&](int g) {
-      Member& mb = *B.m[g];
-      State& s = mb.s;
-      const long long n = s.pr.ntot, maxl = std::min<long long>(P.maxl > 0 ? P.maxl : 10, n);
-      bool zero = true;
-      for (long long i = 0; i < n && zero; ++i) zero = density[den_offs[g] + i] == 0.0;
-      s.stats = erosion_solve_stats{};
-      const long long c0 = s.captures;
-      mb.status = gmres_solve(s, mb.b.p, mb.x.p, zero, maxl, P.tol, &mb.iterations, &mb.residual);
-      mb.captures = s.captures - c0;
-    });
+    auto run = [&] {
+      const auto t_setup = std::chrono::steady_clock::now();
+      for_each(lib.device, order, [&](int g) {
+        Member& mb = *B.m[g];
+        State& s = mb.s;
+        init_state(s, lib.device);
+        s.pc_valid = false;   // the inverses it holds are of another call's geometry
+        Problem pr;
+        pr.P = P;
+        pr.n = (int)npts[g]; pr.M = (int)nbods[g]; pr.nout = (int)nouter[g];
+        const size_t nb = (size_t)pr.n * pr.M;
+        double* dx = s.d_xx.ensure(std::max<size_t>(nb, 1));
+        double* dy = s.d_yy.ensure(std::max<size_t>(nb, 1));
+        h2d(dx, xx + node_offs[g], nb, s.st);
+        h2d(dy, yy + node_offs[g], nb, s.st);
+        setup_problem(s, pr, dx, dy);
+        h2d(mb.x.ensure(s.pr.ntot), density + den_offs[g], (size_t)s.pr.ntot, s.st);
+        build_rhs(s, mb.b.ensure(s.pr.ntot));
+        if (device_norm(s, mb.b.p, s.pr.ntot) == 0.0)
+          throw Error(EROSION_BAD_INPUT, "erosion_solve_batch: zero right-hand side");
+      });
+      B.stats.setup_host_ms =
+          std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_setup).count();
+      for_each(lib.device, order, [&](int g) {
+        Member& mb = *B.m[g];
+        State& s = mb.s;
+        const long long n = s.pr.ntot, maxl = std::min<long long>(P.maxl > 0 ? P.maxl : 10, n);
+        bool zero = true;
+        for (long long i = 0; i < n && zero; ++i) zero = density[den_offs[g] + i] == 0.0;
+        s.stats = erosion_solve_stats{};
+        const long long c0 = s.captures;
+        mb.status = gmres_solve(s, mb.b.p, mb.x.p, zero, maxl, P.tol, &mb.iterations, &mb.residual);
+        mb.captures = s.captures - c0;
+      });
+    };
+    run();
     // handed over once every geometry has ended: a call that fails leaves the
     // caller's densities as they were (12 geometries 104.7 ms, each as it ended 105.1)
     for (int g = 0; g < nbatch; ++g) {
@@ -180,14 +203,17 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
       if (mb.status != EROSION_OK && worst == EROSION_OK) worst = mb.status;
       B.stats.max_true_residual = std::max(B.stats.max_true_residual, mb.residual);
     }
+    trim(B);
     set_status(worst, worst == EROSION_OK ? "" : "a geometry of the ensemble did not converge");
     return worst;
   } catch (const Error& e) {
     for (auto& mb : batch().m) settle(mb->s);
+    trim(batch());
     set_status(e.code, e.what());
     return e.code;
   } catch (const std::exception& e) {
     for (auto& mb : batch().m) settle(mb->s);
+    trim(batch());
     set_status(EROSION_CUDA_ERROR, e.what());
     return EROSION_CUDA_ERROR;
   }

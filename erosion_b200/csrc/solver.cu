@@ -27,6 +27,8 @@ void set_status(int code, const std::string& msg) {
 }
 static int g_num_sms = 148;
 int eb_num_sms() { return g_num_sms; }
+static size_t g_device_bytes = 0;
+size_t eb_device_bytes() { return g_device_bytes; }
 
 void allow_max_dynamic_smem(const void* fn) {
   // once per kernel and device: the driver call takes milliseconds while other
@@ -55,6 +57,7 @@ void ensure_init(State& s) {
   cudaDeviceProp prop;
   EB_CK(cudaGetDeviceProperties(&prop, s.device));
   g_num_sms = prop.multiProcessorCount;
+  g_device_bytes = prop.totalGlobalMem;
   init_state(s, s.device);
 }
 
@@ -1547,31 +1550,48 @@ int gmres_solve(State& s, const double* d_b, double* d_x, bool x0_zero, long lon
   return EROSION_MAXITER;
 }
 
-// Frees every device buffer a State holds (the next call sets it up again).
+// Every device buffer a State holds.
+template <class F>
+static void each_buffer(State& s, F&& f) {
+  for (auto* b : {&s.dker_body, &s.dker_wall, &s.wx, &s.wy, &s.sp, &s.cur, &s.w, &s.rb, &s.sigdotn, &s.d_xx, &s.d_yy,
+                  &s.d_den, &s.d_rhs, &s.d_r, &s.d_w, &s.V, &s.Z, &s.part, &s.hdev, &s.ydev, &s.pc_z, &s.pc_u, &s.k_cur,
+                  &s.k_w, &s.k_h1, &s.k_h2, &s.k_np, &s.cg_Cinv, &s.cg_q, &s.cg_cs, &s.cg_cr, &s.cl_rad, &s.cl.lnd,
+                  &s.cl_stress.lnd})
+    f(*b);
+  for (auto* b : {&s.xy, &s.nrm, &s.dz, &s.cen, &s.d1tmp, &s.ws, &s.partial, &s.bd, &s.pair_out, &s.tile_c, &s.anchor,
+                  &s.selfsum, &s.pc_tw, &s.cl_cen, &s.cl_mp, &s.cl_lam, &s.near.reach})
+    f(*b);
+  for (auto* b : {&s.split_ptr, &s.split_ptr32, &s.split_ptr64t, &s.split_ptr64f, &s.split_ptrw, &s.split_tune,
+                  &s.pc_split_ptr, &s.pc_bad, &s.cg_bad, &s.k_count, &s.cl.near, &s.cl.far, &s.cl.fcls, &s.cl_stress.near,
+                  &s.cl_stress.far, &s.cl_stress.fcls, &s.near.cnt, &s.near.ptr, &s.near.wptr, &s.near.fill,
+                  &s.near.wflag, &s.near.pair_tgt, &s.near.tpairs})
+    f(*b);
+  for (auto* b : {&s.items32, &s.items64, &s.cl.ncnt, &s.cl_stress.ncnt, &s.near.tl}) f(*b);
+  for (auto* b : {&s.tiles, &s.near.bary_work}) f(*b);
+  for (auto* b : {&s.src32, &s.sq32, &s.pc_sq32}) f(*b);
+  for (auto* b : {&s.sq64, &s.pc_sq64}) f(*b);
+  for (auto* b : {&s.pcB, &s.cg_B}) f(*b);
+  f(s.tgt32);
+  f(s.near.mask);
+  f(s.near.info);
+}
+
+size_t state_bytes(State& s) {
+  size_t n = 0;
+  each_buffer(s, [&](auto& b) { n += b.cap * sizeof(*b.p); });
+  return n;
+}
+
+// Frees them (the next call sets them up again), and the captured steps that refer to them.
 void release_state_buffers(State& s) {
-  DBuf<double>* dbs[] = {&s.dker_body, &s.dker_wall, &s.wx, &s.wy, &s.sp, &s.cur, &s.w, &s.rb, &s.sigdotn,
-                         &s.d_xx, &s.d_yy, &s.d_den, &s.d_rhs, &s.d_r, &s.d_w, &s.V, &s.Z, &s.part, &s.hdev,
-                         &s.ydev, &s.pc_z, &s.pc_u};
-  for (auto* b : dbs) b->release();
-  DBuf<double2>* d2s[] = {&s.xy, &s.nrm, &s.dz, &s.cen, &s.d1tmp, &s.ws, &s.partial, &s.bd, &s.pair_out};
-  s.sq64.release();
-  for (auto* b : d2s) b->release();
+  each_buffer(s, [](auto& b) { b.release(); });
   drop_steps(s);
-  s.k_cur.release(); s.k_w.release(); s.k_h1.release(); s.k_h2.release(); s.k_np.release(); s.k_count.release();
-  s.near.release();
   s.lay_n = -1;
-  s.tiles.release(); s.split_ptr.release();
   s.vcap = 0;
   s.zcap = 0;
-  s.pcB.release(); s.pc_tw.release(); s.pc_sq32.release(); s.pc_split_ptr.release(); s.pc_bad.release();
-  s.cg_B.release(); s.cg_Cinv.release(); s.cg_q.release(); s.cg_cs.release(); s.cg_cr.release(); s.cg_bad.release();
   s.cg_ready = false;
   s.pc_valid = false;
-  s.src32.release(); s.sq32.release(); s.tgt32.release(); s.tile_c.release(); s.anchor.release();
-  s.selfsum.release(); s.cl.release(); s.cl_stress.release(); s.cl_cen.release(); s.cl_rad.release(); s.cl_mp.release(); s.cl_lam.release();
-  s.items32.release(); s.items64.release(); s.pc_sq64.release();
-  s.split_ptr32.release(); s.split_ptr64t.release(); s.split_ptrw.release();
-  s.split_tune.release(); s.split_ptr64f.release(); s.tune_N = -1;
+  s.tune_N = -1;
   for (int k = 0; k < kFarKinds; ++k) s.tuned_shape[k] = -1;
   s.dker_body_n = s.dker_wall_n = -1;
   s.geo_valid = false;

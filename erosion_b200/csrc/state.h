@@ -101,10 +101,6 @@ struct Near {
   DBuf<int4> bary_work;
   DBuf<unsigned> mask;
   DBuf<unsigned char> info;  // NearInfo
-  void release() {
-    cnt.release(); ptr.release(); wptr.release(); fill.release(); wflag.release(); reach.release();
-    pair_tgt.release(); tpairs.release(); tl.release(); bary_work.release(); mask.release(); info.release();
-  }
 };
 
 // Near and far lists of the clusters (ClView in kernels.cuh).
@@ -112,9 +108,6 @@ struct ClLists {
   DBuf<int> near, far, fcls;
   DBuf<int2> ncnt;
   DBuf<double> lnd;
-  void release() {
-    near.release(); far.release(); fcls.release(); ncnt.release(); lnd.release();
-  }
 };
 
 struct State {
@@ -337,6 +330,10 @@ double device_norm(State& s, const double* d_v, long long n);
 void harvest_far_timing(State& s);
 
 void release_state_buffers(State& s);
+// Bytes of device memory they take.
+size_t state_bytes(State& s);
+// Memory of the library's device.
+size_t eb_device_bytes();
 // Frees the ensemble solver's members (batch.cu).
 void release_batch();
 

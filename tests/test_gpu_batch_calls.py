@@ -45,3 +45,20 @@ def test_failed_call_leaves_the_densities(lib):
     assert rc == _lib.EROSION_BREAKDOWN
     assert np.array_equal(den, kept, equal_nan=True)
     assert nits.tolist() == [-1, -1]
+
+
+def free_bytes():
+    import torch
+    return torch.cuda.mem_get_info()
+
+
+def test_what_is_kept_is_bounded(lib):
+    """Sixteen geometries whose bases take a gigabyte each: the call may keep a sixteenth of
+    the device's memory, and a gigabyte for streams, graphs and the driver."""
+    lib.erosion_release()
+    before, total = free_bytes()
+    ens = [G.ensemble(1, seed=3 + k, bodies=(100, 100), npts=(512,), porosity=(0.7, 0.7), nout=2048)[0]
+           for k in range(16)]
+    stokes.solve_batch(ens, tol=1e-14, maxl=1100, allow=(_lib.EROSION_OK, _lib.EROSION_MAXITER))
+    assert before - free_bytes()[0] < total / 16 + 2 ** 30
+    lib.erosion_release()
