@@ -171,7 +171,17 @@ int erosion_solve_batch(const erosion_params* p, int32_t nbatch, const int64_t* 
         mb.captures = s.captures - c0;
       });
     };
-    run();
+    bool kept = false;
+    for (auto& mb : B.m) kept = kept || mb->s.V.p;
+    try {
+      run();
+    } catch (const Error& e) {
+      // buffers kept from another ensemble, whose large geometries had other places, may be
+      // what the device has no room for: once more without them
+      if (!e.memory || !kept) throw;
+      for (auto& mb : B.m) release_buffers(*mb);
+      run();
+    }
     // handed over once every geometry has ended: a call that fails leaves the
     // caller's densities as they were (12 geometries 104.7 ms, each as it ended 105.1)
     for (int g = 0; g < nbatch; ++g) {

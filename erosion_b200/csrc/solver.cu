@@ -1109,6 +1109,7 @@ void settle(State& s) {
   if (s.st) cudaStreamSynchronize(s.st);
   for (auto& b : s.br)
     if (b) cudaStreamSynchronize(b);
+  (void)cudaGetLastError();
 }
 
 void ensure_branches(State& s) {

@@ -20,14 +20,16 @@ extern thread_local long long t_launches;   // those of the calling thread
 
 struct Error : std::runtime_error {
   int code;
-  Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
+  bool memory;   // the device had none left
+  Error(int c, const std::string& m, bool oom = false) : std::runtime_error(m), code(c), memory(oom) {}
 };
 
 #define EB_CK(x)                                                                               \
   do {                                                                                         \
     cudaError_t e_ = (x);                                                                      \
     if (e_ != cudaSuccess)                                                                     \
-      throw ::eb::Error(EROSION_CUDA_ERROR, std::string(#x) + ": " + cudaGetErrorString(e_));  \
+      throw ::eb::Error(EROSION_CUDA_ERROR, std::string(#x) + ": " + cudaGetErrorString(e_),   \
+                        e_ == cudaErrorMemoryAllocation);                                      \
   } while (0)
 
 #define EB_LAUNCH_CHECK()  \
@@ -254,8 +256,9 @@ void on_stream(State& s, cudaStream_t st, F&& f) {
   f();
 }
 
-// Waits for what a failed call left in flight on the state's streams: its branches are
-// joined by nothing, and the next call uses the same buffers.
+// Waits for what a failed call left in flight on the state's streams (its branches are
+// joined by nothing, and the next call uses the same buffers), and clears the error that
+// the call reports, which would otherwise be found by the next call's first launch.
 void settle(State& s);
 int eb_num_sms();
 // Creates the branch streams and their events.

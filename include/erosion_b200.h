@@ -220,6 +220,8 @@ void erosion_get_solve_stats(erosion_solve_stats* s);
  * solved with the method erosion_solve applies for the same parameters (one
  * erosion_params for all), on streams of its own, from a pool of up to 16 host
  * threads; the GPU works on as many geometries at a time.
+ * The geometries' device buffers stay for the next call, up to a sixteenth of the
+ * device's memory; erosion_release frees them.
  * Returns EROSION_OK or the first non-OK status of a geometry.  Geometries that
  * reach maxl or stall still return their densities; on any other error (bad
  * input, a non-finite value, a CUDA error) density and nits stay as they were. */
