@@ -68,6 +68,31 @@ def test_velocity(lib, spiral):
             assert err.max() < 3.0 ** -32 + 32 * EPS, (j, comp, float(err.max()))
 
 
+def test_stokeslet_and_rotlet(lib, spiral):
+    """A body's stokeslet and rotlet ride on the same expansions, at the disc's centre: to
+    the rounding of 32 terms of (|log r| + 1) / (4 pi) and of 1 / r."""
+    g = spiral
+    x = nodes(g)[0]
+    c = np.array([stokes.geometry(g)[k][0] for k in ("cx", "cy")], L)
+    tgt = np.r_[0:g.nout, g.nout + N:g.nout + g.M * N]
+    r = x[tgt] - c
+    r2 = (r ** 2).sum(1)
+    for k in range(3):
+        den = np.zeros(g.ntot)
+        den[2 * g.nout + 2 * N * g.M + k] = 1.0   # of the first body
+        u = stokes.matvec(g, den, ibary=0)
+        body = u[2 * g.nout:2 * g.nout + 2 * N * g.M].reshape(g.M, 2, N)
+        got = np.stack([np.concatenate([u[q * g.nout:(q + 1) * g.nout], body[:, q].ravel()]) for q in (0, 1)], 1)
+        if k < 2:
+            ref = r[:, k, None] * r / r2[:, None]
+            ref[:, k] -= np.log(r2) / 2
+            ref, mag = ref / (4 * L(np.pi)), (np.abs(np.log(r2)) / 2 + 1) / (4 * L(np.pi))
+        else:
+            ref, mag = np.stack([r[:, 1], -r[:, 0]], 1) / r2[:, None], 1 / np.sqrt(r2)
+        err = np.sqrt(((got[tgt] - ref) ** 2).sum(1)) / mag
+        assert err.max() < 3.0 ** -32 + 32 * EPS, (k, float(err.max()))
+
+
 def test_strain(lib, spiral):
     g = spiral
     x, n, w, sp = nodes(g)
