@@ -56,11 +56,17 @@ constexpr int CL_MAX_TILES = 4096;       // above this the lists (tiles^2 entrie
 // expansions are two launches more.
 constexpr int kExpandNodes = 3200;
 
+// The binomials in the order in which the lanes of cl_shift_run read them: c[lt][kt][lane]
+// = C(k + l, l) for l = 8 lt + lane / 4, k = 4 kt + lane % 4.
 struct BinomTable {
-  double c[CL_P][CL_P];   // c[l][k] = C(k + l, l)
+  double c[CL_P / 8][CL_P / 4][32];
   constexpr BinomTable() : c{} {
+    double b[CL_P][CL_P] = {};
     for (int l = 0; l < CL_P; ++l)
-      for (int k = 0; k < CL_P; ++k) c[l][k] = (l == 0 || k == 0) ? 1.0 : c[l - 1][k] + c[l][k - 1];
+      for (int k = 0; k < CL_P; ++k) {
+        b[l][k] = (l == 0 || k == 0) ? 1.0 : b[l - 1][k] + b[l][k - 1];
+        c[l / 8][k / 4][4 * (l % 8) + k % 4] = b[l][k];
+      }
   }
 };
 __device__ const BinomTable kBinom{};
@@ -348,7 +354,7 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double
 // (-R'/D)^l and added to the lane's sums, which the warps combine at the end in
 // a fixed order.  Bound by the FP64 pipe, which the tensor-core products share:
 // of ~450 operations per lane for two sources of 32 x 32 terms, 256 are products.
-// The velocity at 400 bodies x 256 nodes takes 101 us, at 200 x 256 67 us, at
+// The velocity at 400 bodies x 256 nodes takes 98 us, at 200 x 256 52 us, at
 // 100 x 256 27 us (all pairs with 32 x 32 terms took 180 us at the first).
 struct ClShared {
   double P[CL_P * CL_P];
@@ -433,10 +439,7 @@ __device__ __forceinline__ void cl_shift(const ClView& L, int t, const double2* 
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = lane >> 2, csrc = (lane >> 1) & 1, cfn = lane & 1;
   constexpr int NL = cl_terms(USE) / 8;
-  for (int e = threadIdx.x; e < NL * 8 * CL_P; e += blockDim.x) {
-    const int ln = e & 31, kt = (e >> 5) % (CL_P / 4), lt = (e >> 5) / (CL_P / 4);
-    sh.P[e] = kBinom.c[8 * lt + (ln >> 2)][4 * kt + (ln & 3)];
-  }
+  for (int e = threadIdx.x; e < NL * 8 * CL_P; e += blockDim.x) sh.P[e] = (&kBinom.c[0][0][0])[e];
   __syncthreads();
   double ax[NL] = {}, ay[NL] = {};
   const int* __restrict__ f = L.fcls + (size_t)t * (2 * CL_NCLS + 1);
@@ -470,9 +473,10 @@ __device__ __forceinline__ void cl_shift(const ClView& L, int t, const double2* 
   __syncthreads();
 }
 
-// The separated sources' velocity at the nodes of cluster blockIdx.x + tile0.
-template <int USE>
-__global__ void __launch_bounds__(256, 2)
+// The separated sources' velocity at the nodes of cluster blockIdx.x + tile0.  MINB: CTAs
+// an SM holds, 2 with 127 registers or 3 with 80 and a few spills (shift_ctas).
+template <int USE, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 k_cl_shift(GeoDev G, ClView L, int tile0, const int4* __restrict__ tiles, const double2* __restrict__ mp,
            const double2* __restrict__ lam, double2* __restrict__ out) {
   __shared__ ClShared sh;
@@ -749,6 +753,12 @@ k_cl_near32(GeoDev G, ClView L, const int2* __restrict__ items, const int4* __re
 
 // Host side.
 namespace eb {
+
+// CTAs per SM of k_cl_shift for that many clusters: two while all of them find a place, at
+// 164, 264 and 294 clusters 27.0, 33.6 and 43.6 us (three: 32.5, 43.8, 49.3), then three, as
+// the clusters past two an SM would make a wave of their own: at 328, 428, 528, 628 and 728
+// clusters 50.2, 63.6, 97.8, 129.9 and 147.1 us (two: 55.0, 73.8, 99.9, 140.9, 165.7).
+inline int shift_ctas(int ntile, int sms) { return ntile <= 2 * sms ? 2 : 3; }
 
 static inline ClView cl_view(const State& s, const ClLists& L) {
   ClView v;

@@ -251,7 +251,8 @@ extern "C" int erosion_matvec_noalloc(const erosion_params* p, int64_t npts, int
     if (expand) {
       k_cl_form<CL_P / 8><<<ntile, 256, 0, st>>>(G, 0, tiles, ccen, crad, sq64, sing ? d_den : nullptr, mp, lam);
       EB_LAUNCH_CHECK();
-      k_cl_shift<CL_ALL><<<ntile, 256, 0, st>>>(G, L, 0, tiles, mp, lam, partial + (size_t)parts * N);
+      const auto shift = shift_ctas(ntile, nd.sms) == 2 ? k_cl_shift<CL_ALL, 2> : k_cl_shift<CL_ALL, 3>;
+      shift<<<ntile, 256, 0, st>>>(G, L, 0, tiles, mp, lam, partial + (size_t)parts * N);
       EB_LAUNCH_CHECK();
     }
     if (M > 0) {

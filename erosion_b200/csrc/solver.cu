@@ -471,7 +471,8 @@ static void launch_expansions(State& s, const double* d_den, double2* out) {
   k_cl_form<CL_P / 8><<<s.ntile, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.sq64.p, s.cl_sing ? d_den : nullptr,
                                        s.cl_mp.p, s.cl_lam.p);
   EB_LAUNCH_CHECK();
-  k_cl_shift<CL_ALL><<<s.ntile, 256, 0, s.st>>>(G, cl_view(s, s.cl), 0, s.tiles.p, s.cl_mp.p, s.cl_lam.p, out);
+  const auto shift = shift_ctas(s.ntile, g_num_sms) == 2 ? k_cl_shift<CL_ALL, 2> : k_cl_shift<CL_ALL, 3>;
+  shift<<<s.ntile, 256, 0, s.st>>>(G, cl_view(s, s.cl), 0, s.tiles.p, s.cl_mp.p, s.cl_lam.p, out);
   EB_LAUNCH_CHECK();
 }
 
@@ -492,7 +493,7 @@ static void launch_wall_coupling(State& s, double2* out) {
   k_cl_form<3><<<s.nwall_tiles, 256, 0, s.st>>>(G, 0, s.tiles.p, s.cl_cen.p, s.cl_rad.p, s.pc_sq64.p, nullptr, s.cl_mp.p,
                                              s.cl_lam.p);
   EB_LAUNCH_CHECK();
-  k_cl_shift<CL_WALL32><<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,
+  k_cl_shift<CL_WALL32, 2><<<s.ntile - s.nwall_tiles, 256, 0, s.st>>>(G, L, s.nwall_tiles, s.tiles.p, s.cl_mp.p,
                                                                    s.cl_lam.p, out + s.pr.N);
   EB_LAUNCH_CHECK();
   join(s, 0);
