@@ -1366,7 +1366,9 @@ static int gmres_cycle(State& s, double* d_r, double* d_x, long long maxl_in, do
     for (long long ll = 1; ll <= last && running; ++ll) {
       if (launched < ll) launch(ll);
       const bool settled = relax_abs <= 0.0 || kind[ll & 1] == 1;   // rho only falls
-      if (ll < last && settled && ll > 1) launch(ll + 1);
+      // a basis that is full grows only once the next step is known to be needed
+      const bool room = ll + 2 <= s.vcap && (!s.pc_active || ll + 1 <= s.zcap);
+      if (ll < last && settled && room && ll > 1) launch(ll + 1);
       EB_CK(cudaEventSynchronize(s.ev_step[ll & 1]));
       count_operator(s, kind[ll & 1]);
       running = hessenberg(ll, host + (size_t)(ll & 1) * (CGS_MAX + 2));
